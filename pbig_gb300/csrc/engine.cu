@@ -227,10 +227,10 @@ struct GridScene {
 // device buffers of one query; fills the matching Params fields
 static int ensure_query_buffers(pbig2_ctx* c, Params& p, uint64_t entry_cap, uint64_t out_cap, uint64_t task_cap,
                                 uint32_t nsc, bool grouped, cudaStream_t st) {
-    CK(c->d_entries.ensure(entry_cap * 4, false, st));
+    CK(c->d_entries.ensure(entry_cap * sizeof(uint4), false, st));
     // list regions: a cell of class c holds at least lo_c boxes, so with
     // E <= entry capacity no list can overflow
-    const uint64_t ecap = c->d_entries.bytes / 4;
+    const uint64_t ecap = c->d_entries.bytes / sizeof(uint4);
     const unsigned long long map = p.class_map ? p.class_map : kClassMapDefault;
     uint64_t loff = 0;
     for (int k = 0; k < kNumLists; k++) {
@@ -248,13 +248,17 @@ static int ensure_query_buffers(pbig2_ctx* c, Params& p, uint64_t entry_cap, uin
         CK(c->d_scene_cursor.ensure((nsc + 1) * 8, false, st));
     }
     p.counts = c->d_counts.as<uint32_t>();
-    p.entries = c->d_entries.as<uint32_t>();
+    p.entries = c->d_entries.as<uint4>();
     p.entry_cap = ecap;
     p.lists = c->d_lists.as<uint2>();
     p.tasks = c->d_tasks.as<uint4>();
     p.task_cap = c->d_tasks.bytes / 16;
     p.out = c->d_out.as<uint2>();
     p.out_cap = c->d_out.bytes / 8;
+    if (p.records) {
+        CK(c->d_recs.ensure(ecap * 4, false, st));
+        p.recs = c->d_recs.as<uint32_t>();
+    }
     return PBIG2_OK;
 }
 
@@ -292,7 +296,7 @@ static cudaError_t record_pipeline(pbig2_ctx* c, const Params& p, int dims, bool
         // keep the grid and lists; clear the pair count and error word
         R(cudaMemsetAsync(&p.ctr->pairs, 0, sizeof(unsigned long long), st));
         R(cudaMemsetAsync(&p.ctr->err, 0, sizeof(unsigned int), st));
-        R(cudaMemsetAsync(&p.ctr->med_next, 0, sizeof(unsigned int), st));
+        R(cudaMemsetAsync(&p.ctr->med_next, 0, 2 * sizeof(unsigned int), st));  // and big_next
         R(cudaEventRecordWithFlags(c->evp[4], st, evf));
     }
     // pairs stored over the host link: the lighter pair kernels run beside
@@ -385,6 +389,7 @@ static int capture_graph(pbig2_ctx* c, const Params& p0, const uint32_t* d_boxes
     CK(cudaStreamSynchronize(st));
     Params p = p0;
     p.dyn = c->d_dims.as<RunDims>();
+    p.open = 1;  // later batches choose their own cell sizes
     p.nboxes = nboxes;
     p.ncells = ncells;
     p.nscenes = nsc;
@@ -426,12 +431,14 @@ static int capture_graph(pbig2_ctx* c, const Params& p0, const uint32_t* d_boxes
 // the new slab holds no merged cell and the block's running count (the sum of
 // the first pass's per-cell counts) stays <= 256. merged[c] = the block root
 // of every cell of a block of two or more cells (the root included), else
-// kUnmerged. Returns the number of such blocks.
-static uint32_t merge_cells(std::vector<uint32_t>& nrs, std::vector<uint32_t>& merged, uint32_t nrc, int dims,
-                            uint32_t limit) {
+// kUnmerged; ext[root] = the block's cells per axis, 21 bits each. Returns the
+// number of such blocks.
+static uint32_t merge_cells(std::vector<uint32_t>& nrs, std::vector<uint32_t>& merged,
+                            std::vector<unsigned long long>& ext, uint32_t nrc, int dims, uint32_t limit) {
     const uint64_t C = nrs.size();
     const uint64_t kLimit = limit;  // NTPB of the shipped build by default (256)
     merged.assign(C, kUnmerged);
+    ext.assign(C, 0);
     const uint64_t nrc2 = (uint64_t)nrc * nrc;
     uint32_t blocks = 0;
     // try to add the slab next to block (root, h x v x u) along axis dir
@@ -481,7 +488,10 @@ static uint32_t merge_cells(std::vector<uint32_t>& nrs, std::vector<uint32_t>& m
             if (gy + v < nrc) progress += grow(i, 1, h, v, u);
             if (dims == 3 && gz + u < nrc) progress += grow(i, 2, h, v, u);
         } while (progress != 0);
-        if (merged[i] == (uint32_t)i) blocks++;
+        if (merged[i] == (uint32_t)i) {
+            ext[i] = (unsigned long long)u << 42 | (unsigned long long)v << 21 | h;
+            blocks++;
+        }
     }
     return blocks;
 }
@@ -586,7 +596,7 @@ static int run_pipeline(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t nboxes, 
     CK(c->h_ctr.ensure(sizeof(Ctr)));
 
     uint64_t entry_cap = (uint64_t)(est_entries * 1.25) + 4096;
-    entry_cap = std::max<uint64_t>(entry_cap, c->d_entries.bytes / 4);
+    entry_cap = std::max<uint64_t>(entry_cap, c->d_entries.bytes / sizeof(uint4));
     uint64_t out_cap = std::max<uint64_t>({c->out_hint, nboxes * 4, 1u << 16});
     out_cap = std::max<uint64_t>(out_cap, c->d_out.bytes / 8);
     uint64_t task_cap = std::max<uint64_t>(c->d_tasks.bytes / 16, 4096);
@@ -609,6 +619,7 @@ static int run_pipeline(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t nboxes, 
     p.nscenes = nsc;
     p.split = split;
     p.max_range = range;
+    for (const Scene& s : tab) p.open |= s.shift >= kOpenShift ? 1u : 0u;
     p.ncells = ncells;
     p.tile_state = c->d_state.as<unsigned long long>();
     p.ctr = c->d_ctr.as<Ctr>();
@@ -625,13 +636,18 @@ static int run_pipeline(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t nboxes, 
         CK(cudaMemsetAsync(p.ctr, 0, sizeof(Ctr), st));
         CK(launch_count(p0, dims, st));
         std::vector<uint32_t> nrs(ncells), merged;
+        std::vector<unsigned long long> ext;
         CK(cudaMemcpyAsync(nrs.data(), p0.counts, ncells * 4, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        c->merged_blocks = merge_cells(nrs, merged, tab[0].nrc, dims, c->merge_limit);
+        c->merged_blocks = merge_cells(nrs, merged, ext, tab[0].nrc, dims, c->merge_limit);
         CK(c->d_merged.ensure(ncells * 4, false, st));
         CK(cudaMemcpyAsync(c->d_merged.p, merged.data(), ncells * 4, cudaMemcpyHostToDevice, st));
-        CK(cudaStreamSynchronize(st));  // `merged` goes out of scope
+        CK(c->d_merged_ext.ensure(ncells * sizeof(ext[0]), false, st));
+        CK(cudaMemcpyAsync(c->d_merged_ext.p, ext.data(), ncells * sizeof(ext[0]), cudaMemcpyHostToDevice, st));
+        CK(cudaStreamSynchronize(st));  // the tables go out of scope
         p.merged = c->d_merged.as<uint32_t>();
+        p.merged_ext = c->d_merged_ext.as<unsigned long long>();
+        p.open = 1;  // a block may be wider than a cell
     }
     bool need_full = true;
     // self/bipartite pairs go straight to the caller's buffer when one is set;
@@ -732,7 +748,7 @@ static int fused_query(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t n, int di
         c->bar_base = 0;
         c->fused_slot = 0;
     }
-    const uint64_t entry_cap = std::max<uint64_t>({c->fused_entry_hint, 8 * n + 4096, c->d_entries.bytes / 4});
+    const uint64_t entry_cap = std::max<uint64_t>({c->fused_entry_hint, 8 * n + 4096, c->d_entries.bytes / sizeof(uint4)});
     const uint64_t out_cap = std::max<uint64_t>({c->out_hint, n * 4, 1u << 16, c->d_out.bytes / 8});
     const uint64_t task_cap = std::max<uint64_t>(c->d_tasks.bytes / 16, 4096);
     const bool use_ext = c->ext_out != nullptr;
@@ -889,7 +905,7 @@ PBIG2_API int pbig2_destroy(pbig2_ctx* c) {
     cudaSetDevice(c->device);
     if (c->own_stream) cudaStreamSynchronize(c->own_stream);
     c->drop_graph();
-    for (DevBuf* b : {&c->d_boxes, &c->d_counts, &c->d_entries, &c->d_bar, &c->d_fctr,
+    for (DevBuf* b : {&c->d_boxes, &c->d_counts, &c->d_entries, &c->d_recs, &c->d_merged, &c->d_merged_ext, &c->d_bar, &c->d_fctr,
                       &c->d_lists, &c->d_tasks, &c->d_state,
                       &c->d_out, &c->d_out2, &c->d_ctr, &c->d_scenes, &c->d_scene_off, &c->d_scene_pair,
                       &c->d_scene_cursor, &c->d_dims, &c->d_scene_tab, &c->d_tune})
@@ -1212,7 +1228,7 @@ PBIG2_API int pbig2_result_records(pbig2_ctx* c, const uint64_t** words, uint64_
     *nwords = c->rice_words;
     *start_i = c->d_counts.as<uint32_t>();
     *ncells = c->last_ncells;
-    *recs = c->d_entries.as<uint32_t>();
+    *recs = c->d_recs.as<uint32_t>();
     *nentries = c->last_entries;
     return PBIG2_OK;
 }
@@ -1224,7 +1240,7 @@ PBIG2_API int pbig2_copy_records(pbig2_ctx* c, uint64_t* words, uint32_t* start_
     cudaStream_t st = c->own_stream;
     if (words && c->rice_words) CK(cudaMemcpyAsync(words, c->result, c->rice_words * 8, cudaMemcpyDefault, st));
     if (start_i && c->last_ncells) CK(cudaMemcpyAsync(start_i, c->d_counts.p, c->last_ncells * 4, cudaMemcpyDefault, st));
-    if (recs && c->last_entries) CK(cudaMemcpyAsync(recs, c->d_entries.p, c->last_entries * 4, cudaMemcpyDefault, st));
+    if (recs && c->last_entries) CK(cudaMemcpyAsync(recs, c->d_recs.p, c->last_entries * 4, cudaMemcpyDefault, st));
     CK(cudaStreamSynchronize(st));
     return PBIG2_OK;
 }

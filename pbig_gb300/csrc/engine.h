@@ -52,7 +52,8 @@ struct pbig2_ctx {
     cudaStream_t own_stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t evp[9] = {};
-    pbig::DevBuf d_merged;  // merged mode: cell -> root table
+    pbig::DevBuf d_merged, d_merged_ext;  // merged mode: cell -> root table; the roots' extents
+    pbig::DevBuf d_recs;    // record mode: box index of every entry
     bool merged_mode = false;
     bool rice_mode = false;      // record mode (PBIG2_OPT_RICE)
     bool result_records = false; // the last result is a record stream

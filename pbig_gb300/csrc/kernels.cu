@@ -10,12 +10,13 @@
 //
 // Box records are the reference's RectInfo (rect.h): 2*D+1 unsigned words.
 // Cell ids follow the reference linearisation gid = (k*nrc + j)*nrc + i.
-// An entry stores the box index and three "starts here" bits: bit d is set
-// when the box's minimum along axis d lies in this cell. The reference-cell
-// rule of calcRightToWrite (pbig.cu:579-603) -- a pair is reported in the
-// cell holding the minimum corner of the two boxes' intersection -- is then
-// exactly (flags_a | flags_b) == 7: along each axis max(min_a, min_b) falls
-// in this cell iff one of the two minima does (both boxes cover the cell).
+// An entry stores the box index, three "starts here" bits -- bit d is set
+// when the box's minimum along axis d lies in this cell -- and the box's part
+// of the cell in 15-bit terms ("entries" below). The reference-cell rule of
+// calcRightToWrite (pbig.cu:579-603) -- a pair is reported in the cell holding
+// the minimum corner of the two boxes' intersection -- is then exactly
+// (flags_a | flags_b) == 7: along each axis max(min_a, min_b) falls in this
+// cell iff one of the two minima does (both boxes cover the cell).
 #include "kernels.cuh"
 
 #include <cstdio>
@@ -260,16 +261,52 @@ __device__ __forceinline__ uint32_t div_magic(uint32_t n, uint32_t d, uint32_t m
     return q * d > n ? q - 1u : q;
 }
 
+// ---- entries -----------------------------------------------------------------
+// An entry is 16 bytes: a word per axis with the box's part of the cell, then
+// {start bits << 29 | box index}. Both corners are counted from the cell's
+// first coordinate and scaled to 1..32765; a lower corner before the cell is 0
+// and an upper one beyond it 32766, so for two boxes of the cell lower <= upper
+// holds for the scaled corners whenever it holds for the real ones, and is the
+// same unless both fall into the cell and are scaled to one value (cells of
+// 2^kOpenShift or wider only). The high half of the word is the lower corner,
+// the low half 32767 minus the upper one: a row's lower corner plus a column's
+// low half is at most 32767 iff that side of the boxes overlaps, and never
+// carries out of 16 bits. An empty entry's first word, 32768 in the low half,
+// overlaps nothing.
+//
+// The pair kernels read the entries of a cell one after the other and never
+// the boxes (only to settle scaled corners that compare equal). With 4-byte
+// entries that named the boxes, fetching them took 0.26 of the 0.42 ms of the
+// medium-cell kernel on the clustered 4M-box scene, 0.29 of 0.39 ms on two
+// million red and blue boxes and 0.69 of 0.94 ms on 512 scenes: a random
+// 28-byte read per entry.
+constexpr uint32_t kTermSpan = 32765u;
+constexpr uint32_t kTermBeyond = 32767u - (kTermSpan + 1u);  // low half of a box that ends beyond the cell
+constexpr uint32_t kTermEmpty = 32768u;
+__device__ __forceinline__ uint4 entry_empty() { return make_uint4(kTermEmpty, 0u, 0u, 0u); }
+
+// x of [0, 2^s) scaled: floor(x * 32765 / 2^s)
+__device__ __forceinline__ uint32_t term_scale(uint32_t x, uint32_t s) {
+    return __umulhi(x << (31u - s), 2u * kTermSpan);
+}
+__device__ __forceinline__ uint32_t term_word(uint32_t lo, uint32_t hi) {
+    return ((lo + 1u) << 16) | (32766u - hi);
+}
+// a box's word in one of its cells, from that of a cell it lies in whole
+__device__ __forceinline__ uint32_t term_cut(uint32_t w, bool starts, bool ends) {
+    return (starts ? w & 0xffff0000u : 0u) | (ends ? w & 0xffffu : kTermBeyond);
+}
+
+// (scatter: the boxes' rows in sbox are overwritten)
 template <int D, bool SCATTER, bool MERGED>
-__device__ __forceinline__ void enumerate_cells(const Params& p, const uint32_t* sbox, uint64_t b0,
-                                                uint32_t nb) {
+__device__ __forceinline__ void enumerate_cells(const Params& p, uint32_t* sbox, uint64_t b0, uint32_t nb) {
     constexpr uint32_t W = 2 * D + 1;
     const uint32_t t = threadIdx.x, lane = t & 31u;
     const uint64_t gi = b0 + t;
     uint32_t cnt = 0, sx = 1, sy = 1, nrc = 0;
     uint64_t base = 0;
     if (t < nb) {
-        const uint32_t* b = sbox + t * W;
+        uint32_t* b = sbox + t * W;
         const Scene sc = p.scenes[find_scene(p, gi)];
         uint32_t err = 0;
 #pragma unroll
@@ -292,6 +329,12 @@ __device__ __forceinline__ void enumerate_cells(const Params& p, const uint32_t*
                 cnt = (uint32_t)c64;
                 nrc = sc.nrc;
                 base = sc.cell_off + ((uint64_t)lo2 * nrc + lo1) * nrc + lo0;
+                if (SCATTER && !MERGED) {  // the row becomes the box's terms, one word per axis
+                    const uint32_t low = (1u << sh) - 1u;
+#pragma unroll
+                    for (int d = 0; d < D; d++)
+                        b[d] = term_word(term_scale(b[2 * d] & low, sh), term_scale(b[2 * d + 1] & low, sh));
+                }
             }
         }
         if (err && !SCATTER) {
@@ -299,6 +342,7 @@ __device__ __forceinline__ void enumerate_cells(const Params& p, const uint32_t*
             atomicAdd(&p.ctr->bad, 1u);
         }
     }
+    if (SCATTER) __syncwarp();
     const uint32_t incl = warp_incl_scan(cnt);
     const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
     const uint32_t excl = incl - cnt;
@@ -319,6 +363,7 @@ __device__ __forceinline__ void enumerate_cells(const Params& p, const uint32_t*
         const uint64_t o_base = __shfl_sync(FULL_MASK, base, o);
         const uint32_t o_mx = __shfl_sync(FULL_MASK, mx, o);
         const uint32_t o_my = __shfl_sync(FULL_MASK, my, o);
+        const uint32_t o_cnt = SCATTER ? __shfl_sync(FULL_MASK, cnt, o) : 0u;
         if (q < total) {
             const uint32_t lq = q - o_excl;  // < 2^26
             const uint32_t rr = div_magic(lq, o_sx, o_mx), i = lq - rr * o_sx;
@@ -326,6 +371,14 @@ __device__ __forceinline__ void enumerate_cells(const Params& p, const uint32_t*
             uint64_t gid = o_base + ((uint64_t)k * o_nrc + j) * o_nrc + i;
             uint32_t f = (i == 0 ? 1u : 0u) | (j == 0 ? 2u : 0u) | ((D == 2 || k == 0) ? 4u : 0u);
             bool take = true;
+            uint4 rec = make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t* ob = sbox + ((t & ~31u) + o) * W;
+            if (SCATTER && !MERGED) {
+                rec.x = term_cut(ob[0], i == 0, i + 1 == o_sx);
+                rec.y = term_cut(ob[1], j == 0, j + 1 == o_sy);
+                // (the last layer: its cells are the last sx*sy)
+                if (D == 3) rec.z = term_cut(ob[2], k == 0, lq + o_sx * o_sy >= o_cnt);
+            }
             if (MERGED) {
                 // merged mode: a cell of a merged block stands for the block's
                 // root, and a box enters the block once, at the minimum corner of
@@ -344,13 +397,31 @@ __device__ __forceinline__ void enumerate_cells(const Params& p, const uint32_t*
                     gid = m;
                     f = (lx >= rx ? 1u : 0u) | (ly >= ry ? 2u : 0u) | ((D == 2 || lz >= rz) ? 4u : 0u);
                 }
+                if (SCATTER && take) {  // the box's part of the block (or of an unmerged cell)
+                    const uint64_t nr = o_nrc, ext = m != kUnmerged ? p.merged_ext[m] : (1ull << 42 | 1ull << 21 | 1ull);
+                    const uint32_t sh = p.scenes[0].shift;  // (one grid in merged mode)
+                    uint32_t root[3] = {(uint32_t)(gid % nr), (uint32_t)((gid / nr) % nr), (uint32_t)(gid / (nr * nr))};
+                    uint32_t w[3] = {0u, 0u, 0u};
+#pragma unroll
+                    for (int d = 0; d < D; d++) {
+                        const uint64_t len = (ext >> (21 * d) & 0x1fffffull) << sh, at = (uint64_t)root[d] << sh;
+                        const uint64_t lo = ob[2 * d] - at, hi = ob[2 * d + 1] - at;  // (lo wraps where it is cut)
+                        w[d] = term_cut(term_word((uint32_t)((lo < len ? lo : 0u) * kTermSpan / len),
+                                                  (uint32_t)((hi < len ? hi : 0u) * kTermSpan / len)),
+                                        lo < len, hi < len);
+                    }
+                    rec.x = w[0];
+                    rec.y = w[1];
+                    rec.z = w[2];
+                }
             }
             if (!take) {
             } else if (SCATTER) {
                 // after the scan a cell's counter holds its end: counting it
                 // down hands out the cell's slots (and leaves its start)
                 const uint64_t pos = (uint64_t)(atomicSub(&p.counts[gid], 1u) - 1u);
-                if (pos < p.entry_cap) p.entries[pos] = (f << kIdBits) | (uint32_t)(wbox0 + o);
+                rec.w = (f << kIdBits) | (uint32_t)(wbox0 + o);
+                if (pos < p.entry_cap) p.entries[pos] = rec;
                 else atomicOr(&p.ctr->err, kErrEntryOvf);
             } else {
                 atomicAdd(&p.counts[gid], 1u);
@@ -811,165 +882,56 @@ __global__ void k_expand(Params p) { expand_cells(p, blockIdx.x * blockDim.x + t
 // ---------------------------------------------------------------------------
 // pair test
 //
-// Three kernels share the per-pair test and the sweeps:
+// Three kernels:
 //   k_pairs_small  cells of 2..32 boxes, 32/WG cells per warp item
 //   k_pairs_med    cells of 33..kMedMax boxes, one cell per warp item,
 //                  staged whole in the warp's shared memory
 //   k_pairs_block  cells of kMedMax+1..kBigMax boxes staged whole by a
-//                  block, and 32x32 tile tasks of larger cells
-// The warp items of the small- and medium-cell kernels run independently (no
-// block barriers); each warp compacts its pairs into its own shared-memory
-// buffer and flushes it to the pair array with one global reservation per
-// flush (the block kernel does the same per block).
-//
-// The test of one (row box, column box) pair is branch free: with every
-// coordinate < 2^29 the six differences max-min are non-negative exactly
-// when the closed intervals overlap, and a negative difference sets bits
-// 29..31; the reference-cell rule adds the "does not start here" bits of
-// both boxes in bits 29..31, so the pair is reported iff the OR of all of
-// them is < 2^29. Wider coordinates use plain comparisons.
+//                  team of four warps, and 32x32 tile tasks of larger cells
+// Warps test and compact independently; each has a shared-memory buffer of
+// pairs that it flushes to the pair array with one global reservation.
+// Cells above the small ones are tested tile by tile (32 rows x 32 columns,
+// "tiles" below).
 // ---------------------------------------------------------------------------
 constexpr int kPairThreads = 256;
 constexpr int kPairWarps = kPairThreads / 32;
-constexpr uint32_t kMissShift = 29;
 constexpr uint32_t kWarpOut = 256;          // per-warp output buffer (pairs), small cells
-constexpr uint32_t kMedOut = 512;           // per-warp output buffer (pairs), medium cells: above the
+constexpr uint32_t kMedOut = 512;           // per-warp output buffer (pairs), other cells: above the
                                             // typical output of one emission step, so it rarely spills
 constexpr uint32_t kSmallSlots = 64;        // per-warp staging, small cells (each cell twice in a row)
-constexpr uint32_t kMedSlots = kMedMax;     // per-warp staging, medium cells
-constexpr uint32_t kBlockSlots = kBigMax;   // per-block staging, big cells
-constexpr uint32_t kBlockOut = 2048;        // per-block output buffer (pairs)
-// big cells per block task: two, so the few hundred big cells of a large
-// scene spread over the blocks (eight per task kept 60 of 304 blocks busy on
-// the clustered 4M-box scene: 0.060 ms; one per task 0.028, two 0.024 ms)
-constexpr uint32_t kBigCellsPerTask = 2;
 
-struct Box {
-    uint32_t x0, x1, y0, y1, z0, z1, f, id;  // f: axes where the box does not start in this cell, << 29
-};
-
-// staging arrays in shared memory: slot i = (a[i], b[i])
-struct Slots {
-    uint4* a;  // x0 x1 y0 y1
-    uint4* b;  // z0 z1 f id
-};
-
-__device__ __forceinline__ void slot_put(const Slots& s, uint32_t i, const Box& x) {
-    s.a[i] = make_uint4(x.x0, x.x1, x.y0, x.y1);
-    s.b[i] = make_uint4(x.z0, x.z1, x.f, x.id);
-}
-__device__ __forceinline__ Box slot_get(const Slots& s, uint32_t i) {
-    const uint4 a = s.a[i], b = s.b[i];
-    Box x;
-    x.x0 = a.x; x.x1 = a.y; x.y0 = a.z; x.y1 = a.w;
-    x.z0 = b.x; x.z1 = b.y; x.f = b.z; x.id = b.w;
-    return x;
-}
-__device__ __forceinline__ uint32_t slot_id(const Slots& s, uint32_t i) { return s.b[i].w; }
-
-// a box that overlaps nothing (pads tiles to multiples of 8 and idle lanes)
-template <bool NARROW>
-__device__ __forceinline__ Box dummy_box() {
-    Box x;
-    x.x0 = x.y0 = x.z0 = NARROW ? (1u << 30) : 0xffffffffu;
-    x.x1 = x.y1 = x.z1 = 0u;
-    x.f = 7u << kMissShift;
-    x.id = 0;
-    return x;
-}
-
-template <int D, bool NARROW>
-__device__ __forceinline__ Box load_box(const Params& p, uint32_t raw) {
-    Box x;
-    x.id = raw & kIdMask;
-    x.f = (~(raw >> kIdBits) & 7u) << kMissShift;
-    if (x.id >= p.nboxes) {  // cannot happen with a consistent grid; never read past the box buffer
-        atomicOr(&p.ctr->err, kErrIndex);
-        return dummy_box<NARROW>();
-    }
-    const uint32_t* b = p.boxes + (uint64_t)x.id * (2 * D + 1);
-    x.x0 = __ldg(b); x.x1 = __ldg(b + 1); x.y0 = __ldg(b + 2); x.y1 = __ldg(b + 3);
-    if (D == 3) { x.z0 = __ldg(b + 4); x.z1 = __ldg(b + 5); }
-    else { x.z0 = 0; x.z1 = 0; }
-    return x;
-}
-
-// closed-interval overlap on every axis (calcOverlaps, pbig.cu:562-577) and
-// the reference-cell rule (calcRightToWrite, pbig.cu:579-603); 1 or 0
-template <int D, bool BIP, bool NARROW>
-__device__ __forceinline__ uint32_t hit_bit(const Box& a, const Box& b, uint32_t split) {
-    uint32_t ok;
-    if (NARROW) {
-        uint32_t t = (b.x1 - a.x0) | (a.x1 - b.x0) | (b.y1 - a.y0) | (a.y1 - b.y0) | (a.f & b.f);
-        if (D == 3) t |= (b.z1 - a.z0) | (a.z1 - b.z0);
-        ok = t < (1u << kMissShift) ? 1u : 0u;
-    } else {
-        ok = ((a.x0 <= b.x1) & (b.x0 <= a.x1) & (a.y0 <= b.y1) & (b.y0 <= a.y1) & ((a.f & b.f) == 0u)) ? 1u : 0u;
-        if (D == 3) ok &= ((a.z0 <= b.z1) & (b.z0 <= a.z1)) ? 1u : 0u;
-    }
-    if (BIP) ok &= ((a.id < split) != (b.id < split)) ? 1u : 0u;
-    return ok;
-}
-
-// circular half sweep over the m boxes in slots [base, base+m): lane l < m
-// tests box l against boxes l+1 .. l+floor(m/2) (mod m), lanes past m/2 one
-// fewer when m is even (the BALANCE=1 sweep of d_matching, pbig.cu:804-825),
-// so each unordered pair is tested once. Bit d of the result: partner l+d.
-template <int D, bool BIP, bool NARROW>
-__device__ __forceinline__ uint32_t sweep_diag(const Slots& s, const Box& me, uint32_t lane, uint32_t base,
-                                               uint32_t m, uint32_t split) {
-    const uint32_t l = lane < m ? lane : 0u;
-    const uint32_t nelm = lane < m ? (lane < (m >> 1) ? (m >> 1) : ((m - 1) >> 1)) : 0u;
-    const uint32_t dmax = m >> 1;
-    uint32_t mask = 0;
-#pragma unroll 4
-    for (uint32_t d = 1; d <= dmax; d++) {
-        uint32_t pr = l + d;
-        if (pr >= m) pr -= m;
-        mask |= (hit_bit<D, BIP, NARROW>(me, slot_get(s, base + pr), split) & (d <= nelm ? 1u : 0u)) << d;
-    }
-    return mask;
-}
-
-// row box against the column boxes in slots [base, base+cols8), cols8 a
-// multiple of 8 (padding slots hold dummy boxes); bit j: column j
-template <int D, bool BIP, bool NARROW>
-__device__ __forceinline__ uint32_t sweep_cols(const Slots& s, const Box& me, uint32_t base, uint32_t cols8,
-                                               uint32_t split) {
-    uint32_t mask = 0;
-    if (cols8 == 32) {
-#pragma unroll
-        for (uint32_t j = 0; j < 32; j++) mask |= hit_bit<D, BIP, NARROW>(me, slot_get(s, base + j), split) << j;
-    } else {
-        for (uint32_t j0 = 0; j0 < cols8; j0 += 8) {
-#pragma unroll
-            for (uint32_t jj = 0; jj < 8; jj++)
-                mask |= hit_bit<D, BIP, NARROW>(me, slot_get(s, base + j0 + jj), split) << (j0 + jj);
-        }
-    }
-    return mask;
-}
 
 // ---- output: warp-private buffer ------------------------------------------
 struct WarpOut {
-    uint2* buf;
+    uint2* buf;    // candidate order: {row entry, column entry}, flag bits and all
     uint32_t n;    // warp-uniform fill
     uint32_t cap;  // buffer capacity (pairs)
     unsigned long long hits = 0;  // record mode: pairs written by this lane
 };
 
+// a buffered word as it is reported: the entries' start bits off, the
+// smaller index first, the blue index counted from the first blue box.
+// (Done here, by full warps, rather than in the emission loops, where on
+// average half the lanes are idle.) Record words are written as they are.
+template <bool BIP, bool REC>
+__device__ __forceinline__ uint2 out_pair(const Params& p, uint2 w) {
+    if (REC) return w;
+    const uint32_t a = w.x & kIdMask, b = w.y & kIdMask;
+    return make_uint2(min(a, b), BIP ? max(a, b) - p.split : max(a, b));
+}
+
 // copy n pairs (8-byte words) from shared memory to p.out[base, base + n):
-// thread t of nt (a multiple of 32) stores 16-byte units laid on the
-// destination's 128-byte lines, so a warp store covers whole lines and only
-// the first and last line of a run are partial. The pair array may be
-// page-locked host memory, where partial lines cost a large share of the
-// link's write bandwidth.
-__device__ __forceinline__ void store_run(const Params& p, unsigned long long base, const uint2* src, uint32_t n,
-                                          uint32_t t, uint32_t nt) {
+// a lane stores 16-byte units laid on the destination's 128-byte lines, so a
+// warp store covers whole lines and only the first and last line of a run
+// are partial. The pair array may be page-locked host memory, where partial
+// lines cost a large share of the link's write bandwidth.
+template <bool BIP, bool REC>
+__device__ __forceinline__ void store_run(const Params& p, unsigned long long base, const uint2* src, uint32_t n) {
+    const uint32_t lane = lane_id();
     if (base + n > p.out_cap) {
-        for (uint32_t k = t; k < n; k += nt) {
+        for (uint32_t k = lane; k < n; k += 32) {
             const unsigned long long g = base + k;
-            if (g < p.out_cap) p.out[g] = src[k];
+            if (g < p.out_cap) p.out[g] = out_pair<BIP, REC>(p, src[k]);
             else atomicOr(&p.ctr->err, kErrOutOvf);
         }
         return;
@@ -978,18 +940,19 @@ __device__ __forceinline__ void store_run(const Params& p, unsigned long long ba
     const uint32_t lead = (uint32_t)(((reinterpret_cast<uintptr_t>(p.out) >> 3) + base) & 15u);
     const uint32_t units = (lead + n + 1) >> 1;
     uint2* dst = p.out + base;
-    for (uint32_t u = t; u < units; u += nt) {
+    for (uint32_t u = lane; u < units; u += 32) {
         const int r = 2 * (int)u - (int)lead;  // first pair of the unit, relative to base
         if (r >= 0 && r + 1 < (int)n) {
-            const uint2 a = src[r], b = src[r + 1];
+            const uint2 a = out_pair<BIP, REC>(p, src[r]), b = out_pair<BIP, REC>(p, src[r + 1]);
             *reinterpret_cast<uint4*>(dst + r) = make_uint4(a.x, a.y, b.x, b.y);
         } else {
-            if (r >= 0 && r < (int)n) dst[r] = src[r];
-            if (r + 1 >= 0 && r + 1 < (int)n) dst[r + 1] = src[r + 1];
+            if (r >= 0 && r < (int)n) dst[r] = out_pair<BIP, REC>(p, src[r]);
+            if (r + 1 >= 0 && r + 1 < (int)n) dst[r + 1] = out_pair<BIP, REC>(p, src[r + 1]);
         }
     }
 }
 
+template <bool BIP, bool REC>
 __device__ __forceinline__ void wflush(const Params& p, WarpOut& o) {
     if (o.n == 0) return;
     const uint32_t lane = lane_id();
@@ -997,17 +960,18 @@ __device__ __forceinline__ void wflush(const Params& p, WarpOut& o) {
     if (lane == 0) base = atomicAdd(&p.ctr->pairs, (unsigned long long)o.n);
     base = __shfl_sync(FULL_MASK, base, 0);
     __syncwarp();
-    store_run(p, base, o.buf, o.n, lane, 32);
+    store_run<BIP, REC>(p, base, o.buf, o.n);
     __syncwarp();
     o.n = 0;
 }
 
 // compaction of the set bits of two masks (ranks from one warp scan of the
 // per-lane popcounts) into the warp buffer, or straight to the pair array
-// when the batch is larger than the buffer
+// when the batch is larger than the buffer. pa, pb: the entry (or box index)
+// of a bit's column; row: this lane's own.
 template <bool BIP, class PA, class PB>
 __device__ __forceinline__ void wemit(const Params& p, WarpOut& o, uint32_t ma, PA pa, uint32_t mb, PB pb,
-                                      uint32_t myid) {
+                                      uint32_t row) {
     const uint32_t lane = lane_id();
     const uint32_t k = __popc(ma) + __popc(mb);
     const uint32_t incl = warp_incl_scan(k);
@@ -1016,7 +980,7 @@ __device__ __forceinline__ void wemit(const Params& p, WarpOut& o, uint32_t ma, 
     bool direct = false;
     unsigned long long gbase = 0;
     if (o.n + total > o.cap) {
-        wflush(p, o);
+        wflush<BIP, false>(p, o);
         if (total > o.cap) {
             direct = true;
             if (lane == 0) gbase = atomicAdd(&p.ctr->pairs, (unsigned long long)total);
@@ -1024,22 +988,17 @@ __device__ __forceinline__ void wemit(const Params& p, WarpOut& o, uint32_t ma, 
         }
     }
     uint32_t w = incl - k;
-    auto pair = [&](uint32_t q) {
-        uint2 pr = make_uint2(min(myid, q), max(myid, q));
-        if (BIP) pr.y -= p.split;
-        return pr;
-    };
     if (!direct) {  // (warp-uniform: the loops below carry no per-pair branch)
         uint2* dst = o.buf + o.n + w;
         while (ma) {
             const uint32_t bit = 31u - __clz(ma);  // highest set bit first
             ma ^= 1u << bit;
-            *dst++ = pair(pa(bit));
+            *dst++ = make_uint2(row, pa(bit));
         }
         while (mb) {
             const uint32_t bit = 31u - __clz(mb);
             mb ^= 1u << bit;
-            *dst++ = pair(pb(bit));
+            *dst++ = make_uint2(row, pb(bit));
         }
         __syncwarp();
         o.n += total;
@@ -1047,7 +1006,7 @@ __device__ __forceinline__ void wemit(const Params& p, WarpOut& o, uint32_t ma, 
     }
     auto put = [&](uint32_t q) {
         const unsigned long long g = gbase + w;
-        if (g < p.out_cap) p.out[g] = pair(q);
+        if (g < p.out_cap) p.out[g] = out_pair<BIP, false>(p, make_uint2(row, q));
         else atomicOr(&p.ctr->err, kErrOutOvf);
         w++;
     };
@@ -1118,7 +1077,7 @@ __device__ __forceinline__ void remit(const Params& p, WarpOut& o, uint32_t ma, 
     bool direct = false;
     unsigned long long gbase = 0;
     if (o.n + total > o.cap) {
-        wflush(p, o);
+        wflush<false, true>(p, o);
         if (total > o.cap) {
             direct = true;
             if (lane == 0) gbase = atomicAdd(&p.ctr->pairs, (unsigned long long)total);
@@ -1141,195 +1100,60 @@ __device__ __forceinline__ void remit(const Params& p, WarpOut& o, uint32_t ma, 
     if (!direct) o.n += total;
 }
 
-// row tile r of a cell staged at slots [off, off + n8): the diagonal tile and
-// every column tile x > r, emitted two tiles at a time
-template <int D, bool BIP, bool NARROW, bool REC, class Emit>
-__device__ __forceinline__ void row_unit(const Params& p, const Slots& s, uint32_t off, uint32_t n, uint32_t r,
-                                         Emit emit) {
-    const uint32_t lane = lane_id();
-    const uint32_t R = (n + 31) >> 5;
-    const uint32_t rows = min(32u, n - 32 * r);
-    const uint32_t rbase = off + 32 * r;
-    const Box me = lane < rows ? slot_get(s, rbase + lane) : dummy_box<NARROW>();
-    const uint32_t md = sweep_diag<D, BIP, NARROW>(s, me, lane, rbase, rows, p.split);
-    if constexpr (REC) {  // records: cell-local row and column indices
-        const uint32_t row = 32 * r + lane;
-        auto ldiag = [&](uint32_t d) {
-            uint32_t pr = lane + d;
-            if (pr >= rows) pr -= rows;
-            return 32 * r + pr;
-        };
-        uint32_t x = r + 1;
-        if (x >= R) {
-            emit(md, ldiag, 0u, ldiag, row);
-            return;
-        }
-        {
-            const uint32_t cb = off + 32 * x, c8 = (min(32u, n - 32 * x) + 7) & ~7u;
-            const uint32_t mc = sweep_cols<D, BIP, NARROW>(s, me, cb, c8, p.split);
-            emit(md, ldiag, mc, [&](uint32_t j) { return 32 * x + j; }, row);
-        }
-        for (x = r + 2; x < R; x += 2) {
-            const uint32_t cb1 = off + 32 * x, c81 = (min(32u, n - 32 * x) + 7) & ~7u;
-            const uint32_t m1 = sweep_cols<D, BIP, NARROW>(s, me, cb1, c81, p.split);
-            uint32_t m2 = 0;
-            if (x + 1 < R)
-                m2 = sweep_cols<D, BIP, NARROW>(s, me, off + 32 * (x + 1), (min(32u, n - 32 * (x + 1)) + 7) & ~7u,
-                                                p.split);
-            emit(m1, [&](uint32_t j) { return 32 * x + j; }, m2, [&](uint32_t j) { return 32 * (x + 1) + j; }, row);
-        }
-        return;
-    }
-    auto pdiag = [&](uint32_t d) {
-        uint32_t pr = lane + d;
-        if (pr >= rows) pr -= rows;
-        return slot_id(s, rbase + pr);
-    };
-    uint32_t x = r + 1;
-    if (x >= R) {
-        emit(md, pdiag, 0u, pdiag, me.id);
-        return;
-    }
-    {
-        const uint32_t cb = off + 32 * x, c8 = (min(32u, n - 32 * x) + 7) & ~7u;
-        const uint32_t mc = sweep_cols<D, BIP, NARROW>(s, me, cb, c8, p.split);
-        emit(md, pdiag, mc, [&](uint32_t j) { return slot_id(s, cb + j); }, me.id);
-    }
-    for (x = r + 2; x < R; x += 2) {
-        const uint32_t cb1 = off + 32 * x, c81 = (min(32u, n - 32 * x) + 7) & ~7u;
-        const uint32_t m1 = sweep_cols<D, BIP, NARROW>(s, me, cb1, c81, p.split);
-        uint32_t m2 = 0, cb2 = cb1;
-        if (x + 1 < R) {
-            cb2 = off + 32 * (x + 1);
-            m2 = sweep_cols<D, BIP, NARROW>(s, me, cb2, (min(32u, n - 32 * (x + 1)) + 7) & ~7u, p.split);
-        }
-        emit(m1, [&](uint32_t j) { return slot_id(s, cb1 + j); }, m2, [&](uint32_t j) { return slot_id(s, cb2 + j); },
-             me.id);
-    }
-}
-
-// Medium-cell staging. With coordinates < 2^29 a slot holds its box as the
-// six signed terms (-x1, x0, -y1, y0, -z1, z0) (then f and the index), and a
-// row box is taken as the partner terms (x0-1, -x1-1, y0-1, -y1-1, z0-1,
-// -z1-1). Each sum row_k + col_k is the gap between the two boxes along one
-// axis and side minus one (a.x0 - c.x1 - 1, c.x0 - a.x1 - 1, ...), so the
-// closed boxes overlap iff the largest of the six sums is negative: one add
-// and five add-max instructions per test, the result's sign bit the hit.
-// Wider coordinates keep the plain layout and comparisons.
-struct SepRow {
-    int t0, t1, t2, t3, t4, t5;
-};
-template <bool NARROW> struct MedRowT { using type = Box; };
-template <> struct MedRowT<true> { using type = SepRow; };
-
-// (with narrow coordinates the b array's space holds the z terms,
-// uint2[kMedSlots], then {f, id}, uint2[kMedSlots]: 8-byte loads of
-// consecutive slots take two wavefronts a warp, not four)
-__device__ __forceinline__ uint2* med_z(const Slots& s) { return reinterpret_cast<uint2*>(s.b); }
-__device__ __forceinline__ uint2* med_fi(const Slots& s) { return reinterpret_cast<uint2*>(s.b) + kMedSlots; }
-
-template <bool NARROW>
-__device__ __forceinline__ void med_slot_put(const Slots& s, uint32_t i, const Box& x) {
-    if constexpr (NARROW) {
-        s.a[i] = make_uint4(0u - x.x1, x.x0, 0u - x.y1, x.y0);
-        med_z(s)[i] = make_uint2(0u - x.z1, x.z0);
-        med_fi(s)[i] = make_uint2(x.f, x.id);
-    } else {
-        slot_put(s, i, x);
-    }
-}
-
-// a staged medium-cell box in slot_get's form
-template <bool NARROW>
-__device__ __forceinline__ Box med_slot_get(const Slots& s, uint32_t i) {
-    if constexpr (NARROW) {
-        const uint4 a = s.a[i];
-        const uint2 z = med_z(s)[i], fi = med_fi(s)[i];
-        Box x;
-        x.x0 = a.x; x.x1 = a.y; x.y0 = a.z; x.y1 = a.w;
-        x.z0 = z.x; x.z1 = z.y; x.f = fi.x; x.id = fi.y;
-        return x;
-    } else {
-        return slot_get(s, i);
-    }
-}
-
-template <bool NARROW>
-__device__ __forceinline__ uint32_t med_slot_id(const Slots& s, uint32_t i) {
-    if constexpr (NARROW) return med_fi(s)[i].y;
-    else return slot_id(s, i);
-}
-
-// the row form of a staged box (st: slot_get of its slot)
-template <bool NARROW>
-__device__ __forceinline__ typename MedRowT<NARROW>::type med_row(const Box& st) {
-    if constexpr (NARROW) {  // slot_get maps (-x1, x0, -y1, y0, -z1, z0) to (x0, x1, y0, y1, z0, z1)
-        return SepRow{(int)st.x1 - 1, (int)st.x0 - 1, (int)st.y1 - 1, (int)st.y0 - 1, (int)st.z1 - 1, (int)st.z0 - 1};
-    } else {
-        return st;
-    }
-}
-
-// bit 31 set iff row box r and column box (ca, cz) overlap
-template <int D>
-__device__ __forceinline__ uint32_t sep_hit(const SepRow& r, const uint4& ca, const uint2& cz) {
-    int m = r.t0 + (int)ca.x;
-    m = __viaddmax_s32(r.t1, (int)ca.y, m);
-    m = __viaddmax_s32(r.t2, (int)ca.z, m);
-    m = __viaddmax_s32(r.t3, (int)ca.w, m);
-    if (D == 3) {
-        m = __viaddmax_s32(r.t4, (int)cz.x, m);
-        m = __viaddmax_s32(r.t5, (int)cz.y, m);
-    }
-    return (uint32_t)m;
-}
-
 // ---- small cells ------------------------------------------------------------
 // lane group g (WG lanes) holds cell item*G+g of the class list, lane r its
-// box r; the circular half sweep runs inside the group.
-template <int D, int WG, bool NARROW, bool REC>
-__device__ __forceinline__ Box small_fetch(const Params& p, int list, uint64_t nl, uint64_t ci, uint32_t r,
-                                           uint32_t& n, uint32_t& gid) {
-    n = 0;
-    gid = 0;
-    uint32_t start = 0;
-    if (ci < nl) {
-        const uint2 sn = p.lists[p.list_off[list] + ci];
-        start = sn.x;
-        n = sn.y;
-        if (REC) {  // the list holds the cell id; its start is in the counters after the scatter
-            gid = sn.x;
-            start = gid < p.ncells ? p.counts[gid] : 0xffffffffu;
-        }
-        if (n > WG || (uint64_t)start + n > p.entry_cap) n = 0;  // inconsistent grid: skip
+// entry r; the circular half sweep runs inside the group: lane l < n tests
+// its box against boxes l+1 .. l+floor(n/2) (mod n), lanes past n/2 one fewer
+// when n is even (the BALANCE=1 sweep of d_matching, pbig.cu:804-825), so each
+// unordered pair is tested once. The group's cell is staged twice in a row, so
+// partner r+d needs no wrap. A row is its entry with each word's halves
+// swapped: row plus column holds the two sides of an axis, so the boxes
+// overlap iff the largest sums of both halves are below 32768 -- a u16x2
+// add-max per axis. The
+// reference-cell and red/blue rules are applied once per cell from ballots.
+
+// the hits of `mask` (bit d: partner slot i + d) that hold on the whole coordinates
+template <int D>
+__device__ __noinline__ uint32_t small_exact(const uint32_t* boxes, uint64_t nboxes, const uint4* s, uint32_t i,
+                                             uint32_t mask) {
+    uint32_t keep = 0;
+    while (mask) {
+        const uint32_t d = __ffs(mask) - 1;
+        mask &= mask - 1;
+        const uint32_t a = s[i].w & kIdMask, b = s[i + d].w & kIdMask;
+        if (a >= nboxes || b >= nboxes) continue;  // cannot happen with a consistent grid
+        const uint32_t *x = boxes + (uint64_t)a * (2 * D + 1), *y = boxes + (uint64_t)b * (2 * D + 1);
+        bool hit = true;
+#pragma unroll
+        for (int k = 0; k < D; k++)
+            hit = hit && __ldg(x + 2 * k) <= __ldg(y + 2 * k + 1) && __ldg(y + 2 * k) <= __ldg(x + 2 * k + 1);
+        keep |= (hit ? 1u : 0u) << d;
     }
-    return r < n ? load_box<D, NARROW>(p, p.entries[start + r]) : dummy_box<NARROW>();
+    return keep;
 }
 
-template <int D, int WG, bool BIP, bool NARROW, bool REC>
-__device__ __forceinline__ void small_sweep(const Params& p, const Slots& s, WarpOut& o, const Box& me, uint32_t n,
-                                            uint32_t lane, uint32_t g, uint32_t r, uint32_t gid) {
-    if constexpr (NARROW && !REC) {
-        // the medium-cell test: boxes staged as separation terms, one add and
-        // add-max instructions per test; the group's cell staged twice in a
-        // row, so partner r+d needs no wrap; the reference-cell and red/blue
-        // rules applied once per cell from ballots. Slot i: s.a[i] the x and y
-        // terms, then in s.b's space the z terms (8 bytes per slot, so a
-        // warp's loads take two wavefronts) and the box index.
-        const uint32_t gb = g * (2 * WG);
-        uint2* zz = reinterpret_cast<uint2*>(s.b);
-        uint32_t* ids = reinterpret_cast<uint32_t*>(s.b) + 2 * kSmallSlots;
+template <int D, int WG, bool BIP, bool REC, bool FRESH = false>
+__device__ __forceinline__ void small_items(const Params& p, uint4* s, WarpOut& o, int list, uint64_t first,
+                                            uint64_t stride) {
+    constexpr uint32_t G = 32 / WG;
+    const uint32_t lane = lane_id(), g = lane / WG, r = lane % WG, gb = g * (2 * WG);
+    const uint64_t nl = mn64(ctr_read<FRESH>(&p.ctr->n_list[list]), p.list_cap[list]);
+    const uint64_t nitems = (nl + G - 1) / G;
+    for (uint64_t item = first; item < nitems; item += stride) {
+        const uint64_t ci = item * G + g;
+        uint32_t n = 0, gid = 0, start = 0;
+        if (ci < nl) {
+            const uint2 sn = p.lists[p.list_off[list] + ci];
+            gid = sn.x;  // record mode: the list holds the cell id; its start is in the counters after the scatter
+            start = REC ? (gid < p.ncells ? p.counts[gid] : 0xffffffffu) : sn.x;
+            n = sn.y;
+            if (n > WG || (uint64_t)start + n > p.entry_cap) n = 0;  // inconsistent grid: skip
+        }
+        const uint4 me = r < n ? p.entries[start + r] : entry_empty();
+        __syncwarp();  // (the last item's slots are read)
         if (r < n) {
-            const uint4 xa = make_uint4(0u - me.x1, me.x0, 0u - me.y1, me.y0);
-            s.a[gb + r] = xa;
-            s.a[gb + n + r] = xa;
-            if (D == 3) {
-                const uint2 zt = make_uint2(0u - me.z1, me.z0);
-                zz[gb + r] = zt;
-                zz[gb + n + r] = zt;
-            }
-            ids[gb + r] = me.id;
-            ids[gb + n + r] = me.id;
+            s[gb + r] = me;
+            s[gb + n + r] = me;
         }
         __syncwarp();
         const uint32_t nelm = r < n ? (r < (n >> 1) ? (n >> 1) : ((n - 1) >> 1)) : 0u;
@@ -1337,79 +1161,49 @@ __device__ __forceinline__ void small_sweep(const Params& p, const Slots& s, War
         // bit j: group lane j is a partner the rules exclude
         const uint32_t sh = WG == 32 ? 0u : g * WG;
         const uint32_t nm = n >= 32u ? FULL_MASK : ((1u << n) - 1u);
-        const uint32_t fa = me.f >> kMissShift;
-        const uint32_t m0 = (__ballot_sync(FULL_MASK, (fa & 1u) != 0u) >> sh) & nm;
-        const uint32_t m1 = (__ballot_sync(FULL_MASK, (fa & 2u) != 0u) >> sh) & nm;
-        const uint32_t m2 = (__ballot_sync(FULL_MASK, (fa & 4u) != 0u) >> sh) & nm;
-        uint32_t deny = ((fa & 1u) ? m0 : 0u) | ((fa & 2u) ? m1 : 0u) | ((fa & 4u) ? m2 : 0u);
+        const bool f0 = ((me.w >> kIdBits) & 1u) == 0u, f1 = ((me.w >> (kIdBits + 1)) & 1u) == 0u;
+        const bool f2 = ((me.w >> (kIdBits + 2)) & 1u) == 0u;
+        const uint32_t m0 = (__ballot_sync(FULL_MASK, f0) >> sh) & nm;
+        const uint32_t m1 = (__ballot_sync(FULL_MASK, f1) >> sh) & nm;
+        const uint32_t m2 = (__ballot_sync(FULL_MASK, f2) >> sh) & nm;
+        uint32_t deny = (f0 ? m0 : 0u) | (f1 ? m1 : 0u) | (f2 ? m2 : 0u);
         if (BIP) {
-            const uint32_t red = (__ballot_sync(FULL_MASK, me.id < p.split) >> sh) & nm;
-            deny |= me.id < p.split ? red : (~red & nm);
+            const bool is_red = (me.w & kIdMask) < p.split;
+            const uint32_t red = (__ballot_sync(FULL_MASK, is_red) >> sh) & nm;
+            deny |= is_red ? red : (~red & nm);
         }
         // bit d: partner (r + d) mod n
         uint32_t rot = 0;
         if (r < n) rot = n >= 32u ? __funnelshift_r(deny, deny, r) : (((deny >> r) | (deny << (n - r))) & nm);
-        const SepRow row{(int)me.x0 - 1, -(int)me.x1 - 1, (int)me.y0 - 1, -(int)me.y1 - 1, (int)me.z0 - 1,
-                         -(int)me.z1 - 1};
-        uint32_t mask = 0;
+        const uint32_t rx = __byte_perm(me.x, 0u, 0x1032), ry = __byte_perm(me.y, 0u, 0x1032);
+        const uint32_t rz = __byte_perm(me.z, 0u, 0x1032);
+        uint32_t miss = 0, top = 0;
 #pragma unroll
         for (uint32_t d = 1; d <= WG / 2; d++) {
             if (d > dlim) break;
-            const uint32_t i = gb + r + d;
-            const uint4 ca = s.a[i];
-            const uint2 cz = D == 3 ? zz[i] : make_uint2(0u, 0u);
-            mask |= (sep_hit<D>(row, ca, cz) >> 31) << d;
+            const uint4 c = s[gb + r + d];
+            uint32_t m = __viaddmax_u16x2(ry, c.y, rx + c.x);
+            if (D == 3) m = __viaddmax_u16x2(rz, c.z, m);
+            m = __vmaxu2(m, __byte_perm(m, 0u, 0x1032));
+            top = __vmaxs2(top, m);
+            miss |= (m >> 31) << d;
         }
-        mask &= ~rot & ((2u << nelm) - 2u);
-        auto pid = [&](uint32_t d) { return ids[gb + r + d]; };
-        wemit<BIP>(p, o, mask, pid, 0u, pid, me.id);
-        return;
-    }
-    slot_put(s, lane, me);
-    __syncwarp();
-    const uint32_t gb = g * WG;
-    const uint32_t nelm = r < n ? (r < (n >> 1) ? (n >> 1) : ((n - 1) >> 1)) : 0u;
-    // partners a lane of the warp needs at most: the sweep stops there rather
-    // than at WG/2 (a cell of 17 boxes in a 32-lane group needs 8, not 16)
-    const uint32_t dlim = __reduce_max_sync(FULL_MASK, nelm);
-    uint32_t mask = 0;
-#pragma unroll
-    for (uint32_t d = 1; d <= WG / 2; d++) {
-        if (d > dlim) break;
-        uint32_t pr = r + d;
-        if (pr >= n) pr -= n;
-        if (pr >= WG) pr = 0;  // idle lanes (n = 0) stay inside the group
-        mask |= (hit_bit<D, BIP, NARROW>(me, slot_get(s, gb + pr), p.split) & (d <= nelm ? 1u : 0u)) << d;
-    }
-    if constexpr (REC) {
-        auto ploc = [&](uint32_t d) {
-            uint32_t pr = r + d;
-            if (pr >= n) pr -= n;
-            return pr;
-        };
-        const uint32_t gmask = WG == 32 ? FULL_MASK : (((1u << WG) - 1u) << (g * WG));
-        remit(p, o, mask, ploc, 0u, ploc, r, gid, gmask);
-    } else {
-        auto pid = [&](uint32_t d) {
-            uint32_t pr = r + d;
-            if (pr >= n) pr -= n;
-            return slot_id(s, gb + pr);
-        };
-        wemit<BIP>(p, o, mask, pid, 0u, pid, me.id);
-    }
-}
-
-template <int D, int WG, bool BIP, bool NARROW, bool REC, bool FRESH = false>
-__device__ __forceinline__ void small_items(const Params& p, const Slots& s, WarpOut& o, int list, uint64_t first,
-                                            uint64_t stride) {
-    constexpr uint32_t G = 32 / WG;
-    const uint32_t lane = lane_id(), g = lane / WG, r = lane % WG;
-    const uint64_t nl = mn64(ctr_read<FRESH>(&p.ctr->n_list[list]), p.list_cap[list]);
-    const uint64_t nitems = (nl + G - 1) / G;
-    for (uint64_t item = first; item < nitems; item += stride) {
-        uint32_t n1, gid;
-        const Box a = small_fetch<D, WG, NARROW, REC>(p, list, nl, item * G + g, r, n1, gid);
-        small_sweep<D, WG, BIP, NARROW, REC>(p, s, o, a, n1, lane, g, r, gid);
+        uint32_t mask = ~miss & ~rot & ((2u << nelm) - 2u);
+        // a largest sum of 32767 may be two corners of one scaled value
+        if (p.open && top == 0x7fff7fffu && mask) mask = small_exact<D>(p.boxes, p.nboxes, s, gb + r, mask);
+        __syncwarp();
+        if constexpr (REC) {
+            auto ploc = [&](uint32_t d) {
+                uint32_t pr = r + d;
+                if (pr >= n) pr -= n;
+                return pr;
+            };
+            const uint32_t gmask = WG == 32 ? FULL_MASK : (((1u << WG) - 1u) << (g * WG));
+            remit(p, o, mask, ploc, 0u, ploc, r, gid, gmask);
+        } else {
+            auto pid = [&](uint32_t d) { return s[gb + r + d].w; };
+            wemit<BIP>(p, o, mask, pid, 0u, pid, me.w);
+        }
     }
 }
 
@@ -1419,156 +1213,300 @@ __device__ __forceinline__ void rec_hits(const Params& p, const WarpOut& o) {
     if (lane_id() == 0 && h) atomicAdd(&p.ctr->rec_pairs, h);
 }
 
-// the four small-cell lists, warp gw of nw; per-warp staging in s_a, s_b
-// (kSmallSlots each) and an output buffer of kWarpOut pairs
-template <int D, bool BIP, bool NARROW, bool REC, bool FRESH = false>
-__device__ __forceinline__ void small_pass(const Params& p, uint4* s_a, uint4* s_b, uint2* s_out, uint64_t gw,
-                                           uint64_t nw) {
-    const Slots s{s_a, s_b};
+// the four small-cell lists, warp gw of nw; per-warp staging of kSmallSlots
+// entries in s and an output buffer of kWarpOut pairs
+template <int D, bool BIP, bool REC, bool FRESH = false>
+__device__ __forceinline__ void small_pass(const Params& p, uint4* s, uint2* s_out, uint64_t gw, uint64_t nw) {
     WarpOut o{s_out, 0, kWarpOut};
     // classes interleaved over the warps so every warp gets a similar mix
-    small_items<D, 32, BIP, NARROW, REC, FRESH>(p, s, o, 3, gw, nw);
-    small_items<D, 16, BIP, NARROW, REC, FRESH>(p, s, o, 2, (gw + nw / 4) % nw, nw);
-    small_items<D, 8, BIP, NARROW, REC, FRESH>(p, s, o, 1, (gw + nw / 2) % nw, nw);
-    small_items<D, 4, BIP, NARROW, REC, FRESH>(p, s, o, 0, (gw + 3 * nw / 4) % nw, nw);
-    wflush(p, o);
+    small_items<D, 32, BIP, REC, FRESH>(p, s, o, 3, gw, nw);
+    small_items<D, 16, BIP, REC, FRESH>(p, s, o, 2, (gw + nw / 4) % nw, nw);
+    small_items<D, 8, BIP, REC, FRESH>(p, s, o, 1, (gw + nw / 2) % nw, nw);
+    small_items<D, 4, BIP, REC, FRESH>(p, s, o, 0, (gw + 3 * nw / 4) % nw, nw);
+    wflush<BIP, REC>(p, o);
     if (REC) rec_hits(p, o);
 }
 
-template <int D, bool BIP, bool NARROW, bool REC = false>
+template <int D, bool BIP, bool REC = false>
 __global__ void __launch_bounds__(kPairThreads, 5) k_pairs_small(Params p) {
-    __shared__ uint4 s_a[kPairWarps][kSmallSlots], s_b[kPairWarps][kSmallSlots];
+    __shared__ uint4 s_slot[kPairWarps][kSmallSlots];
     __shared__ uint2 s_out[kPairWarps][kWarpOut];
     const uint32_t warp = threadIdx.x >> 5;
-    small_pass<D, BIP, NARROW, REC>(p, s_a[warp], s_b[warp], s_out[warp], (uint64_t)blockIdx.x * kPairWarps + warp,
-                                    (uint64_t)gridDim.x * kPairWarps);
+    small_pass<D, BIP, REC>(p, s_slot[warp], s_out[warp], (uint64_t)blockIdx.x * kPairWarps + warp,
+                            (uint64_t)gridDim.x * kPairWarps);
+}
+
+// ---- tiles ------------------------------------------------------------------
+// Cells above the small ones are tested tile by tile, 32 rows against 32
+// columns, staged in shared memory as pairs of columns: a word holds one term
+// of two boxes, so an add, five u16x2 add-max instructions and two shared
+// loads test two columns. The kernels are bound by these instructions (the
+// integer pipe issues one of them every other clock; the plain add has a
+// second pipe). With 32-bit terms of one column the shared loads alone would
+// allow 20 tests/ns per SM, and a sweep with a partner of its own per lane 10;
+// a tile against itself is therefore swept whole and masked, rather than in a
+// half sweep.
+//
+// Slot 8b + g of a tile is that bit of the masks and holds box 4g + b; column
+// pair j holds the boxes 2j and 2j + 1. So the signs of two pairs, spread over
+// bytes by one prmt, go to bit g of every byte, and the columns of a partial
+// tile end with group ceil(n/4).
+//
+// Cells of 2^15 or wider: a sum of exactly 32767 may be two corners that share
+// a scaled value, which leaves the test open when no other sum is larger. The
+// sweep keeps the largest signed value it saw (32767 is the largest there is),
+// and a tile that met one is tested again on the whole coordinates (about 1 %
+// of the tiles of random boxes).
+//
+// Red/blue queries stage the two colours apart, so their tiles are red rows
+// against blue columns (or the other way, whichever takes fewer steps), and a
+// cell of one colour costs no more than reading its entries.
+constexpr uint32_t kMedTiles = kMedMax / 32 + 1;   // (+ 1: two colours, each rounded up to whole tiles)
+constexpr uint32_t kBigTiles = kBigMax / 32 + 1;
+constexpr uint32_t kHugeTiles = 3;                 // a row tile and two column tiles
+constexpr uint32_t kTileBytes = 16 * (sizeof(uint4) + sizeof(uint2)) + 32 * sizeof(uint32_t);
+
+struct Tiles {
+    uint4* xy;      // 16 per tile: {x1, x0, y1, y0} terms of a column pair, the second column in the high halves
+    uint2* z;       // 16 per tile: {z1, z0}
+    uint32_t* raw;  // 32 per tile: the entries' last words (start bits << 29 | box index)
+    __device__ __forceinline__ Tiles(unsigned char* m, uint32_t tiles)
+        : xy(reinterpret_cast<uint4*>(m)), z(reinterpret_cast<uint2*>(xy + 16 * tiles)),
+          raw(reinterpret_cast<uint32_t*>(z + 16 * tiles)) {}
+};
+
+// box e of a tile <-> its slot
+__device__ __forceinline__ uint32_t tile_slot(uint32_t e) { return ((e & 3u) << 3) | (e >> 2); }
+__device__ __forceinline__ uint32_t tile_box(uint32_t s) { return ((s & 7u) << 2) | (s >> 3); }
+__device__ __forceinline__ uint32_t tile_fill(uint32_t n, uint32_t x) { return min(32u, n - 32u * x); }
+
+// column pair j of tile x: entries a and b
+template <int D>
+__device__ __forceinline__ void tile_put_pair(const Tiles& t, uint32_t x, uint32_t j, const uint4& a, const uint4& b) {
+    t.xy[16 * x + j] = make_uint4(__byte_perm(a.x, b.x, 0x5410), __byte_perm(a.x, b.x, 0x7632),
+                                  __byte_perm(a.y, b.y, 0x5410), __byte_perm(a.y, b.y, 0x7632));
+    if (D == 3) t.z[16 * x + j] = make_uint2(__byte_perm(a.z, b.z, 0x5410), __byte_perm(a.z, b.z, 0x7632));
+    const uint32_t s = 32 * x + tile_slot(2 * j);
+    t.raw[s] = a.w;
+    t.raw[s + 8] = b.w;
+}
+
+// one entry into slot `slot` of tile x
+template <int D>
+__device__ __forceinline__ void tile_put(const Tiles& t, uint32_t x, uint32_t slot, const uint4& e) {
+    const uint32_t box = tile_box(slot), j = 16 * x + (box >> 1);
+    unsigned short* a = reinterpret_cast<unsigned short*>(t.xy + j) + (box & 1u);
+    a[0] = (unsigned short)e.x;
+    a[2] = (unsigned short)(e.x >> 16);
+    a[4] = (unsigned short)e.y;
+    a[6] = (unsigned short)(e.y >> 16);
+    if (D == 3) {
+        unsigned short* b = reinterpret_cast<unsigned short*>(t.z + j) + (box & 1u);
+        b[0] = (unsigned short)e.z;
+        b[2] = (unsigned short)(e.z >> 16);
+    }
+    t.raw[32 * x + slot] = e.w;
+}
+
+// empty slots of a group's last tile (red/blue: the slots are filled one by one)
+template <int D>
+__device__ __forceinline__ void tile_clear_rest(const Tiles& t, uint32_t tile, uint32_t n) {
+    const uint32_t slot = lane_id();
+    if ((n & 31u) != 0u && tile_box(slot) >= (n & 31u)) tile_put<D>(t, tile, slot, entry_empty());
+}
+
+__device__ __forceinline__ uint4 entry_at(const Params& p, uint32_t start, uint32_t e, uint32_t n) {
+    return e < n ? p.entries[start + e] : entry_empty();
+}
+
+// a row: this lane's slot of a tile, each term in both halves of its word,
+// and a full mask per axis that it does not start on
+template <int D>
+struct Row {
+    uint32_t t[2 * D];
+    uint32_t raw, f0, f1, f2;
+};
+template <int D>
+__device__ __forceinline__ Row<D> tile_row(const Tiles& t, uint32_t x) {
+    const uint32_t lane = lane_id(), box = tile_box(lane), sel = box & 1u ? 0x3232u : 0x1010u;
+    const uint4 a = t.xy[16 * x + (box >> 1)];
+    Row<D> r;
+    r.t[0] = __byte_perm(a.y, 0u, sel);  // (a row's lower corner meets the columns' upper ones)
+    r.t[1] = __byte_perm(a.x, 0u, sel);
+    r.t[2] = __byte_perm(a.w, 0u, sel);
+    r.t[3] = __byte_perm(a.z, 0u, sel);
+    if (D == 3) {
+        const uint2 z = t.z[16 * x + (box >> 1)];
+        r.t[2 * D - 2] = __byte_perm(z.y, 0u, sel);
+        r.t[2 * D - 1] = __byte_perm(z.x, 0u, sel);
+    }
+    r.raw = t.raw[32 * x + lane];
+    r.f0 = (r.raw >> kIdBits) & 1u ? 0u : ~0u;
+    r.f1 = (r.raw >> (kIdBits + 1)) & 1u ? 0u : ~0u;
+    r.f2 = (r.raw >> (kIdBits + 2)) & 1u ? 0u : ~0u;
+    return r;
+}
+
+template <int D>
+__device__ __forceinline__ uint32_t tile_pair(const Tiles& t, const Row<D>& r, uint32_t i) {
+    const uint4 c = t.xy[i];
+    uint32_t m = __viaddmax_u16x2(r.t[1], c.y, r.t[0] + c.x);  // (the halves of the plain add carry nothing)
+    m = __viaddmax_u16x2(r.t[2], c.z, m);
+    m = __viaddmax_u16x2(r.t[3], c.w, m);
+    if (D == 3) {
+        const uint2 z = t.z[i];
+        m = __viaddmax_u16x2(r.t[2 * D - 2], z.x, m);
+        m = __viaddmax_u16x2(r.t[2 * D - 1], z.y, m);
+    }
+    return m;
+}
+// column pairs i and i + 1: a miss sets the bit `bits` has in its byte
+template <int D>
+__device__ __forceinline__ void tile_group(const Tiles& t, const Row<D>& r, uint32_t i, uint32_t bits, uint32_t& miss,
+                                           uint32_t& top) {
+    const uint32_t m = tile_pair<D>(t, r, i), n = tile_pair<D>(t, r, i + 1);
+    uint32_t signs;  // a byte per half: all its sign bit
+    asm("prmt.b32 %0, %1, %2, 0xfdb9;" : "=r"(signs) : "r"(m), "r"(n));
+    top = __vimax3_s16x2(top, m, n);
+    miss |= signs & bits;
+}
+
+// the same tile on the whole coordinates: the column boxes pass from lane to
+// lane (rare, so it reads the boxes rather than keep them staged)
+template <int D>
+__device__ __noinline__ uint32_t tile_exact(const uint32_t* boxes, uint64_t nboxes, uint32_t row, uint32_t col,
+                                            uint32_t rows, uint32_t cols) {
+    const uint32_t e = tile_box(lane_id());
+    const uint32_t ri = row & kIdMask, ci = col & kIdMask;
+    uint32_t a[2 * D], b[2 * D];
+    const bool rv = e < rows && ri < nboxes, cv = e < cols && ci < nboxes;
+#pragma unroll
+    for (int k = 0; k < 2 * D; k++) {
+        a[k] = rv ? __ldg(boxes + (uint64_t)ri * (2 * D + 1) + k) : 0u;
+        b[k] = cv ? __ldg(boxes + (uint64_t)ci * (2 * D + 1) + k) : 0u;
+    }
+    uint32_t mask = 0;
+    for (uint32_t j = 0; j < 32; j++) {
+        bool hit = true;
+#pragma unroll
+        for (int d = 0; d < D; d++)
+            hit = hit & (a[2 * d] <= __shfl_sync(FULL_MASK, b[2 * d + 1], j)) &
+                  (__shfl_sync(FULL_MASK, b[2 * d], j) <= a[2 * d + 1]);
+        mask |= (hit ? 1u : 0u) << j;
+    }
+    const uint32_t there = __ballot_sync(FULL_MASK, cv);
+    return rv ? mask & there : 0u;
+}
+
+// the bits of the slots of groups `groups` .. 7
+__device__ __forceinline__ uint32_t tile_beyond(uint32_t groups) { return ((0xffu << groups) & 0xffu) * 0x01010101u; }
+
+// row tile against column tile x of `cols` boxes: bit s set iff this lane's
+// box and slot s overlap and the reference-cell rule reports them here
+template <int D>
+__device__ __forceinline__ uint32_t tile_hits(const Params& p, const Tiles& t, const Row<D>& r, uint32_t rows,
+                                              uint32_t x, uint32_t cols) {
+    uint32_t miss = 0, top = 0;
+    if (cols > 24u) {
+#pragma unroll
+        for (uint32_t g = 0; g < 8; g++) tile_group<D>(t, r, 16 * x + 2 * g, 0x01010101u << g, miss, top);
+    } else {
+        const uint32_t groups = ((cols + 7u) >> 3) * 2u;
+        uint32_t bits = 0x01010101u;
+        for (uint32_t g = 0; g < groups; g += 2, bits <<= 2) {
+            tile_group<D>(t, r, 16 * x + 2 * g, bits, miss, top);
+            tile_group<D>(t, r, 16 * x + 2 * g + 2, bits << 1, miss, top);
+        }
+        miss |= tile_beyond(groups);
+    }
+    const uint32_t raw = t.raw[32 * x + lane_id()];
+    uint32_t mask = ~miss;
+    if (p.open) {
+        const uint32_t low = top ^ 0x7fff7fffu;  // a zero half: a sum of 32767 was the largest of its pair
+        if (__any_sync(FULL_MASK, ((low - 0x00010001u) & ~low & 0x80008000u) != 0u))
+            mask = tile_exact<D>(p.boxes, p.nboxes, r.raw, raw, rows, cols);
+    }
+    const uint32_t m0 = __ballot_sync(FULL_MASK, ((raw >> kIdBits) & 1u) == 0u);
+    const uint32_t m1 = __ballot_sync(FULL_MASK, ((raw >> (kIdBits + 1)) & 1u) == 0u);
+    const uint32_t m2 = __ballot_sync(FULL_MASK, ((raw >> (kIdBits + 2)) & 1u) == 0u);
+    return mask & ~((m0 & r.f0) | (m1 & r.f1) | (m2 & r.f2));
+}
+
+// the slots after this lane's, for a tile against itself
+__device__ __forceinline__ uint32_t after_lane() { return 0xfffffffeu << lane_id(); }
+
+// the pairs of one or two column tiles of a row tile; gid and the tiles'
+// first box in the cell are for record mode
+template <bool BIP, bool REC>
+__device__ __forceinline__ void tile_emit(const Params& p, const Tiles& t, WarpOut& o, uint32_t row, uint32_t ma,
+                                          uint32_t xa, uint32_t mb, uint32_t xb, uint32_t row0, uint32_t col0a,
+                                          uint32_t col0b, uint32_t gid) {
+    if constexpr (REC) {
+        remit(p, o, ma, [&](uint32_t b) { return col0a + tile_box(b); }, mb,
+              [&](uint32_t b) { return col0b + tile_box(b); }, row0 + tile_box(lane_id()), gid, FULL_MASK);
+    } else {
+        const uint32_t *ca = t.raw + 32 * xa, *cb = t.raw + 32 * xb;
+        wemit<BIP>(p, o, ma, [&](uint32_t b) { return ca[b]; }, mb, [&](uint32_t b) { return cb[b]; }, row);
+    }
+}
+
+// A staged cell's rows and columns as tiles: self queries have n boxes in
+// tiles 0, 1, ...; red/blue queries the red boxes in tiles 0, 1, ... and the
+// blue ones in the last tile, the one before, ...
+struct CellTiles {
+    uint32_t rows, cols;  // boxes
+    int row0, row_step, col0, col_step;
+    __device__ __forceinline__ uint32_t row_tiles() const { return (rows + 31u) >> 5; }
+    __device__ __forceinline__ uint32_t col_tiles() const { return (cols + 31u) >> 5; }
+    __device__ __forceinline__ uint32_t row_tile(uint32_t r) const { return (uint32_t)(row0 + row_step * (int)r); }
+    __device__ __forceinline__ uint32_t col_tile(uint32_t x) const { return (uint32_t)(col0 + col_step * (int)x); }
+};
+// red/blue: the colour whose tiles make fewer steps (whole row tiles, quarters of column tiles) is the columns
+__device__ __forceinline__ CellTiles cell_tiles_bip(uint32_t red, uint32_t blue, uint32_t tiles) {
+    const int last = (int)tiles - 1;
+    if (((red + 31u) >> 5) * ((blue + 7u) >> 3) <= ((blue + 31u) >> 5) * ((red + 7u) >> 3))
+        return CellTiles{red, blue, 0, 1, last, -1};
+    return CellTiles{blue, red, last, -1, 0, 1};
+}
+
+// a red/blue entry into its colour's tiles: box rank e of its colour
+template <int D>
+__device__ __forceinline__ void tile_put_colour(const Tiles& t, uint32_t tiles, bool is_red, uint32_t e, const uint4& w) {
+    tile_put<D>(t, is_red ? e >> 5 : tiles - 1 - (e >> 5), tile_slot(e & 31u), w);
+}
+
+// row tile r of a staged cell against its column tiles from x (self: from r),
+// `count` of them at most, two per emission step
+template <int D, bool BIP, bool REC>
+__device__ __forceinline__ void row_sweep(const Params& p, const Tiles& t, WarpOut& o, const CellTiles& c, uint32_t r,
+                                          uint32_t x, uint32_t count, uint32_t gid) {
+    const uint32_t rows = tile_fill(c.rows, r), end = min(c.col_tiles(), x + count);
+    const Row<D> row = tile_row<D>(t, c.row_tile(r));
+    for (; x < end; x += 2) {
+        const uint32_t xa = c.col_tile(x);
+        uint32_t ma = tile_hits<D>(p, t, row, rows, xa, tile_fill(c.cols, x));
+        if (!BIP && x == r) ma &= after_lane();
+        uint32_t mb = 0, xb = xa;
+        if (x + 1 < end) {
+            xb = c.col_tile(x + 1);
+            mb = tile_hits<D>(p, t, row, rows, xb, tile_fill(c.cols, x + 1));
+        }
+        tile_emit<BIP, REC>(p, t, o, row.raw, ma, xa, mb, xb, 32 * r, 32 * x, 32 * (x + 1), gid);
+    }
 }
 
 // ---- medium cells: one per warp item, staged whole ---------------------------
-// The reference-cell rule and the red/blue rule are applied per 32-column
-// tile with ballots (bit j: column j may pair with this lane's row box), so
-// the per-pair work is the overlap test alone: six differences whose OR has
-// bit 31 set iff some pair of intervals is disjoint, pushed into the hit
-// mask with one funnel shift (mask = mask << 1 | hit).
-
-// columns [c0, c0 + ncol) of the staged cell that row box `me` may pair with
-template <bool BIP, bool NARROW>
-__device__ __forceinline__ uint32_t tile_allow(const Params& p, const Slots& s, uint32_t c0, uint32_t ncol,
-                                               const Box& me) {
-    const uint32_t lane = lane_id();
-    const bool v = lane < ncol;
-    uint32_t bf, bid;
-    if constexpr (NARROW) {
-        const uint2 fi = med_fi(s)[c0 + (v ? lane : 0u)];
-        bf = fi.x;
-        bid = fi.y;
-    } else {
-        const uint4 b = s.b[c0 + (v ? lane : 0u)];
-        bf = b.z;
-        bid = b.w;
-    }
-    const uint32_t f = v ? bf >> kMissShift : 0u;
-    const uint32_t vm = __ballot_sync(FULL_MASK, v);
-    const uint32_t m0 = __ballot_sync(FULL_MASK, (f & 1u) != 0u);
-    const uint32_t m1 = __ballot_sync(FULL_MASK, (f & 2u) != 0u);
-    const uint32_t m2 = __ballot_sync(FULL_MASK, (f & 4u) != 0u);
-    const uint32_t fa = me.f >> kMissShift;
-    uint32_t allow = vm & ~(((fa & 1u) ? m0 : 0u) | ((fa & 2u) ? m1 : 0u) | ((fa & 4u) ? m2 : 0u));
-    if (BIP) {
-        const uint32_t red = __ballot_sync(FULL_MASK, v && bid < p.split);
-        allow &= (me.id < p.split) ? ~red : red;
-    }
-    return allow;
-}
-
-// bit 31 set iff row box a and column box (ca, cz) are disjoint on some axis
-template <int D, bool NARROW>
-__device__ __forceinline__ uint32_t miss_word(const Box& a, const uint4& ca, const uint2& cz) {
-    if (NARROW) {
-        uint32_t t = (ca.y - a.x0) | (a.x1 - ca.x) | (ca.w - a.y0) | (a.y1 - ca.z);
-        if (D == 3) t |= (cz.y - a.z0) | (a.z1 - cz.x);
-        return t;
-    }
-    bool ok = (a.x0 <= ca.y) & (ca.x <= a.x1) & (a.y0 <= ca.w) & (ca.z <= a.y1);
-    if (D == 3) ok &= (a.z0 <= cz.y) & (cz.x <= a.z1);
-    return ok ? 0u : 0x80000000u;
-}
-
-__device__ __forceinline__ uint32_t push_hit(uint32_t mask, uint32_t miss) { return __funnelshift_l(~miss, mask, 1); }
-
-template <int D, bool NARROW, class Row>
-__device__ __forceinline__ uint32_t test_slot(const Slots& s, const Row& me, uint32_t mask, uint32_t i) {
-    const uint4 ca = s.a[i];
-    const uint2 cz = D == 3 ? (NARROW ? med_z(s)[i] : *reinterpret_cast<const uint2*>(&s.b[i])) : make_uint2(0u, 0u);
-    if constexpr (NARROW) return __funnelshift_l(sep_hit<D>(me, ca, cz), mask, 1);
-    else return push_hit(mask, miss_word<D, false>(me, ca, cz));
-}
-
-// row box against columns [c0, c0 + cnt), cnt a multiple of 8 up to 32;
-// bit cnt-1-j of the result: column j
-template <int D, bool NARROW, class Row>
-__device__ __forceinline__ uint32_t sweep_tile(const Slots& s, const Row& me, uint32_t c0, uint32_t cnt) {
-    uint32_t mask = 0;
-    if (cnt == 32) {
-#pragma unroll
-        for (uint32_t j = 0; j < 32; j++) mask = test_slot<D, NARROW>(s, me, mask, c0 + j);
-    } else {
-        for (uint32_t j0 = 0; j0 < cnt; j0 += 8) {
-#pragma unroll
-            for (uint32_t jj = 0; jj < 8; jj++) mask = test_slot<D, NARROW>(s, me, mask, c0 + j0 + jj);
-        }
-    }
-    return mask;
-}
-
-// circular half sweep of the m rows staged at [rb, rb + m): lane l < m tests
-// partners l+1 .. l+floor(m/2) (mod m), lanes past m/2 one fewer when m is
-// even (the BALANCE=1 sweep of d_matching, pbig.cu:804-825), so each
-// unordered pair is tested once; bit dmax-d of the result: partner l+d
-template <int D, bool NARROW, class Row>
-__device__ __forceinline__ uint32_t sweep_diag2(const Slots& s, const Row& me, uint32_t l, uint32_t rb, uint32_t m) {
-    uint32_t mask = 0;
-    if (m == 32) {
-#pragma unroll
-        for (uint32_t d = 1; d <= 16; d++) mask = test_slot<D, NARROW>(s, me, mask, rb + ((l + d) & 31u));
-    } else {
-        const uint32_t dmax = m >> 1;
-#pragma unroll 4
-        for (uint32_t d = 1; d <= dmax; d++) {
-            uint32_t pr = l + d;
-            if (pr >= m) pr -= m;
-            mask = test_slot<D, NARROW>(s, me, mask, rb + pr);
-        }
-    }
-    return mask;
-}
-
-// the allow mask of the diagonal tile in sweep_diag2's bit order, with the
-// half-sweep limit applied
-__device__ __forceinline__ uint32_t diag_allow(uint32_t allow, uint32_t lane, uint32_t m) {
-    if (lane >= m) return 0u;
-    const uint32_t dmax = m >> 1;
-    if (dmax == 0) return 0u;
-    uint32_t rot;  // bit d: partner (lane + d) mod m
-    if (m == 32) rot = __funnelshift_r(allow, allow, lane);
-    else rot = ((allow >> lane) | (allow << (m - lane))) & ((1u << m) - 1u);
-    uint32_t a = (__brev(rot) >> (31u - dmax)) & ((1u << dmax) - 1u);
-    if ((m & 1u) == 0u && lane >= dmax) a &= ~1u;  // even m: the opposite partner once
-    return a;
-}
-
 // the medium-cell list, warp gw of nw (the one-launch kernel: items in a
 // fixed stride; the medium-cell kernel: every warp takes items from one
-// counter); wsm: the warp's kMedWarpBytes of shared memory (staging slots,
-// then the output buffer)
-constexpr uint32_t kMedWarpBytes = kMedSlots * 2 * sizeof(uint4) + kMedOut * sizeof(uint2);
+// counter); wsm: the warp's kMedWarpBytes of shared memory (tiles, then the
+// output buffer)
+constexpr uint32_t kMedWarpBytes = kMedTiles * kTileBytes + kMedOut * sizeof(uint2);
 
-template <int D, bool BIP, bool NARROW, bool REC, bool FRESH = false>
+template <int D, bool BIP, bool REC, bool FRESH = false>
 __device__ __forceinline__ void med_pass(const Params& p, unsigned char* wsm, uint64_t gw, uint64_t nw) {
     const uint32_t lane = lane_id();
-    uint4* base = reinterpret_cast<uint4*>(wsm);
-    const Slots s{base, base + kMedSlots};
-    WarpOut o{reinterpret_cast<uint2*>(base + 2 * kMedSlots), 0, kMedOut};
+    const Tiles t(wsm, kMedTiles);
+    WarpOut o{reinterpret_cast<uint2*>(wsm + kMedTiles * kTileBytes), 0, kMedOut};
     const uint64_t nl = mn64(ctr_read<FRESH>(&p.ctr->n_list[kListMed]), p.list_cap[kListMed]);
     auto cell = [&](uint64_t item) {
         const uint2 sn = p.lists[p.list_off[kListMed] + item];
@@ -1576,74 +1514,47 @@ __device__ __forceinline__ void med_pass(const Params& p, unsigned char* wsm, ui
         const uint32_t start = REC ? (gid < p.ncells ? p.counts[gid] : 0xffffffffu) : sn.x;
         const uint32_t n = sn.y;
         if (n > kMedMax || (uint64_t)start + n > p.entry_cap) return;  // inconsistent grid: skip
-        const uint32_t R = (n + 31) >> 5;
-        // stage: all entry ids first, then all boxes (loads in flight together)
-        uint32_t raw[kMedSlots / 32];
+        CellTiles c{n, n, 0, 1, 0, 1};
+        if (!BIP) {  // a lane takes one column pair of each two tiles (all loads in flight together)
+            constexpr uint32_t kPer = kMedMax / 64;
+            uint4 a[kPer], b[kPer];
 #pragma unroll
-        for (uint32_t k = 0; k < kMedSlots / 32; k++) {
-            const uint32_t e = lane + 32 * k;
-            raw[k] = e < n ? p.entries[start + e] : 0u;
-        }
+            for (uint32_t k = 0; k < kPer; k++) {
+                a[k] = entry_at(p, start, 64 * k + 2 * lane, n);
+                b[k] = entry_at(p, start, 64 * k + 2 * lane + 1, n);
+            }
 #pragma unroll
-        for (uint32_t k = 0; k < kMedSlots / 32; k++) {
-            const uint32_t e = lane + 32 * k;
-            if (e < 32 * R) med_slot_put<NARROW>(s, e, e < n ? load_box<D, NARROW>(p, raw[k]) : dummy_box<NARROW>());
+            for (uint32_t k = 0; k < kPer; k++)
+                if (64 * k < n) tile_put_pair<D>(t, 2 * k + (lane >> 4), lane & 15u, a[k], b[k]);
+        } else {
+            constexpr uint32_t kPer = kMedMax / 32;
+            uint4 w[kPer];
+            uint32_t reds[kPer], red = 0;
+#pragma unroll
+            for (uint32_t k = 0; k < kPer; k++) w[k] = entry_at(p, start, 32 * k + lane, n);
+#pragma unroll
+            for (uint32_t k = 0; k < kPer; k++) {
+                reds[k] = __ballot_sync(FULL_MASK, 32 * k + lane < n && (w[k].w & kIdMask) < p.split);
+                red += __popc(reds[k]);
+            }
+            if (red == 0u || red == n) return;  // one colour: no pair
+            uint32_t r0 = 0, b0 = 0;  // boxes of each colour before chunk k
+#pragma unroll
+            for (uint32_t k = 0; k < kPer; k++) {
+                const uint32_t left = n > 32 * k ? min(32u, n - 32 * k) : 0u;
+                const uint32_t rr = __popc(reds[k] & ((1u << lane) - 1u));
+                const bool is_red = (reds[k] >> lane) & 1u;
+                if (lane < left) tile_put_colour<D>(t, kMedTiles, is_red, is_red ? r0 + rr : b0 + (lane - rr), w[k]);
+                r0 += __popc(reds[k]);
+                b0 += left - __popc(reds[k]);
+            }
+            tile_clear_rest<D>(t, (red - 1) >> 5, red);
+            tile_clear_rest<D>(t, kMedTiles - 1 - ((n - red - 1) >> 5), n - red);
+            c = cell_tiles_bip(red, n - red, kMedTiles);
         }
         __syncwarp();
-        for (uint32_t r = 0; r < R; r++) {
-            const uint32_t rows = min(32u, n - 32 * r), rb = 32 * r;
-            const Box me = med_slot_get<NARROW>(s, rb + lane);  // lanes >= rows hold a padding box, masked below
-            const auto row = med_row<NARROW>(me);
-            const uint32_t l = lane < rows ? lane : 0u;
-            const uint32_t dm = sweep_diag2<D, NARROW>(s, row, l, rb, rows) &
-                                diag_allow(tile_allow<BIP, NARROW>(p, s, rb, rows, me), lane, rows);
-            const uint32_t dmax = rows >> 1;
-            auto pdiag = [&](uint32_t k) {
-                uint32_t pr = l + dmax - k;
-                if (pr >= rows) pr -= rows;
-                return med_slot_id<NARROW>(s, rb + pr);
-            };
-            uint32_t pend = dm;  // the diagonal's hits wait for the first column tile
-            bool have = true;
-            for (uint32_t x = r + 1; x < R; x++) {
-                const uint32_t c0 = 32 * x, ncol = min(32u, n - c0);
-                uint32_t allow = tile_allow<BIP, NARROW>(p, s, c0, ncol, me);
-                if (lane >= rows) allow = 0u;
-                uint32_t mc = 0;
-                const uint32_t cnt = (ncol + 7) & ~7u;
-                if (__any_sync(FULL_MASK, allow != 0u))
-                    mc = sweep_tile<D, NARROW>(s, row, c0, cnt) & (__brev(allow) >> (32u - cnt));
-                auto pcol = [&](uint32_t k) { return med_slot_id<NARROW>(s, c0 + cnt - 1 - k); };
-                if constexpr (REC) {
-                    auto lcol = [&](uint32_t k) { return c0 + cnt - 1 - k; };
-                    auto ldiag = [&](uint32_t k) {
-                        uint32_t pr = l + dmax - k;
-                        if (pr >= rows) pr -= rows;
-                        return rb + pr;
-                    };
-                    if (have) remit(p, o, pend, ldiag, mc, lcol, rb + lane, gid, FULL_MASK);
-                    else remit(p, o, mc, lcol, 0u, lcol, rb + lane, gid, FULL_MASK);
-                    have = false;
-                } else if (have) {
-                    wemit<BIP>(p, o, pend, pdiag, mc, pcol, me.id);
-                    have = false;
-                } else {
-                    wemit<BIP>(p, o, mc, pcol, 0u, pcol, me.id);
-                }
-            }
-            if (have) {
-                if constexpr (REC) {
-                    auto ldiag = [&](uint32_t k) {
-                        uint32_t pr = l + dmax - k;
-                        if (pr >= rows) pr -= rows;
-                        return rb + pr;
-                    };
-                    remit(p, o, pend, ldiag, 0u, ldiag, rb + lane, gid, FULL_MASK);
-                } else {
-                    wemit<BIP>(p, o, pend, pdiag, 0u, pdiag, me.id);
-                }
-            }
-        }
+        const uint32_t R = c.row_tiles();
+        for (uint32_t r = 0; r < R; r++) row_sweep<D, BIP, REC>(p, t, o, c, r, BIP ? 0u : r, ~0u >> 1, gid);
         __syncwarp();
     };
     // items taken one at a time from a counter, so warps whose cells were
@@ -1663,217 +1574,122 @@ __device__ __forceinline__ void med_pass(const Params& p, unsigned char* wsm, ui
             cell(item);
         }
     }
-    wflush(p, o);
+    wflush<BIP, REC>(p, o);
     if (REC) rec_hits(p, o);
 }
 
-template <int D, bool BIP, bool NARROW, bool REC = false>
-__global__ void __launch_bounds__(kPairThreads, 3) k_pairs_med(Params p) {
+template <int D, bool BIP, bool REC = false>
+__global__ void __launch_bounds__(kPairThreads, 4) k_pairs_med(Params p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t warp = threadIdx.x >> 5;
-    med_pass<D, BIP, NARROW, REC>(p, smem_raw + warp * kMedWarpBytes, (uint64_t)blockIdx.x * kPairWarps + warp,
-                                  (uint64_t)gridDim.x * kPairWarps);
+    med_pass<D, BIP, REC>(p, smem_raw + warp * kMedWarpBytes, (uint64_t)blockIdx.x * kPairWarps + warp,
+                          (uint64_t)gridDim.x * kPairWarps);
 }
 
-// ---- big cells (block staged) and huge cells (tiles) -----------------------
-// a barrier of the whole block, or (SUB) of its first kPairThreads threads
+// ---- big cells (staged by a team of warps) and huge cells (tile tasks) -------
+// A team of four warps stages a big cell and shares its tiles. Small teams, so
+// that those waiting for a cell's entries or for their last warp are few among
+// the eight on an SM: with teams of eight warps, three an SM, half the issue
+// slots were empty (1.10 ms for the cells of 129..512 boxes of the crowded
+// 4M-box scene, against 0.78 ms).
+constexpr int kTeamWarps = 4;
+constexpr int kTeamThreads = 32 * kTeamWarps;
+
+struct TeamSmem {
+    uint4 tiles[kBigTiles * kTileBytes / sizeof(uint4)];  // a big cell's; huge cells: kHugeTiles per warp
+    uint2 out[kTeamWarps][kMedOut];
+    uint2 cell;          // the team's cell {start, n}; n = 0: none is left
+    uint32_t red, blue;  // red/blue: boxes of each colour placed so far
+    uint32_t next_unit;
+    uint32_t pad[3];
+};
+static_assert(kTeamWarps * kHugeTiles <= kBigTiles, "huge cells' tiles in a big cell's");
+
+// a barrier of the team: the block, or (SUB) a quarter of the one-launch kernel's
 template <bool SUB>
-__device__ __forceinline__ void block_sync() {
-    if constexpr (SUB) asm volatile("bar.sync 1, %0;" ::"n"(kPairThreads) : "memory");
+__device__ __forceinline__ void team_sync() {
+    if constexpr (SUB) asm volatile("bar.sync %0, %1;" ::"r"(1u + threadIdx.x / kTeamThreads), "n"(kTeamThreads) : "memory");
     else __syncthreads();
 }
 
-struct BlockSmem {
-    uint4 a[kBlockSlots];
-    uint4 b[kBlockSlots];
-    uint2 out[kBlockOut];
-    uint32_t out_n, first_ovf;
-    unsigned long long gbase;
-    uint32_t cell_start[kBigCellsPerTask], cell_n[kBigCellsPerTask], cell_off[kBigCellsPerTask + 1];
-    uint32_t unit_pref[kBigCellsPerTask + 1];
-    uint32_t k, tot, units;
-    unsigned long long nbt[2];
-    uint32_t cell_gid[kBigCellsPerTask];  // record mode: cell ids
-    unsigned long long hits;              // record mode: pairs written by the block
-};
-
-// block-buffer compaction (shared reservation per warp call); when the
-// buffer is full the warp reserves global space itself
-template <bool BIP, class PA, class PB>
-__device__ __forceinline__ void bemit(const Params& p, BlockSmem& s, uint32_t ma, PA pa, uint32_t mb, PB pb,
-                                      uint32_t myid) {
-    const uint32_t lane = lane_id();
-    const uint32_t k = __popc(ma) + __popc(mb);
-    const uint32_t incl = warp_incl_scan(k);
-    const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
-    if (total == 0) return;
-    uint32_t pos = 0;
-    unsigned long long gbase = 0;
-    if (lane == 0) {
-        pos = atomicAdd(&s.out_n, total);
-        if (pos + total > kBlockOut) {
-            atomicMin(&s.first_ovf, pos);
-            gbase = atomicAdd(&p.ctr->pairs, (unsigned long long)total);
+// one big cell: staged by the team's threads, then its warps take units of a
+// row tile and up to two column tiles from a counter. s.next_unit and the
+// colour counts are zero at the start.
+template <int D, bool BIP, bool REC, bool SUB>
+__device__ __forceinline__ void big_cell(const Params& p, TeamSmem& s, WarpOut& o, uint2 sn) {
+    const uint32_t lane = lane_id(), tid = threadIdx.x % kTeamThreads, warp = tid >> 5;
+    const Tiles t(reinterpret_cast<unsigned char*>(s.tiles), kBigTiles);
+    const uint32_t gid = sn.x, n = sn.y;  // record mode: the list holds the cell id, its start is in the counters
+    const uint32_t start = REC ? (gid < p.ncells ? p.counts[gid] : 0xffffffffu) : sn.x;
+    if (n > kBigMax || (uint64_t)start + n > p.entry_cap) return;  // inconsistent grid: skip (the whole team)
+    CellTiles c{n, n, 0, 1, 0, 1};
+    if (!BIP) {
+        constexpr uint32_t kPer = kBigMax / 2 / kTeamThreads;
+        uint4 a[kPer], b[kPer];
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; k++) {
+            const uint32_t q = tid + kTeamThreads * k;  // column pair
+            a[k] = entry_at(p, start, 2 * q, n);
+            b[k] = entry_at(p, start, 2 * q + 1, n);
         }
-    }
-    pos = __shfl_sync(FULL_MASK, pos, 0);
-    gbase = __shfl_sync(FULL_MASK, gbase, 0);
-    const bool direct = pos + total > kBlockOut;
-    uint32_t w = incl - k;
-    auto put = [&](uint32_t q) {
-        uint2 pr = make_uint2(min(myid, q), max(myid, q));
-        if (BIP) pr.y -= p.split;
-        if (!direct) {
-            s.out[pos + w] = pr;
-        } else {
-            const unsigned long long g = gbase + w;
-            if (g < p.out_cap) p.out[g] = pr;
-            else atomicOr(&p.ctr->err, kErrOutOvf);
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; k++) {
+            const uint32_t q = tid + kTeamThreads * k;
+            if (32 * (q >> 4) < n) tile_put_pair<D>(t, q >> 4, q & 15u, a[k], b[k]);
         }
-        w++;
-    };
-    while (ma) {
-        const uint32_t bit = __ffs(ma) - 1;
-        ma &= ma - 1;
-        put(pa(bit));
-    }
-    while (mb) {
-        const uint32_t bit = __ffs(mb) - 1;
-        mb &= mb - 1;
-        put(pb(bit));
-    }
-}
-
-// block-buffer record step (the words of a warp step go to the block buffer
-// or, when it is full, straight to global memory)
-template <class LA, class LB>
-__device__ __forceinline__ void bremit(const Params& p, BlockSmem& s, uint32_t ma, LA la, uint32_t mb, LB lb,
-                                       uint32_t row, uint32_t gid) {
-    const uint32_t lane = lane_id();
-    const uint32_t wa = rec_words(__popc(ma)), wb = rec_words(__popc(mb));
-    const uint32_t any = __ballot_sync(FULL_MASK, (wa | wb) != 0u);
-    const bool hdr = any != 0u && lane == (uint32_t)(__ffs(any) - 1);
-    const uint32_t k = wa + wb + (hdr ? 2u : 0u);
-    const uint32_t incl = warp_incl_scan(k);
-    const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
-    if (total == 0) return;
-    const unsigned long long hits = warp_sum_u64(__popc(ma) + __popc(mb));
-    uint32_t pos = 0;
-    unsigned long long gbase = 0;
-    if (lane == 0) {
-        atomicAdd(&s.hits, hits);
-        pos = atomicAdd(&s.out_n, total);
-        if (pos + total > kBlockOut) {
-            atomicMin(&s.first_ovf, pos);
-            gbase = atomicAdd(&p.ctr->pairs, (unsigned long long)total);
-        }
-    }
-    pos = __shfl_sync(FULL_MASK, pos, 0);
-    gbase = __shfl_sync(FULL_MASK, gbase, 0);
-    const bool direct = pos + total > kBlockOut;
-    const bool keep = !direct || gbase + total <= p.out_cap;
-    if (direct && !keep && lane == 0) atomicOr(&p.ctr->err, kErrOutOvf);
-    unsigned long long* dst = direct ? reinterpret_cast<unsigned long long*>(p.out) + gbase
-                                     : reinterpret_cast<unsigned long long*>(s.out + pos);
-    uint32_t w = incl - k;
-    if (hdr && keep) {
-        dst[w] = kRiceUnused;
-        dst[w + 1] = gid;
-    }
-    if (hdr) w += 2;
-    if (wa) rec_write(dst + w, keep, row, ma, la);
-    if (wb) rec_write(dst + w + wa, keep, row, mb, lb);
-}
-
-template <int D, bool BIP, bool NARROW, bool REC, bool FRESH = false, bool SUB = false>
-__device__ void big_task(const Params& p, BlockSmem& s, uint64_t task) {
-    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
-    const Slots sl{s.a, s.b};
-    auto emit = [&](uint32_t ma, auto pa, uint32_t mb, auto pb, uint32_t myid) { bemit<BIP>(p, s, ma, pa, mb, pb, myid); };
-    const uint64_t nl = mn64(ctr_read<FRESH>(&p.ctr->n_list[kListBig]), p.list_cap[kListBig]);
-    uint64_t cur = task * kBigCellsPerTask;
-    const uint64_t end = mn64(cur + kBigCellsPerTask, nl);
-    while (cur < end) {
-        if (warp == 0) {
-            uint32_t n = 0, st = 0;
-            const bool v = lane < kBigCellsPerTask && cur + lane < end;
-            uint32_t gid = 0;
-            if (v) {
-                const uint2 sn = p.lists[p.list_off[kListBig] + cur + lane];
-                st = sn.x;
-                n = sn.y;
-                if (REC) {  // the list holds the cell id; its start is in the counters
-                    gid = sn.x;
-                    st = gid < p.ncells ? p.counts[gid] : 0xffffffffu;
-                }
-                if (n > kBigMax || (uint64_t)st + n > p.entry_cap) n = 0;  // inconsistent grid: skip
-            }
-            const uint32_t n8 = (n + 7) & ~7u;
-            const uint32_t inc = warp_incl_scan(n8);
-            const uint32_t fits = __ballot_sync(FULL_MASK, v && inc <= kBlockSlots);
-            const uint32_t k = __popc(fits);  // fits is a run of low bits
-            const uint32_t units = lane < k ? (n + 31) >> 5 : 0u;
-            const uint32_t uinc = warp_incl_scan(units);
-            if (lane < k) {
-                s.cell_start[lane] = st;
-                s.cell_gid[lane] = gid;
-                s.cell_n[lane] = n;
-                s.cell_off[lane] = inc - n8;
-                s.unit_pref[lane + 1] = uinc;
-            }
+        team_sync<SUB>();
+    } else {
+        constexpr uint32_t kPer = kBigMax / kTeamThreads;
+        uint4 w[kPer];
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; k++) w[k] = entry_at(p, start, tid + kTeamThreads * k, n);
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; k++) {
+            const uint32_t first = 32 * (warp + kTeamWarps * k);  // this warp's 32 entries
+            if (first >= n) continue;
+            const uint32_t left = min(32u, n - first);
+            const bool is_red = lane < left && (w[k].w & kIdMask) < p.split;
+            const uint32_t reds = __ballot_sync(FULL_MASK, is_red), nr = __popc(reds);
+            uint32_t r0 = 0, b0 = 0;
             if (lane == 0) {
-                s.unit_pref[0] = 0;
-                if (k == 0) s.k = s.tot = s.units = 0;
+                r0 = atomicAdd(&s.red, nr);
+                b0 = atomicAdd(&s.blue, left - nr);
             }
-            if (k > 0 && lane == k - 1) {
-                s.cell_off[k] = inc;
-                s.k = k;
-                s.tot = inc;
-                s.units = uinc;
-            }
+            r0 = __shfl_sync(FULL_MASK, r0, 0);
+            b0 = __shfl_sync(FULL_MASK, b0, 0);
+            const uint32_t rr = __popc(reds & ((1u << lane) - 1u));
+            if (lane < left) tile_put_colour<D>(t, kBigTiles, is_red, is_red ? r0 + rr : b0 + (lane - rr), w[k]);
         }
-        block_sync<SUB>();
-        const uint32_t K = s.k, tot = s.tot, U = s.units;
-        if (K == 0) break;  // uniform: every thread read the same K
-        for (uint32_t e = t; e < tot; e += kPairThreads) {
-            uint32_t c = 0;  // last cell whose slots start at or before e
-#pragma unroll
-            for (uint32_t step = 4; step; step >>= 1)
-                if (c + step < K && s.cell_off[c + step] <= e) c += step;
-            const uint32_t local = e - s.cell_off[c];
-            slot_put(sl, e, local < s.cell_n[c] ? load_box<D, NARROW>(p, p.entries[s.cell_start[c] + local])
-                                                : dummy_box<NARROW>());
+        team_sync<SUB>();
+        const uint32_t red = s.red;
+        if (red == 0u || red == n) return;  // one colour: no pair
+        if (warp == 0) tile_clear_rest<D>(t, (red - 1) >> 5, red);
+        if (warp == 1) tile_clear_rest<D>(t, kBigTiles - 1 - ((n - red - 1) >> 5), n - red);
+        c = cell_tiles_bip(red, n - red, kBigTiles);
+        team_sync<SUB>();
+    }
+    // units in the order of their row tiles: row r's first unit is `before`
+    const uint32_t R = c.row_tiles(), X = c.col_tiles();
+    uint32_t r = 0, before = 0;
+    for (;;) {
+        uint32_t u = 0;
+        if (lane == 0) u = atomicAdd(&s.next_unit, 1u);
+        u = __shfl_sync(FULL_MASK, u, 0);
+        uint32_t units;
+        while (r < R && u >= before + (units = (X - (BIP ? 0u : r) + 1u) >> 1)) {
+            before += units;
+            r++;
         }
-        block_sync<SUB>();
-        for (uint32_t u = warp; u < U; u += kPairWarps) {
-            uint32_t c = 0;
-#pragma unroll
-            for (uint32_t step = 4; step; step >>= 1)
-                if (c + step < K && s.unit_pref[c + step] <= u) c += step;
-            if constexpr (REC) {
-                const uint32_t gid = s.cell_gid[c];
-                auto remit_b = [&](uint32_t ma, auto la, uint32_t mb, auto lb, uint32_t row) {
-                    bremit(p, s, ma, la, mb, lb, row, gid);
-                };
-                row_unit<D, BIP, NARROW, true>(p, sl, s.cell_off[c], s.cell_n[c], u - s.unit_pref[c], remit_b);
-            } else {
-                row_unit<D, BIP, NARROW, false>(p, sl, s.cell_off[c], s.cell_n[c], u - s.unit_pref[c], emit);
-            }
-        }
-        block_sync<SUB>();
-        cur += K;
+        if (r >= R) break;
+        row_sweep<D, BIP, REC>(p, t, o, c, r, (BIP ? 0u : r) + 2 * (u - before), 2, gid);
     }
 }
 
-// huge cells: one tile task {start, n, r, x0} per warp; boxes gathered per
-// tile into the warp's 64 slots (32 rows, 32 columns)
-template <int D, bool BIP, bool NARROW, bool REC, bool FRESH = false>
-__device__ __forceinline__ void huge_item(const Params& p, BlockSmem& s, uint64_t item, uint32_t slot0) {
+// huge cells: one tile task {start, n, r, x0} per warp; the row tile and two
+// column tiles at a time staged in the warp's own tiles
+template <int D, bool BIP, bool REC>
+__device__ __forceinline__ void huge_item(const Params& p, const Tiles& t, WarpOut& o, const uint4& tk) {
     const uint32_t lane = lane_id();
-    const Slots sl{s.a, s.b};
-    const uint64_t nt = mn64(ctr_read<FRESH>(&p.ctr->need_tasks), p.task_cap);
-    if (item >= nt) return;
-    const uint4 tk = p.tasks[item];
     const uint32_t gid = tk.x;  // record mode: the cell id; its start is in the counters
     const uint32_t start = REC ? (gid < p.ncells ? p.counts[gid] : 0xffffffffu) : tk.x;
     const uint32_t n = tk.y, r = tk.z, x0 = tk.w;
@@ -1884,97 +1700,83 @@ __device__ __forceinline__ void huge_item(const Params& p, BlockSmem& s, uint64_
     const uint32_t R = (n + 31) >> 5;
     const uint32_t x1 = min(x0 + kTaskCols, R);
     if ((uint64_t)start + n > p.entry_cap || r >= R || x0 >= R) return;
-    const uint32_t rows = min(32u, n - 32 * r);
-    const Box me = lane < rows ? load_box<D, NARROW>(p, p.entries[start + 32 * r + lane]) : dummy_box<NARROW>();
-    slot_put(sl, slot0 + lane, me);
+    const uint32_t rows = tile_fill(n, r), j = lane & 15u;
+    if (lane < 16u)
+        tile_put_pair<D>(t, 0, j, entry_at(p, start, 32 * r + 2 * j, n), entry_at(p, start, 32 * r + 2 * j + 1, n));
     __syncwarp();
-    for (uint32_t x = x0; x < x1; x++) {
-        if (x == r) {
-            const uint32_t md = sweep_diag<D, BIP, NARROW>(sl, me, lane, slot0, rows, p.split);
-            if constexpr (REC) {
-                auto ld = [&](uint32_t d) {
-                    uint32_t pr = lane + d;
-                    if (pr >= rows) pr -= rows;
-                    return 32 * r + pr;
-                };
-                bremit(p, s, md, ld, 0u, ld, 32 * r + lane, gid);
-            } else {
-                auto pd = [&](uint32_t d) {
-                    uint32_t pr = lane + d;
-                    if (pr >= rows) pr -= rows;
-                    return slot_id(sl, slot0 + pr);
-                };
-                bemit<BIP>(p, s, md, pd, 0u, pd, me.id);
-            }
-        } else {
-            const uint32_t cols = min(32u, n - 32 * x);
-            slot_put(sl, slot0 + 32 + lane,
-                     lane < cols ? load_box<D, NARROW>(p, p.entries[start + 32 * x + lane]) : dummy_box<NARROW>());
-            __syncwarp();
-            const uint32_t mc = sweep_cols<D, BIP, NARROW>(sl, me, slot0 + 32, (cols + 7) & ~7u, p.split);
-            if constexpr (REC) {
-                auto lc = [&](uint32_t j) { return 32 * x + j; };
-                bremit(p, s, mc, lc, 0u, lc, 32 * r + lane, gid);
-            } else {
-                auto pc = [&](uint32_t j) { return slot_id(sl, slot0 + 32 + j); };
-                bemit<BIP>(p, s, mc, pc, 0u, pc, me.id);
-            }
-        }
+    const Row<D> row = tile_row<D>(t, 0);
+    for (uint32_t x = x0; x < x1; x += 2) {
+        const uint32_t e = 32 * x + 2 * lane, end = min(n, 32 * x1);
+        __syncwarp();  // (the last columns are read)
+        tile_put_pair<D>(t, 1 + (lane >> 4), j, entry_at(p, start, e, end), entry_at(p, start, e + 1, end));
         __syncwarp();
+        uint32_t m[2] = {0u, 0u};
+#pragma unroll
+        for (uint32_t k = 0; k < 2; k++) {
+            if (x + k >= x1) continue;
+            m[k] = tile_hits<D>(p, t, row, rows, 1 + k, tile_fill(n, x + k));
+            if (x + k == r) m[k] &= after_lane();
+            if (BIP) {
+                const uint32_t red = __ballot_sync(FULL_MASK, (t.raw[32 * (1 + k) + lane] & kIdMask) < p.split);
+                m[k] &= (row.raw & kIdMask) < p.split ? ~red : red;
+            }
+        }
+        tile_emit<BIP, REC>(p, t, o, row.raw, m[0], 1, m[1], 2, 32 * r, 32 * x, 32 * (x + 1), gid);
     }
+    __syncwarp();
 }
 
-// big-cell tasks and huge-cell tile tasks, block blk of nblk (SUB: run by
-// the block's first kPairThreads threads alone)
-template <int D, bool BIP, bool NARROW, bool REC, bool FRESH = false, bool SUB = false>
-__device__ __forceinline__ void block_pass(const Params& p, BlockSmem& s, uint64_t blk, uint64_t nblk) {
-    const uint32_t t = threadIdx.x, warp = t >> 5;
-    if (t == 0) {
-        s.out_n = 0;
-        s.first_ovf = kBlockOut;
-        s.hits = 0;
-        const uint64_t nb = mn64(ctr_read<FRESH>(&p.ctr->n_list[kListBig]), p.list_cap[kListBig]);
-        const uint64_t nt = mn64(ctr_read<FRESH>(&p.ctr->need_tasks), p.task_cap);
-        s.nbt[0] = (nb + kBigCellsPerTask - 1) / kBigCellsPerTask;
-        s.nbt[1] = (nt + kPairWarps - 1) / kPairWarps;
-    }
-    block_sync<SUB>();
-    const uint64_t total = s.nbt[0] + s.nbt[1];
-    for (uint64_t bt = blk; bt < total; bt += nblk) {
-        if (bt < s.nbt[0]) big_task<D, BIP, NARROW, REC, FRESH, SUB>(p, s, bt);
-        else huge_item<D, BIP, NARROW, REC, FRESH>(p, s, (bt - s.nbt[0]) * kPairWarps + warp, warp * 64);
-        block_sync<SUB>();
-        const uint32_t on = s.out_n, ovf = s.first_ovf;
-        const uint32_t nv = min(on, ovf);
-        const bool last = bt + nblk >= total;
-        if (nv >= kBlockOut / 2 || on > nv || (last && on > 0)) {
-            if (t == 0) s.gbase = nv ? atomicAdd(&p.ctr->pairs, (unsigned long long)nv) : 0ull;
-            block_sync<SUB>();
-            store_run(p, s.gbase, s.out, nv, t, kPairThreads);
-            block_sync<SUB>();
-            if (t == 0) {
-                s.out_n = 0;
-                s.first_ovf = kBlockOut;
+// big cells, then the tile tasks of huge cells: team `team` of nteam. Big
+// cells are taken from a counter (the one-launch kernel: in a fixed stride),
+// the next one while the team is at work on its own.
+template <int D, bool BIP, bool REC, bool FRESH = false, bool SUB = false>
+__device__ __forceinline__ void team_pass(const Params& p, TeamSmem& s, uint64_t team, uint64_t nteam) {
+    const uint32_t tid = threadIdx.x % kTeamThreads, warp = tid >> 5;
+    WarpOut o{s.out[warp], 0, kMedOut};
+    const uint64_t nb = mn64(ctr_read<FRESH>(&p.ctr->n_list[kListBig]), p.list_cap[kListBig]);
+    const uint64_t nt = mn64(ctr_read<FRESH>(&p.ctr->need_tasks), p.task_cap);
+    uint64_t item = team;
+    auto fetch = [&]() {
+        if (!FRESH) item = atomicAdd(&p.ctr->big_next, 1u);
+        const uint2 sn = item < nb ? p.lists[p.list_off[kListBig] + item] : make_uint2(0u, 0u);
+        item += nteam;
+        return sn;
+    };
+    uint2 next = make_uint2(0u, 0u);
+    if (nb > 0) {  // (uniform)
+        if (tid == 0) next = fetch();
+        for (;;) {
+            if (tid == 0) {
+                s.cell = next;
+                s.red = s.blue = s.next_unit = 0u;
             }
-            block_sync<SUB>();
+            team_sync<SUB>();
+            const uint2 sn = s.cell;
+            if (sn.y == 0u) break;
+            if (tid == 0) next = fetch();
+            big_cell<D, BIP, REC, SUB>(p, s, o, sn);
+            team_sync<SUB>();
         }
     }
-    if (REC && t == 0 && s.hits) atomicAdd(&p.ctr->rec_pairs, s.hits);
+    const Tiles t(reinterpret_cast<unsigned char*>(s.tiles) + warp * kHugeTiles * kTileBytes, kHugeTiles);
+    for (uint64_t i = team * kTeamWarps + warp; i < nt; i += nteam * kTeamWarps) huge_item<D, BIP, REC>(p, t, o, p.tasks[i]);
+    wflush<BIP, REC>(p, o);
+    if (REC) rec_hits(p, o);
 }
 
-template <int D, bool BIP, bool NARROW, bool REC = false>
-__global__ void __launch_bounds__(kPairThreads, 2) k_pairs_block(Params p) {
+template <int D, bool BIP, bool REC = false>
+__global__ void __launch_bounds__(kTeamThreads, 8) k_pairs_block(Params p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    block_pass<D, BIP, NARROW, REC>(p, *reinterpret_cast<BlockSmem*>(smem_raw), blockIdx.x, gridDim.x);
+    team_pass<D, BIP, REC>(p, *reinterpret_cast<TeamSmem*>(smem_raw), blockIdx.x, gridDim.x);
 }
 
-// record mode, after the pair kernels: entries become the plain box indices
-// the record decoder reads (the reference's Recs array)
+// record mode, after the pair kernels: the entries' box indices, which the
+// record decoder reads (the reference's Recs array)
 __global__ void k_strip_entries(Params pin) {
     const Params p = resolve(pin);
     const uint64_t n = mn64(p.ctr->entries, p.entry_cap);
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        p.entries[i] &= kIdMask;
+        p.recs[i] = p.entries[i].w & kIdMask;
 }
 
 // ---------------------------------------------------------------------------
@@ -2095,10 +1897,8 @@ constexpr uint32_t kFusedWarps = kFusedThreads / 32;
 constexpr uint32_t kFusedChunks = (uint32_t)(kFusedMaxCells / kScanChunk);
 constexpr uint32_t kFusedLocalCells = 8192;  // grids of up to 8192 cells: 128-cell chunks, totals per block
 constexpr uint32_t kGridWaitLimit = 1u << 20;  // polls of 64 ns or more: the wait ends after a second at most
-constexpr uint32_t kSmallWarpBytes = 2 * kSmallSlots * sizeof(uint4) + kWarpOut * sizeof(uint2);
+constexpr uint32_t kSmallWarpBytes = kSmallSlots * sizeof(uint4) + kWarpOut * sizeof(uint2);
 static_assert(kFusedChunks % kFusedThreads == 0, "chunk prefixes per thread");
-static_assert(2 * kMedSlots * sizeof(uint2) <= kMedSlots * sizeof(uint4), "medium-cell z terms and {f, id} in the b array");
-static_assert(kSmallSlots * sizeof(uint2) + kSmallSlots * sizeof(uint32_t) <= kSmallSlots * sizeof(uint4), "small-cell z terms and indices in the b array");
 
 // barrier number k of this launch (k counts the barriers passed so far)
 __device__ __forceinline__ bool grid_barrier(const FusedArgs& a, uint32_t k) {
@@ -2198,7 +1998,7 @@ __device__ __forceinline__ uint32_t tune_scene_fast(const uint32_t* boxes, uint6
     return best;
 }
 
-template <int D, bool NARROW>
+template <int D>
 __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArgs a) {
     Params p = pin;  // the grid's size is set below
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -2239,6 +2039,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArg
         a.scenes[0] = Scene{0u, (uint32_t)p.nboxes, shift, nrc, 0ull, range, 0u};
     }
     __syncthreads();
+    p.open = shift >= kOpenShift ? 1u : 0u;
     p.scenes = &s_scene;  // the count and the scatter read the scene from shared memory
     if (a.zero_cells) {
         uint4* c4 = reinterpret_cast<uint4*>(p.counts);
@@ -2358,15 +2159,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArg
         for (uint64_t i = 4 * (p.ncells / 4) + gt; i < p.ncells; i += nt) p.counts[i] = 0u;
     }
     if (fits) {
-        unsigned char* ws = smem_raw + warp * kSmallWarpBytes;
-        uint4* sa = reinterpret_cast<uint4*>(ws);
-        small_pass<D, false, NARROW, false, true>(p, sa, sa + kSmallSlots, reinterpret_cast<uint2*>(sa + 2 * kSmallSlots),
-                                            gw, nw);
+        uint4* ws = reinterpret_cast<uint4*>(smem_raw + warp * kSmallWarpBytes);
+        small_pass<D, false, false, true>(p, ws, reinterpret_cast<uint2*>(ws + kSmallSlots), gw, nw);
         __syncthreads();
-        med_pass<D, false, NARROW, false, true>(p, smem_raw + warp * kMedWarpBytes, gw, nw);
+        med_pass<D, false, false, true>(p, smem_raw + warp * kMedWarpBytes, gw, nw);
         __syncthreads();
-        if (t < kPairThreads)  // (the block pass is laid out for kPairThreads threads)
-            block_pass<D, false, NARROW, false, true, true>(p, *reinterpret_cast<BlockSmem*>(smem_raw), blk, nblk);
+        constexpr uint32_t kTeams = kFusedThreads / kTeamThreads;
+        team_pass<D, false, false, true, true>(p, reinterpret_cast<TeamSmem*>(smem_raw)[t / kTeamThreads],
+                                               blk * kTeams + t / kTeamThreads, nblk * kTeams);
     }
     // the last block to finish copies the run counters to the host (one
     // more arrival per block on the barriers' count)
@@ -2404,13 +2204,13 @@ static int g_sm_count = 0;
 
 static size_t med_smem() { return (size_t)kPairWarps * kMedWarpBytes; }
 
-size_t pair_smem_bytes() { return sizeof(BlockSmem); }
+size_t pair_smem_bytes() { return sizeof(TeamSmem); }
 
-template <int D, bool B, bool N, bool R = false>
+template <int D, bool B, bool R = false>
 static cudaError_t init_variant() {
-    cudaError_t e = cudaFuncSetAttribute(k_pairs_med<D, B, N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)med_smem());
+    cudaError_t e = cudaFuncSetAttribute(k_pairs_med<D, B, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)med_smem());
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_pairs_block<D, B, N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BlockSmem));
+    e = cudaFuncSetAttribute(k_pairs_block<D, B, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TeamSmem));
     return e;
 }
 
@@ -2418,7 +2218,8 @@ static int g_fused_blocks = 0;
 
 static size_t fused_smem() {
     size_t b = (size_t)kFusedWarps * kMedWarpBytes;
-    b = b > sizeof(BlockSmem) ? b : sizeof(BlockSmem);
+    const size_t team = sizeof(TeamSmem) * (kFusedThreads / kTeamThreads);
+    b = b > team ? b : team;
     b = b > (size_t)kFusedWarps * kSmallWarpBytes ? b : (size_t)kFusedWarps * kSmallWarpBytes;
     b = b > (size_t)kFusedChunks * 4 ? b : (size_t)kFusedChunks * 4;
     b = b > (size_t)kFusedThreads * 7 * 4 ? b : (size_t)kFusedThreads * 7 * 4;
@@ -2427,25 +2228,23 @@ static size_t fused_smem() {
 
 int fused_blocks() { return g_fused_blocks; }
 
-template <int D, bool N>
+template <int D>
 static cudaError_t launch_fused_t(const Params& p, const FusedArgs& a, cudaStream_t st) {
     Params pp = p;
     FusedArgs aa = a;
     void* args[] = {&pp, &aa};
-    return cudaLaunchCooperativeKernel((const void*)k_fused<D, N>, dim3((unsigned)g_fused_blocks), dim3(kFusedThreads),
+    return cudaLaunchCooperativeKernel((const void*)k_fused<D>, dim3((unsigned)g_fused_blocks), dim3(kFusedThreads),
                                       args, fused_smem(), st);
 }
 
 cudaError_t launch_fused(const Params& p, const FusedArgs& a, int dims, cudaStream_t st) {
     if (g_fused_blocks <= 0) return cudaErrorNotSupported;
-    const bool narrow = p.max_range <= (1u << kMissShift);
-    if (narrow) return dims == 2 ? launch_fused_t<2, true>(p, a, st) : launch_fused_t<3, true>(p, a, st);
-    return dims == 2 ? launch_fused_t<2, false>(p, a, st) : launch_fused_t<3, false>(p, a, st);
+    return dims == 2 ? launch_fused_t<2>(p, a, st) : launch_fused_t<3>(p, a, st);
 }
 
-template <int D, bool N>
+template <int D>
 static cudaError_t init_fused() {
-    return cudaFuncSetAttribute(k_fused<D, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem());
+    return cudaFuncSetAttribute(k_fused<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem());
 }
 
 cudaError_t kernels_init() {
@@ -2455,35 +2254,27 @@ cudaError_t kernels_init() {
         if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
         if ((e = cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     }
+    if ((e = init_variant<2, false>()) != cudaSuccess) return e;
+    if ((e = init_variant<3, false>()) != cudaSuccess) return e;
+    if ((e = init_variant<2, true>()) != cudaSuccess) return e;
+    if ((e = init_variant<3, true>()) != cudaSuccess) return e;
     if ((e = init_variant<2, false, true>()) != cudaSuccess) return e;
     if ((e = init_variant<3, false, true>()) != cudaSuccess) return e;
-    if ((e = init_variant<2, true, true>()) != cudaSuccess) return e;
-    if ((e = init_variant<3, true, true>()) != cudaSuccess) return e;
-    if ((e = init_variant<2, false, false>()) != cudaSuccess) return e;
-    if ((e = init_variant<3, false, false>()) != cudaSuccess) return e;
-    if ((e = init_variant<2, true, false>()) != cudaSuccess) return e;
-    if ((e = init_variant<3, true, false>()) != cudaSuccess) return e;
-    if ((e = init_variant<2, false, true, true>()) != cudaSuccess) return e;
-    if ((e = init_variant<3, false, true, true>()) != cudaSuccess) return e;
-    if ((e = init_variant<2, false, false, true>()) != cudaSuccess) return e;
-    if ((e = init_variant<3, false, false, true>()) != cudaSuccess) return e;
     int nb = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pairs_small<3, false, true>, kPairThreads, 0)) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pairs_small<3, false>, kPairThreads, 0)) != cudaSuccess) return e;
     g_blocks_small = nb > 0 ? nb : 1;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pairs_med<3, false, true>, kPairThreads, med_smem())) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pairs_med<3, false>, kPairThreads, med_smem())) != cudaSuccess) return e;
     g_blocks_med = nb > 0 ? nb : 1;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pairs_block<3, false, true>, kPairThreads, sizeof(BlockSmem))) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pairs_block<3, false>, kTeamThreads, sizeof(TeamSmem))) != cudaSuccess) return e;
     g_blocks_block = nb > 0 ? nb : 1;
     // one-launch queries: one block per SM, all resident (cooperative launch)
-    if ((e = init_fused<2, true>()) != cudaSuccess) return e;
-    if ((e = init_fused<3, true>()) != cudaSuccess) return e;
-    if ((e = init_fused<2, false>()) != cudaSuccess) return e;
-    if ((e = init_fused<3, false>()) != cudaSuccess) return e;
+    if ((e = init_fused<2>()) != cudaSuccess) return e;
+    if ((e = init_fused<3>()) != cudaSuccess) return e;
     {
         int dev = 0, coop = 0, nf = 0;
         if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
         if ((e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev)) != cudaSuccess) return e;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nf, k_fused<3, true>, kFusedThreads, fused_smem())) !=
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nf, k_fused<3>, kFusedThreads, fused_smem())) !=
             cudaSuccess)
             return e;
         g_fused_blocks = coop && nf >= 1 ? g_sm_count : 0;
@@ -2581,27 +2372,27 @@ cudaError_t launch_expand(const Params& p, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-template <int D, bool B, bool N, bool R = false>
+template <int D, bool B, bool R = false>
 static cudaError_t launch_pairs_t(const Params& p, int sm_count, cudaStream_t st, cudaEvent_t* ev, unsigned evf,
                                   const PairOverlap* ov) {
     if (ov && !R && ov->side_sms > 0 && ov->side_sms < sm_count) {
         cudaError_t e;
         if ((e = cudaEventRecord(ov->fork, st)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(ov->side, ov->fork, 0)) != cudaSuccess) return e;
-        k_pairs_small<D, B, N, R><<<ov->side_sms * g_blocks_small, kPairThreads, 0, ov->side>>>(p);
+        k_pairs_small<D, B, R><<<ov->side_sms * g_blocks_small, kPairThreads, 0, ov->side>>>(p);
         if (ev) cudaEventRecordWithFlags(ev[0], ov->side, evf);
-        k_pairs_block<D, B, N, R><<<ov->side_sms * g_blocks_block, kPairThreads, sizeof(BlockSmem), ov->side>>>(p);
-        k_pairs_med<D, B, N, R><<<(sm_count - ov->side_sms) * g_blocks_med, kPairThreads, med_smem(), st>>>(p);
+        k_pairs_block<D, B, R><<<ov->side_sms * g_blocks_block, kTeamThreads, sizeof(TeamSmem), ov->side>>>(p);
+        k_pairs_med<D, B, R><<<(sm_count - ov->side_sms) * g_blocks_med, kPairThreads, med_smem(), st>>>(p);
         if (ev) cudaEventRecordWithFlags(ev[1], st, evf);
         if ((e = cudaEventRecord(ov->join, ov->side)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(st, ov->join, 0)) != cudaSuccess) return e;
         return cudaGetLastError();
     }
-    k_pairs_small<D, B, N, R><<<sm_count * g_blocks_small, kPairThreads, 0, st>>>(p);
+    k_pairs_small<D, B, R><<<sm_count * g_blocks_small, kPairThreads, 0, st>>>(p);
     if (ev) cudaEventRecordWithFlags(ev[0], st, evf);
-    k_pairs_med<D, B, N, R><<<sm_count * g_blocks_med, kPairThreads, med_smem(), st>>>(p);
+    k_pairs_med<D, B, R><<<sm_count * g_blocks_med, kPairThreads, med_smem(), st>>>(p);
     if (ev) cudaEventRecordWithFlags(ev[1], st, evf);
-    k_pairs_block<D, B, N, R><<<sm_count * g_blocks_block, kPairThreads, sizeof(BlockSmem), st>>>(p);
+    k_pairs_block<D, B, R><<<sm_count * g_blocks_block, kTeamThreads, sizeof(TeamSmem), st>>>(p);
     if (R) k_strip_entries<<<(unsigned)(sm_count * 4), 512, 0, st>>>(p);
     return cudaGetLastError();
 }
@@ -2609,20 +2400,13 @@ static cudaError_t launch_pairs_t(const Params& p, int sm_count, cudaStream_t st
 cudaError_t launch_pairs(const Params& p, int dims, int sm_count, cudaStream_t st, cudaEvent_t* ev, unsigned evf,
                          const PairOverlap* ov) {
     const bool bip = p.split != kNoSplit;
-    const bool narrow = p.max_range <= (1u << kMissShift);
     if (p.records) {  // record mode: self queries
         if (bip) return cudaErrorInvalidValue;
-        if (narrow) return dims == 2 ? launch_pairs_t<2, false, true, true>(p, sm_count, st, ev, evf, ov)
-                                     : launch_pairs_t<3, false, true, true>(p, sm_count, st, ev, evf, ov);
-        return dims == 2 ? launch_pairs_t<2, false, false, true>(p, sm_count, st, ev, evf, ov)
-                         : launch_pairs_t<3, false, false, true>(p, sm_count, st, ev, evf, ov);
+        return dims == 2 ? launch_pairs_t<2, false, true>(p, sm_count, st, ev, evf, ov)
+                         : launch_pairs_t<3, false, true>(p, sm_count, st, ev, evf, ov);
     }
-    if (narrow) {
-        if (dims == 2) return bip ? launch_pairs_t<2, true, true>(p, sm_count, st, ev, evf, ov) : launch_pairs_t<2, false, true>(p, sm_count, st, ev, evf, ov);
-        return bip ? launch_pairs_t<3, true, true>(p, sm_count, st, ev, evf, ov) : launch_pairs_t<3, false, true>(p, sm_count, st, ev, evf, ov);
-    }
-    if (dims == 2) return bip ? launch_pairs_t<2, true, false>(p, sm_count, st, ev, evf, ov) : launch_pairs_t<2, false, false>(p, sm_count, st, ev, evf, ov);
-    return bip ? launch_pairs_t<3, true, false>(p, sm_count, st, ev, evf, ov) : launch_pairs_t<3, false, false>(p, sm_count, st, ev, evf, ov);
+    if (dims == 2) return bip ? launch_pairs_t<2, true>(p, sm_count, st, ev, evf, ov) : launch_pairs_t<2, false>(p, sm_count, st, ev, evf, ov);
+    return bip ? launch_pairs_t<3, true>(p, sm_count, st, ev, evf, ov) : launch_pairs_t<3, false>(p, sm_count, st, ev, evf, ov);
 }
 
 cudaError_t launch_group_by_scene(const Params& p, const unsigned long long* scene_pair_off,

@@ -21,6 +21,7 @@ enum : uint32_t {
 };
 
 constexpr uint32_t kNoSplit = 0xffffffffu;
+constexpr uint32_t kOpenShift = 15;  // from this cell shift on, two coordinates of a cell may share an entry term
 constexpr int kIdBits = 29;
 constexpr uint32_t kIdMask = (1u << kIdBits) - 1u;
 
@@ -144,6 +145,8 @@ struct Ctr {
     unsigned int need_tasks;            // tile tasks needed
     unsigned int max_cell;              // largest cell (or merged block) of two or more boxes
     unsigned int med_next;              // next medium-cell item (items are taken one at a time)
+    unsigned int big_next;              // next big-cell item, likewise
+    unsigned int pad;
     unsigned long long entries;         // E
     unsigned long long pairs;           // pairs found (may exceed capacity)
     unsigned long long tests;           // sum of n(n-1)/2 over cells
@@ -173,10 +176,11 @@ struct Params {
     uint32_t* scene_table;        // batched queries: scene of box 256*b, per b (built by launch_scene_table)
     uint32_t nscenes;
     uint32_t split;               // bipartite: global index of the first blue box
-    uint32_t max_range;           // largest scene range (selects the pair-test arithmetic)
+    uint32_t max_range;           // largest scene range
+    uint32_t open;                // some cell is 2^15 or wider: equal entry terms need the coordinates
     uint32_t* counts;             // [ncells] per-cell counts; cell ends after the scan, starts after the scatter
     uint64_t ncells;
-    uint32_t* entries;            // [entry_cap]: flags<<29 | global box index
+    uint4* entries;               // [entry_cap]: a word per axis, then flags<<29 | global box index
     uint64_t entry_cap;
     uint2* lists;                 // kNumLists regions of {start, n}
     uint64_t list_off[kNumLists]; // region offsets into lists
@@ -189,6 +193,8 @@ struct Params {
     Ctr* ctr;
     const RunDims* dyn;           // when set, overrides nboxes / ncells / nscenes
     const uint32_t* merged;       // merged mode (one scene): cell -> root of its merged block, or kUnmerged
+    const unsigned long long* merged_ext; // ... and of a root: its block's cells per axis, 21 bits each
+    uint32_t* recs;               // record mode: [entry_cap] box indices, written after the pair kernels
     uint32_t records;             // record mode: work lists hold {cell id, n}; the pair kernels write the
                                   // reference's Rice record stream (8-byte words) instead of pairs
     unsigned long long class_map; // cell size -> work list (0: kClassMapDefault)

@@ -12,7 +12,7 @@
 // call allocates nothing.
 //
 // The scratch array is a file-scope __device__ array of kScratchBytes
-// (16 MiB): every GPU that loads the library holds it until the process
+// (24 MiB): every GPU that loads the library holds it until the process
 // exits. Every call shares it and it keeps the last call's contents, so the
 // call clears what must start at zero; calls that overlap on the GPU (two
 // host threads, or two streams) race on it and must be serialized by the
@@ -31,7 +31,7 @@
 
 namespace pbig {
 
-static constexpr size_t kScratchBytes = 16u << 20;
+static constexpr size_t kScratchBytes = 24u << 20;
 
 // limits of one allocation-free query (so that everything fits the scratch)
 static constexpr uint64_t kNaMaxBoxes = 1u << 18;    // 262,144 boxes
@@ -138,7 +138,7 @@ PBIG2_API int pbig2_self_intersect_noalloc(const uint32_t* d_boxes, uint64_t n, 
     p.counts = (uint32_t*)take(ncells * 4 + 16);
     const uint64_t tiles = scan_tiles(ncells);
     p.tile_state = (unsigned long long*)take(scan_state_bytes(ncells));
-    p.entries = (uint32_t*)take(kNaMaxEntries * 4);
+    p.entries = (uint4*)take(kNaMaxEntries * sizeof(uint4));
     p.entry_cap = kNaMaxEntries;
     const uint64_t lo[kNumLists] = {2, 5, 9, 17, 33, kMedMax + 1, kBigMax + 1};
     uint64_t loff = 0;
@@ -150,7 +150,7 @@ PBIG2_API int pbig2_self_intersect_noalloc(const uint32_t* d_boxes, uint64_t n, 
     p.lists = (uint2*)take(loff * 8);
     p.tasks = (uint4*)take(kNaMaxTasks * 16);
     p.task_cap = kNaMaxTasks;
-    if (off > kScratchBytes) return na_fail(PBIG2_ECAPACITY, "scratch layout exceeds 16 MiB");
+    if (off > kScratchBytes) return na_fail(PBIG2_ECAPACITY, "scratch layout exceeds 24 MiB");
 
     Scene sc{};
     sc.box_off = 0;
@@ -167,6 +167,7 @@ PBIG2_API int pbig2_self_intersect_noalloc(const uint32_t* d_boxes, uint64_t n, 
     p.nscenes = 1;
     p.split = kNoSplit;
     p.max_range = range;
+    p.open = shift >= kOpenShift ? 1u : 0u;
     p.ncells = ncells;
     p.out = reinterpret_cast<uint2*>(d_pairs);
     p.out_cap = pair_cap;
