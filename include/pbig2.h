@@ -344,8 +344,10 @@ PBIG2_API int pbig2_scene_copy(pbig2_scene* scene, int which, uint32_t* dst, uin
  * refuse grids of 2^32 - 1 cells or more. */
 PBIG2_API uint64_t pbig2_grid_cells(uint32_t range, uint32_t shift, uint32_t dims);
 
-/* Cell-size autotuner: the shift the engine would pick for these boxes
- * (host memory), from a sample of at most `sample` boxes. */
+/* Cell-size autotuner of batched and serving scenes, for boxes in host
+ * memory, from a sample of at most `sample` of them. (Self and red/blue
+ * queries with PBIG2_AUTO choose on the device, with a cost model of their
+ * own.) */
 PBIG2_API int pbig2_tune_shift(const uint32_t* boxes, uint64_t n, uint32_t dims, uint32_t range,
                                uint64_t sample, uint32_t* shift);
 

@@ -85,20 +85,16 @@ uint32_t nrc_for(uint32_t range, uint32_t shift) {
 }
 
 // --------------------------------------------------------------------------
-// autotuner: cost(s) = kCell*C(s) + kEntry*E(s) + kTest*T(s) in seconds
-// (C cells, E box-in-cell entries, T pair tests; tune_cost in kernels.cuh),
-// estimated from a sample. T is counted exactly on the sample (cell
-// occupancy by hashing) and scaled by (n/m)^2, since a pair of boxes
-// survives sampling with probability (m/n)^2. A test costs more once the
-// tests sit in cells beyond the medium-cell kernel's reach: with the
-// entry-weighted mean occupancy m = 2T/E + 1, kTest is scaled by
-// max(1, m / kOccTest). The constants are fitted on GB300 cell-size sweeps
-// (2-D/3-D, uniform/clustered, single scenes and a 4096-scene batch), where
-// they pick the fastest size or one within 2%; per unit, an entry costs
-// ~16 ps in the count and scatter plus its fetch and sweep in the pair
-// kernels, a test ~1 ps in the medium-cell kernel and ~2 ps in the block
-// kernel. Batched queries run the same model on the device, one warp per
-// scene, with T = E^2 / 2C (k_tune_scenes).
+// autotuner of pbig2_tune_shift and of new scenes in a serving batch: cost(s) =
+// kCell*C(s) + kEntry*E(s) + kTest*T(s) in seconds (C cells, E box-in-cell
+// entries, T pair tests; tune_cost in kernels.cuh), estimated from a sample.
+// T is counted exactly on the sample (cell occupancy by hashing) and scaled by
+// (n/m)^2, since a pair of boxes survives sampling with probability (m/n)^2;
+// with the entry-weighted mean occupancy m = 2T/E + 1, kTest is scaled by
+// max(1, m / kOccTest). Batched queries run the same model on the device, one
+// warp per scene, with T = E^2 / 2C (k_tune_scenes); its constants were fitted
+// to earlier pair kernels, and on the batches measured it still picks the
+// fastest size. Self and red/blue queries choose with k_tune_query.
 // --------------------------------------------------------------------------
 
 // pair tests of the sample at one cell size: occupancy of the sample's cells
@@ -262,50 +258,47 @@ static int ensure_query_buffers(pbig2_ctx* c, Params& p, uint64_t entry_cap, uin
     return PBIG2_OK;
 }
 
-// the launches of one pipeline pass (also what a graph captures): counters
-// and scan state reset, count, scan, expand, scatter, the three pair
-// kernels and, for batches, grouping of the pairs by scene
+// the launches of one pipeline pass (also what a graph captures): count,
+// scan, scatter, the three pair kernels and, for batches, grouping of the
+// pairs by scene. The kernel that ends the pass copies the run counters to
+// c->h_ctr. Single-scene queries run the tuner first (which clears the run
+// counters); `full` false repeats the pair kernels on the grid that is there.
 static int g_record_line = 0;  // line of the call that failed in record_pipeline
 
-static cudaError_t record_pipeline(pbig2_ctx* c, const Params& p, int dims, bool grouped, uint32_t nsc,
-                                   bool full, cudaStream_t st) {
+static cudaError_t record_pipeline(pbig2_ctx* c, const Params& p, int dims, bool grouped, uint32_t nsc, bool full,
+                                   const TuneArgs* tune, cudaStream_t st) {
     cudaError_t e;
     (void)cudaGetLastError();  // launch checks below must not see older, unrelated errors
-    // inside a stream capture an event record must be an external node to be timed
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if ((e = cudaStreamIsCapturing(st, &cap)) != cudaSuccess) return e;
-    const unsigned evf = cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
 #define R(x)                          \
     if ((e = (x)) != cudaSuccess) {   \
         g_record_line = __LINE__;     \
         return e;                     \
     }
     if (full) {
-        R(cudaMemsetAsync(p.ctr, 0, sizeof(Ctr), st));
+        if (tune) {
+            R(launch_tune_query(p, *tune, dims, st));
+        } else {
+            R(cudaMemsetAsync(p.ctr, 0, sizeof(Ctr), st));
+        }
         if (p.scene_table) R(launch_scene_table(p, st));
-        R(cudaEventRecordWithFlags(c->evp[0], st, evf));
         R(launch_count(p, dims, st));
-        R(cudaEventRecordWithFlags(c->evp[1], st, evf));
         R(launch_scan(p, st));
-        R(cudaEventRecordWithFlags(c->evp[2], st, evf));
-        R(launch_expand(p, st));
-        R(cudaEventRecordWithFlags(c->evp[3], st, evf));
         R(launch_scatter(p, dims, st));
-        R(cudaEventRecordWithFlags(c->evp[4], st, evf));
     } else {
-        // keep the grid and lists; clear the pair count and error word
+        // keep the grid and lists; clear the pair count, the error word and the item counters
         R(cudaMemsetAsync(&p.ctr->pairs, 0, sizeof(unsigned long long), st));
+        R(cudaMemsetAsync(&p.ctr->rec_pairs, 0, sizeof(unsigned long long), st));
         R(cudaMemsetAsync(&p.ctr->err, 0, sizeof(unsigned int), st));
-        R(cudaMemsetAsync(&p.ctr->med_next, 0, 2 * sizeof(unsigned int), st));  // and big_next
-        R(cudaEventRecordWithFlags(c->evp[4], st, evf));
+        R(cudaMemsetAsync(&p.ctr->med_next, 0, 3 * sizeof(unsigned int), st));  // med_next, big_next, done
     }
+    Params pp = p;
+    pp.ctr_host = grouped ? nullptr : static_cast<Ctr*>(c->h_ctr.p);
     // pairs stored over the host link: the lighter pair kernels run beside
     // the medium-cell kernel (two fifths of the SMs unless set)
     PairOverlap ov{c->side_stream, c->ev_fork, c->ev_join,
                    c->host_split > 0 ? c->host_split : (2 * c->sm_count + 2) / 5};
     const bool overlap = c->ext_host && p.out == c->ext_out && c->host_split >= 0 && !p.records;
-    R(launch_pairs(p, dims, c->sm_count, st, &c->evp[7], evf, overlap ? &ov : nullptr));  // records evp[7], evp[8]
-    R(cudaEventRecordWithFlags(c->evp[5], st, evf));
+    R(launch_pairs(pp, dims, c->sm_count, st, overlap ? &ov : nullptr));
     if (grouped) {
         unsigned long long* hist = c->d_scene_cursor.as<unsigned long long>();
         unsigned long long* offs = c->d_scene_pair.as<unsigned long long>();
@@ -313,17 +306,16 @@ static cudaError_t record_pipeline(pbig2_ctx* c, const Params& p, int dims, bool
         R(launch_scene_hist(p, hist, st));
         R(launch_scene_offsets(p, hist, offs, nsc, st));
         R(cudaMemsetAsync(hist, 0, (nsc + 1) * 8, st));
-        R(launch_group_by_scene(p, offs, hist, c->d_out2.as<uint2>(), st));
+        pp.ctr_host = static_cast<Ctr*>(c->h_ctr.p);
+        R(launch_group_by_scene(pp, offs, hist, c->d_out2.as<uint2>(), st));
     }
-    R(cudaEventRecordWithFlags(c->ev1, st, evf));
 #undef R
     return cudaSuccess;
 }
 
 // result bookkeeping after a pass: pair count, per-scene offsets, stats
 static int finish_query(pbig2_ctx* c, const Ctr& h, uint64_t nboxes, uint64_t ncells, uint32_t nsc,
-                        const std::vector<GridScene>& scenes, bool grouped, int launches, cudaStream_t st,
-                        bool phases = true) {
+                        const std::vector<GridScene>& scenes, bool grouped, int launches, cudaStream_t st) {
     c->result_records = c->rice_mode && !grouped;
     c->rice_words = c->result_records ? h.pairs : 0;
     c->npairs = c->result_records ? h.rec_pairs : h.pairs;
@@ -339,22 +331,15 @@ static int finish_query(pbig2_ctx* c, const Ctr& h, uint64_t nboxes, uint64_t nc
         c->scene_pair_off.assign(1, 0);
         c->scene_pair_off.push_back(c->npairs);
     }
-    float ms = 0;
-    if (phases) cudaEventElapsedTime(&ms, c->ev0, c->ev1);
-    double phase[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int k = 0; k < 5 && phases; k++) {
-        float x = 0;
-        if (cudaEventElapsedTime(&x, c->evp[k], c->evp[k + 1]) == cudaSuccess) phase[k] = x;
-    }
-    if (phases) {
-        float x = 0;
-        if (grouped && cudaEventElapsedTime(&x, c->evp[5], c->ev1) == cudaSuccess) phase[5] = x;
-        // (the pair kernels may overlap: a phase that ends before the
-        // previous one reads 0)
-        if (cudaEventElapsedTime(&x, c->evp[4], c->evp[7]) == cudaSuccess) phase[6] = std::max(0.f, x);
-        if (cudaEventElapsedTime(&x, c->evp[7], c->evp[8]) == cudaSuccess) phase[7] = std::max(0.f, x);
-        if (cudaEventElapsedTime(&x, c->evp[8], c->evp[5]) == cudaSuccess) phase[8] = std::max(0.f, x);
-    }
+    // phase times from the kernels' own clock stamps (one-launch queries have none)
+    const auto between = [&](int a, int b) {
+        return h.stamp[a] && h.stamp[b] > h.stamp[a] ? (double)(h.stamp[b] - h.stamp[a]) * 1e-6 : 0.0;
+    };
+    const int pairs_end = grouped ? kStampGroup : kStampEnd;
+    const double phase[9] = {between(kStampCount, kStampScan), between(kStampScan, kStampScatter), 0.0,
+                             between(kStampScatter, kStampSmall), between(kStampSmall, pairs_end),
+                             grouped ? between(kStampGroup, kStampEnd) : 0.0, between(kStampSmall, kStampMed),
+                             between(kStampMed, kStampBlock), between(kStampBlock, pairs_end)};
     c->last_err = h.err;
     pbig2_stats& s = c->stats;
     s.boxes = nboxes;
@@ -372,9 +357,8 @@ static int finish_query(pbig2_ctx* c, const Ctr& h, uint64_t nboxes, uint64_t nc
     s.scenes = nsc;
     s.kernels = (uint32_t)launches;
     s.grid_retries = 0;  // set by the caller after a coarser-grid rerun
-    s.device_ms = ms;
+    s.device_ms = between(kStampStart, kStampEnd);
     for (int k = 0; k < 9; k++) s.phase_ms[k] = phase[k];
-    (void)cudaGetLastError();  // a timing query on an unrecorded event is not an error of the query
     if (h.bad) return fail(PBIG2_EINPUT, "%u boxes violate the input contract (error bits 0x%x) and were skipped",
                            h.bad, h.err);
     return PBIG2_OK;
@@ -396,8 +380,7 @@ static int capture_graph(pbig2_ctx* c, const Params& p0, const uint32_t* d_boxes
     cudaStream_t cs = c->own_stream;
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = record_pipeline(c, p, dims, true, nsc, true, cs);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(c->h_ctr.p, p.ctr, sizeof(Ctr), cudaMemcpyDeviceToHost, cs);
+    cudaError_t e = record_pipeline(c, p, dims, true, nsc, true, nullptr, cs);
     cudaError_t e2 = cudaStreamEndCapture(cs, &g);
     if (e != cudaSuccess || e2 != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -420,7 +403,7 @@ static int capture_graph(pbig2_ctx* c, const Params& p0, const uint32_t* d_boxes
     G.entry_cap = p.entry_cap;
     G.out_cap = p.out_cap;
     G.class_map = c->class_map;  // the option (0: automatic), as graph_fits compares it
-    G.launches = 13;  // scene table, count (2), scan (2), expand, scatter, pairs (3), scene grouping (3)
+    G.launches = 12;  // scene table, count (2), scan (2), scatter, pairs (3), scene grouping (3)
     G.buffers = c->buffers_sig();
     return PBIG2_OK;
 }
@@ -496,9 +479,63 @@ static uint32_t merge_cells(std::vector<uint32_t>& nrs, std::vector<uint32_t>& m
     return blocks;
 }
 
-static int run_pipeline(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t nboxes, int dims, uint32_t range,
-                        const std::vector<GridScene>& scenes, uint32_t split, double est_entries,
-                        cudaStream_t st, bool group) {
+// what a finished pass says about its buffers: grows the capacities in `need`
+// and returns kAgain for another pass (need.full: from the count on), or the
+// error, or PBIG2_OK
+struct Need {
+    uint64_t entries, out, tasks;
+    bool full;
+    uint64_t cells;  // (single-scene queries)
+};
+constexpr int kAgain = -1001;
+
+static int check_pass(const Params& p, const Ctr& h, Need& need) {
+    if (h.err & kErrWait) return fail(PBIG2_ETIMEOUT, "a bounded device wait gave up (scan bulk copy)");
+    if (h.err & kErrRecCell)
+        return fail(PBIG2_ECAPACITY, "a cell of 65536 boxes or more cannot be written as records");
+    if (h.err & kErrIndex) return fail(PBIG2_ECUDA, "inconsistent cell lists (error bits 0x%x)", h.err);
+    if (h.err & kErrGridRoom) {  // the pass stopped at the tuner
+        need.cells = h.cells;
+        need.full = true;
+        return kAgain;
+    }
+    if ((h.err & kErrEntryOvf) || h.entries > p.entry_cap) {
+        if (h.entries >= (1ull << 32))
+            return fail(PBIG2_ENOMEM, "%llu cell entries exceed the 2^32 limit of one query",
+                        (unsigned long long)h.entries);
+        need.entries = h.entries + h.entries / 16 + 4096;
+        need.full = true;
+        return kAgain;
+    }
+    if (h.err & kErrTaskOvf) {
+        need.tasks = (uint64_t)h.need_tasks + 1024;
+        need.full = true;
+        return kAgain;
+    }
+    if ((h.err & kErrOutOvf) || h.pairs > p.out_cap) {
+        need.out = std::max<uint64_t>(need.out, h.pairs + h.pairs / 8 + 1024);
+        need.full = false;
+        return kAgain;
+    }
+    return PBIG2_OK;
+}
+
+// One pass and the wait for it; h: its run counters.
+static int run_pass(pbig2_ctx* c, const Params& p, int dims, bool grouped, uint32_t nsc, bool full,
+                    const TuneArgs* tune, cudaStream_t st, Ctr& h) {
+    const cudaError_t re = record_pipeline(c, p, dims, grouped, nsc, full, tune, st);
+    if (re != cudaSuccess)
+        return fail(PBIG2_ECUDA, "pipeline launch (engine.cu:%d): %s", g_record_line, cudaGetErrorString(re));
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return fail(PBIG2_ECUDA, "pipeline failed: %s", cudaGetErrorString(e));
+    memcpy(&h, c->h_ctr.p, sizeof(Ctr));
+    return PBIG2_OK;
+}
+
+// A batched query of two or more scenes: the scene table from the host, the
+// pairs grouped by scene.
+static int run_batch(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t nboxes, int dims, uint32_t range,
+                     const std::vector<GridScene>& scenes, double est_entries, cudaStream_t st) {
     const uint32_t nsc = (uint32_t)scenes.size();
     c->last_err = 0;
     c->fused_dirty = true;  // this pipeline leaves cell starts in the counters
@@ -517,27 +554,21 @@ static int run_pipeline(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t nboxes, 
         s.nrc = nrc_for(range, g.shift);
         s.range = range;
         s.pad = 0;
-        if (g.grid_of == (int)i) {
-            s.cell_off = ncells;
-            const uint64_t cc = grid_cells(range, g.shift, dims);  // saturating
-            ncells = cc > ~0ull - ncells ? ~0ull : ncells + cc;
-        } else {
-            s.cell_off = tab[g.grid_of].cell_off;
-        }
+        s.cell_off = ncells;
+        const uint64_t cc = grid_cells(range, g.shift, dims);  // saturating
+        ncells = cc > ~0ull - ncells ? ~0ull : ncells + cc;
         box_off[i] = (uint32_t)g.box_off;
     }
     box_off[nsc] = (uint32_t)nboxes;
     if (ncells >= (1ull << 32) - 1)
         return fail(PBIG2_EINVAL, "grid too fine: %llu cells (limit 2^32)", (unsigned long long)ncells);
-    const bool grouped = group && nsc > 1;
 
     // a captured graph serves this query if the buffers it was captured with
     // are large enough and the fixed arguments match
     pbig2_ctx::Graph& G = c->graph;
-    const bool graph_fits = c->use_graph && grouped && G.exec && G.boxes == d_boxes && G.dims == dims &&
-                            G.range == range && G.split == split && nboxes <= G.nboxes_cap &&
-                            ncells <= G.ncells_cap && nsc <= G.nscenes_cap && G.buffers == c->buffers_sig() &&
-                            G.class_map == c->class_map;
+    const bool graph_fits = c->use_graph && G.exec && G.boxes == d_boxes && G.dims == dims && G.range == range &&
+                            nboxes <= G.nboxes_cap && ncells <= G.ncells_cap && nsc <= G.nscenes_cap &&
+                            G.buffers == c->buffers_sig() && G.class_map == c->class_map;
 
     // tables -> pinned staging -> device (before the pipeline or graph)
     const size_t tab_bytes = nsc * sizeof(Scene), off_bytes = (nsc + 1) * sizeof(uint32_t);
@@ -547,6 +578,7 @@ static int run_pipeline(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t nboxes, 
     rd.nboxes = nboxes;
     rd.ncells = ncells;
     rd.nscenes = nsc;
+    rd.open = 1;
     memcpy(c->h_stage.p, tab.data(), tab_bytes);
     memcpy((char*)c->h_stage.p + tab_bytes, box_off.data(), off_bytes);
     memcpy((char*)c->h_stage.p + tab_bytes + off_bytes, &rd, sizeof rd);
@@ -563,7 +595,6 @@ static int run_pipeline(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t nboxes, 
     Ctr h{};
     int launches = 0;
     if (graph_fits) {
-        CK(cudaEventRecord(c->ev0, st));
         CK(cudaGraphLaunch(G.exec, st));
         cudaError_t e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) {
@@ -583,7 +614,7 @@ static int run_pipeline(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t nboxes, 
             c->out_hint = std::max<uint64_t>(c->out_hint, h.pairs + h.pairs / 8);
             est_entries = std::max(est_entries, (double)h.entries * 1.1);
         } else {
-            const int rf = finish_query(c, h, nboxes, ncells, nsc, scenes, grouped, launches, st);
+            const int rf = finish_query(c, h, nboxes, ncells, nsc, scenes, true, launches, st);
             c->stats.class_map = c->class_map ? c->class_map : kClassMapDefault;
             return rf;
         }
@@ -594,52 +625,174 @@ static int run_pipeline(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t nboxes, 
     CK(c->d_state.ensure(scan_state_bytes(ncells), false, st));
     CK(c->d_ctr.ensure(sizeof(Ctr), false, st));
     CK(c->h_ctr.ensure(sizeof(Ctr)));
+    CK(c->d_scene_tab.ensure(scene_table_entries(nboxes) * 4, false, st));
 
-    uint64_t entry_cap = (uint64_t)(est_entries * 1.25) + 4096;
-    entry_cap = std::max<uint64_t>(entry_cap, c->d_entries.bytes / sizeof(uint4));
-    uint64_t out_cap = std::max<uint64_t>({c->out_hint, nboxes * 4, 1u << 16});
-    out_cap = std::max<uint64_t>(out_cap, c->d_out.bytes / 8);
-    uint64_t task_cap = std::max<uint64_t>(c->d_tasks.bytes / 16, 4096);
+    Need need{};
+    need.entries = std::max<uint64_t>((uint64_t)(est_entries * 1.25) + 4096, c->d_entries.bytes / sizeof(uint4));
+    need.out = std::max<uint64_t>({c->out_hint, nboxes * 4, 1u << 16, c->d_out.bytes / 8});
+    need.tasks = std::max<uint64_t>(c->d_tasks.bytes / 16, 4096);
+    need.full = true;
 
     Params p{};
     p.boxes = d_boxes;
     p.nboxes = nboxes;
-    if (c->up_red || c->up_blue) {  // the count uploads the boxes (self and red/blue queries)
-        p.up_red = c->up_red;
-        p.up_blue = c->up_blue;
-        p.up_split = c->up_split;
-        p.box_copy = const_cast<uint32_t*>(d_boxes);
-    }
     p.scenes = c->d_scenes.as<Scene>();
     p.scene_box_off = c->d_scene_off.as<uint32_t>();
-    if (grouped) {  // many scenes: the scene of every 256th box, for the scene lookups of the kernels
-        CK(c->d_scene_tab.ensure(scene_table_entries(nboxes) * 4, false, st));
-        p.scene_table = c->d_scene_tab.as<uint32_t>();
-    }
+    p.scene_table = c->d_scene_tab.as<uint32_t>();  // the scene of every 256th box, for the kernels' scene lookups
     p.nscenes = nsc;
-    p.split = split;
+    p.split = kNoSplit;
     p.max_range = range;
-    for (const Scene& s : tab) p.open |= s.shift >= kOpenShift ? 1u : 0u;
+    p.open = 1;
     p.ncells = ncells;
     p.tile_state = c->d_state.as<unsigned long long>();
     p.ctr = c->d_ctr.as<Ctr>();
-    p.dyn = nullptr;
     p.class_map = c->class_map ? c->class_map : kClassMapDefault;
     c->merged_blocks = 0;
-    bool one_grid = true;  // a single scene, or red and blue sharing one grid
-    for (uint32_t i = 0; i < nsc; i++) one_grid = one_grid && scenes[i].grid_of == 0;
-    if (c->merged_mode && one_grid && !grouped) {
+    c->result_ext = false;
+    int rc = kAgain;
+    for (int attempt = 0; attempt < 6 && rc == kAgain; attempt++) {
+        rc = ensure_query_buffers(c, p, need.entries, need.out, need.tasks, nsc, true, st);
+        if (rc) return rc;
+        rc = run_pass(c, p, dims, true, nsc, need.full, nullptr, st, h);
+        if (rc) return rc;
+        launches += (need.full ? 6 : 0) + 6;  // scene table, count (2), scan (2), scatter; pairs (3), grouping (3)
+        rc = check_pass(p, h, need);
+    }
+    if (rc == kAgain) return fail(PBIG2_ENOMEM, "capacity retries exhausted");
+    if (rc) return rc;
+    c->out_hint = std::max<uint64_t>(c->out_hint, h.pairs + h.pairs / 8);
+    rc = finish_query(c, h, nboxes, ncells, nsc, scenes, true, launches, st);
+    c->stats.class_map = p.class_map;
+    if (rc != PBIG2_OK && rc != PBIG2_EINPUT) return rc;
+    // capture this query's pipeline for later batches of the same shape
+    if (G.exec && G.buffers != c->buffers_sig()) c->drop_graph();
+    if (c->use_graph && !G.exec) {
+        int rg = capture_graph(c, p, d_boxes, nboxes, ncells, nsc, dims, range, kNoSplit, need.entries, st);
+        if (rg) return rg;
+    }
+    return rc;
+}
+
+// The boxes of a single-scene query: `boxes` on the device, red first and blue
+// behind it. Boxes in page-locked host memory stay there until the count
+// copies them (up_red, up_blue: their device-mapped addresses).
+struct SingleScene {
+    const uint32_t* boxes;
+    const uint32_t* up_red;
+    const uint32_t* up_blue;
+    uint64_t n_red, n;
+    bool bip;
+    int dims;
+    uint32_t range;
+};
+
+// up to this many boxes a query is launched whole, the grid and its size known
+// to the device alone, into buffers for eight cells and six entries a box (a
+// query that needs more runs again); beyond, the tuner's result is read first
+constexpr uint64_t kBlindBoxes = 1u << 25;
+
+// A self or red/blue query of one scene at cell shift `shift` (PBIG2_AUTO:
+// chosen on the device). used: the cell shift it ran at.
+static int run_single(pbig2_ctx* c, const SingleScene& q, uint32_t shift, cudaStream_t st, uint32_t* used) {
+    c->last_err = 0;
+    c->fused_dirty = true;  // this pipeline leaves cell starts in the counters
+    c->merged_blocks = 0;
+    c->result_ext = false;
+    if (q.n > (uint64_t)kIdMask + 1)
+        return fail(PBIG2_EINVAL, "a query holds at most 2^29 boxes (got %llu)", (unsigned long long)q.n);
+    if (c->rice_mode && q.bip) return fail(PBIG2_EINVAL, "record mode serves self queries only");
+    const bool blind = !c->merged_mode && q.n <= kBlindBoxes;
+    Need need{};
+    const uint64_t have_cells = c->d_counts.bytes >= 64 ? (c->d_counts.bytes - 16) / 4 : 0;
+    need.cells = blind ? std::max<uint64_t>(8 * q.n + (1u << 20), have_cells) : 0;
+    if (shift != PBIG2_AUTO) {
+        need.cells = grid_cells(q.range, shift, q.dims);  // saturating
+        if (need.cells >= (1ull << 32) - 1)
+            return fail(PBIG2_EINVAL, "grid too fine: %llu cells (limit 2^32)", (unsigned long long)need.cells);
+    }
+    CK(c->d_ctr.ensure(sizeof(Ctr), false, st));
+    CK(c->h_ctr.ensure(sizeof(Ctr)));
+    CK(c->d_scenes.ensure(2 * sizeof(Scene), false, st));
+    CK(c->d_scene_off.ensure(3 * sizeof(uint32_t), false, st));
+    CK(c->d_dims.ensure(sizeof(RunDims), false, st));
+    CK(c->d_tune_cost.ensure(kTuneScratchBytes, true, st));
+
+    Params p{};
+    p.boxes = q.boxes;
+    p.nboxes = q.n;
+    if (q.up_red || q.up_blue) {
+        p.up_red = q.up_red;
+        p.up_blue = q.up_blue;
+        p.up_split = q.n_red;
+        p.box_copy = const_cast<uint32_t*>(q.boxes);
+    }
+    p.scenes = c->d_scenes.as<Scene>();
+    p.scene_box_off = c->d_scene_off.as<uint32_t>();
+    p.nscenes = q.bip ? 2 : 1;
+    p.split = q.bip ? (uint32_t)q.n_red : kNoSplit;
+    p.max_range = q.range;
+    p.ctr = c->d_ctr.as<Ctr>();
+    p.dyn = c->d_dims.as<RunDims>();
+    p.class_map = c->class_map ? c->class_map : kClassMapDefault;
+    p.records = c->rice_mode ? 1u : 0u;
+
+    TuneArgs ta{};
+    const bool on_host = q.up_red || q.up_blue;
+    ta.red = on_host ? q.up_red : q.boxes;
+    ta.blue = on_host ? q.up_blue : q.boxes + q.n_red * (2 * (uint64_t)q.dims + 1);
+    ta.n_red = q.n_red;
+    ta.n = q.n;
+    ta.bip = q.bip ? 1u : 0u;
+    ta.range = q.range;
+    ta.shift = shift == PBIG2_AUTO ? kTuneShift : shift;
+    ta.raise_from = ta.raise_to = 32;
+    for (const auto& r : c->raised)
+        if (r.n == q.n && r.dims == q.dims && r.range == q.range) {
+            ta.raise_from = r.from;
+            ta.raise_to = r.to;
+        }
+    ta.max_cells = 4000000000ull;
+    ta.scenes = c->d_scenes.as<Scene>();
+    ta.box_off = c->d_scene_off.as<uint32_t>();
+    ta.dims = c->d_dims.as<RunDims>();
+    ta.scratch = c->d_tune_cost.as<unsigned long long>();
+
+    need.entries = std::max<uint64_t>(6 * q.n + 4096, c->d_entries.bytes / sizeof(uint4));
+    need.out = std::max<uint64_t>({c->out_hint, q.n * 4, 1u << 16, c->d_out.bytes / 8});
+    need.tasks = std::max<uint64_t>(c->d_tasks.bytes / 16, 4096);
+    need.full = true;
+    Ctr h{};
+    int launches = 0, rc = PBIG2_OK;
+    if (!blind) {
+        ta.room_cells = ~0ull;
+        CK(launch_tune_query(p, ta, q.dims, st));
+        CK(cudaMemcpyAsync(c->h_ctr.p, p.ctr, sizeof(Ctr), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        memcpy(&h, c->h_ctr.p, sizeof(Ctr));
+        launches++;
+        need.entries = std::max<uint64_t>((uint64_t)((double)std::max(h.est_entries, (unsigned long long)q.n) * 1.25) + 4096,
+                                          c->d_entries.bytes / sizeof(uint4));
+        need.cells = h.cells;
+    }
+    const auto grid_room = [&]() {
+        CK(c->d_counts.ensure(need.cells * 4 + 16, false, st));  // zeroed by every pass
+        CK(c->d_state.ensure(scan_state_bytes(need.cells), false, st));
+        p.counts = c->d_counts.as<uint32_t>();
+        p.ncells = ta.room_cells = need.cells;
+        p.tile_state = c->d_state.as<unsigned long long>();
+        return (int)PBIG2_OK;
+    };
+    if ((rc = grid_room())) return rc;
+    if (c->merged_mode) {
         // first pass: plain counts; merge on the host; the pass below then
         // counts, bins and tests per merged block
-        Params p0 = p;
-        p0.counts = c->d_counts.as<uint32_t>();
-        CK(cudaMemsetAsync(p.ctr, 0, sizeof(Ctr), st));
-        CK(launch_count(p0, dims, st));
+        const uint64_t ncells = h.cells;
+        CK(launch_count(p, q.dims, st));
         std::vector<uint32_t> nrs(ncells), merged;
         std::vector<unsigned long long> ext;
-        CK(cudaMemcpyAsync(nrs.data(), p0.counts, ncells * 4, cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(nrs.data(), p.counts, ncells * 4, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        c->merged_blocks = merge_cells(nrs, merged, ext, tab[0].nrc, dims, c->merge_limit);
+        c->merged_blocks = merge_cells(nrs, merged, ext, nrc_for(q.range, h.shift), q.dims, c->merge_limit);
         CK(c->d_merged.ensure(ncells * 4, false, st));
         CK(cudaMemcpyAsync(c->d_merged.p, merged.data(), ncells * 4, cudaMemcpyHostToDevice, st));
         CK(c->d_merged_ext.ensure(ncells * sizeof(ext[0]), false, st));
@@ -648,76 +801,35 @@ static int run_pipeline(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t nboxes, 
         p.merged = c->d_merged.as<uint32_t>();
         p.merged_ext = c->d_merged_ext.as<unsigned long long>();
         p.open = 1;  // a block may be wider than a cell
+        ta.shift = h.shift;
     }
-    bool need_full = true;
-    // self/bipartite pairs go straight to the caller's buffer when one is set;
-    // a result that does not fit is redone into the context's buffer
-    p.records = (c->rice_mode && !grouped) ? 1u : 0u;
-    if (p.records && split != kNoSplit) return fail(PBIG2_EINVAL, "record mode serves self queries only");
-    bool use_ext = c->ext_out != nullptr && !grouped && !p.records;
-    c->result_ext = false;
-    for (int attempt = 0; attempt < 6; attempt++) {
-        int rc = ensure_query_buffers(c, p, entry_cap, use_ext ? 1 : out_cap, task_cap, nsc, grouped, st);
+    // pairs go straight to the caller's buffer when one is set; a result that
+    // does not fit is redone into the context's buffer
+    bool use_ext = c->ext_out != nullptr && !p.records;
+    rc = kAgain;
+    for (int attempt = 0; attempt < 6 && rc == kAgain; attempt++) {
+        if ((rc = grid_room())) return rc;
+        rc = ensure_query_buffers(c, p, need.entries, use_ext ? 1 : need.out, need.tasks, p.nscenes, false, st);
         if (rc) return rc;
         if (use_ext) {
             p.out = c->ext_out;
             p.out_cap = c->ext_cap;
         }
-        if (attempt == 0) CK(cudaEventRecord(c->ev0, st));
-        {
-            const cudaError_t re = record_pipeline(c, p, dims, grouped, nsc, need_full, st);
-            if (re != cudaSuccess)
-                return fail(PBIG2_ECUDA, "pipeline launch (engine.cu:%d): %s", g_record_line, cudaGetErrorString(re));
-        }
-        launches += need_full ? 6 : 0;  // count, scan (3), expand, scatter
-        launches += 3 + (grouped ? 3 : 0) + (p.records ? 1 : 0) + (need_full && p.scene_table ? 1 : 0);
-        CK(cudaMemcpyAsync(c->h_ctr.p, p.ctr, sizeof(Ctr), cudaMemcpyDeviceToHost, st));
-        cudaError_t e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) {
-            return fail(PBIG2_ECUDA, "pipeline failed: %s", cudaGetErrorString(e));
-        }
-        memcpy(&h, c->h_ctr.p, sizeof(Ctr));
-        if (h.err & kErrWait) {
-            return fail(PBIG2_ETIMEOUT, "a bounded device wait gave up (scan bulk copy)");
-        }
-        if (h.err & kErrRecCell)
-            return fail(PBIG2_ECAPACITY, "a cell of 65536 boxes or more cannot be written as records");
-        if (h.err & kErrIndex) {
-            return fail(PBIG2_ECUDA, "inconsistent cell lists (error bits 0x%x)", h.err);
-        }
-        if ((h.err & kErrEntryOvf) || h.entries > p.entry_cap) {
-            if (h.entries >= (1ull << 32))
-                return fail(PBIG2_ENOMEM, "%llu cell entries exceed the 2^32 limit of one query",
-                            (unsigned long long)h.entries);
-            entry_cap = h.entries + h.entries / 16 + 4096;
-            need_full = true;
-            continue;
-        }
-        if (h.err & kErrTaskOvf) {
-            task_cap = (uint64_t)h.need_tasks + 1024;
-            need_full = true;
-            continue;
-        }
-        if ((h.err & kErrOutOvf) || h.pairs > p.out_cap) {
-            out_cap = std::max<uint64_t>(out_cap, h.pairs + h.pairs / 8 + 1024);
-            use_ext = false;
-            need_full = false;
-            continue;
-        }
-        break;
+        rc = run_pass(c, p, q.dims, false, p.nscenes, need.full, &ta, st, h);
+        if (rc) return rc;
+        launches += (need.full ? 6 : 0) + 3 + (p.records ? 1 : 0);  // tuner, count (2), scan (2), scatter; pairs (3)
+        rc = check_pass(p, h, need);
+        if (rc == kAgain && !need.full) use_ext = false;
     }
+    if (rc == kAgain) return fail(PBIG2_ENOMEM, "capacity retries exhausted");
+    if (rc) return rc;
     c->result_ext = use_ext;
-    if (h.err & (kErrEntryOvf | kErrTaskOvf | kErrOutOvf)) return fail(PBIG2_ENOMEM, "capacity retries exhausted");
     c->out_hint = std::max<uint64_t>(c->out_hint, h.pairs + h.pairs / 8);
-    int rc = finish_query(c, h, nboxes, ncells, nsc, scenes, grouped, launches, st);
+    std::vector<GridScene> sc{{0, q.n, h.shift, 0}};
+    if (q.bip) sc.push_back({q.n_red, q.n - q.n_red, h.shift, 0});
+    *used = h.shift;
+    rc = finish_query(c, h, q.n, h.cells, p.nscenes, sc, false, launches, st);
     c->stats.class_map = p.class_map;
-    if (rc != PBIG2_OK && rc != PBIG2_EINPUT) return rc;
-    // capture this query's pipeline for later batches of the same shape
-    if (G.exec && G.buffers != c->buffers_sig()) c->drop_graph();
-    if (c->use_graph && grouped && !G.exec) {
-        int rg = capture_graph(c, p, d_boxes, nboxes, ncells, nsc, dims, range, split, entry_cap, st);
-        if (rg) return rg;
-    }
     return rc;
 }
 
@@ -817,7 +929,7 @@ static int fused_query(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t n, int di
     c->out_hint = std::max<uint64_t>(c->out_hint, h.pairs + h.pairs / 8);
     c->merged_blocks = 0;
     std::vector<GridScene> sc{{0, n, h.shift, 0}};
-    rc = finish_query(c, h, n, h.cells, 1, sc, false, 1, st, false);
+    rc = finish_query(c, h, n, h.cells, 1, sc, false, 1, st);
     c->stats.class_map = p.class_map;
     c->stats.device_ms = h.t_end > h.t_start ? (double)(h.t_end - h.t_start) * 1e-6 : 0.0;  // the kernel's own clock
     return rc;
@@ -825,21 +937,6 @@ static int fused_query(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t n, int di
 
 static cudaStream_t pick_stream(pbig2_ctx* c, void* stream) {
     return stream ? (cudaStream_t)stream : c->own_stream;
-}
-
-// strided sample of device-resident boxes (host copy) for the autotuner
-static int sample_device_boxes(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t n, int dims, uint64_t m,
-                               cudaStream_t st, std::vector<uint32_t>& out) {
-    const int W = 2 * dims + 1;
-    m = std::min<uint64_t>(m, n);
-    out.resize(m * W);
-    if (m == 0) return PBIG2_OK;
-    CK(c->h_stage.ensure(m * W * 4));
-    const uint64_t stride = n / m;
-    CK(cudaMemcpy2DAsync(c->h_stage.p, W * 4, d_boxes, stride * W * 4, W * 4, m, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    memcpy(out.data(), c->h_stage.p, m * W * 4);
-    return PBIG2_OK;
 }
 
 // device-mapped address of page-locked host memory, or null (pageable memory)
@@ -885,9 +982,6 @@ PBIG2_API int pbig2_create(int device, pbig2_ctx** out) {
     c->device = device;
     cudaError_t e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
-    if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
-    for (int k = 0; k < 9 && e == cudaSuccess; k++) e = cudaEventCreate(&c->evp[k]);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming);
@@ -908,14 +1002,10 @@ PBIG2_API int pbig2_destroy(pbig2_ctx* c) {
     for (DevBuf* b : {&c->d_boxes, &c->d_counts, &c->d_entries, &c->d_recs, &c->d_merged, &c->d_merged_ext, &c->d_bar, &c->d_fctr,
                       &c->d_lists, &c->d_tasks, &c->d_state,
                       &c->d_out, &c->d_out2, &c->d_ctr, &c->d_scenes, &c->d_scene_off, &c->d_scene_pair,
-                      &c->d_scene_cursor, &c->d_dims, &c->d_scene_tab, &c->d_tune})
+                      &c->d_scene_cursor, &c->d_dims, &c->d_scene_tab, &c->d_tune, &c->d_tune_cost})
         b->release();
     c->h_ctr.release();
     c->h_stage.release();
-    if (c->ev0) cudaEventDestroy(c->ev0);
-    if (c->ev1) cudaEventDestroy(c->ev1);
-    for (cudaEvent_t ev : c->evp)
-        if (ev) cudaEventDestroy(ev);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
     if (c->side_stream) cudaStreamDestroy(c->side_stream);
@@ -941,47 +1031,6 @@ PBIG2_API int pbig2_tune_shift(const uint32_t* boxes, uint64_t n, uint32_t dims,
     return PBIG2_OK;
 }
 
-// autotuner with a per-context memo: a query whose size, dims, range and
-// mean box extent (over 256 strided boxes) match an earlier one within 5%
-// reuses that choice
-constexpr uint64_t kMemoRows = 256;
-
-static double mean_extent(const uint32_t* boxes, uint64_t n_avail, int dims) {
-    const int W = 2 * dims + 1;
-    const uint64_t m = std::min<uint64_t>(n_avail, kMemoRows);
-    double ext = 0;
-    for (uint64_t i = 0; i < m; i++) {
-        const uint32_t* b = boxes + (uint64_t)((unsigned __int128)i * n_avail / m) * W;
-        for (int d = 0; d < dims; d++) ext += (double)b[2 * d + 1] - (double)b[2 * d];
-    }
-    return m ? ext / (double)(m * dims) : 0;
-}
-
-static bool memo_find(pbig2_ctx* c, uint64_t n, int dims, uint32_t range, double ext, TuneResult& tr) {
-    for (const auto& e : c->memo)
-        if (e.dims == dims && e.range == range && std::fabs((double)e.n - (double)n) <= 0.05 * (double)n &&
-            std::fabs(e.ext - ext) <= 0.05 * std::max(1.0, e.ext)) {
-            tr = TuneResult{e.shift, e.est_e * (double)n / std::max(1.0, (double)e.n), 0, 0};
-            return true;
-        }
-    return false;
-}
-
-static void memo_put(pbig2_ctx* c, uint64_t n, int dims, uint32_t range, double ext, const TuneResult& tr) {
-    if (c->memo.size() >= 64) c->memo.erase(c->memo.begin());
-    c->memo.push_back({n, dims, range, ext, tr.shift, tr.est_entries});
-}
-
-static TuneResult memo_tune(pbig2_ctx* c, const uint32_t* boxes, uint64_t n_avail, uint64_t n, int dims,
-                            uint32_t range, uint64_t sample) {
-    const double ext = mean_extent(boxes, n_avail, dims);
-    TuneResult tr{};
-    if (memo_find(c, n, dims, range, ext, tr)) return tr;
-    tr = tune_shift_sample(boxes, n_avail, n, dims, range, sample);
-    memo_put(c, n, dims, range, ext, tr);
-    return tr;
-}
-
 // A box outside the tuner's sample can cover 2^26 cells or more at the cell
 // size chosen from the sample; the count kernel then skips it as an input
 // error (kErrCellOvf). A query whose cell sizes were chosen automatically is
@@ -990,10 +1039,16 @@ static bool coarser_grid_helps(const pbig2_ctx* c, int rc) {
     return rc == PBIG2_EINPUT && (c->last_err & kErrCellOvf) != 0;
 }
 
-// later queries of a remembered scene start at the cell size that fitted
-static void memo_raise(pbig2_ctx* c, uint64_t n, int dims, uint32_t range, uint32_t from, uint32_t to) {
-    for (auto& e : c->memo)
-        if (e.n == n && e.dims == dims && e.range == range && e.shift == from) e.shift = to;
+// later queries of this size that choose the same cell size start at the one that fitted
+static void remember_raise(pbig2_ctx* c, uint64_t n, int dims, uint32_t range, uint32_t from, uint32_t to) {
+    for (auto& r : c->raised)
+        if (r.n == n && r.dims == dims && r.range == range) {
+            r.from = from;
+            r.to = to;
+            return;
+        }
+    if (c->raised.size() >= 64) c->raised.erase(c->raised.begin());
+    c->raised.push_back({n, dims, range, from, to});
 }
 
 static int self_or_bip(pbig2_ctx* c, const uint32_t* red, uint64_t n_red, const uint32_t* blue, uint64_t n_blue,
@@ -1036,65 +1091,16 @@ static int self_or_bip(pbig2_ctx* c, const uint32_t* red, uint64_t n_red, const 
         if (n_blue) CK(cudaMemcpyAsync(c->d_boxes.as<uint32_t>() + n_red * W, blue, n_blue * W * 4, k, st));
         d_boxes = c->d_boxes.as<uint32_t>();
     }
-    // choose the cell size (from a sample of the union for red/blue)
-    TuneResult tr{};
-    std::vector<uint32_t> smp;
-    const uint64_t kSample = 4096;
-    if (cell_shift != PBIG2_AUTO) {
-        tr.shift = cell_shift;
-    } else if (loc == PBIG2_HOST && !bip) {
-        tr = memo_tune(c, red, n, n, (int)dims, range, kSample);
-    } else {
-        if (loc == PBIG2_HOST) {
-            const uint64_t m = std::min<uint64_t>(n, kSample);
-            smp.resize(m * W);
-            for (uint64_t i = 0; i < m; i++) {
-                const uint64_t g = (uint64_t)((unsigned __int128)i * n / m);
-                const uint32_t* src = g < n_red ? red + g * W : blue + (g - n_red) * W;
-                memcpy(&smp[i * W], src, W * 4);
-            }
-            tr = memo_tune(c, smp.data(), smp.size() / W, n, (int)dims, range, kSample);
-        } else {
-            // device-resident boxes: 256 rows recognise a remembered scene;
-            // the full sample crosses to the host only when none matches
-            int rc = sample_device_boxes(c, d_boxes, n, (int)dims, kMemoRows, st, smp);
-            if (rc) return rc;
-            const double ext = mean_extent(smp.data(), smp.size() / W, (int)dims);
-            if (!memo_find(c, n, (int)dims, range, ext, tr)) {
-                rc = sample_device_boxes(c, d_boxes, n, (int)dims, kSample, st, smp);
-                if (rc) return rc;
-                tr = tune_shift_sample(smp.data(), smp.size() / W, n, (int)dims, range, kSample);
-                memo_put(c, n, (int)dims, range, ext, tr);
-            }
-        }
-    }
-    std::vector<GridScene> sc;
-    if (!bip) {
-        sc.push_back({0, n, tr.shift, 0});
-    } else {
-        sc.push_back({0, n_red, tr.shift, 0});
-        sc.push_back({n_red, n_blue, tr.shift, 0});
-    }
-    if (fused) {
-        c->up_red = m_red;
-        c->up_blue = m_blue;
-        c->up_split = n_red;
-    }
-    int rc = run_pipeline(c, d_boxes, n, (int)dims, range, sc, bip ? (uint32_t)n_red : kNoSplit,
-                          std::max(tr.est_entries, (double)n), st, false);
+    const SingleScene q{d_boxes, fused ? m_red : nullptr, fused ? m_blue : nullptr, n_red, n, bip, (int)dims, range};
+    uint32_t shift = cell_shift;
+    int rc = run_single(c, q, cell_shift, st, &shift);
     if (cell_shift == PBIG2_AUTO && coarser_grid_helps(c, rc)) {
-        const uint32_t first = tr.shift;
-        while (coarser_grid_helps(c, rc) && tr.shift < 31) {
-            tr.shift++;
-            for (auto& g : sc) g.shift = tr.shift;
-            rc = run_pipeline(c, d_boxes, n, (int)dims, range, sc, bip ? (uint32_t)n_red : kNoSplit,
-                              std::max(tr.est_entries, (double)n), st, false);
-        }
-        memo_raise(c, n, (int)dims, range, first, tr.shift);
-        c->stats.grid_retries = tr.shift - first;
+        const uint32_t first = shift;
+        while (coarser_grid_helps(c, rc) && shift < 31) rc = run_single(c, q, shift + 1, st, &shift);
+        remember_raise(c, n, (int)dims, range, first, shift);
+        c->stats.grid_retries = shift - first;
     }
-    c->up_red = c->up_blue = nullptr;
-    c->scene_shifts.assign(1, tr.shift);
+    c->scene_shifts.assign(1, shift);
     *npairs = c->npairs;
     return rc;
 }
@@ -1163,7 +1169,13 @@ PBIG2_API int pbig2_batch_intersect(pbig2_ctx* c, const uint32_t* boxes, const u
         sc[i] = GridScene{a, ns, shift, (int)i};
         est_e += e;
     }
-    rc = run_pipeline(c, d_boxes, n, (int)dims, range, sc, kNoSplit, est_e, st, true);
+    // (a batch of one scene is a query of that scene)
+    const auto run = [&]() {
+        uint32_t used = 0;
+        if (n_scenes > 1) return run_batch(c, d_boxes, n, (int)dims, range, sc, est_e, st);
+        return run_single(c, SingleScene{d_boxes, nullptr, nullptr, n, n, false, (int)dims, range}, sc[0].shift, st, &used);
+    };
+    rc = run();
     // automatic cell sizes: coarser grids for every scene while a box does
     // not fit (the failing scene is not known)
     uint32_t retries = 0;
@@ -1175,7 +1187,7 @@ PBIG2_API int pbig2_batch_intersect(pbig2_ctx* c, const uint32_t* boxes, const u
                 raised = true;
             }
         if (!raised) break;
-        rc = run_pipeline(c, d_boxes, n, (int)dims, range, sc, kNoSplit, est_e, st, true);
+        rc = run();
         retries++;
     }
     c->stats.grid_retries = retries;

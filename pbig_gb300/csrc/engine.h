@@ -50,8 +50,6 @@ struct pbig2_ctx {
     int device = 0;
     int sm_count = 0;
     cudaStream_t own_stream = nullptr;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    cudaEvent_t evp[9] = {};
     pbig::DevBuf d_merged, d_merged_ext;  // merged mode: cell -> root table; the roots' extents
     pbig::DevBuf d_recs;    // record mode: box index of every entry
     bool merged_mode = false;
@@ -62,7 +60,7 @@ struct pbig2_ctx {
     uint32_t merged_blocks = 0;  // merged blocks of the last query
     uint32_t last_err = 0;       // error bits of the last pipeline pass
     pbig::DevBuf d_boxes, d_counts, d_entries, d_lists, d_tasks, d_state, d_out, d_out2, d_ctr,
-        d_scenes, d_scene_off, d_scene_pair, d_scene_cursor, d_dims, d_scene_tab, d_tune;
+        d_scenes, d_scene_off, d_scene_pair, d_scene_cursor, d_dims, d_scene_tab, d_tune, d_tune_cost;
     pbig::HostPinned h_ctr, h_stage;
     // caller's pair buffer for self/bipartite queries (pbig2_set_pair_output)
     uint2* ext_out = nullptr;
@@ -72,11 +70,6 @@ struct pbig2_ctx {
     // the medium-cell kernel (PBIG2_OPT_HOST_SPLIT; 0 = automatic, < 0 = off)
     int host_split = 0;
     cudaStream_t side_stream = nullptr;
-    // page-locked host input of the running query, uploaded by the count
-    // kernel (device-mapped addresses; null: the boxes are on the device)
-    const uint32_t* up_red = nullptr;
-    const uint32_t* up_blue = nullptr;
-    uint64_t up_split = 0;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     bool result_ext = false;  // the last result went to ext_out
     // last result
@@ -124,7 +117,8 @@ struct pbig2_ctx {
     // work-list class map of later queries (PBIG2_OPT_CLASS_MAP; 0: automatic)
     unsigned long long class_map = 0;
     uint32_t merge_limit = 256;  // merged mode's block limit (PBIG2_OPT_MERGE_LIMIT)
-    // autotuner memo: (n, dims, range, mean extent) -> shift
-    struct TuneMemo { uint64_t n; int dims; uint32_t range; double ext; uint32_t shift; double est_e; };
-    std::vector<TuneMemo> memo;
+    // scenes whose automatic cell size had to be raised (a box outside the
+    // tuner's sample did not fit): a choice of `from` becomes `to`
+    struct Raised { uint64_t n; int dims; uint32_t range, from, to; };
+    std::vector<Raised> raised;
 };

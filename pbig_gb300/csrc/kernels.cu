@@ -3,8 +3,8 @@
 //   k_count    boxes -> per-cell counts                (src/pbig/pbig.cu:174-221)
 //   k_scan     counts -> cell starts + cell work lists (host thrust scan, pbig.cu:1497-1505,
 //              and the job list of sched_phase, pbig.cu:1586-1688)
-//   k_expand   tile tasks for cells too big for shared memory (sched_phase's 256-row jobs)
-//   k_scatter  boxes -> cell entry lists               (d_mapping, pbig.cu:321-427)
+//   k_scatter  boxes -> cell entry lists               (d_mapping, pbig.cu:321-427), and tile tasks
+//              for cells too big for shared memory     (sched_phase's 256-row jobs)
 //   k_pairs    per-cell all-pairs test with the reference-cell rule and compacted output
 //              (d_matching + prefix_scan, pbig.cu:429-543, 562-603, 641-932)
 //
@@ -53,9 +53,55 @@ __device__ __forceinline__ Params resolve(const Params& in) {
         p.nboxes = p.dyn->nboxes;
         p.ncells = p.dyn->ncells;
         p.nscenes = p.dyn->nscenes;
+        p.open |= p.dyn->open;
     }
     return p;
 }
+
+__device__ __forceinline__ unsigned long long now_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// the query's clock: a kernel's first block notes when it starts
+__device__ __forceinline__ void stamp(const Params& p, int k) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.ctr->stamp[k] = now_ns();
+}
+
+// the run counters to page-locked host memory (one thread; the counters were
+// changed through L2 by other blocks)
+__device__ __forceinline__ void ctr_to_host(const Ctr* ctr, Ctr* host) {
+    constexpr uint32_t kWords = sizeof(Ctr) / sizeof(unsigned long long);
+    static_assert(sizeof(Ctr) % sizeof(unsigned long long) == 0, "run counters in 8-byte words");
+    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(ctr);
+    unsigned long long* dst = reinterpret_cast<unsigned long long*>(host);
+    unsigned long long w[kWords];
+#pragma unroll
+    for (uint32_t k = 0; k < kWords; k++) w[k] = __ldcg(src + k);
+#pragma unroll
+    for (uint32_t k = 0; k < kWords; k++) dst[k] = w[k];
+    __threadfence_system();
+}
+
+// at the end of a query's last kernel (p.ctr_host set): its last block to
+// finish hands the run counters to the host, so no copy follows the kernel
+__device__ __forceinline__ void query_end(const Params& p) {
+    if (!p.ctr_host) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&p.ctr->done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            p.ctr->stamp[kStampEnd] = now_ns();
+            __threadfence();
+            ctr_to_host(p.ctr, p.ctr_host);
+        }
+    }
+}
+
+// (where the last two kernels run beside each other)
+__global__ void k_query_end(Params p) { query_end(p); }
 
 // the last scene s in [lo, hi) with scene_box_off[s] <= gi
 __device__ __forceinline__ uint32_t search_scene(const Params& p, uint64_t gi, uint32_t lo, uint32_t hi) {
@@ -190,6 +236,260 @@ __global__ void k_tune_scenes(const uint32_t* boxes, const unsigned long long* o
         const SceneTune best = tune_scene_warp(boxes, a, offs[sc + 1] > a ? offs[sc + 1] - a : 0, dims, range, 4.0e9);
         if (lane_id() == 0) out[sc] = best;
     }
+}
+
+// ---------------------------------------------------------------------------
+// the cell size of a single-scene query: block b of kTuneBlocks weighs the
+// candidate s0 - 2 + b (s0 = log2 of the sample's mean extent) with the cost
+// model on a strided sample: C cells, E entries, and T tests. A cell holds
+// about E/m entries for every box whose lower corner lies in it (m boxes in
+// the sample), so T is (E/m)^2 times the pairs of sampled corners that share a
+// cell (counted in a shared-memory hash table), times (n/m)^2, since a pair
+// survives sampling with probability (m/n)^2. The last block to finish takes
+// the cheapest, the finest on a tie, or, when none qualifies, weighs every
+// coarser size itself. It then writes the query's tables.
+//
+// Latency is all that counts here, so one thread does the arithmetic in double
+// precision (its rate is a sixty-fourth: 30 us with every thread at it) and
+// the others count in integers. Counting every cell of the sampled boxes
+// took 40 us when they were dealt out evenly over the threads, and 115 to 300
+// us with a thread per box, which waited for its largest. On the host the
+// sample's way there and back took 20 us or more, and a scene not seen before
+// two milliseconds of hashing; scenes were recognised by size and mean extent,
+// and one taken for another could run at a cell size that made it ten times
+// slower.
+// ---------------------------------------------------------------------------
+constexpr int kTuneThreads = 1024;
+constexpr uint32_t kTuneBlocks = 8;          // s0 - 2 .. s0 + 5
+constexpr uint32_t kTuneSlots = 8192;        // hash table {cell + 1, corners}, twice the sample
+constexpr int kTunePer = (int)(kTuneSample / kTuneThreads);
+constexpr size_t kTuneSmem = kTuneSlots * 2 * sizeof(uint32_t);
+static_assert(kTuneSlots == 2 * kTuneSample && kTuneThreads == 1024, "tuner table and sums");
+static_assert((1 + 2 * kTuneBlocks) * sizeof(unsigned long long) <= kTuneScratchBytes, "tuner scratch");
+
+// a box's coordinates, wherever its row begins, in two or three 16-byte loads
+// (every row is a line or two of its own, and each load instruction looks all
+// of a warp's lines up: with a load per word the sample alone took 12 us). The
+// loads cover aligned 16 bytes that hold at least a byte of the row, so they
+// stay in its memory page.
+template <int D>
+__device__ __forceinline__ void load_row(const uint32_t* b, uint32_t (&v)[2 * D]) {
+    const uint32_t o = (uint32_t)(reinterpret_cast<uintptr_t>(b) >> 2) & 3u;
+    const uint4* q = reinterpret_cast<const uint4*>(b - o);
+    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+    const uint4 q0 = __ldg(q), q1 = o + 2 * D > 4 ? __ldg(q + 1) : z, q2 = o + 2 * D > 8 ? __ldg(q + 2) : z;
+    uint32_t w[11] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, q2.y, q2.z};
+    if (o & 1u) {
+#pragma unroll
+        for (int k = 0; k < 10; k++) w[k] = w[k + 1];
+    }
+#pragma unroll
+    for (int k = 0; k < 2 * D; k++) v[k] = o & 2u ? w[k + 2] : w[k];
+}
+
+struct TuneShared {
+    uint32_t part[2][kTuneThreads / 32];
+    int s0;
+    uint32_t state;  // the last block: a size was found; another block: not the last
+};
+
+// two sums over the block, each below 2^32 (every thread gets them)
+__device__ __forceinline__ uint2 block_sums(TuneShared& s, uint32_t x, uint32_t y) {
+    x = __reduce_add_sync(FULL_MASK, x);
+    y = __reduce_add_sync(FULL_MASK, y);
+    __syncthreads();
+    if (lane_id() == 0) {
+        s.part[0][threadIdx.x >> 5] = x;
+        s.part[1][threadIdx.x >> 5] = y;
+    }
+    __syncthreads();
+    return make_uint2(__reduce_add_sync(FULL_MASK, s.part[0][lane_id()]),
+                      __reduce_add_sync(FULL_MASK, s.part[1][lane_id()]));
+}
+
+// cells of the grid at shift sh, ~0 for 2^32 per two axes or more (beyond every limit here)
+template <int D>
+__device__ __forceinline__ uint64_t tune_grid(uint32_t range, uint32_t sh) {
+    const uint64_t nrc = nrc_dev(range, (int)sh);
+    return nrc >= 65536ull ? ~0ull : D == 3 ? nrc * nrc * nrc : nrc * nrc;
+}
+
+// what the cost of cell shift sh takes: the sample's entries and pairs of
+// corners in a cell; false when the size does not qualify (block-uniform)
+template <int D>
+__device__ bool tune_weigh(TuneShared& s, uint32_t* key, const uint32_t (&lo)[kTunePer][D],
+                           const uint32_t (&hi)[kTunePer][D], const bool (&ok)[kTunePer], uint32_t m, uint32_t range,
+                           uint32_t sh, uint64_t max_cells, uint32_t& entries, uint32_t& pairs) {
+    const uint32_t t = threadIdx.x, nrc = nrc_dev(range, (int)sh);
+    if (tune_grid<D>(range, sh) > max_cells) return false;
+    uint32_t e = 0, huge = 0;
+#pragma unroll
+    for (int j = 0; j < kTunePer; j++) {
+        if (!ok[j]) continue;
+        unsigned long long c = 1;
+#pragma unroll
+        for (int d = 0; d < D; d++) {
+            const unsigned long long k = (hi[j][d] >> sh) - (lo[j][d] >> sh) + 1;
+            c = c >= (1ull << 26) ? c : c * k;
+        }
+        huge |= c >= (1ull << 26) ? 1u : 0u;
+        e += (uint32_t)(c < (1ull << 19) ? c : (1ull << 19));  // (2^18 over the sample is too many)
+    }
+    const uint2 sums = block_sums(s, e, huge);
+    entries = sums.x;
+    if (sums.y || entries > 64u * m) return false;  // a box that would not fit; too many entries per box
+    uint32_t* cnt = key + kTuneSlots;
+    for (uint32_t i = t; i < kTuneSlots / 2; i += kTuneThreads) reinterpret_cast<uint4*>(key)[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    uint32_t found = 0;  // < 2^23
+#pragma unroll
+    for (int j = 0; j < kTunePer; j++) {
+        if (!ok[j]) continue;
+        const uint32_t z = D == 3 ? lo[j][D - 1] >> sh : 0u;
+        const uint32_t id = (z * nrc + (lo[j][1] >> sh)) * nrc + (lo[j][0] >> sh) + 1u;  // (C < 2^32)
+        uint32_t h = (id * 0x9e3779b1u) >> 19;
+        for (uint32_t probe = 0; probe < kTuneSlots; probe++, h = (h + 1) & (kTuneSlots - 1)) {
+            const uint32_t old = atomicCAS(&key[h], 0u, id);
+            if (old != 0u && old != id) continue;
+            found += atomicAdd(&cnt[h], 1u);  // a new member pairs with every earlier one
+            break;
+        }
+    }
+    static_assert(kTuneSlots == 1u << 13, "13 bits of the hash");
+    pairs = block_sums(s, found, 0u).x;
+    return true;
+}
+
+// the cost model (one thread): C cells, the sample's counts, m of n boxes. Of
+// a red/blue query's tests those of one colour are left out.
+__device__ double tune_cost_query(uint64_t C, uint32_t entries, uint32_t pairs, uint32_t m, uint64_t n, bool bip, double& E) {
+    const double per_box = (double)entries / (double)m, f = per_box * ((double)n / (double)m);
+    E = per_box * (double)n;
+    return kQueryCell * (double)C + kQueryEntry * E + (bip ? 0.5 : 1.0) * kQueryTest * ((double)pairs * f * f);
+}
+
+template <int D>
+__global__ void __launch_bounds__(kTuneThreads, 1) k_tune_query(Params p, TuneArgs a) {
+    extern __shared__ __align__(16) uint32_t table[];
+    __shared__ TuneShared s;
+    constexpr uint32_t W = 2 * D + 1;
+    const uint32_t t = threadIdx.x;
+    const unsigned long long began = now_ns();
+    uint32_t shift = a.shift;
+    double est = (double)a.n;
+    if (a.shift == kTuneShift) {
+        const uint32_t m = (uint32_t)mn64(a.n, kTuneSample);
+        uint32_t lo[kTunePer][D], hi[kTunePer][D];
+        bool ok[kTunePer];
+        unsigned long long ext = 0;
+        uint32_t good = 0;
+#pragma unroll
+        for (int j = 0; j < kTunePer; j++) {
+            const uint32_t k = t + (uint32_t)j * kTuneThreads;
+            ok[j] = k < m;
+            static_assert(kTuneSample == 1u << 12, "row k * n / m of a full sample");
+            const uint64_t g = !ok[j] ? 0ull : a.n > kTuneSample ? (uint64_t)k * a.n >> 12 : k;
+            const uint32_t* b = g < a.n_red ? a.red + g * W : a.blue + (g - a.n_red) * W;
+            uint32_t v[2 * D] = {};
+            if (ok[j]) load_row<D>(b, v);
+#pragma unroll
+            for (int d = 0; d < D; d++) {
+                lo[j][d] = v[2 * d];
+                hi[j][d] = v[2 * d + 1];
+            }
+#pragma unroll
+            for (int d = 0; d < D; d++) ok[j] = ok[j] && lo[j][d] <= hi[j][d] && hi[j][d] < a.range;
+            if (ok[j]) {
+#pragma unroll
+                for (int d = 0; d < D; d++) ext += (unsigned long long)(hi[j][d] - lo[j][d]) + 1;
+                good++;
+            }
+        }
+        // (ext: up to 2^46 over the block, in three sums)
+        const uint2 lo_mid = block_sums(s, (uint32_t)ext & 0xffffu, (uint32_t)(ext >> 16) & 0xffffu);
+        const uint2 top = block_sums(s, (uint32_t)(ext >> 32), good);
+        ext = ((unsigned long long)top.x << 32) + ((unsigned long long)lo_mid.y << 16) + lo_mid.x;
+        if (t == 0) {
+            const unsigned long long mean = ext / ((top.y ? top.y : 1u) * (unsigned long long)D);
+            s.s0 = mean < 2ull ? 0 : 63 - __clzll((long long)mean);
+        }
+        __syncthreads();
+        const int s0 = s.s0, s_lo = s0 - 2 > 0 ? s0 - 2 : 0, s_win = s0 + 3 < 31 ? s0 + 3 : 31;
+        const int mine = s_lo + (int)blockIdx.x;
+        uint32_t e = 0, pairs = 0;
+        // s0 + 4 and s0 + 5 (of boxes of two sizes the mean says little) where s0 + 3
+        // makes at most 64 cells a box; scenes sparser than that in their range stay
+        // with s0 + 3 at most
+        const int s_far = tune_grid<D>(a.range, (uint32_t)s_win) <= 64 * a.n ? (s0 + 5 < 31 ? s0 + 5 : 31) : s_win;
+        const bool fits = m > 0 && mine <= s_far &&
+                          tune_weigh<D>(s, table, lo, hi, ok, m, a.range, (uint32_t)mine, a.max_cells, e, pairs);
+        double best = 1e300, E = 0.0;  // (thread 0)
+        if (t == 0) {
+            const double cost = fits ? tune_cost_query(tune_grid<D>(a.range, (uint32_t)mine), e, pairs, m, a.n, a.bip, E) : 1e300;
+            a.scratch[1 + 2 * blockIdx.x] = (unsigned long long)__double_as_longlong(cost);
+            a.scratch[2 + 2 * blockIdx.x] = (unsigned long long)__double_as_longlong(E);
+            __threadfence();
+            const bool last = atomicAdd(a.scratch, 1ull) == gridDim.x - 1;
+            if (last) {
+                __threadfence();
+                for (uint32_t b = 0; b < gridDim.x; b++) {
+                    const double c = __longlong_as_double((long long)__ldcg(a.scratch + 1 + 2 * b));
+                    if (c < best) {
+                        best = c;
+                        shift = (uint32_t)s_lo + b;
+                        est = __longlong_as_double((long long)__ldcg(a.scratch + 2 + 2 * b));
+                    }
+                }
+            }
+            s.state = !last || best < 1e300 ? 1u : 0u;
+        }
+        __syncthreads();
+        if (s.state == 0u) {
+            // a few huge boxes in the sample can disqualify all of those: every
+            // coarser size, on grids in proportion to the boxes
+            const uint64_t far = mn64(a.max_cells, a.n * 64 > 4096 ? a.n * 64 : 4096);
+            for (int w = s_win + 1; w <= 31 && m > 0; w++) {
+                const bool qualifies = tune_weigh<D>(s, table, lo, hi, ok, m, a.range, (uint32_t)w, far, e, pairs);
+                if (t == 0 && qualifies) {
+                    const double cost = tune_cost_query(tune_grid<D>(a.range, (uint32_t)w), e, pairs, m, a.n, a.bip, E);
+                    if (cost < best) {
+                        best = cost;
+                        shift = (uint32_t)w;
+                        est = E;
+                    }
+                }
+                __syncthreads();
+            }
+            if (t == 0 && best == 1e300) {  // the coarsest grid that is not a single cell
+                shift = 31;
+                while (shift > 0 && nrc_dev(a.range, (int)shift - 1) <= 1) shift--;
+                est = (double)a.n;
+            }
+        }
+        if (t != 0 || shift == kTuneShift) return;  // (another block writes the tables)
+        if (shift == a.raise_from) shift = a.raise_to;
+    }
+    if (t != 0) return;
+    if (a.shift == kTuneShift) a.scratch[0] = 0;
+    const uint32_t nrc = nrc_dev(a.range, (int)shift);
+    const uint64_t C = D == 3 ? (uint64_t)nrc * nrc * nrc : (uint64_t)nrc * nrc;
+    const uint32_t n_scenes = a.bip ? 2u : 1u;
+    a.scenes[0] = Scene{0u, (uint32_t)(a.bip ? a.n_red : a.n), shift, nrc, 0ull, a.range, 0u};
+    a.box_off[0] = 0u;
+    a.box_off[n_scenes] = (uint32_t)a.n;
+    if (a.bip) {
+        a.scenes[1] = Scene{(uint32_t)a.n_red, (uint32_t)(a.n - a.n_red), shift, nrc, 0ull, a.range, 0u};
+        a.box_off[1] = (uint32_t)a.n_red;
+    }
+    const bool room = C <= a.room_cells;
+    *a.dims = RunDims{room ? a.n : 0ull, room ? C : 0ull, n_scenes, shift >= kOpenShift ? 1u : 0u};
+    Ctr c{};
+    if (!room) c.err = kErrGridRoom;
+    c.cells = C;
+    c.shift = shift;
+    c.est_entries = (unsigned long long)fmin(est, 1e18);
+    c.stamp[kStampStart] = began;
+    *p.ctr = c;
 }
 
 // ---------------------------------------------------------------------------
@@ -430,14 +730,22 @@ __device__ __forceinline__ void enumerate_cells(const Params& p, uint32_t* sbox,
     }
 }
 
-// counts = 0 before a pass (the scatter leaves every cell's start there)
+// counts = 0 before a pass (the scatter leaves every cell's start there), and
+// the scan's tile records
 __global__ void k_zero_counts(Params pin) {
     const Params p = resolve(pin);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        p.ctr->stamp[kStampCount] = now_ns();
+        if (p.ctr->stamp[kStampStart] == 0ull) p.ctr->stamp[kStampStart] = p.ctr->stamp[kStampCount];
+    }
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t n4 = p.ncells / 4;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     uint4* c4 = reinterpret_cast<uint4*>(p.counts);
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) c4[i] = make_uint4(0, 0, 0, 0);
-    for (uint64_t i = 4 * n4 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.ncells; i += stride) p.counts[i] = 0;
+    for (uint64_t i = t; i < n4; i += stride) c4[i] = make_uint4(0, 0, 0, 0);
+    for (uint64_t i = 4 * n4 + t; i < p.ncells; i += stride) p.counts[i] = 0;
+    const uint64_t r4 = scan_tiles(p.ncells) * (kTileRecBytes / 16);
+    uint4* s4 = reinterpret_cast<uint4*>(p.tile_state);
+    for (uint64_t i = t; i < r4; i += stride) s4[i] = make_uint4(0, 0, 0, 0);
 }
 
 // tiles of TILE boxes: blk, blk + nblk, ... (blockDim.x == TILE)
@@ -459,9 +767,44 @@ __global__ void __launch_bounds__(kBoxThreads) k_count(Params pin) {
     box_pass<D, false, MERGED>(resolve(pin), sbox, blockIdx.x, gridDim.x);
 }
 
+// ---------------------------------------------------------------------------
+// expand: cells larger than kBigMax get tile tasks {cell, row tile r, column
+// tiles [x0,x1)} with 32-box tiles, x >= r, at most 8 column tiles a task.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kTaskCols = 8;
+
+// a run counter that a pass reads: FRESH (one-launch queries, where phases
+// of the same kernel change the counters) reads it past L1; the separate
+// kernels of the regular pipeline read it plainly (a load past L1 there
+// measured 20 % slower medium-cell and twice slower block passes)
+template <bool FRESH>
+__device__ __forceinline__ uint32_t ctr_read(const unsigned int* a) { return FRESH ? __ldcg(a) : *a; }
+
+// huge cells i0, i0 + stride, ...
+template <bool FRESH = false>
+__device__ __forceinline__ void expand_cells(const Params& p, uint32_t i0, uint32_t stride) {
+    const uint32_t nh = mn64(ctr_read<FRESH>(&p.ctr->n_list[kListHuge]), p.list_cap[kListHuge]);
+    for (uint32_t i = i0; i < nh; i += stride) {
+        const uint2 sn = p.lists[p.list_off[kListHuge] + i];
+        const uint32_t n = sn.y;
+        const uint32_t R = (n + 31) >> 5;
+        uint32_t cnt = 0;
+        for (uint32_t r = 0; r < R; r++) cnt += (R - r + kTaskCols - 1) / kTaskCols;
+        const uint32_t b = atomicAdd(&p.ctr->need_tasks, cnt);
+        uint32_t k = 0;
+        for (uint32_t r = 0; r < R; r++)
+            for (uint32_t x0 = r; x0 < R; x0 += kTaskCols, k++)
+                if ((uint64_t)b + k < p.task_cap) p.tasks[b + k] = make_uint4(sn.x, n, r, x0);
+        if ((uint64_t)b + cnt > p.task_cap) atomicOr(&p.ctr->err, kErrTaskOvf);
+    }
+}
+
+// (with the tile tasks of huge cells: a launch of their own took 4 to 6 us)
 template <int D, bool MERGED>
 __global__ void __launch_bounds__(kBoxThreads) k_scatter(Params pin) {
     __shared__ __align__(16) uint32_t sbox[kBoxThreads * (2 * D + 1)];
+    stamp(pin, kStampScatter);
+    expand_cells(pin, blockIdx.x * kBoxThreads + threadIdx.x, gridDim.x * kBoxThreads);
     box_pass<D, true, MERGED>(resolve(pin), sbox, blockIdx.x, gridDim.x);
 }
 
@@ -504,7 +847,7 @@ struct TileRec {                         // 64 bytes per tile
     uint32_t chunk[kScanChunks];         // entries per chunk
     uint32_t pad[6];
 };
-static_assert(sizeof(TileRec) == 64, "tile record layout");
+static_assert(sizeof(TileRec) == kTileRecBytes && kScanTile == kTileCells, "tile record layout");
 
 static_assert(kMedMax == 128 && kBigMax == 512, "list bounds are powers of two (the class map's buckets)");
 // the work list of a cell of n >= 2 boxes under the class map
@@ -615,6 +958,7 @@ __device__ __forceinline__ void scan_prefix_block(const Params& p) {
 __global__ void __launch_bounds__(kReduceThreads, 4) k_scan_reduce(Params pin) {
     __shared__ uint32_t s_last;
     const Params p = resolve(pin);
+    stamp(p, kStampScan);
     const uint32_t warp = threadIdx.x >> 5;
     const uint64_t chunks = (p.ncells + kScanChunk - 1) / kScanChunk;
     TileRec* rec = reinterpret_cast<TileRec*>(p.tile_state);
@@ -844,40 +1188,6 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan_cells(Params pin) {
     }
     scan_stats_flush(p, stats);
 }
-
-// ---------------------------------------------------------------------------
-// expand: cells larger than kBigMax get tile tasks {cell, row tile r, column
-// tiles [x0,x1)} with 32-box tiles, x >= r, at most 8 column tiles a task.
-// ---------------------------------------------------------------------------
-constexpr uint32_t kTaskCols = 8;
-
-// a run counter that a pass reads: FRESH (one-launch queries, where phases
-// of the same kernel change the counters) reads it past L1; the separate
-// kernels of the regular pipeline read it plainly (a load past L1 there
-// measured 20 % slower medium-cell and twice slower block passes)
-template <bool FRESH>
-__device__ __forceinline__ uint32_t ctr_read(const unsigned int* a) { return FRESH ? __ldcg(a) : *a; }
-
-// huge cells i0, i0 + stride, ...
-template <bool FRESH = false>
-__device__ __forceinline__ void expand_cells(const Params& p, uint32_t i0, uint32_t stride) {
-    const uint32_t nh = mn64(ctr_read<FRESH>(&p.ctr->n_list[kListHuge]), p.list_cap[kListHuge]);
-    for (uint32_t i = i0; i < nh; i += stride) {
-        const uint2 sn = p.lists[p.list_off[kListHuge] + i];
-        const uint32_t n = sn.y;
-        const uint32_t R = (n + 31) >> 5;
-        uint32_t cnt = 0;
-        for (uint32_t r = 0; r < R; r++) cnt += (R - r + kTaskCols - 1) / kTaskCols;
-        const uint32_t b = atomicAdd(&p.ctr->need_tasks, cnt);
-        uint32_t k = 0;
-        for (uint32_t r = 0; r < R; r++)
-            for (uint32_t x0 = r; x0 < R; x0 += kTaskCols, k++)
-                if ((uint64_t)b + k < p.task_cap) p.tasks[b + k] = make_uint4(sn.x, n, r, x0);
-        if ((uint64_t)b + cnt > p.task_cap) atomicOr(&p.ctr->err, kErrTaskOvf);
-    }
-}
-
-__global__ void k_expand(Params p) { expand_cells(p, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x); }
 
 // ---------------------------------------------------------------------------
 // pair test
@@ -1228,7 +1538,9 @@ __device__ __forceinline__ void small_pass(const Params& p, uint4* s, uint2* s_o
 }
 
 template <int D, bool BIP, bool REC = false>
-__global__ void __launch_bounds__(kPairThreads, 5) k_pairs_small(Params p) {
+__global__ void __launch_bounds__(kPairThreads, 5) k_pairs_small(Params pin) {
+    const Params p = resolve(pin);
+    stamp(p, kStampSmall);
     __shared__ uint4 s_slot[kPairWarps][kSmallSlots];
     __shared__ uint2 s_out[kPairWarps][kWarpOut];
     const uint32_t warp = threadIdx.x >> 5;
@@ -1579,7 +1891,9 @@ __device__ __forceinline__ void med_pass(const Params& p, unsigned char* wsm, ui
 }
 
 template <int D, bool BIP, bool REC = false>
-__global__ void __launch_bounds__(kPairThreads, 4) k_pairs_med(Params p) {
+__global__ void __launch_bounds__(kPairThreads, 4) k_pairs_med(Params pin) {
+    const Params p = resolve(pin);
+    stamp(p, kStampMed);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t warp = threadIdx.x >> 5;
     med_pass<D, BIP, REC>(p, smem_raw + warp * kMedWarpBytes, (uint64_t)blockIdx.x * kPairWarps + warp,
@@ -1765,9 +2079,12 @@ __device__ __forceinline__ void team_pass(const Params& p, TeamSmem& s, uint64_t
 }
 
 template <int D, bool BIP, bool REC = false>
-__global__ void __launch_bounds__(kTeamThreads, 8) k_pairs_block(Params p) {
+__global__ void __launch_bounds__(kTeamThreads, 8) k_pairs_block(Params pin) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    const Params p = resolve(pin);
+    stamp(p, kStampBlock);
     team_pass<D, BIP, REC>(p, *reinterpret_cast<TeamSmem*>(smem_raw), blockIdx.x, gridDim.x);
+    query_end(p);
 }
 
 // record mode, after the pair kernels: the entries' box indices, which the
@@ -1800,7 +2117,7 @@ __device__ __forceinline__ unsigned long long warp_scene_reserve(unsigned long l
 __global__ void k_group_by_scene(Params pin, const unsigned long long* scene_pair_off,
                                  unsigned long long* scene_cursor, uint2* dst, unsigned long long n) {
     const Params p = resolve(pin);
-    n = mn64(p.ctr->pairs, p.out_cap);
+    n = mn64(__ldcg(&p.ctr->pairs), p.out_cap);
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
     const unsigned long long n32 = (n + 31) & ~31ull;  // whole warps iterate together
     for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n32; i += stride) {
@@ -1814,10 +2131,12 @@ __global__ void k_group_by_scene(Params pin, const unsigned long long* scene_pai
             dst[scene_pair_off[sc] + base + rank] = make_uint2(pr.x - off, pr.y - off);
         }
     }
+    query_end(p);
 }
 
 __global__ void k_scene_hist(Params pin, unsigned long long* hist, unsigned long long n) {
     const Params p = resolve(pin);
+    stamp(p, kStampGroup);
     n = mn64(p.ctr->pairs, p.out_cap);
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
     const unsigned long long n32 = (n + 31) & ~31ull;
@@ -1924,12 +2243,12 @@ __device__ __forceinline__ bool grid_barrier(const FusedArgs& a, uint32_t k) {
     return s_ok != 0u;
 }
 
-// the tuner's model (k_tune_scenes) for one scene of n boxes at row 0, in
-// single precision over exact integer sums: the one-launch path cannot wait
+// the query's cost model for one scene of n boxes at row 0, with T = E^2 / 2C
+// on 64 sampled boxes, in single precision over exact integer sums: the one-launch path cannot wait
 // for double-precision divisions. Grids of at most max_cells cells, so a
 // box covers at most max_cells cells and every per-box product fits 32 bits.
 __device__ __forceinline__ uint32_t tune_scene_fast(const uint32_t* boxes, uint64_t n, int dims, uint32_t range,
-                                                    uint64_t max_cells) {
+                                                    uint64_t max_cells, uint32_t warps) {
     const uint32_t lane = lane_id();
     const uint32_t W = 2 * (uint32_t)dims + 1;
     const uint64_t m = n < kTuneRows ? n : kTuneRows;
@@ -1982,9 +2301,10 @@ __device__ __forceinline__ uint32_t tune_scene_fast(const uint32_t* boxes, uint6
         if (e > 64u * (uint32_t)m) continue;
         const float E = (float)e * scale, Cf = (float)C;
         const float T = E * E / (2.0f * Cf);
-        const float occ = 2.0f * T / (E > 1.0f ? E : 1.0f) + 1.0f;
-        const float f = occ / (float)kTuneOcc > 1.0f ? occ / (float)kTuneOcc : 1.0f;
-        const float cost = (float)kTuneCell * Cf + (float)kTuneEntry * E + (float)kTuneTest * f * T;
+        // (fewer cells than warps leave warps idle: 30 000 boxes of one
+        // density took 35 us on 512 cells and 26 us on 4096)
+        const float idle = (float)warps > Cf ? (float)warps / Cf : 1.0f;
+        const float cost = (float)kQueryCell * Cf + (float)kQueryEntry * E + (float)kQueryTest * idle * T;
         if (cost < best_cost) {
             best_cost = cost;
             best = (uint32_t)s;
@@ -2012,11 +2332,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArg
     const uint64_t gt = blk * kFusedThreads + t, nt = nblk * kFusedThreads;
     const uint32_t range = p.max_range;
     uint32_t nbar = 0;
-    if (blk == 0 && t == 0) {
-        unsigned long long now;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-        p.ctr->t_start = now;
-    }
+    if (blk == 0 && t == 0) p.ctr->t_start = now_ns();
 #define FUSED_BARRIER()                                        \
     if (!grid_barrier(a, nbar++)) {                            \
         if (t == 0) atomicOr(&p.ctr->err, (unsigned)kErrWait); \
@@ -2025,7 +2341,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArg
     // P0
     if (warp == 0) {
         uint32_t sh = a.shift;
-        if (sh == kFusedTune) sh = tune_scene_fast(p.boxes, p.nboxes, D, range, kFusedMaxCells);
+        if (sh == kFusedTune) sh = tune_scene_fast(p.boxes, p.nboxes, D, range, kFusedMaxCells, (uint32_t)nw);
         if (lane == 0) s_shift = sh;
     }
     __syncthreads();
@@ -2177,20 +2493,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArg
         asm volatile("atom.acq_rel.gpu.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(a.bar) : "memory");
         if ((int32_t)(old - a.bar_base) == (int32_t)((nbar + 1) * nblk - 1)) {
             __threadfence();
-            constexpr uint32_t kWords = sizeof(Ctr) / sizeof(unsigned long long);
-            static_assert(sizeof(Ctr) % sizeof(unsigned long long) == 0, "run counters in 8-byte words");
-            const unsigned long long* src = reinterpret_cast<const unsigned long long*>(p.ctr);
-            unsigned long long w[kWords];
-#pragma unroll
-            for (uint32_t k = 0; k < kWords; k++) w[k] = __ldcg(src + k);
-            Ctr* h = a.ctr_host;
-            unsigned long long* dst = reinterpret_cast<unsigned long long*>(h);
-#pragma unroll
-            for (uint32_t k = 0; k < kWords; k++) dst[k] = w[k];
-            h->barriers = nbar + 1;
-            unsigned long long now;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-            h->t_end = now;
+            ctr_to_host(p.ctr, a.ctr_host);
+            a.ctr_host->barriers = nbar + 1;
+            a.ctr_host->t_end = now_ns();
             __threadfence_system();
         }
     }
@@ -2260,6 +2565,8 @@ cudaError_t kernels_init() {
     if ((e = init_variant<3, true>()) != cudaSuccess) return e;
     if ((e = init_variant<2, false, true>()) != cudaSuccess) return e;
     if ((e = init_variant<3, false, true>()) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_tune_query<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTuneSmem)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_tune_query<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTuneSmem)) != cudaSuccess) return e;
     int nb = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pairs_small<3, false>, kPairThreads, 0)) != cudaSuccess) return e;
     g_blocks_small = nb > 0 ? nb : 1;
@@ -2287,8 +2594,6 @@ cudaError_t launch_scene_hist(const Params& p, unsigned long long* hist, cudaStr
     k_scene_hist<<<(unsigned)((g_sm_count > 0 ? g_sm_count : 152) * 8), 256, 0, st>>>(p, hist, 0);
     return cudaGetLastError();
 }
-
-uint64_t scan_tiles(uint64_t ncells) { return (ncells + kScanTile - 1) / kScanTile; }
 
 uint64_t scene_table_entries(uint64_t nboxes) { return (nboxes >> kSceneTableShift) + 2; }
 
@@ -2342,14 +2647,17 @@ cudaError_t launch_scan(const Params& p, cudaStream_t st) {
     // reduce: two chunks per warp item, 4 resident blocks per SM
     const uint64_t rblocks = (chunks + 2 * (kReduceThreads / 32) - 1) / (2 * (kReduceThreads / 32));
     const unsigned g2 = (unsigned)(rblocks < cap ? (rblocks ? rblocks : 1) : cap);
-    cudaError_t e = cudaMemsetAsync(p.tile_state, 0, scan_state_bytes(p.ncells), st);
-    if (e != cudaSuccess) return e;
     k_scan_reduce<<<g2, kReduceThreads, 0, st>>>(p);
     k_scan_cells<<<g, kScanThreads, 0, st>>>(p);
     return cudaGetLastError();
 }
 
-size_t scan_state_bytes(uint64_t ncells) { return scan_tiles(ncells) * sizeof(TileRec); }
+cudaError_t launch_tune_query(const Params& p, const TuneArgs& a, int dims, cudaStream_t st) {
+    const unsigned blocks = a.shift == kTuneShift ? kTuneBlocks : 1u;
+    if (dims == 2) k_tune_query<2><<<blocks, kTuneThreads, kTuneSmem, st>>>(p, a);
+    else k_tune_query<3><<<blocks, kTuneThreads, kTuneSmem, st>>>(p, a);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_scene_offsets(const Params& p, const unsigned long long* hist, unsigned long long* off,
                                  uint32_t nscenes_cap, cudaStream_t st) {
@@ -2367,46 +2675,38 @@ cudaError_t launch_tune_scenes(const uint32_t* boxes, const unsigned long long* 
     return cudaGetLastError();
 }
 
-cudaError_t launch_expand(const Params& p, cudaStream_t st) {
-    k_expand<<<64, 256, 0, st>>>(p);
-    return cudaGetLastError();
-}
-
 template <int D, bool B, bool R = false>
-static cudaError_t launch_pairs_t(const Params& p, int sm_count, cudaStream_t st, cudaEvent_t* ev, unsigned evf,
-                                  const PairOverlap* ov) {
+static cudaError_t launch_pairs_t(const Params& p, int sm_count, cudaStream_t st, const PairOverlap* ov) {
     if (ov && !R && ov->side_sms > 0 && ov->side_sms < sm_count) {
         cudaError_t e;
+        Params q = p;
+        q.ctr_host = nullptr;  // the query ends behind both streams
         if ((e = cudaEventRecord(ov->fork, st)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(ov->side, ov->fork, 0)) != cudaSuccess) return e;
-        k_pairs_small<D, B, R><<<ov->side_sms * g_blocks_small, kPairThreads, 0, ov->side>>>(p);
-        if (ev) cudaEventRecordWithFlags(ev[0], ov->side, evf);
-        k_pairs_block<D, B, R><<<ov->side_sms * g_blocks_block, kTeamThreads, sizeof(TeamSmem), ov->side>>>(p);
-        k_pairs_med<D, B, R><<<(sm_count - ov->side_sms) * g_blocks_med, kPairThreads, med_smem(), st>>>(p);
-        if (ev) cudaEventRecordWithFlags(ev[1], st, evf);
+        k_pairs_small<D, B, R><<<ov->side_sms * g_blocks_small, kPairThreads, 0, ov->side>>>(q);
+        k_pairs_block<D, B, R><<<ov->side_sms * g_blocks_block, kTeamThreads, sizeof(TeamSmem), ov->side>>>(q);
+        k_pairs_med<D, B, R><<<(sm_count - ov->side_sms) * g_blocks_med, kPairThreads, med_smem(), st>>>(q);
         if ((e = cudaEventRecord(ov->join, ov->side)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(st, ov->join, 0)) != cudaSuccess) return e;
+        k_query_end<<<1, 32, 0, st>>>(p);
         return cudaGetLastError();
     }
     k_pairs_small<D, B, R><<<sm_count * g_blocks_small, kPairThreads, 0, st>>>(p);
-    if (ev) cudaEventRecordWithFlags(ev[0], st, evf);
     k_pairs_med<D, B, R><<<sm_count * g_blocks_med, kPairThreads, med_smem(), st>>>(p);
-    if (ev) cudaEventRecordWithFlags(ev[1], st, evf);
     k_pairs_block<D, B, R><<<sm_count * g_blocks_block, kTeamThreads, sizeof(TeamSmem), st>>>(p);
     if (R) k_strip_entries<<<(unsigned)(sm_count * 4), 512, 0, st>>>(p);
     return cudaGetLastError();
 }
 
-cudaError_t launch_pairs(const Params& p, int dims, int sm_count, cudaStream_t st, cudaEvent_t* ev, unsigned evf,
-                         const PairOverlap* ov) {
+cudaError_t launch_pairs(const Params& p, int dims, int sm_count, cudaStream_t st, const PairOverlap* ov) {
     const bool bip = p.split != kNoSplit;
     if (p.records) {  // record mode: self queries
         if (bip) return cudaErrorInvalidValue;
-        return dims == 2 ? launch_pairs_t<2, false, true>(p, sm_count, st, ev, evf, ov)
-                         : launch_pairs_t<3, false, true>(p, sm_count, st, ev, evf, ov);
+        return dims == 2 ? launch_pairs_t<2, false, true>(p, sm_count, st, ov)
+                         : launch_pairs_t<3, false, true>(p, sm_count, st, ov);
     }
-    if (dims == 2) return bip ? launch_pairs_t<2, true>(p, sm_count, st, ev, evf, ov) : launch_pairs_t<2, false>(p, sm_count, st, ev, evf, ov);
-    return bip ? launch_pairs_t<3, true>(p, sm_count, st, ev, evf, ov) : launch_pairs_t<3, false>(p, sm_count, st, ev, evf, ov);
+    if (dims == 2) return bip ? launch_pairs_t<2, true>(p, sm_count, st, ov) : launch_pairs_t<2, false>(p, sm_count, st, ov);
+    return bip ? launch_pairs_t<3, true>(p, sm_count, st, ov) : launch_pairs_t<3, false>(p, sm_count, st, ov);
 }
 
 cudaError_t launch_group_by_scene(const Params& p, const unsigned long long* scene_pair_off,

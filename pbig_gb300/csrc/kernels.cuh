@@ -17,7 +17,8 @@ enum : uint32_t {
     kErrTaskOvf = 64u,    // tile-task buffer too small
     kErrCellOvf = 128u,   // one box covers >= 2^31 cells
     kErrIndex = 256u,     // more than 2^29 boxes in one launch
-    kErrRecCell = 512u    // record mode: a cell of 65536 boxes or more (the record format's limit)
+    kErrRecCell = 512u,   // record mode: a cell of 65536 boxes or more (the record format's limit)
+    kErrGridRoom = 1024u  // the chosen grid has more cells than the buffers: nothing was run on it
 };
 
 constexpr uint32_t kNoSplit = 0xffffffffu;
@@ -81,6 +82,11 @@ __host__ __device__ inline uint64_t grid_cells(uint32_t range, uint32_t shift, i
 // The products are rounded one at a time (no fused multiply-add), so that
 // host and device compute the same costs.
 constexpr double kTuneCell = 2.4e-12, kTuneEntry = 80.0e-12, kTuneTest = 0.9e-12, kTuneOcc = 96.0;
+// Self and red/blue queries of one scene: fitted to the kernels that read
+// entries with their terms (device time of 7 workloads, 2-D and 3-D, at 4 to 5
+// cell sizes each: 65 us + 3.1 ps C + 41 ps E + 0.46 ps T + 0.6 ps per pair; it
+// picks the fastest size of every one). Tests cost the same in cells of any size.
+constexpr double kQueryCell = 3.1e-12, kQueryEntry = 41.0e-12, kQueryTest = 0.46e-12;
 
 __host__ __device__ inline double tune_mul(double a, double b) {
 #ifdef __CUDA_ARCH__
@@ -146,18 +152,21 @@ struct Ctr {
     unsigned int max_cell;              // largest cell (or merged block) of two or more boxes
     unsigned int med_next;              // next medium-cell item (items are taken one at a time)
     unsigned int big_next;              // next big-cell item, likewise
-    unsigned int pad;
+    unsigned int done;                  // blocks of the query's last kernel that have finished
     unsigned long long entries;         // E
     unsigned long long pairs;           // pairs found (may exceed capacity)
     unsigned long long tests;           // sum of n(n-1)/2 over cells
     unsigned long long comp_pairs;      // sum of n*n/2 over cells of n >= 2 (the reference's numCompPairs)
     unsigned long long jobs;            // sum of ceil(n/256) over cells of n >= 2 (its 256-row jobs)
     unsigned long long rec_pairs;       // record mode: pairs in the records (pairs counts 8-byte words)
-    unsigned long long cells;           // one-launch queries: cells of the grid the kernel chose
-    unsigned int shift;                 // one-launch queries: its cell shift
+    unsigned long long cells;           // cells of the grid the device chose (single-scene queries)
+    unsigned int shift;                 // its cell shift
     unsigned int barriers;              // one-launch queries: grid barriers the launch passed
     unsigned long long t_start, t_end;  // one-launch queries: device time (ns) at the start and the end
+    unsigned long long est_entries;     // single-scene queries: E as estimated from the tuner's sample
+    unsigned long long stamp[9];        // device time (ns) when the kernels of a phase began (kStamp*)
 };
+enum { kStampStart, kStampCount, kStampScan, kStampScatter, kStampSmall, kStampMed, kStampBlock, kStampGroup, kStampEnd };
 
 // query sizes read from device memory (graph replays: one captured graph
 // serves every batch up to the capacities it was captured with)
@@ -165,7 +174,7 @@ struct RunDims {
     unsigned long long nboxes;
     unsigned long long ncells;
     unsigned int nscenes;
-    unsigned int pad;
+    unsigned int open;   // Params::open (either sets it)
 };
 
 struct Params {
@@ -187,11 +196,12 @@ struct Params {
     uint64_t list_cap[kNumLists];
     uint4* tasks;                 // huge-cell tile tasks {start, n, r, x0}
     uint64_t task_cap;
-    unsigned long long* tile_state; // scan tile records (128 bytes per 4096 cells)
+    unsigned long long* tile_state; // scan tile records (kTileRecBytes per kTileCells cells)
     uint2* out;                   // pairs
     uint64_t out_cap;
     Ctr* ctr;
-    const RunDims* dyn;           // when set, overrides nboxes / ncells / nscenes
+    Ctr* ctr_host;                // page-locked copy of ctr, written when the last kernel of the query ends (or null)
+    const RunDims* dyn;           // when set, overrides nboxes / ncells / nscenes, adds to open
     const uint32_t* merged;       // merged mode (one scene): cell -> root of its merged block, or kUnmerged
     const unsigned long long* merged_ext; // ... and of a root: its block's cells per axis, 21 bits each
     uint32_t* recs;               // record mode: [entry_cap] box indices, written after the pair kernels
@@ -213,10 +223,37 @@ constexpr uint32_t kUnmerged = 0x0fffff11u;  // a cell outside every merged bloc
 // launchers (all asynchronous on `st`); dims is 2 or 3
 // grids: sized from p.nboxes / p.ncells (which must then be upper bounds
 // of the device-side sizes when p.dyn is set)
+// launch_count zeroes the counters and the scan's tile records first
 cudaError_t launch_count(const Params& p, int dims, cudaStream_t st);
 cudaError_t launch_scan(const Params& p, cudaStream_t st);
-cudaError_t launch_expand(const Params& p, cudaStream_t st);
 cudaError_t launch_scatter(const Params& p, int dims, cudaStream_t st);
+
+// The grid of a single-scene query (red/blue: both colours on one grid),
+// chosen on the device: zeroes p.ctr and writes the scene table (p.scenes,
+// p.scene_box_off), `dims` and ctr->cells, shift, est_entries, so that the
+// kernels behind it need nothing from the host. `shift`: the cell shift, or
+// kTuneShift for the cost model on a strided sample of 4096 boxes, over grids
+// of at most max_cells cells. A choice of raise_from becomes raise_to. A grid
+// of more than room_cells cells sets kErrGridRoom and leaves the kernels
+// behind it nothing to do.
+constexpr uint32_t kTuneShift = 0xffffffffu;
+constexpr uint64_t kTuneSample = 4096;
+struct TuneArgs {
+    const uint32_t* red;    // boxes [0, n_red) and [n_red, n) (device memory or mapped host memory)
+    const uint32_t* blue;
+    uint64_t n_red, n;
+    uint32_t bip;           // two scenes
+    uint32_t range;
+    uint32_t shift;
+    uint32_t raise_from, raise_to;
+    uint64_t max_cells, room_cells;
+    Scene* scenes;
+    uint32_t* box_off;
+    RunDims* dims;
+    unsigned long long* scratch;  // 2 words per block, zero at the start and left zero
+};
+constexpr size_t kTuneScratchBytes = 256;
+cudaError_t launch_tune_query(const Params& p, const TuneArgs& a, int dims, cudaStream_t st);
 // exclusive scan of nscenes+1 per-scene pair counts (one block)
 // per-scene cell sizes of a batched query (one warp per scene, a strided
 // sample of up to 64 boxes of each scene, T estimated as E^2 / 2C); offs:
@@ -236,19 +273,17 @@ struct PairOverlap {
     int side_sms;
 };
 
-// ev (optional, 2 events) is recorded after the small-cell and after the
-// medium-cell kernel (with an overlap: after the small-cell kernel on the side
-// stream and after the medium-cell kernel on st)
-cudaError_t launch_pairs(const Params& p, int dims, int sm_count, cudaStream_t st, cudaEvent_t* ev = nullptr,
-                         unsigned ev_flags = cudaEventRecordDefault, const PairOverlap* ov = nullptr);
+cudaError_t launch_pairs(const Params& p, int dims, int sm_count, cudaStream_t st, const PairOverlap* ov = nullptr);
 cudaError_t launch_group_by_scene(const Params& p, const unsigned long long* scene_pair_off,
                                   unsigned long long* scene_cursor, uint2* dst, cudaStream_t st);
 cudaError_t launch_scene_hist(const Params& p, unsigned long long* hist, cudaStream_t st);
 // p.scene_table for p.nboxes boxes (scene_table_entries of them)
 cudaError_t launch_scene_table(const Params& p, cudaStream_t st);
 uint64_t scene_table_entries(uint64_t nboxes);
-uint64_t scan_tiles(uint64_t ncells);
-size_t scan_state_bytes(uint64_t ncells);  // scan tile records
+// scan tile records: kTileRecBytes per kTileCells cells
+constexpr uint64_t kTileCells = 4096, kTileRecBytes = 64;
+__host__ __device__ inline uint64_t scan_tiles(uint64_t ncells) { return (ncells + kTileCells - 1) / kTileCells; }
+inline size_t scan_state_bytes(uint64_t ncells) { return scan_tiles(ncells) * kTileRecBytes; }
 size_t pair_smem_bytes();
 cudaError_t kernels_init();
 

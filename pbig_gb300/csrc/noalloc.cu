@@ -178,7 +178,6 @@ PBIG2_API int pbig2_self_intersect_noalloc(const uint32_t* d_boxes, uint64_t n, 
     if (e == cudaSuccess) e = cudaMemsetAsync(p.ctr, 0, sizeof(Ctr), st);
     if (e == cudaSuccess) e = launch_count(p, (int)dims, st);
     if (e == cudaSuccess) e = launch_scan(p, st);
-    if (e == cudaSuccess) e = launch_expand(p, st);
     if (e == cudaSuccess) e = launch_scatter(p, (int)dims, st);
     int sms = 0;
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

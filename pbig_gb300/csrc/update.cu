@@ -458,6 +458,7 @@ int build_grid(pbig2_scene* s, cudaStream_t st) {
     p.ctr = s->ctrbuf.as<Ctr>();
     p.lists = s->lists.as<uint2>();
     SCK(cudaMemsetAsync(p.ctr, 0, sizeof(Ctr), st));
+    SCK(cudaMemsetAsync(p.tile_state, 0, scan_state_bytes(p.ncells), st));
     SCK(launch_scan(p, st));
     k_res_starts<<<grid_for(s->ncells, 256, sms), 256, 0, st>>>(s->cnt.as<uint32_t>(), s->tmp.as<uint32_t>(), g);
     SCK(cudaGetLastError());
