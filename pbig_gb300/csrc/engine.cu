@@ -241,7 +241,9 @@ static int ensure_query_buffers(pbig2_ctx* c, Params& p, uint64_t entry_cap, uin
     if (grouped) {
         CK(c->d_out2.ensure(c->d_out.bytes, false, st));
         CK(c->d_scene_pair.ensure((nsc + 1) * 8, false, st));
-        CK(c->d_scene_cursor.ensure((nsc + 1) * 8, false, st));
+        CK(c->d_scene_cursor.ensure(2 * (nsc + 1) * 8, false, st));  // pair counts, then cursors
+        CK(c->d_group.ensure(group_count_bytes(nsc), false, st));
+        CK(c->h_pair_off.ensure((nsc + 1) * 8));
     }
     p.counts = c->d_counts.as<uint32_t>();
     p.entries = c->d_entries.as<uint4>();
@@ -300,14 +302,16 @@ static cudaError_t record_pipeline(pbig2_ctx* c, const Params& p, int dims, bool
     const bool overlap = c->ext_host && p.out == c->ext_out && c->host_split >= 0 && !p.records;
     R(launch_pairs(pp, dims, c->sm_count, st, overlap ? &ov : nullptr));
     if (grouped) {
-        unsigned long long* hist = c->d_scene_cursor.as<unsigned long long>();
-        unsigned long long* offs = c->d_scene_pair.as<unsigned long long>();
-        R(cudaMemsetAsync(hist, 0, (nsc + 1) * 8, st));
-        R(launch_scene_hist(p, hist, st));
-        R(launch_scene_offsets(p, hist, offs, nsc, st));
-        R(cudaMemsetAsync(hist, 0, (nsc + 1) * 8, st));
-        pp.ctr_host = static_cast<Ctr*>(c->h_ctr.p);
-        R(launch_group_by_scene(pp, offs, hist, c->d_out2.as<uint2>(), st));
+        GroupArgs g{};
+        g.hist = c->d_scene_cursor.as<unsigned long long>();
+        g.cursor = g.hist + nsc + 1;
+        g.off = c->d_scene_pair.as<unsigned long long>();
+        g.off_host = static_cast<unsigned long long*>(c->h_pair_off.p);
+        g.block_counts = c->d_group.as<uint32_t>();
+        g.dst = c->d_out2.as<uint2>();
+        g.ctr_host = static_cast<Ctr*>(c->h_ctr.p);
+        R(cudaMemsetAsync(g.hist, 0, 2 * (nsc + 1) * 8, st));
+        R(launch_group_by_scene(pp, g, st));
     }
 #undef R
     return cudaSuccess;
@@ -315,7 +319,7 @@ static cudaError_t record_pipeline(pbig2_ctx* c, const Params& p, int dims, bool
 
 // result bookkeeping after a pass: pair count, per-scene offsets, stats
 static int finish_query(pbig2_ctx* c, const Ctr& h, uint64_t nboxes, uint64_t ncells, uint32_t nsc,
-                        const std::vector<GridScene>& scenes, bool grouped, int launches, cudaStream_t st) {
+                        const std::vector<GridScene>& scenes, bool grouped, int launches) {
     c->result_records = c->rice_mode && !grouped;
     c->rice_words = c->result_records ? h.pairs : 0;
     c->npairs = c->result_records ? h.rec_pairs : h.pairs;
@@ -323,10 +327,8 @@ static int finish_query(pbig2_ctx* c, const Ctr& h, uint64_t nboxes, uint64_t nc
     c->last_entries = h.entries;
     c->result = grouped ? c->d_out2.as<uint2>() : c->result_ext ? c->ext_out : c->d_out.as<uint2>();
     if (grouped) {
-        CK(c->h_stage.ensure((nsc + 1) * 8));
-        CK(cudaMemcpyAsync(c->h_stage.p, c->d_scene_pair.p, (nsc + 1) * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        c->scene_pair_off.assign((const uint64_t*)c->h_stage.p, (const uint64_t*)c->h_stage.p + nsc + 1);
+        const uint64_t* off = static_cast<const uint64_t*>(c->h_pair_off.p);  // (written by the grouping)
+        c->scene_pair_off.assign(off, off + nsc + 1);
     } else {
         c->scene_pair_off.assign(1, 0);
         c->scene_pair_off.push_back(c->npairs);
@@ -614,7 +616,7 @@ static int run_batch(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t nboxes, int
             c->out_hint = std::max<uint64_t>(c->out_hint, h.pairs + h.pairs / 8);
             est_entries = std::max(est_entries, (double)h.entries * 1.1);
         } else {
-            const int rf = finish_query(c, h, nboxes, ncells, nsc, scenes, true, launches, st);
+            const int rf = finish_query(c, h, nboxes, ncells, nsc, scenes, true, launches);
             c->stats.class_map = c->class_map ? c->class_map : kClassMapDefault;
             return rf;
         }
@@ -661,7 +663,7 @@ static int run_batch(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t nboxes, int
     if (rc == kAgain) return fail(PBIG2_ENOMEM, "capacity retries exhausted");
     if (rc) return rc;
     c->out_hint = std::max<uint64_t>(c->out_hint, h.pairs + h.pairs / 8);
-    rc = finish_query(c, h, nboxes, ncells, nsc, scenes, true, launches, st);
+    rc = finish_query(c, h, nboxes, ncells, nsc, scenes, true, launches);
     c->stats.class_map = p.class_map;
     if (rc != PBIG2_OK && rc != PBIG2_EINPUT) return rc;
     // capture this query's pipeline for later batches of the same shape
@@ -828,7 +830,7 @@ static int run_single(pbig2_ctx* c, const SingleScene& q, uint32_t shift, cudaSt
     std::vector<GridScene> sc{{0, q.n, h.shift, 0}};
     if (q.bip) sc.push_back({q.n_red, q.n - q.n_red, h.shift, 0});
     *used = h.shift;
-    rc = finish_query(c, h, q.n, h.cells, p.nscenes, sc, false, launches, st);
+    rc = finish_query(c, h, q.n, h.cells, p.nscenes, sc, false, launches);
     c->stats.class_map = p.class_map;
     return rc;
 }
@@ -929,7 +931,7 @@ static int fused_query(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t n, int di
     c->out_hint = std::max<uint64_t>(c->out_hint, h.pairs + h.pairs / 8);
     c->merged_blocks = 0;
     std::vector<GridScene> sc{{0, n, h.shift, 0}};
-    rc = finish_query(c, h, n, h.cells, 1, sc, false, 1, st);
+    rc = finish_query(c, h, n, h.cells, 1, sc, false, 1);
     c->stats.class_map = p.class_map;
     c->stats.device_ms = h.t_end > h.t_start ? (double)(h.t_end - h.t_start) * 1e-6 : 0.0;  // the kernel's own clock
     return rc;
@@ -1002,9 +1004,10 @@ PBIG2_API int pbig2_destroy(pbig2_ctx* c) {
     for (DevBuf* b : {&c->d_boxes, &c->d_counts, &c->d_entries, &c->d_recs, &c->d_merged, &c->d_merged_ext, &c->d_bar, &c->d_fctr,
                       &c->d_lists, &c->d_tasks, &c->d_state,
                       &c->d_out, &c->d_out2, &c->d_ctr, &c->d_scenes, &c->d_scene_off, &c->d_scene_pair,
-                      &c->d_scene_cursor, &c->d_dims, &c->d_scene_tab, &c->d_tune, &c->d_tune_cost})
+                      &c->d_scene_cursor, &c->d_dims, &c->d_scene_tab, &c->d_tune, &c->d_tune_cost, &c->d_group})
         b->release();
     c->h_ctr.release();
+    c->h_pair_off.release();
     c->h_stage.release();
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);

@@ -60,8 +60,8 @@ struct pbig2_ctx {
     uint32_t merged_blocks = 0;  // merged blocks of the last query
     uint32_t last_err = 0;       // error bits of the last pipeline pass
     pbig::DevBuf d_boxes, d_counts, d_entries, d_lists, d_tasks, d_state, d_out, d_out2, d_ctr,
-        d_scenes, d_scene_off, d_scene_pair, d_scene_cursor, d_dims, d_scene_tab, d_tune, d_tune_cost;
-    pbig::HostPinned h_ctr, h_stage;
+        d_scenes, d_scene_off, d_scene_pair, d_scene_cursor, d_dims, d_scene_tab, d_tune, d_tune_cost, d_group;
+    pbig::HostPinned h_ctr, h_stage, h_pair_off;
     // caller's pair buffer for self/bipartite queries (pbig2_set_pair_output)
     uint2* ext_out = nullptr;
     uint64_t ext_cap = 0;
@@ -96,9 +96,9 @@ struct pbig2_ctx {
         uintptr_t h = 0;
         for (const pbig::DevBuf* b : {&d_counts, &d_entries, &d_lists, &d_tasks, &d_state, &d_out, &d_out2,
                                       &d_ctr, &d_scenes, &d_scene_off, &d_scene_pair, &d_scene_cursor, &d_dims,
-                                      &d_scene_tab})
+                                      &d_scene_tab, &d_group})
             h = h * 1000003u + (uintptr_t)b->p;
-        return h * 1000003u + (uintptr_t)h_ctr.p;
+        return (h * 1000003u + (uintptr_t)h_ctr.p) * 1000003u + (uintptr_t)h_pair_off.p;
     }
     void drop_graph() {
         if (graph.exec) cudaGraphExecDestroy(graph.exec);

@@ -1449,7 +1449,12 @@ __device__ __forceinline__ void small_items(const Params& p, uint4* s, WarpOut& 
     const uint32_t lane = lane_id(), g = lane / WG, r = lane % WG, gb = g * (2 * WG);
     const uint64_t nl = mn64(ctr_read<FRESH>(&p.ctr->n_list[list]), p.list_cap[list]);
     const uint64_t nitems = (nl + G - 1) / G;
-    for (uint64_t item = first; item < nitems; item += stride) {
+    // a batch's warp takes items next to each other, so that its pairs leave it
+    // in long runs of one scene (4 % slower here than every stride-th item, and
+    // less than half the time in the grouping)
+    const uint64_t per = (nitems + stride - 1) / stride;
+    const uint64_t step = p.scene_table ? 1 : stride, end = p.scene_table ? mn64((first + 1) * per, nitems) : nitems;
+    for (uint64_t item = p.scene_table ? first * per : first; item < end; item += step) {
         const uint64_t ci = item * G + g;
         uint32_t n = 0, gid = 0, start = 0;
         if (ci < nl) {
@@ -1869,21 +1874,26 @@ __device__ __forceinline__ void med_pass(const Params& p, unsigned char* wsm, ui
         for (uint32_t r = 0; r < R; r++) row_sweep<D, BIP, REC>(p, t, o, c, r, BIP ? 0u : r, ~0u >> 1, gid);
         __syncwarp();
     };
-    // items taken one at a time from a counter, so warps whose cells were
-    // larger end no later than the others (on the clustered 4M-box scene
-    // 0.444 ms, against 0.499 ms for a fixed stride over the list and
-    // 0.455-0.50 ms for a fixed stride over its first half to seven eighths).
-    // A one-launch query's warps take one or two cells each: there the
-    // counter's round trip costs more than the balance gains.
+    // items taken from a counter, so warps whose cells were larger end no
+    // later than the others (with one cell at a time 0.444 ms on the clustered
+    // 4M-box scene when this was tried, against 0.499 ms for a fixed stride
+    // over the list), of a batch 16 at a time and fewer as the list ends, so
+    // that its pairs leave the warp in long runs of one scene (512 scenes 0.58
+    // ms here, with one at a time 0.56, with 15 to the end 0.60; the grouping
+    // takes 0.17 ms instead of 0.27). A one-launch query's warps take one or
+    // two cells each: there the counter's round trip costs more than the
+    // balance gains.
     if constexpr (FRESH) {
         for (uint64_t item = gw; item < nl; item += nw) cell(item);
     } else {
+        uint32_t run = 0;
+        uint64_t item = 0;
         for (;;) {
-            uint64_t item = 0;
-            if (lane == 0) item = atomicAdd(&p.ctr->med_next, 1u);
+            run = p.scene_table ? max((uint32_t)mn64((nl - item) / (4 * nw), 16), 1u) : 1u;
+            if (lane == 0) item = atomicAdd(&p.ctr->med_next, run);
             item = __shfl_sync(FULL_MASK, item, 0);
             if (item >= nl) break;
-            cell(item);
+            for (const uint64_t end = mn64(item + run, nl); item < end; item++) cell(item);
         }
     }
     wflush<BIP, REC>(p, o);
@@ -2099,59 +2109,151 @@ __global__ void k_strip_entries(Params pin) {
 // ---------------------------------------------------------------------------
 // group pairs by scene (batched queries): a pair's scene is the scene of its
 // first box; pairs are written to their scene's range with scene-local ids.
+//
+// As one pass of a radix sort by scene: each block counts a run of the pairs
+// per scene in shared memory (k_scene_hist, which keeps the block's counts and
+// adds them to the scenes' totals) and, once the totals are offsets, reserves
+// its part of every scene it met with one atomic and places its pairs from
+// shared-memory counters (k_group_by_scene). Pairs come out of the pair kernels
+// in runs of one scene, so each warp takes a run of its own and keeps the
+// bounds of the scene it is in: a lookup, five loads one after the other, is
+// made where the scene changes only. With a lookup per warp step 512 scenes of
+// 18.4 M pairs took 470 us, with one per pair 288 us, and with the warps adding
+// to the scenes' totals themselves 326 us (eight scenes of 1.3 M pairs, all on
+// a few counters' heels, 79 us). More than kGroupScenes scenes still do that:
+// their counters do not fit the shared memory, and are many.
 // ---------------------------------------------------------------------------
-// lanes of a warp holding pairs of the same scene share one atomic (pairs
-// come out of the pair kernels in runs of one scene)
-__device__ __forceinline__ unsigned long long warp_scene_reserve(unsigned long long* ctr, uint32_t sc, bool valid,
-                                                                  uint32_t& rank) {
-    const uint32_t lane = lane_id();
-    const uint32_t key = valid ? sc : 0xffffffffu;
-    const uint32_t same = __match_any_sync(FULL_MASK, key);
-    const uint32_t leader = __ffs(same) - 1;
-    rank = __popc(same & ((1u << lane) - 1u));
-    unsigned long long base = 0;
-    if (valid && lane == leader) base = atomicAdd(&ctr[sc], (unsigned long long)__popc(same));
-    return __shfl_sync(FULL_MASK, base, leader);
+constexpr int kGroupThreads = 512;
+constexpr int kGroupAhead = 4;            // warp steps of pairs loaded together
+constexpr uint32_t kGroupScenes = 8192;   // 12 bytes of counters each: two blocks an SM
+constexpr size_t kGroupBytes = sizeof(unsigned long long) + sizeof(uint32_t);
+
+// the scene a warp is in: its boxes [lo, hi)
+struct SceneRun {
+    uint32_t scene = 0, lo = 0, hi = 0;
+};
+
+// warp step over the boxes gi of the valid lanes: each scene among them, with
+// the lanes that have it; change() where it is not the one before
+template <class C, class F>
+__device__ __forceinline__ void warp_by_scene(const Params& p, SceneRun& run, uint32_t gi, bool valid, C change, F lanes) {
+    uint32_t left = __ballot_sync(FULL_MASK, valid);
+    while (left) {
+        uint32_t mine = __ballot_sync(FULL_MASK, gi >= run.lo && gi < run.hi) & left;
+        if (mine == 0u) {  // another scene: that of the first lane left
+            const uint32_t x = __shfl_sync(FULL_MASK, gi, __ffs(left) - 1);
+            const uint32_t s = find_scene(p, x);
+            change(s);
+            run.scene = s;
+            run.lo = p.scene_box_off[s];
+            run.hi = p.scene_box_off[s + 1];
+            mine = __ballot_sync(FULL_MASK, gi >= run.lo && gi < run.hi) & left;
+            if (mine == 0u) return;  // (cannot happen: every box has its scene)
+        }
+        lanes(mine);
+        left &= ~mine;
+    }
 }
 
-__global__ void k_group_by_scene(Params pin, const unsigned long long* scene_pair_off,
-                                 unsigned long long* scene_cursor, uint2* dst, unsigned long long n) {
+// step(pair, whether the lane has one) over this warp's run of the pairs, a
+// few steps' loads in flight together
+template <class F>
+__device__ __forceinline__ void group_pairs(const Params& p, F step) {
+    const unsigned long long n = mn64(__ldcg(&p.ctr->pairs), p.out_cap);
+    const unsigned long long warps = (unsigned long long)gridDim.x * (kGroupThreads / 32);
+    const unsigned long long per = ((n + 31) / 32 + warps - 1) / warps * 32;
+    const unsigned long long first = per * ((unsigned long long)blockIdx.x * (kGroupThreads / 32) + (threadIdx.x >> 5));
+    const unsigned long long end = first + per < n ? first + per : n;
+    for (unsigned long long i = first; i < end; i += 32 * kGroupAhead) {
+        uint2 pr[kGroupAhead];
+#pragma unroll
+        for (int k = 0; k < kGroupAhead; k++) {
+            const unsigned long long at = i + 32 * k + lane_id();
+            pr[k] = at < end ? p.out[at] : make_uint2(0u, 0u);
+        }
+#pragma unroll
+        for (int k = 0; k < kGroupAhead; k++) step(pr[k], i + 32 * k + lane_id() < end);
+    }
+}
+
+// LOCAL: the block's counters are in shared memory
+template <bool LOCAL>
+__global__ void __launch_bounds__(kGroupThreads, 2) k_scene_hist(Params pin, unsigned long long* hist, uint32_t* block_counts) {
+    extern __shared__ unsigned long long group_smem[];
     const Params p = resolve(pin);
-    n = mn64(__ldcg(&p.ctr->pairs), p.out_cap);
-    const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-    const unsigned long long n32 = (n + 31) & ~31ull;  // whole warps iterate together
-    for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n32; i += stride) {
-        const bool valid = i < n;
-        const uint2 pr = valid ? p.out[i] : make_uint2(0u, 0u);
-        const uint32_t sc = valid ? find_scene(p, pr.x) : 0u;
-        uint32_t rank;
-        const unsigned long long base = warp_scene_reserve(scene_cursor, sc, valid, rank);
-        if (valid) {
-            const uint32_t off = p.scene_box_off[sc];
-            dst[scene_pair_off[sc] + base + rank] = make_uint2(pr.x - off, pr.y - off);
+    stamp(p, kStampGroup);
+    const uint32_t lane = lane_id();
+    uint32_t* counts = reinterpret_cast<uint32_t*>(group_smem);
+    if constexpr (LOCAL) {
+        for (uint32_t s = threadIdx.x; s < p.nscenes; s += kGroupThreads) counts[s] = 0u;
+        __syncthreads();
+    }
+    SceneRun run;
+    uint32_t have = 0;  // pairs of the scene the warp is in, not yet added to its counter
+    const auto add = [&](uint32_t) {
+        if (lane == 0 && have) {
+            if constexpr (LOCAL) atomicAdd(&counts[run.scene], have);
+            else atomicAdd(&hist[run.scene], (unsigned long long)have);
+        }
+        have = 0;
+    };
+    group_pairs(p, [&](uint2 pr, bool valid) {
+        warp_by_scene(p, run, pr.x, valid, add, [&](uint32_t mine) { have += __popc(mine); });
+    });
+    add(0u);
+    if constexpr (LOCAL) {
+        __syncthreads();
+        for (uint32_t s = threadIdx.x; s < p.nscenes; s += kGroupThreads) {
+            const uint32_t c = counts[s];
+            block_counts[(uint64_t)blockIdx.x * p.nscenes + s] = c;
+            if (c) atomicAdd(&hist[s], (unsigned long long)c);
         }
     }
+}
+
+template <bool LOCAL>
+__global__ void __launch_bounds__(kGroupThreads, 2) k_group_by_scene(Params pin, const unsigned long long* scene_pair_off,
+                                                                     unsigned long long* scene_cursor,
+                                                                     const uint32_t* block_counts, uint2* dst) {
+    extern __shared__ unsigned long long group_smem[];  // a scene's part of dst for this block, then its pairs so far
+    const Params p = resolve(pin);
+    const uint32_t lane = lane_id();
+    uint32_t* placed = reinterpret_cast<uint32_t*>(group_smem + p.nscenes);
+    if constexpr (LOCAL) {
+        for (uint32_t s = threadIdx.x; s < p.nscenes; s += kGroupThreads) {
+            const uint32_t c = block_counts[(uint64_t)blockIdx.x * p.nscenes + s];
+            if (c) group_smem[s] = scene_pair_off[s] + atomicAdd(&scene_cursor[s], (unsigned long long)c);
+            placed[s] = 0u;
+        }
+        __syncthreads();
+    }
+    SceneRun run;
+    uint2* part = dst;  // of the scene the warp is in
+    const auto change = [&](uint32_t s) { part = dst + (LOCAL ? group_smem[s] : scene_pair_off[s]); };
+    group_pairs(p, [&](uint2 pr, bool valid) {
+        warp_by_scene(p, run, pr.x, valid, change, [&](uint32_t mine) {
+            const uint32_t leader = __ffs(mine) - 1;
+            unsigned long long at = 0;
+            if constexpr (LOCAL) {
+                uint32_t k = 0;
+                if (lane == leader) k = atomicAdd(&placed[run.scene], (uint32_t)__popc(mine));
+                at = __shfl_sync(FULL_MASK, k, leader);
+            } else {
+                if (lane == leader) at = atomicAdd(&scene_cursor[run.scene], (unsigned long long)__popc(mine));
+                at = __shfl_sync(FULL_MASK, at, leader);
+            }
+            if ((mine >> lane) & 1u)
+                part[at + __popc(mine & ((1u << lane) - 1u))] = make_uint2(pr.x - run.lo, pr.y - run.lo);
+        });
+    });
     query_end(p);
 }
 
-__global__ void k_scene_hist(Params pin, unsigned long long* hist, unsigned long long n) {
-    const Params p = resolve(pin);
-    stamp(p, kStampGroup);
-    n = mn64(p.ctr->pairs, p.out_cap);
-    const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-    const unsigned long long n32 = (n + 31) & ~31ull;
-    for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n32; i += stride) {
-        const bool valid = i < n;
-        const uint32_t sc = valid ? find_scene(p, p.out[i].x) : 0u;
-        uint32_t rank;
-        warp_scene_reserve(hist, sc, valid, rank);
-    }
-}
-
 // exclusive scan of the per-scene pair counts: off[s] = sum of hist[< s],
-// off[nscenes] = total; one block, 1024 threads, chunks of 1024 scenes
+// off[nscenes] = total, also to page-locked host memory; one block, 1024
+// threads, chunks of 1024 scenes
 __global__ void __launch_bounds__(1024) k_scene_offsets(Params pin, const unsigned long long* hist,
-                                                        unsigned long long* off) {
+                                                        unsigned long long* off, unsigned long long* off_host) {
     const Params p = resolve(pin);
     __shared__ unsigned long long s_w[32];
     __shared__ unsigned long long s_carry;
@@ -2180,7 +2282,10 @@ __global__ void __launch_bounds__(1024) k_scene_offsets(Params pin, const unsign
         }
         __syncthreads();
         const unsigned long long incl = x + (warp ? s_w[warp - 1] : 0ull) + s_carry;
-        if (i <= p.nscenes) off[i] = incl - v;
+        if (i <= p.nscenes) {
+            off[i] = incl - v;
+            off_host[i] = incl - v;
+        }
         __syncthreads();
         if (t == 1023) s_carry = incl;
         __syncthreads();
@@ -2565,6 +2670,8 @@ cudaError_t kernels_init() {
     if ((e = init_variant<3, true>()) != cudaSuccess) return e;
     if ((e = init_variant<2, false, true>()) != cudaSuccess) return e;
     if ((e = init_variant<3, false, true>()) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_scene_hist<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kGroupScenes * sizeof(uint32_t)))) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_group_by_scene<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kGroupScenes * kGroupBytes))) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(k_tune_query<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTuneSmem)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(k_tune_query<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTuneSmem)) != cudaSuccess) return e;
     int nb = 0;
@@ -2587,12 +2694,6 @@ cudaError_t kernels_init() {
         g_fused_blocks = coop && nf >= 1 ? g_sm_count : 0;
     }
     return cudaSuccess;
-}
-
-cudaError_t launch_scene_hist(const Params& p, unsigned long long* hist, cudaStream_t st) {
-    // the pair count is read on the device
-    k_scene_hist<<<(unsigned)((g_sm_count > 0 ? g_sm_count : 152) * 8), 256, 0, st>>>(p, hist, 0);
-    return cudaGetLastError();
 }
 
 uint64_t scene_table_entries(uint64_t nboxes) { return (nboxes >> kSceneTableShift) + 2; }
@@ -2659,13 +2760,6 @@ cudaError_t launch_tune_query(const Params& p, const TuneArgs& a, int dims, cuda
     return cudaGetLastError();
 }
 
-cudaError_t launch_scene_offsets(const Params& p, const unsigned long long* hist, unsigned long long* off,
-                                 uint32_t nscenes_cap, cudaStream_t st) {
-    (void)nscenes_cap;
-    k_scene_offsets<<<1, 1024, 0, st>>>(p, hist, off);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_tune_scenes(const uint32_t* boxes, const unsigned long long* offs, uint32_t nscenes, int dims,
                                uint32_t range, SceneTune* out, cudaStream_t st) {
     if (nscenes == 0) return cudaSuccess;
@@ -2709,11 +2803,26 @@ cudaError_t launch_pairs(const Params& p, int dims, int sm_count, cudaStream_t s
     return bip ? launch_pairs_t<3, true>(p, sm_count, st, ov) : launch_pairs_t<3, false>(p, sm_count, st, ov);
 }
 
-cudaError_t launch_group_by_scene(const Params& p, const unsigned long long* scene_pair_off,
-                                  unsigned long long* scene_cursor, uint2* dst, cudaStream_t st) {
-    // the pair count is read on the device
-    k_group_by_scene<<<(unsigned)((g_sm_count > 0 ? g_sm_count : 152) * 8), 256, 0, st>>>(p, scene_pair_off,
-                                                                                          scene_cursor, dst, 0);
+static unsigned group_blocks() { return (unsigned)((g_sm_count > 0 ? g_sm_count : 152) * 2); }
+
+size_t group_count_bytes(uint32_t nscenes) {
+    return nscenes <= kGroupScenes ? (size_t)group_blocks() * nscenes * sizeof(uint32_t) : 0;
+}
+
+cudaError_t launch_group_by_scene(const Params& p, const GroupArgs& g, cudaStream_t st) {
+    // the pair count is read on the device; the scenes may be fewer than p.nscenes
+    const bool local = p.nscenes <= kGroupScenes;
+    const size_t n = local ? p.nscenes : 0;
+    const unsigned blocks = group_blocks();
+    if (local) k_scene_hist<true><<<blocks, kGroupThreads, n * sizeof(uint32_t), st>>>(p, g.hist, g.block_counts);
+    else k_scene_hist<false><<<blocks, kGroupThreads, 0, st>>>(p, g.hist, nullptr);
+    k_scene_offsets<<<1, 1024, 0, st>>>(p, g.hist, g.off, g.off_host);
+    Params q = p;
+    q.ctr_host = g.ctr_host;  // the query ends here
+    if (local)
+        k_group_by_scene<true><<<blocks, kGroupThreads, n * kGroupBytes, st>>>(q, g.off, g.cursor,
+                                                                                             g.block_counts, g.dst);
+    else k_group_by_scene<false><<<blocks, kGroupThreads, 0, st>>>(q, g.off, g.cursor, nullptr, g.dst);
     return cudaGetLastError();
 }
 

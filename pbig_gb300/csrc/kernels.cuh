@@ -254,14 +254,11 @@ struct TuneArgs {
 };
 constexpr size_t kTuneScratchBytes = 256;
 cudaError_t launch_tune_query(const Params& p, const TuneArgs& a, int dims, cudaStream_t st);
-// exclusive scan of nscenes+1 per-scene pair counts (one block)
 // per-scene cell sizes of a batched query (one warp per scene, a strided
 // sample of up to 64 boxes of each scene, T estimated as E^2 / 2C); offs:
 // nscenes+1 box offsets in device memory
 cudaError_t launch_tune_scenes(const uint32_t* boxes, const unsigned long long* offs, uint32_t nscenes, int dims,
                                uint32_t range, SceneTune* out, cudaStream_t st);
-cudaError_t launch_scene_offsets(const Params& p, const unsigned long long* hist, unsigned long long* off,
-                                 uint32_t nscenes_cap, cudaStream_t st);
 // Pairs bound for page-locked host memory are limited by the host link, not
 // by the kernels: with an overlap the small-cell and block kernels run on
 // `side` over side_sms SMs while the medium-cell kernel runs on the others,
@@ -274,9 +271,19 @@ struct PairOverlap {
 };
 
 cudaError_t launch_pairs(const Params& p, int dims, int sm_count, cudaStream_t st, const PairOverlap* ov = nullptr);
-cudaError_t launch_group_by_scene(const Params& p, const unsigned long long* scene_pair_off,
-                                  unsigned long long* scene_cursor, uint2* dst, cudaStream_t st);
-cudaError_t launch_scene_hist(const Params& p, unsigned long long* hist, cudaStream_t st);
+// the pairs of p.out grouped by scene into dst, the scenes' pair offsets on the
+// device and the host, and the end of the query (Params::ctr_host)
+struct GroupArgs {
+    unsigned long long* hist;    // [nscenes + 1] zero
+    unsigned long long* cursor;  // [nscenes + 1] zero
+    unsigned long long* off;     // [nscenes + 1]
+    unsigned long long* off_host;
+    uint32_t* block_counts;      // group_count_bytes(nscenes)
+    uint2* dst;
+    Ctr* ctr_host;
+};
+size_t group_count_bytes(uint32_t nscenes);
+cudaError_t launch_group_by_scene(const Params& p, const GroupArgs& g, cudaStream_t st);
 // p.scene_table for p.nboxes boxes (scene_table_entries of them)
 cudaError_t launch_scene_table(const Params& p, cudaStream_t st);
 uint64_t scene_table_entries(uint64_t nboxes);
