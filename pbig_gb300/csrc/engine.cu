@@ -676,10 +676,12 @@ static int run_batch(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t nboxes, int
 }
 
 // The boxes of a single-scene query: `boxes` on the device, red first and blue
-// behind it. Boxes in page-locked host memory stay there until the count
-// copies them (up_red, up_blue: their device-mapped addresses).
+// behind it, or in an array of their own (`blue`). Boxes in page-locked host
+// memory stay there until the count copies them to `boxes` (up_red, up_blue:
+// their device-mapped addresses).
 struct SingleScene {
     const uint32_t* boxes;
+    const uint32_t* blue;
     const uint32_t* up_red;
     const uint32_t* up_blue;
     uint64_t n_red, n;
@@ -721,6 +723,7 @@ static int run_single(pbig2_ctx* c, const SingleScene& q, uint32_t shift, cudaSt
 
     Params p{};
     p.boxes = q.boxes;
+    p.blue = q.blue;
     p.nboxes = q.n;
     if (q.up_red || q.up_blue) {
         p.up_red = q.up_red;
@@ -741,7 +744,7 @@ static int run_single(pbig2_ctx* c, const SingleScene& q, uint32_t shift, cudaSt
     TuneArgs ta{};
     const bool on_host = q.up_red || q.up_blue;
     ta.red = on_host ? q.up_red : q.boxes;
-    ta.blue = on_host ? q.up_blue : q.boxes + q.n_red * (2 * (uint64_t)q.dims + 1);
+    ta.blue = on_host ? q.up_blue : q.blue ? q.blue : q.boxes + q.n_red * (2 * (uint64_t)q.dims + 1);
     ta.n_red = q.n_red;
     ta.n = q.n;
     ta.bip = q.bip ? 1u : 0u;
@@ -846,39 +849,54 @@ static bool fused_eligible(const pbig2_ctx* c, uint64_t n, int dims, uint32_t ra
     return cell_shift == PBIG2_AUTO || grid_cells(range, cell_shift, dims) <= kFusedMaxCells;
 }
 
-static int fused_query(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t n, int dims, uint32_t range,
-                       uint32_t cell_shift, cudaStream_t st) {
+// a small query small enough to test every pair (a grid of one cell, which a
+// range above 2^31 has not); a caller's class map asks for the grid's passes
+static bool all_pairs_eligible(const pbig2_ctx* c, uint64_t n, uint32_t range, uint32_t cell_shift) {
+    return cell_shift == PBIG2_AUTO && n <= kAllPairsBoxes && range <= (1u << 31) && c->class_map == 0 && !c->want_grid &&
+           !c->fused_stall_test;
+}
+
+// boxes [0, n_red) at red and, for a red/blue query, [n_red, n) at blue
+static int fused_query(pbig2_ctx* c, const uint32_t* red, uint64_t n_red, const uint32_t* blue, uint64_t n, int dims,
+                       uint32_t range, uint32_t cell_shift, cudaStream_t st) {
     c->last_err = 0;
-    const uint64_t cells_cap = cell_shift == PBIG2_AUTO ? kFusedMaxCells : grid_cells(range, cell_shift, dims);
-    void* counts_before = c->d_counts.p;
-    CK(c->d_counts.ensure(cells_cap * 4 + 16, false, st));
-    if (c->d_counts.p != counts_before) c->fused_dirty = true;
-    CK(c->d_state.ensure(kFusedMaxCells / 512 * 4 + 8192 * 4, false, st));  // chunk totals, then small-grid cell ends
+    const bool bip = blue != nullptr, all = all_pairs_eligible(c, n, range, cell_shift);
     CK(c->h_ctr.ensure(sizeof(Ctr)));
-    CK(c->d_scenes.ensure(sizeof(Scene), false, st));
     if (!c->d_bar.p || !c->d_fctr.p) {
         CK(c->d_bar.ensure(sizeof(unsigned int), true, st));
         CK(c->d_fctr.ensure(2 * sizeof(Ctr), true, st));
         c->bar_base = 0;
         c->fused_slot = 0;
     }
-    const uint64_t entry_cap = std::max<uint64_t>({c->fused_entry_hint, 8 * n + 4096, c->d_entries.bytes / sizeof(uint4)});
     const uint64_t out_cap = std::max<uint64_t>({c->out_hint, n * 4, 1u << 16, c->d_out.bytes / 8});
-    const uint64_t task_cap = std::max<uint64_t>(c->d_tasks.bytes / 16, 4096);
     const bool use_ext = c->ext_out != nullptr;
     Ctr* slots = c->d_fctr.as<Ctr>();
     Params p{};
-    p.boxes = d_boxes;
+    p.boxes = red;
+    p.blue = blue;
     p.nboxes = n;
-    p.scenes = c->d_scenes.as<Scene>();
-    p.nscenes = 1;
-    p.split = kNoSplit;
+    p.nscenes = bip ? 2 : 1;
+    p.split = bip ? (uint32_t)n_red : kNoSplit;
     p.max_range = range;
-    p.tile_state = c->d_state.as<unsigned long long>();
     p.class_map = c->class_map ? c->class_map : kClassMapOneLaunch;
-    int rc = ensure_query_buffers(c, p, entry_cap, use_ext ? 1 : out_cap, task_cap, 1, false, st);
-    if (rc) return rc;
     p.ctr = slots + c->fused_slot;
+    int rc;
+    if (all) {
+        CK(c->d_out.ensure(use_ext ? 8 : out_cap * 8, false, st));
+        p.out = c->d_out.as<uint2>();
+        p.out_cap = c->d_out.bytes / 8;
+        p.entry_cap = ~0ull;
+    } else {
+        const uint64_t cells_cap = cell_shift == PBIG2_AUTO ? kFusedMaxCells : grid_cells(range, cell_shift, dims);
+        const uint64_t entry_cap = std::max<uint64_t>({c->fused_entry_hint, 8 * n + 4096, c->d_entries.bytes / sizeof(uint4)});
+        const uint64_t task_cap = std::max<uint64_t>(c->d_tasks.bytes / 16, 4096);
+        void* counts_before = c->d_counts.p;
+        CK(c->d_counts.ensure(cells_cap * 4 + 16, false, st));
+        if (c->d_counts.p != counts_before) c->fused_dirty = true;
+        CK(c->d_state.ensure(kFusedMaxCells / 512 * 4 + 8192 * 4, false, st));  // chunk totals, then small-grid cell ends
+        p.tile_state = c->d_state.as<unsigned long long>();
+        if ((rc = ensure_query_buffers(c, p, entry_cap, use_ext ? 1 : out_cap, task_cap, 1, false, st))) return rc;
+    }
     if (use_ext) {
         p.out = c->ext_out;
         p.out_cap = c->ext_cap;
@@ -890,7 +908,6 @@ static int fused_query(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t n, int di
     c->fused_stall_test = false;
     a.chunk_sum = c->d_state.as<uint32_t>();
     a.ends = c->d_state.as<uint32_t>() + kFusedMaxCells / 512;
-    a.scenes = c->d_scenes.as<Scene>();
     a.ctr_next = slots + (c->fused_slot ^ 1);
     a.zero_cells = c->fused_dirty ? std::min<uint64_t>(kFusedMaxCells, c->d_counts.bytes / 4) : 0;
     a.shift = cell_shift == PBIG2_AUTO ? kFusedTune : cell_shift;
@@ -899,12 +916,30 @@ static int fused_query(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t n, int di
     Ctr* hc = static_cast<Ctr*>(c->h_ctr.p);
     hc->barriers = 0xffffffffu;
     a.ctr_host = hc;
-    CK(launch_fused(p, a, dims, st));
+    if (all) {
+        hc->done = 0;
+        p.ctr_host = hc;
+        CK(launch_all_pairs(p, a.ctr_next, dims, st));
+    } else {
+        CK(launch_fused(p, a, dims, st));
+    }
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail(PBIG2_ECUDA, "one-launch query failed: %s", cudaGetErrorString(e));
     Ctr h{};
     memcpy(&h, hc, sizeof(Ctr));
-    if (h.barriers == 0xffffffffu) {  // no block copied the counters: read them
+    if (all) {  // as a grid of one cell reports itself
+        const uint64_t v = n - h.bad;
+        h.cells = 1;
+        while ((1ull << h.shift) < range) h.shift++;
+        h.entries = v;
+        h.tests = v * (v ? v - 1 : 0) / 2;
+        h.comp_pairs = v >= 2 ? v * v / 2 : 0;
+        h.jobs = v >= 2 ? (v + 255) / 256 : 0;
+        h.max_cell = v >= 2 ? (unsigned)v : 0;
+        h.t_start = h.stamp[kStampStart];
+        h.t_end = h.stamp[kStampEnd];
+        for (auto& s : h.stamp) s = 0;  // (no phases)
+    } else if (h.barriers == 0xffffffffu) {  // no block copied the counters: read them
         CK(cudaMemcpy(&h, p.ctr, sizeof(Ctr), cudaMemcpyDeviceToHost));
         h.err |= kErrWait;
     }
@@ -918,9 +953,13 @@ static int fused_query(pbig2_ctx* c, const uint32_t* d_boxes, uint64_t n, int di
         c->fused_dirty = true;
         return fail(PBIG2_ETIMEOUT, "a bounded device wait gave up (grid barrier of a one-launch query)");
     }
-    c->bar_base += h.barriers * (unsigned int)fused_blocks();
     c->fused_slot ^= 1;
-    c->fused_dirty = false;
+    if (!all) {
+        c->bar_base += h.barriers * (unsigned int)fused_blocks();
+        // (a query left to the regular pipeline touched no counters)
+        if (!(h.err & kErrGridRoom)) c->fused_dirty = false;
+    }
+    if (h.err & kErrGridRoom) return kFusedRedo;
     if (h.err & kErrIndex) return fail(PBIG2_ECUDA, "inconsistent cell lists (error bits 0x%x)", h.err);
     if ((h.err & (kErrEntryOvf | kErrTaskOvf | kErrOutOvf)) || h.entries > p.entry_cap || h.pairs > p.out_cap) {
         c->fused_entry_hint = std::max<uint64_t>(c->fused_entry_hint, h.entries + h.entries / 8 + 4096);
@@ -1066,10 +1105,24 @@ static int self_or_bip(pbig2_ctx* c, const uint32_t* red, uint64_t n_red, const 
     const bool bip = blue != nullptr;
     const uint64_t n = n_red + n_blue;
     const uint32_t* d_boxes = nullptr;
-    if (!bip && fused_eligible(c, n, (int)dims, range, cell_shift)) {
-        int rc = stage_boxes_in(c, red, n * W, loc, st, &d_boxes);
+    // device-resident red and blue boxes stay in their two arrays
+    const bool two = bip && loc == PBIG2_DEVICE;
+    const auto stage = [&]() {
+        if (loc == PBIG2_DEVICE) {
+            d_boxes = red;
+            return (int)PBIG2_OK;
+        }
+        CK(c->d_boxes.ensure(n * W * 4 + 16, false, st));
+        if (n_red) CK(cudaMemcpyAsync(c->d_boxes.p, red, n_red * W * 4, cudaMemcpyHostToDevice, st));
+        if (n_blue) CK(cudaMemcpyAsync(c->d_boxes.as<uint32_t>() + n_red * W, blue, n_blue * W * 4, cudaMemcpyHostToDevice, st));
+        d_boxes = c->d_boxes.as<uint32_t>();
+        return (int)PBIG2_OK;
+    };
+    if (fused_eligible(c, n, (int)dims, range, cell_shift)) {
+        int rc = stage();
         if (rc) return rc;
-        rc = fused_query(c, d_boxes, n, (int)dims, range, cell_shift, st);
+        const uint32_t* d_blue = !bip ? nullptr : two ? blue : d_boxes + n_red * W;
+        rc = fused_query(c, d_boxes, n_red, d_blue, n, (int)dims, range, cell_shift, st);
         if (rc != kFusedRedo) {
             c->scene_shifts.assign(1, c->stats.cell_shift);
             *npairs = c->npairs;
@@ -1084,17 +1137,10 @@ static int self_or_bip(pbig2_ctx* c, const uint32_t* red, uint64_t n_red, const 
     if (fused) {
         CK(c->d_boxes.ensure(n * W * 4 + 16, false, st));
         d_boxes = c->d_boxes.as<uint32_t>();
-    } else if (!bip) {
-        int rc = stage_boxes_in(c, red, n_red * W, loc, st, &d_boxes);
-        if (rc) return rc;
-    } else {
-        CK(c->d_boxes.ensure(n * W * 4 + 16, false, st));
-        const cudaMemcpyKind k = loc == PBIG2_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-        if (n_red) CK(cudaMemcpyAsync(c->d_boxes.p, red, n_red * W * 4, k, st));
-        if (n_blue) CK(cudaMemcpyAsync(c->d_boxes.as<uint32_t>() + n_red * W, blue, n_blue * W * 4, k, st));
-        d_boxes = c->d_boxes.as<uint32_t>();
+    } else if (int rc = stage()) {
+        return rc;
     }
-    const SingleScene q{d_boxes, fused ? m_red : nullptr, fused ? m_blue : nullptr, n_red, n, bip, (int)dims, range};
+    const SingleScene q{d_boxes, two ? blue : nullptr, fused ? m_red : nullptr, fused ? m_blue : nullptr, n_red, n, bip, (int)dims, range};
     uint32_t shift = cell_shift;
     int rc = run_single(c, q, cell_shift, st, &shift);
     if (cell_shift == PBIG2_AUTO && coarser_grid_helps(c, rc)) {
@@ -1176,7 +1222,7 @@ PBIG2_API int pbig2_batch_intersect(pbig2_ctx* c, const uint32_t* boxes, const u
     const auto run = [&]() {
         uint32_t used = 0;
         if (n_scenes > 1) return run_batch(c, d_boxes, n, (int)dims, range, sc, est_e, st);
-        return run_single(c, SingleScene{d_boxes, nullptr, nullptr, n, n, false, (int)dims, range}, sc[0].shift, st, &used);
+        return run_single(c, SingleScene{d_boxes, nullptr, nullptr, nullptr, n, n, false, (int)dims, range}, sc[0].shift, st, &used);
     };
     rc = run();
     // automatic cell sizes: coarser grids for every scene while a box does

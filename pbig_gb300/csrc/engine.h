@@ -113,6 +113,7 @@ struct pbig2_ctx {
     int fused_slot = 0;
     bool fused_dirty = true;     // the counters may hold values another pipeline left (or are new)
     uint64_t fused_entry_hint = 0;
+    bool want_grid = false;      // the running query's cell size is what the caller is after
     bool fused_stall_test = false;  // the next launch's barriers never complete (test of the bounded wait)
     // work-list class map of later queries (PBIG2_OPT_CLASS_MAP; 0: automatic)
     unsigned long long class_map = 0;

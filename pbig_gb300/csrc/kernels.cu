@@ -500,20 +500,6 @@ __global__ void __launch_bounds__(kTuneThreads, 1) k_tune_query(Params p, TuneAr
 // ---------------------------------------------------------------------------
 constexpr int kBoxThreads = 256;
 
-template <int D>
-__device__ __forceinline__ void stage_boxes(const Params& p, uint64_t b0, uint32_t nb, uint32_t* sbox) {
-    constexpr uint32_t W = 2 * D + 1;
-    const uint32_t* src = p.boxes + b0 * W;
-    const uint32_t nwords = nb * W;
-    if (((reinterpret_cast<uintptr_t>(src) & 15u) == 0) && (nwords & 3u) == 0) {
-        const uint4* s4 = reinterpret_cast<const uint4*>(src);
-        uint4* d4 = reinterpret_cast<uint4*>(sbox);
-        for (uint32_t k = threadIdx.x; k < nwords / 4; k += blockDim.x) d4[k] = __ldg(s4 + k);
-    } else {
-        for (uint32_t k = threadIdx.x; k < nwords; k += blockDim.x) sbox[k] = __ldg(src + k);
-    }
-}
-
 __device__ __forceinline__ void copy_words(const uint32_t* src, uint32_t* dst, uint32_t nwords) {
     if ((((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0) && (nwords & 3u) == 0) {
         const uint4* s4 = reinterpret_cast<const uint4*>(src);
@@ -524,22 +510,41 @@ __device__ __forceinline__ void copy_words(const uint32_t* src, uint32_t* dst, u
     }
 }
 
+// a tile of boxes into shared memory: boxes [0, split) at red, the rest at blue
+template <int D>
+__device__ __forceinline__ void stage_two(const uint32_t* red, const uint32_t* blue, uint64_t split, uint64_t b0,
+                                          uint32_t nb, uint32_t* sbox) {
+    constexpr uint32_t W = 2 * D + 1;
+    if (b0 + nb <= split || b0 >= split) {
+        copy_words(b0 < split ? red + b0 * W : blue + (b0 - split) * W, sbox, nb * W);
+    } else {  // the tile straddles red and blue
+        const uint64_t sw = split * W;
+        for (uint32_t k = threadIdx.x; k < nb * W; k += blockDim.x) {
+            const uint64_t gw = b0 * W + k;
+            sbox[k] = gw < sw ? __ldg(red + gw) : __ldg(blue + (gw - sw));
+        }
+    }
+}
+
+template <int D>
+__device__ __forceinline__ void stage_boxes(const Params& p, uint64_t b0, uint32_t nb, uint32_t* sbox) {
+    if (p.blue) stage_two<D>(p.boxes, p.blue, p.split, b0, nb, sbox);
+    else copy_words(p.boxes + b0 * (2 * D + 1), sbox, nb * (2 * D + 1));
+}
+
+// the coordinates of box id, red and blue in one array or two
+template <int D>
+__device__ __forceinline__ const uint32_t* box_row(const uint32_t* boxes, const uint32_t* blue, uint32_t split, uint32_t id) {
+    return blue && id >= split ? blue + (uint64_t)(id - split) * (2 * D + 1) : boxes + (uint64_t)id * (2 * D + 1);
+}
+
 // the count's upload: a tile of boxes from page-locked host memory into
 // shared memory (the host link is the bound, so the count's own work hides
 // under it), then on to the device copy
 template <int D>
 __device__ __forceinline__ void stage_upload(const Params& p, uint64_t b0, uint32_t nb, uint32_t* sbox) {
     constexpr uint32_t W = 2 * D + 1;
-    const uint64_t split = p.up_split;
-    if (b0 + nb <= split || b0 >= split) {
-        copy_words(b0 < split ? p.up_red + b0 * W : p.up_blue + (b0 - split) * W, sbox, nb * W);
-    } else {  // the tile straddles red and blue
-        const uint64_t sw = split * W;
-        for (uint32_t k = threadIdx.x; k < nb * W; k += blockDim.x) {
-            const uint64_t gw = b0 * W + k;
-            sbox[k] = gw < sw ? __ldg(p.up_red + gw) : __ldg(p.up_blue + (gw - sw));
-        }
-    }
+    stage_two<D>(p.up_red, p.up_blue, p.up_split, b0, nb, sbox);
     __syncthreads();
     uint32_t* dst = p.box_copy + b0 * W;
     if (((reinterpret_cast<uintptr_t>(dst) & 15u) == 0) && ((nb * W) & 3u) == 0) {
@@ -1424,15 +1429,15 @@ __device__ __forceinline__ void remit(const Params& p, WarpOut& o, uint32_t ma, 
 
 // the hits of `mask` (bit d: partner slot i + d) that hold on the whole coordinates
 template <int D>
-__device__ __noinline__ uint32_t small_exact(const uint32_t* boxes, uint64_t nboxes, const uint4* s, uint32_t i,
-                                             uint32_t mask) {
+__device__ __noinline__ uint32_t small_exact(const uint32_t* boxes, const uint32_t* blue, uint32_t split,
+                                             uint64_t nboxes, const uint4* s, uint32_t i, uint32_t mask) {
     uint32_t keep = 0;
     while (mask) {
         const uint32_t d = __ffs(mask) - 1;
         mask &= mask - 1;
         const uint32_t a = s[i].w & kIdMask, b = s[i + d].w & kIdMask;
         if (a >= nboxes || b >= nboxes) continue;  // cannot happen with a consistent grid
-        const uint32_t *x = boxes + (uint64_t)a * (2 * D + 1), *y = boxes + (uint64_t)b * (2 * D + 1);
+        const uint32_t *x = box_row<D>(boxes, blue, split, a), *y = box_row<D>(boxes, blue, split, b);
         bool hit = true;
 #pragma unroll
         for (int k = 0; k < D; k++)
@@ -1505,7 +1510,7 @@ __device__ __forceinline__ void small_items(const Params& p, uint4* s, WarpOut& 
         }
         uint32_t mask = ~miss & ~rot & ((2u << nelm) - 2u);
         // a largest sum of 32767 may be two corners of one scaled value
-        if (p.open && top == 0x7fff7fffu && mask) mask = small_exact<D>(p.boxes, p.nboxes, s, gb + r, mask);
+        if (p.open && top == 0x7fff7fffu && mask) mask = small_exact<D>(p.boxes, p.blue, p.split, p.nboxes, s, gb + r, mask);
         __syncwarp();
         if constexpr (REC) {
             auto ploc = [&](uint32_t d) {
@@ -1691,16 +1696,16 @@ __device__ __forceinline__ void tile_group(const Tiles& t, const Row<D>& r, uint
 // the same tile on the whole coordinates: the column boxes pass from lane to
 // lane (rare, so it reads the boxes rather than keep them staged)
 template <int D>
-__device__ __noinline__ uint32_t tile_exact(const uint32_t* boxes, uint64_t nboxes, uint32_t row, uint32_t col,
-                                            uint32_t rows, uint32_t cols) {
+__device__ __noinline__ uint32_t tile_exact(const uint32_t* boxes, const uint32_t* blue, uint32_t split,
+                                            uint64_t nboxes, uint32_t row, uint32_t col, uint32_t rows, uint32_t cols) {
     const uint32_t e = tile_box(lane_id());
     const uint32_t ri = row & kIdMask, ci = col & kIdMask;
     uint32_t a[2 * D], b[2 * D];
     const bool rv = e < rows && ri < nboxes, cv = e < cols && ci < nboxes;
 #pragma unroll
     for (int k = 0; k < 2 * D; k++) {
-        a[k] = rv ? __ldg(boxes + (uint64_t)ri * (2 * D + 1) + k) : 0u;
-        b[k] = cv ? __ldg(boxes + (uint64_t)ci * (2 * D + 1) + k) : 0u;
+        a[k] = rv ? __ldg(box_row<D>(boxes, blue, split, ri) + k) : 0u;
+        b[k] = cv ? __ldg(box_row<D>(boxes, blue, split, ci) + k) : 0u;
     }
     uint32_t mask = 0;
     for (uint32_t j = 0; j < 32; j++) {
@@ -1741,7 +1746,7 @@ __device__ __forceinline__ uint32_t tile_hits(const Params& p, const Tiles& t, c
     if (p.open) {
         const uint32_t low = top ^ 0x7fff7fffu;  // a zero half: a sum of 32767 was the largest of its pair
         if (__any_sync(FULL_MASK, ((low - 0x00010001u) & ~low & 0x80008000u) != 0u))
-            mask = tile_exact<D>(p.boxes, p.nboxes, r.raw, raw, rows, cols);
+            mask = tile_exact<D>(p.boxes, p.blue, p.split, p.nboxes, r.raw, raw, rows, cols);
     }
     const uint32_t m0 = __ballot_sync(FULL_MASK, ((raw >> kIdBits) & 1u) == 0u);
     const uint32_t m1 = __ballot_sync(FULL_MASK, ((raw >> (kIdBits + 1)) & 1u) == 0u);
@@ -2294,6 +2299,114 @@ __global__ void __launch_bounds__(1024) k_scene_offsets(Params pin, const unsign
 
 
 // ---------------------------------------------------------------------------
+// queries of a few thousand boxes: every pair of 32x32 tiles of the boxes,
+// rows in registers, columns in the warp's shared memory, whole coordinates --
+// no grid, no phases to wait for. 1024 boxes take 3.5 us here and took 22 us in
+// the one-launch kernel, most of it latency between its grid barriers. An invalid box (its
+// row then overlaps nothing) is reported by the tile of its row or column
+// against itself (red/blue: by the first tile that it is in).
+// ---------------------------------------------------------------------------
+template <int D>
+struct WholeBox {
+    uint32_t lo[D], hi[D];
+};
+template <int D>
+__device__ __forceinline__ WholeBox<D> whole_box(const Params& p, const uint32_t* boxes, uint32_t i, uint32_t n, bool report) {
+    WholeBox<D> b;
+    uint32_t err = 0;
+    if (i < n) {
+        const uint32_t* r = boxes + (uint64_t)i * (2 * D + 1);
+#pragma unroll
+        for (int d = 0; d < D; d++) {
+            b.lo[d] = __ldg(r + 2 * d);
+            b.hi[d] = __ldg(r + 2 * d + 1);
+        }
+        if (__ldg(r + 2 * D) != i) err |= kErrRid;
+#pragma unroll
+        for (int d = 0; d < D; d++) {
+            if (b.lo[d] >= p.max_range || b.hi[d] >= p.max_range) err |= kErrRange;
+            if (b.lo[d] > b.hi[d]) err |= kErrInverted;
+        }
+        if (err && report) {
+            atomicOr(&p.ctr->err, err);
+            atomicAdd(&p.ctr->bad, 1u);
+        }
+    }
+    if (i >= n || err) {
+#pragma unroll
+        for (int d = 0; d < D; d++) {
+            b.lo[d] = 0xffffffffu;
+            b.hi[d] = 0u;
+        }
+    }
+    return b;
+}
+
+constexpr uint32_t kAllOut = 256;  // per-warp output buffer (pairs)
+
+template <int D, bool BIP>
+__global__ void __launch_bounds__(kPairThreads) k_all_pairs(Params p, Ctr* ctr_next) {
+    __shared__ uint4 s_xy[kPairWarps][32];
+    __shared__ uint2 s_z[kPairWarps][32];
+    __shared__ uint2 s_out[kPairWarps][kAllOut];
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        p.ctr->stamp[kStampStart] = now_ns();
+        *ctr_next = Ctr{};
+    }
+    uint4* xy = s_xy[warp];
+    uint2* zz = s_z[warp];
+    WarpOut o{s_out[warp], 0, kAllOut};
+    const uint32_t n = (uint32_t)p.nboxes, rows = BIP ? p.split : n, cols = BIP ? n - p.split : n;
+    const uint32_t* blue = BIP ? (p.blue ? p.blue : p.boxes + (uint64_t)p.split * (2 * D + 1)) : p.boxes;
+    const uint32_t first = BIP ? p.split : 0u;  // index of the first column
+    const uint32_t R = (rows + 31) >> 5, X = (cols + 31) >> 5;
+    // self: the triangle of tiles x >= r folded into rows of F + 1, F = R
+    // rounded up to an even number: row k and row F - 1 - k together
+    const uint32_t F = (R + 1) & ~1u;
+    const uint32_t tasks = BIP ? R * X : F / 2 * (F + 1);
+    for (uint32_t task = blockIdx.x * kPairWarps + warp; task < tasks; task += gridDim.x * kPairWarps) {
+        uint32_t r, x;
+        if (BIP) {
+            r = task / X;
+            x = task - r * X;
+        } else {
+            const uint32_t k = task / (F + 1), c = task - k * (F + 1);
+            r = c > k ? k : F - 1 - k;
+            x = c > k ? c - 1 : F - 1 - c;
+            if (r >= R || x >= R) continue;
+        }
+        const WholeBox<D> me = whole_box<D>(p, p.boxes, 32 * r + lane, rows, BIP ? x == 0 : x == r);
+        const WholeBox<D> col = whole_box<D>(p, blue, 32 * x + lane, cols, BIP && r == 0);
+        __syncwarp();  // (the last columns are read)
+        xy[lane] = make_uint4(col.lo[0], col.hi[0], col.lo[1], col.hi[1]);
+        if (D == 3) zz[lane] = make_uint2(col.lo[D - 1], col.hi[D - 1]);
+        __syncwarp();
+        uint32_t mask = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 32; j++) {
+            const uint4 c = xy[j];
+            bool hit = me.lo[0] <= c.y && c.x <= me.hi[0] && me.lo[1] <= c.w && c.z <= me.hi[1];
+            if (D == 3) {
+                const uint2 z = zz[j];
+                hit = hit && me.lo[D - 1] <= z.y && z.x <= me.hi[D - 1];
+            }
+            mask |= (hit ? 1u : 0u) << j;
+        }
+        if (!BIP && x == r) mask &= after_lane();
+        const auto id = [&](uint32_t b) { return first + 32 * x + b; };
+        wemit<BIP>(p, o, mask, id, 0u, id, 32 * r + lane);
+    }
+    if (BIP && (R == 0 || X == 0)) {  // one colour: its boxes are still checked
+        const uint32_t count = R ? rows : cols;
+        for (uint32_t i = blockIdx.x * kPairThreads + threadIdx.x; i < count; i += gridDim.x * kPairThreads)
+            whole_box<D>(p, R ? p.boxes : blue, i, count, true);
+    }
+    wflush<BIP, false>(p, o);
+    query_end(p);
+}
+
+// ---------------------------------------------------------------------------
 // one-launch queries of small scenes: a cooperative launch whose blocks run
 // the whole pipeline, phase after phase, separated by grid barriers
 //   P0   every block: the cell size (warp 0 runs the tuner's model on 64
@@ -2320,6 +2433,7 @@ constexpr uint32_t kFusedThreads = 2 * kPairThreads;
 constexpr uint32_t kFusedWarps = kFusedThreads / 32;
 constexpr uint32_t kFusedChunks = (uint32_t)(kFusedMaxCells / kScanChunk);
 constexpr uint32_t kFusedLocalCells = 8192;  // grids of up to 8192 cells: 128-cell chunks, totals per block
+constexpr uint32_t kFusedLeave = 32;  // no cell shift: the query is left to the regular pipeline
 constexpr uint32_t kGridWaitLimit = 1u << 20;  // polls of 64 ns or more: the wait ends after a second at most
 constexpr uint32_t kSmallWarpBytes = kSmallSlots * sizeof(uint4) + kWarpOut * sizeof(uint2);
 static_assert(kFusedChunks % kFusedThreads == 0, "chunk prefixes per thread");
@@ -2352,10 +2466,10 @@ __device__ __forceinline__ bool grid_barrier(const FusedArgs& a, uint32_t k) {
 // on 64 sampled boxes, in single precision over exact integer sums: the one-launch path cannot wait
 // for double-precision divisions. Grids of at most max_cells cells, so a
 // box covers at most max_cells cells and every per-box product fits 32 bits.
-__device__ __forceinline__ uint32_t tune_scene_fast(const uint32_t* boxes, uint64_t n, int dims, uint32_t range,
-                                                    uint64_t max_cells, uint32_t warps) {
+template <int dims, bool BIP>
+__device__ __forceinline__ uint32_t tune_scene_fast(const Params& p, uint32_t range, uint64_t max_cells, uint32_t warps) {
     const uint32_t lane = lane_id();
-    const uint32_t W = 2 * (uint32_t)dims + 1;
+    const uint64_t n = p.nboxes;
     const uint64_t m = n < kTuneRows ? n : kTuneRows;
     uint32_t lo[2][3] = {{0, 0, 0}, {0, 0, 0}}, hi[2][3] = {{0, 0, 0}, {0, 0, 0}};
     bool ok[2] = {false, false};
@@ -2364,7 +2478,7 @@ __device__ __forceinline__ uint32_t tune_scene_fast(const uint32_t* boxes, uint6
     for (int j = 0; j < 2; j++) {
         const uint64_t k = lane + 32u * j;
         if (k >= m) continue;
-        const uint32_t* b = boxes + (k * n / m) * W;
+        const uint32_t* b = box_row<dims>(p.boxes, p.blue, p.split, (uint32_t)(k * n / m));
         bool v = true;
         for (int d = 0; d < dims; d++) {
             lo[j][d] = __ldg(b + 2 * d);
@@ -2383,6 +2497,8 @@ __device__ __forceinline__ uint32_t tune_scene_fast(const uint32_t* boxes, uint6
     const unsigned long long mean = ext / ((good ? good : 1ull) * (unsigned long long)dims);
     const int s0 = mean < 2 ? 0 : 63 - __clzll(mean);
     const int s_win = s0 + 3 < 31 ? s0 + 3 : 31;
+    // red and blue boxes too sparse in their range for these grids: the regular pipeline's
+    if (BIP && tune_grid<dims>(range, (uint32_t)s_win) > max_cells) return kFusedLeave;
     const float scale = (float)n / (float)(m ? m : 1);
     const uint64_t far_cap = n * 64 > 4096 ? n * 64 : 4096;
     float best_cost = 3.0e38f;
@@ -2409,7 +2525,7 @@ __device__ __forceinline__ uint32_t tune_scene_fast(const uint32_t* boxes, uint6
         // (fewer cells than warps leave warps idle: 30 000 boxes of one
         // density took 35 us on 512 cells and 26 us on 4096)
         const float idle = (float)warps > Cf ? (float)warps / Cf : 1.0f;
-        const float cost = (float)kQueryCell * Cf + (float)kQueryEntry * E + (float)kQueryTest * idle * T;
+        const float cost = (float)kQueryCell * Cf + (float)kQueryEntry * E + (BIP ? 0.5f : 1.0f) * (float)kQueryTest * idle * T;
         if (cost < best_cost) {
             best_cost = cost;
             best = (uint32_t)s;
@@ -2423,12 +2539,13 @@ __device__ __forceinline__ uint32_t tune_scene_fast(const uint32_t* boxes, uint6
     return best;
 }
 
-template <int D>
+template <int D, bool BIP>
 __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArgs a) {
     Params p = pin;  // the grid's size is set below
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t s_shift;
-    __shared__ Scene s_scene;
+    __shared__ Scene s_scene[2];
+    __shared__ uint32_t s_off[3];
     __shared__ unsigned long long s_wsum[kFusedWarps];
     __shared__ uint32_t s_csum[kFusedLocalCells / 128];
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
@@ -2446,22 +2563,36 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArg
     // P0
     if (warp == 0) {
         uint32_t sh = a.shift;
-        if (sh == kFusedTune) sh = tune_scene_fast(p.boxes, p.nboxes, D, range, kFusedMaxCells, (uint32_t)nw);
+        if (sh == kFusedTune) sh = tune_scene_fast<D, BIP>(p, range, kFusedMaxCells, (uint32_t)nw);
         if (lane == 0) s_shift = sh;
     }
     __syncthreads();
-    const uint32_t shift = s_shift, nrc = nrc_dev(range, (int)shift);
+    const bool leave = BIP && s_shift == kFusedLeave;  // (the same in every block)
+    const uint32_t shift = leave ? 0u : s_shift, nrc = leave ? 0u : nrc_dev(range, (int)shift);
     p.ncells = D == 3 ? (uint64_t)nrc * nrc * nrc : (uint64_t)nrc * nrc;
-    if (t == 0) s_scene = Scene{0u, (uint32_t)p.nboxes, shift, nrc, 0ull, range, 0u};
+    if (t == 0) {
+        const uint32_t red = BIP ? p.split : (uint32_t)p.nboxes;
+        s_scene[0] = Scene{0u, red, shift, nrc, 0ull, range, 0u};
+        s_off[0] = 0u;
+        s_off[1] = red;
+        if (BIP) {
+            s_scene[1] = Scene{red, (uint32_t)p.nboxes - red, shift, nrc, 0ull, range, 0u};
+            s_off[2] = (uint32_t)p.nboxes;
+        }
+    }
     if (blk == 0 && t == 0) {
         *a.ctr_next = Ctr{};
         p.ctr->cells = p.ncells;
         p.ctr->shift = shift;
-        a.scenes[0] = Scene{0u, (uint32_t)p.nboxes, shift, nrc, 0ull, range, 0u};
+        if (leave) atomicOr(&p.ctr->err, (unsigned)kErrGridRoom);
     }
     __syncthreads();
     p.open = shift >= kOpenShift ? 1u : 0u;
-    p.scenes = &s_scene;  // the count and the scatter read the scene from shared memory
+    p.scenes = s_scene;  // the count and the scatter read the scenes from shared memory
+    p.scene_box_off = s_off;
+    unsigned long long total = 0;
+    bool fits = false;
+    if (!leave) {
     if (a.zero_cells) {
         uint4* c4 = reinterpret_cast<uint4*>(p.counts);
         for (uint64_t i = gt; i < a.zero_cells / 4; i += nt) c4[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -2474,8 +2605,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArg
     FUSED_BARRIER()
     // P2: chunk entry totals and prefixes, then the cells
     uint32_t* pre = reinterpret_cast<uint32_t*>(smem_raw);
-    unsigned long long total = 0;
-    bool fits;
     if (p.ncells <= kFusedLocalCells) {
         const uint32_t nch = (uint32_t)((p.ncells + 127) / 128);
         for (uint32_t ch = warp; ch < nch; ch += kFusedWarps) {
@@ -2571,6 +2700,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArg
         box_pass<D, true, false, kFusedThreads>(pe, sbox, blk, nblk);
     }
     FUSED_BARRIER()
+    }
 #undef FUSED_BARRIER
     // P4: the counters zeroed for the next launch (the pair passes read the
     // work lists, not the counters), then the pairs
@@ -2581,12 +2711,12 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArg
     }
     if (fits) {
         uint4* ws = reinterpret_cast<uint4*>(smem_raw + warp * kSmallWarpBytes);
-        small_pass<D, false, false, true>(p, ws, reinterpret_cast<uint2*>(ws + kSmallSlots), gw, nw);
+        small_pass<D, BIP, false, true>(p, ws, reinterpret_cast<uint2*>(ws + kSmallSlots), gw, nw);
         __syncthreads();
-        med_pass<D, false, false, true>(p, smem_raw + warp * kMedWarpBytes, gw, nw);
+        med_pass<D, BIP, false, true>(p, smem_raw + warp * kMedWarpBytes, gw, nw);
         __syncthreads();
         constexpr uint32_t kTeams = kFusedThreads / kTeamThreads;
-        team_pass<D, false, false, true, true>(p, reinterpret_cast<TeamSmem*>(smem_raw)[t / kTeamThreads],
+        team_pass<D, BIP, false, true, true>(p, reinterpret_cast<TeamSmem*>(smem_raw)[t / kTeamThreads],
                                                blk * kTeams + t / kTeamThreads, nblk * kTeams);
     }
     // the last block to finish copies the run counters to the host (one
@@ -2638,23 +2768,40 @@ static size_t fused_smem() {
 
 int fused_blocks() { return g_fused_blocks; }
 
-template <int D>
+cudaError_t launch_all_pairs(const Params& p, Ctr* ctr_next, int dims, cudaStream_t st) {
+    const uint64_t red = p.split == kNoSplit ? p.nboxes : p.split, blue = p.nboxes - (p.split == kNoSplit ? 0 : p.split);
+    const uint64_t R = (red + 31) / 32, X = (blue + 31) / 32;
+    const uint64_t tiles = p.split == kNoSplit ? R * (R + 1) / 2 : R * X, cap = (uint64_t)(g_sm_count > 0 ? g_sm_count : 152) * 2;
+    const uint64_t b = (tiles + kPairWarps - 1) / kPairWarps;
+    const unsigned g = (unsigned)(b < cap ? (b ? b : 1) : cap);
+    if (p.split != kNoSplit) {
+        if (dims == 2) k_all_pairs<2, true><<<g, kPairThreads, 0, st>>>(p, ctr_next);
+        else k_all_pairs<3, true><<<g, kPairThreads, 0, st>>>(p, ctr_next);
+    } else {
+        if (dims == 2) k_all_pairs<2, false><<<g, kPairThreads, 0, st>>>(p, ctr_next);
+        else k_all_pairs<3, false><<<g, kPairThreads, 0, st>>>(p, ctr_next);
+    }
+    return cudaGetLastError();
+}
+
+template <int D, bool B>
 static cudaError_t launch_fused_t(const Params& p, const FusedArgs& a, cudaStream_t st) {
     Params pp = p;
     FusedArgs aa = a;
     void* args[] = {&pp, &aa};
-    return cudaLaunchCooperativeKernel((const void*)k_fused<D>, dim3((unsigned)g_fused_blocks), dim3(kFusedThreads),
+    return cudaLaunchCooperativeKernel((const void*)k_fused<D, B>, dim3((unsigned)g_fused_blocks), dim3(kFusedThreads),
                                       args, fused_smem(), st);
 }
 
 cudaError_t launch_fused(const Params& p, const FusedArgs& a, int dims, cudaStream_t st) {
     if (g_fused_blocks <= 0) return cudaErrorNotSupported;
-    return dims == 2 ? launch_fused_t<2>(p, a, st) : launch_fused_t<3>(p, a, st);
+    if (p.split != kNoSplit) return dims == 2 ? launch_fused_t<2, true>(p, a, st) : launch_fused_t<3, true>(p, a, st);
+    return dims == 2 ? launch_fused_t<2, false>(p, a, st) : launch_fused_t<3, false>(p, a, st);
 }
 
-template <int D>
+template <int D, bool B>
 static cudaError_t init_fused() {
-    return cudaFuncSetAttribute(k_fused<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem());
+    return cudaFuncSetAttribute(k_fused<D, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem());
 }
 
 cudaError_t kernels_init() {
@@ -2682,13 +2829,15 @@ cudaError_t kernels_init() {
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pairs_block<3, false>, kTeamThreads, sizeof(TeamSmem))) != cudaSuccess) return e;
     g_blocks_block = nb > 0 ? nb : 1;
     // one-launch queries: one block per SM, all resident (cooperative launch)
-    if ((e = init_fused<2>()) != cudaSuccess) return e;
-    if ((e = init_fused<3>()) != cudaSuccess) return e;
+    if ((e = init_fused<2, false>()) != cudaSuccess) return e;
+    if ((e = init_fused<3, false>()) != cudaSuccess) return e;
+    if ((e = init_fused<2, true>()) != cudaSuccess) return e;
+    if ((e = init_fused<3, true>()) != cudaSuccess) return e;
     {
         int dev = 0, coop = 0, nf = 0;
         if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
         if ((e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev)) != cudaSuccess) return e;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nf, k_fused<3>, kFusedThreads, fused_smem())) !=
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nf, k_fused<3, true>, kFusedThreads, fused_smem())) !=
             cudaSuccess)
             return e;
         g_fused_blocks = coop && nf >= 1 ? g_sm_count : 0;

@@ -179,6 +179,7 @@ struct RunDims {
 
 struct Params {
     const uint32_t* boxes;        // RectInfo records, 2*D+1 words each
+    const uint32_t* blue;         // red/blue boxes in two arrays: the blue ones ([split, nboxes)); null: in boxes
     uint64_t nboxes;              // boxes over all scenes
     const Scene* scenes;          // scene table (device)
     const uint32_t* scene_box_off;// nscenes+1 box offsets (device)
@@ -295,28 +296,37 @@ size_t pair_smem_bytes();
 cudaError_t kernels_init();
 
 // ---- one-launch queries of small scenes -----------------------------------
-// A self query of at most kFusedMaxBoxes boxes runs as one cooperative
-// launch: the cell size (chosen on the device when `shift` is kFusedTune,
-// grids of at most kFusedMaxCells cells), the count, the scan, the scatter
-// and every pair pass, separated by grid barriers whose waits are bounded
-// (kErrWait). p must carry the device boxes, counts (kFusedMaxCells or the
-// given grid), entries, lists, tasks, out and ctr, whose counters must be
-// zero at launch; the kernel zeroes ctr_next for the launch after it, writes
-// the chosen grid (ctr->cells, ctr->shift) and the scene table for the host,
+// A self or red/blue query of at most kFusedMaxBoxes boxes runs as one
+// cooperative launch: the cell size (chosen on the device when `shift` is
+// kFusedTune, grids of at most kFusedMaxCells cells; red and blue boxes too
+// sparse for those set kErrGridRoom and are left to the regular pipeline), the
+// count, the scan, the scatter and every pair pass, separated by grid barriers
+// whose waits are bounded (kErrWait). p must carry the device boxes, counts
+// (kFusedMaxCells or the given grid), entries, lists, tasks, out and ctr, whose
+// counters must be zero at launch; the kernel zeroes ctr_next for the launch
+// after it, writes the chosen grid (ctr->cells, ctr->shift) for the host,
 // leaves the counters of its grid zero, and its last block to finish copies
 // the run counters to ctr_host with the number of barrier arrivals per block
-// the launch made (ctr_host->barriers; unchanged when a wait gave up). Counters that may hold anything else (another pipeline
-// used them, or they are new) are zeroed first when zero_cells says so.
+// the launch made (ctr_host->barriers; unchanged when a wait gave up). Counters
+// that may hold anything else (another pipeline used them, or they are new) are
+// zeroed first when zero_cells says so.
+//
+// Of at most kAllPairsBoxes boxes every pair is tested, as on a grid of one
+// cell, in an ordinary launch: p's boxes, out, ctr and ctr_host are used, and
+// the slots of run counters as above.
 constexpr uint64_t kFusedMaxBoxes = 1u << 18;
 constexpr uint64_t kFusedMaxCells = 1u << 20;
 constexpr uint32_t kFusedTune = 0xffffffffu;
+// (per query with the call around it, three-dimensional scenes of one density,
+// all pairs against the grid: 32 against 51 us of 1024 boxes, 38 against 51 of
+// 4096, 47 against 52 of 6144, 59 against 53 of 8192; red and blue cross at 12288)
+constexpr uint64_t kAllPairsBoxes = 6144;
 
 struct FusedArgs {
     unsigned int* bar;        // arrival counter of the grid barriers (only ever increases)
     unsigned int bar_base;    // its value when the launch starts
     uint32_t* chunk_sum;      // entry totals of 512-cell chunks (kFusedMaxCells / 512 words)
     uint32_t* ends;           // cell ends of grids of at most 8192 cells (8192 words)
-    Scene* scenes;            // the scene table for the host, written by the kernel
     Ctr* ctr_next;            // the run counters of the next launch (zeroed by this one)
     Ctr* ctr_host;            // page-locked host copy of the final counters, written by the last block
     uint64_t zero_cells;      // counters to zero before the count (0: they are zero)
@@ -325,5 +335,6 @@ struct FusedArgs {
 // blocks of a one-launch query (0: not available on this device)
 int fused_blocks();
 cudaError_t launch_fused(const Params& p, const FusedArgs& a, int dims, cudaStream_t st);
+cudaError_t launch_all_pairs(const Params& p, Ctr* ctr_next, int dims, cudaStream_t st);
 
 }  // namespace pbig

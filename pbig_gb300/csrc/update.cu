@@ -521,7 +521,9 @@ PBIG2_API int pbig2_scene_create(pbig2_ctx* c, const uint32_t* boxes, uint64_t n
     if (n == 0 || n > (uint64_t)kIdMask + 1) return api_fail(PBIG2_EINVAL, "a scene holds 1 .. 2^29 boxes");
     // the full query first: its pairs, its cell size, and the input checks
     uint64_t np = 0;
+    c->want_grid = true;
     int rc = pbig2_self_intersect(c, boxes, n, dims, range, cell_shift, boxes_loc, nullptr, &np);
+    c->want_grid = false;
     if (rc != PBIG2_OK) return rc == PBIG2_EINPUT ? api_fail(PBIG2_EINPUT, "a scene's boxes must all be valid") : rc;
     pbig2_stats st{};
     pbig2_get_stats(c, &st);
