@@ -602,51 +602,64 @@ __device__ __forceinline__ uint32_t term_cut(uint32_t w, bool starts, bool ends)
     return (starts ? w & 0xffff0000u : 0u) | (ends ? w & 0xffffu : kTermBeyond);
 }
 
+// a box's cells: cnt of them, sx along x and sy along y, from cell `base` of a
+// grid of nrc cells per axis; none of an invalid box
+struct BoxCells {
+    uint32_t cnt = 0, sx = 1, sy = 1, nrc = 0;
+    uint64_t base = 0;
+};
+// b: the box's row in shared memory (TERMS: it becomes the box's terms, one
+// word per axis); REPORT: an invalid box is counted
+template <int D, bool TERMS, bool REPORT>
+__device__ __forceinline__ BoxCells box_cells(const Params& p, uint32_t* b, uint64_t gi) {
+    BoxCells c;
+    const Scene sc = p.scenes[find_scene(p, gi)];
+    uint32_t err = 0;
+#pragma unroll
+    for (int d = 0; d < D; d++) {
+        if (b[2 * d] >= sc.range || b[2 * d + 1] >= sc.range) err |= kErrRange;
+        if (b[2 * d] > b[2 * d + 1]) err |= kErrInverted;
+    }
+    if (b[2 * D] != (uint32_t)(gi - sc.box_off)) err |= kErrRid;
+    if (gi > kIdMask) err |= kErrIndex;
+    if (!err) {
+        const uint32_t sh = sc.shift;
+        const uint32_t lo0 = b[0] >> sh, lo1 = b[2] >> sh, lo2 = D == 3 ? (b[4] >> sh) : 0u;
+        const uint32_t sx = (b[1] >> sh) - lo0 + 1, sy = (b[3] >> sh) - lo1 + 1;
+        const uint32_t sz = D == 3 ? (b[5] >> sh) - lo2 + 1 : 1u;
+        const uint64_t c64 = (uint64_t)sx * sy * sz;
+        if (c64 >= (1ull << 26)) {
+            err |= kErrCellOvf;
+        } else {
+            c.cnt = (uint32_t)c64;
+            c.sx = sx;
+            c.sy = sy;
+            c.nrc = sc.nrc;
+            c.base = sc.cell_off + ((uint64_t)lo2 * c.nrc + lo1) * c.nrc + lo0;
+            if (TERMS) {
+                const uint32_t low = (1u << sh) - 1u;
+#pragma unroll
+                for (int d = 0; d < D; d++)
+                    b[d] = term_word(term_scale(b[2 * d] & low, sh), term_scale(b[2 * d + 1] & low, sh));
+            }
+        }
+    }
+    if (err && REPORT) {
+        atomicOr(&p.ctr->err, err);
+        atomicAdd(&p.ctr->bad, 1u);
+    }
+    return c;
+}
+
 // (scatter: the boxes' rows in sbox are overwritten)
 template <int D, bool SCATTER, bool MERGED>
 __device__ __forceinline__ void enumerate_cells(const Params& p, uint32_t* sbox, uint64_t b0, uint32_t nb) {
     constexpr uint32_t W = 2 * D + 1;
     const uint32_t t = threadIdx.x, lane = t & 31u;
-    const uint64_t gi = b0 + t;
-    uint32_t cnt = 0, sx = 1, sy = 1, nrc = 0;
-    uint64_t base = 0;
-    if (t < nb) {
-        uint32_t* b = sbox + t * W;
-        const Scene sc = p.scenes[find_scene(p, gi)];
-        uint32_t err = 0;
-#pragma unroll
-        for (int d = 0; d < D; d++) {
-            if (b[2 * d] >= sc.range || b[2 * d + 1] >= sc.range) err |= kErrRange;
-            if (b[2 * d] > b[2 * d + 1]) err |= kErrInverted;
-        }
-        if (b[2 * D] != (uint32_t)(gi - sc.box_off)) err |= kErrRid;
-        if (gi > kIdMask) err |= kErrIndex;
-        if (!err) {
-            const uint32_t sh = sc.shift;
-            const uint32_t lo0 = b[0] >> sh, lo1 = b[2] >> sh, lo2 = D == 3 ? (b[4] >> sh) : 0u;
-            sx = (b[1] >> sh) - lo0 + 1;
-            sy = (b[3] >> sh) - lo1 + 1;
-            const uint32_t sz = D == 3 ? (b[5] >> sh) - lo2 + 1 : 1u;
-            const uint64_t c64 = (uint64_t)sx * sy * sz;
-            if (c64 >= (1ull << 26)) {
-                err |= kErrCellOvf;
-            } else {
-                cnt = (uint32_t)c64;
-                nrc = sc.nrc;
-                base = sc.cell_off + ((uint64_t)lo2 * nrc + lo1) * nrc + lo0;
-                if (SCATTER && !MERGED) {  // the row becomes the box's terms, one word per axis
-                    const uint32_t low = (1u << sh) - 1u;
-#pragma unroll
-                    for (int d = 0; d < D; d++)
-                        b[d] = term_word(term_scale(b[2 * d] & low, sh), term_scale(b[2 * d + 1] & low, sh));
-                }
-            }
-        }
-        if (err && !SCATTER) {
-            atomicOr(&p.ctr->err, err);
-            atomicAdd(&p.ctr->bad, 1u);
-        }
-    }
+    BoxCells c;
+    if (t < nb) c = box_cells<D, SCATTER && !MERGED, !SCATTER>(p, sbox + t * W, b0 + t);
+    const uint32_t cnt = c.cnt, sx = c.sx, sy = c.sy, nrc = c.nrc;
+    const uint64_t base = c.base;
     if (SCATTER) __syncwarp();
     const uint32_t incl = warp_incl_scan(cnt);
     const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
@@ -753,11 +766,11 @@ __global__ void k_zero_counts(Params pin) {
     for (uint64_t i = t; i < r4; i += stride) s4[i] = make_uint4(0, 0, 0, 0);
 }
 
-// tiles of TILE boxes: blk, blk + nblk, ... (blockDim.x == TILE)
-template <int D, bool SCATTER, bool MERGED, uint32_t TILE = kBoxThreads>
+// tiles of kBoxThreads boxes: blk, blk + nblk, ...
+template <int D, bool SCATTER, bool MERGED>
 __device__ __forceinline__ void box_pass(const Params& p, uint32_t* sbox, uint64_t blk, uint64_t nblk) {
-    for (uint64_t b0 = blk * TILE; b0 < p.nboxes; b0 += nblk * TILE) {
-        const uint32_t nb = (uint32_t)mn64(TILE, p.nboxes - b0);
+    for (uint64_t b0 = blk * kBoxThreads; b0 < p.nboxes; b0 += nblk * kBoxThreads) {
+        const uint32_t nb = (uint32_t)mn64(kBoxThreads, p.nboxes - b0);
         if (!SCATTER && p.box_copy) stage_upload<D>(p, b0, nb, sbox);
         else stage_boxes<D>(p, b0, nb, sbox);
         __syncthreads();
@@ -778,17 +791,20 @@ __global__ void __launch_bounds__(kBoxThreads) k_count(Params pin) {
 // ---------------------------------------------------------------------------
 constexpr uint32_t kTaskCols = 8;
 
-// a run counter that a pass reads: FRESH (one-launch queries, where phases
-// of the same kernel change the counters) reads it past L1; the separate
-// kernels of the regular pipeline read it plainly (a load past L1 there
-// measured 20 % slower medium-cell and twice slower block passes)
+// the size of a work list (kNumLists: the tile tasks) that a pass reads.
+// FRESH: one-launch queries, where the counters change while the kernel runs;
+// they are read past L1 once, together, before the passes (a read in each pass
+// was half a microsecond each time). The separate kernels read them plainly.
 template <bool FRESH>
-__device__ __forceinline__ uint32_t ctr_read(const unsigned int* a) { return FRESH ? __ldcg(a) : *a; }
+__device__ __forceinline__ uint32_t list_size(const Params& p, int k) {
+    if (FRESH) return p.list_sizes[k];
+    return k < kNumLists ? p.ctr->n_list[k] : p.ctr->need_tasks;
+}
 
 // huge cells i0, i0 + stride, ...
 template <bool FRESH = false>
 __device__ __forceinline__ void expand_cells(const Params& p, uint32_t i0, uint32_t stride) {
-    const uint32_t nh = mn64(ctr_read<FRESH>(&p.ctr->n_list[kListHuge]), p.list_cap[kListHuge]);
+    const uint32_t nh = mn64(FRESH ? __ldcg(&p.ctr->n_list[kListHuge]) : p.ctr->n_list[kListHuge], p.list_cap[kListHuge]);
     for (uint32_t i = i0; i < nh; i += stride) {
         const uint2 sn = p.lists[p.list_off[kListHuge] + i];
         const uint32_t n = sn.y;
@@ -1452,7 +1468,7 @@ __device__ __forceinline__ void small_items(const Params& p, uint4* s, WarpOut& 
                                             uint64_t stride) {
     constexpr uint32_t G = 32 / WG;
     const uint32_t lane = lane_id(), g = lane / WG, r = lane % WG, gb = g * (2 * WG);
-    const uint64_t nl = mn64(ctr_read<FRESH>(&p.ctr->n_list[list]), p.list_cap[list]);
+    const uint64_t nl = mn64(list_size<FRESH>(p, list), p.list_cap[list]);
     const uint64_t nitems = (nl + G - 1) / G;
     // a batch's warp takes items next to each other, so that its pairs leave it
     // in long runs of one scene (4 % slower here than every stride-th item, and
@@ -1829,7 +1845,7 @@ __device__ __forceinline__ void med_pass(const Params& p, unsigned char* wsm, ui
     const uint32_t lane = lane_id();
     const Tiles t(wsm, kMedTiles);
     WarpOut o{reinterpret_cast<uint2*>(wsm + kMedTiles * kTileBytes), 0, kMedOut};
-    const uint64_t nl = mn64(ctr_read<FRESH>(&p.ctr->n_list[kListMed]), p.list_cap[kListMed]);
+    const uint64_t nl = mn64(list_size<FRESH>(p, kListMed), p.list_cap[kListMed]);
     auto cell = [&](uint64_t item) {
         const uint2 sn = p.lists[p.list_off[kListMed] + item];
         const uint32_t gid = sn.x;  // record mode: the cell id (its start is in the counters)
@@ -2062,8 +2078,8 @@ template <int D, bool BIP, bool REC, bool FRESH = false, bool SUB = false>
 __device__ __forceinline__ void team_pass(const Params& p, TeamSmem& s, uint64_t team, uint64_t nteam) {
     const uint32_t tid = threadIdx.x % kTeamThreads, warp = tid >> 5;
     WarpOut o{s.out[warp], 0, kMedOut};
-    const uint64_t nb = mn64(ctr_read<FRESH>(&p.ctr->n_list[kListBig]), p.list_cap[kListBig]);
-    const uint64_t nt = mn64(ctr_read<FRESH>(&p.ctr->need_tasks), p.task_cap);
+    const uint64_t nb = mn64(list_size<FRESH>(p, kListBig), p.list_cap[kListBig]);
+    const uint64_t nt = mn64(list_size<FRESH>(p, kNumLists), p.task_cap);
     uint64_t item = team;
     auto fetch = [&]() {
         if (!FRESH) item = atomicAdd(&p.ctr->big_next, 1u);
@@ -2462,6 +2478,77 @@ __device__ __forceinline__ bool grid_barrier(const FusedArgs& a, uint32_t k) {
     return s_ok != 0u;
 }
 
+// The count and the scatter of a one-launch query. A block takes an even part
+// of the boxes (at most kFusedThreads at a time) and deals their cells out over
+// all its threads, so that a warp whose boxes cover hundreds of cells each does
+// not keep the next barrier waiting: on 50 000 red and blue boxes, one in a
+// hundred of them large, the last warp of the scatter came 16 us after the
+// first (50 us the kernel, 33 with the cells dealt out). A part that is one tile
+// stays in shared memory from the count to the scatter.
+struct DealtTile {
+    uint32_t* rows;  // the boxes' rows, then terms
+    uint4* box;      // {first cell, cells along x | along y << 16, and their multipliers}
+    uint32_t* ends;  // cells of the boxes up to and with this one
+    uint32_t* warp;  // [kFusedThreads / 32]
+};
+constexpr uint32_t kDealtBytes = kFusedThreads * (7 * sizeof(uint32_t) + sizeof(uint4) + sizeof(uint32_t)) + kFusedWarps * sizeof(uint32_t);
+__device__ __forceinline__ DealtTile dealt_tile(unsigned char* m) {
+    DealtTile s;
+    s.box = reinterpret_cast<uint4*>(m);
+    s.rows = reinterpret_cast<uint32_t*>(s.box + kFusedThreads);
+    s.ends = s.rows + 7 * kFusedThreads;
+    s.warp = s.ends + kFusedThreads;
+    return s;
+}
+
+// boxes [b0, b0 + nb) into the tile; their cells in all
+template <int D, bool REPORT>
+__device__ __forceinline__ uint32_t deal_boxes(const Params& p, const DealtTile& s, uint64_t b0, uint32_t nb) {
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    __syncthreads();  // (the last tile is read)
+    stage_boxes<D>(p, b0, nb, s.rows);
+    __syncthreads();
+    BoxCells c;
+    if (t < nb) c = box_cells<D, true, REPORT>(p, s.rows + t * (2 * D + 1), b0 + t);
+    // (grids of at most 2^20 cells: cells, and cells per axis, in 32 and 16 bits)
+    s.box[t] = make_uint4((uint32_t)c.base, c.sx | c.sy << 16, magic_of(c.sx), magic_of(c.sy));
+    const uint32_t incl = warp_incl_scan(c.cnt);
+    if (lane == 31) s.warp[warp] = incl;
+    __syncthreads();
+    const uint32_t w = lane < kFusedWarps ? s.warp[lane] : 0u, upto = warp_incl_scan(w);
+    s.ends[t] = incl + __shfl_sync(FULL_MASK, upto - w, warp);
+    __syncthreads();
+    return __shfl_sync(FULL_MASK, upto, 31);
+}
+
+template <int D, bool SCATTER>
+__device__ __forceinline__ void deal_cells(const Params& p, const DealtTile& s, uint64_t b0, uint32_t total, uint32_t nrc) {
+    for (uint32_t e = threadIdx.x; e < total; e += kFusedThreads) {
+        uint32_t o = 0;  // the box: the first whose end lies beyond e
+#pragma unroll
+        for (uint32_t step = kFusedThreads / 2; step; step >>= 1)
+            if (s.ends[o + step - 1] <= e) o += step;
+        const uint32_t lq = e - (o ? s.ends[o - 1] : 0u), cnt = s.ends[o] - (o ? s.ends[o - 1] : 0u);
+        const uint4 b = s.box[o];
+        const uint32_t sx = b.y & 0xffffu, sy = b.y >> 16;
+        const uint32_t rr = div_magic(lq, sx, b.z), i = lq - rr * sx;
+        const uint32_t k = div_magic(rr, sy, b.w), j = rr - k * sy;
+        const uint32_t gid = b.x + (k * nrc + j) * nrc + i;
+        if (SCATTER) {
+            const uint32_t* ob = s.rows + o * (2 * D + 1);
+            const uint32_t f = (i == 0 ? 1u : 0u) | (j == 0 ? 2u : 0u) | ((D == 2 || k == 0) ? 4u : 0u);
+            const uint4 rec = make_uint4(term_cut(ob[0], i == 0, i + 1 == sx), term_cut(ob[1], j == 0, j + 1 == sy),
+                                         D == 3 ? term_cut(ob[2], k == 0, lq + sx * sy >= cnt) : 0u,
+                                         (f << kIdBits) | (uint32_t)(b0 + o));
+            const uint32_t pos = atomicSub(&p.counts[gid], 1u) - 1u;
+            if (pos < p.entry_cap) p.entries[pos] = rec;
+            else atomicOr(&p.ctr->err, kErrEntryOvf);
+        } else {
+            atomicAdd(&p.counts[gid], 1u);
+        }
+    }
+}
+
 // the query's cost model for one scene of n boxes at row 0, with T = E^2 / 2C
 // on 64 sampled boxes, in single precision over exact integer sums: the one-launch path cannot wait
 // for double-precision divisions. Grids of at most max_cells cells, so a
@@ -2600,11 +2687,17 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArg
         FUSED_BARRIER()
     }
     // P1: count
-    uint32_t* sbox = reinterpret_cast<uint32_t*>(smem_raw);
-    box_pass<D, false, false, kFusedThreads>(p, sbox, blk, nblk);
+    const DealtTile tile = dealt_tile(smem_raw);
+    const uint64_t part = ((p.nboxes + nblk - 1) / nblk + 3) & ~3ull;  // (parts begin at multiples of 16 bytes)
+    const uint64_t part0 = mn64(blk * part, p.nboxes), part1 = mn64(part0 + part, p.nboxes);
+    uint32_t dealt = 0;
+    for (uint64_t b0 = part0; b0 < part1; b0 += kFusedThreads) {
+        dealt = deal_boxes<D, true>(p, tile, b0, (uint32_t)mn64(kFusedThreads, part1 - b0));
+        deal_cells<D, false>(p, tile, b0, dealt, nrc);
+    }
     FUSED_BARRIER()
     // P2: chunk entry totals and prefixes, then the cells
-    uint32_t* pre = reinterpret_cast<uint32_t*>(smem_raw);
+    uint32_t* pre = reinterpret_cast<uint32_t*>(smem_raw + kDealtBytes);  // (the tile stays)
     if (p.ncells <= kFusedLocalCells) {
         const uint32_t nch = (uint32_t)((p.ncells + 127) / 128);
         for (uint32_t ch = warp; ch < nch; ch += kFusedWarps) {
@@ -2697,7 +2790,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArg
         expand_cells<true>(p, (uint32_t)gt, (uint32_t)nt);
         Params pe = p;
         if (p.ncells <= kFusedLocalCells) pe.counts = a.ends;
-        box_pass<D, true, false, kFusedThreads>(pe, sbox, blk, nblk);
+        for (uint64_t b0 = part0; b0 < part1; b0 += kFusedThreads) {
+            if (part > kFusedThreads) dealt = deal_boxes<D, false>(pe, tile, b0, (uint32_t)mn64(kFusedThreads, part1 - b0));
+            deal_cells<D, true>(pe, tile, b0, dealt, nrc);
+        }
     }
     FUSED_BARRIER()
     }
@@ -2709,6 +2805,11 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArg
         for (uint64_t i = gt; i < p.ncells / 4; i += nt) c4[i] = make_uint4(0u, 0u, 0u, 0u);
         for (uint64_t i = 4 * (p.ncells / 4) + gt; i < p.ncells; i += nt) p.counts[i] = 0u;
     }
+    __shared__ uint32_t s_sizes[kNumLists + 1];
+    p.list_sizes = s_sizes;
+    if (t <= (uint32_t)kNumLists)
+        s_sizes[t] = __ldcg(t < (uint32_t)kNumLists ? &p.ctr->n_list[t] : &p.ctr->need_tasks);
+    __syncthreads();  // (the sizes are there and the tile is read)
     if (fits) {
         uint4* ws = reinterpret_cast<uint4*>(smem_raw + warp * kSmallWarpBytes);
         small_pass<D, BIP, false, true>(p, ws, reinterpret_cast<uint2*>(ws + kSmallSlots), gw, nw);
@@ -2761,8 +2862,7 @@ static size_t fused_smem() {
     const size_t team = sizeof(TeamSmem) * (kFusedThreads / kTeamThreads);
     b = b > team ? b : team;
     b = b > (size_t)kFusedWarps * kSmallWarpBytes ? b : (size_t)kFusedWarps * kSmallWarpBytes;
-    b = b > (size_t)kFusedChunks * 4 ? b : (size_t)kFusedChunks * 4;
-    b = b > (size_t)kFusedThreads * 7 * 4 ? b : (size_t)kFusedThreads * 7 * 4;
+    b = b > kDealtBytes + (size_t)kFusedChunks * 4 ? b : kDealtBytes + (size_t)kFusedChunks * 4;
     return b;
 }
 

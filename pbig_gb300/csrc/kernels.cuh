@@ -195,6 +195,7 @@ struct Params {
     uint2* lists;                 // kNumLists regions of {start, n}
     uint64_t list_off[kNumLists]; // region offsets into lists
     uint64_t list_cap[kNumLists];
+    const uint32_t* list_sizes;   // one-launch queries, pair passes: the lists' sizes, then the tile tasks'
     uint4* tasks;                 // huge-cell tile tasks {start, n, r, x0}
     uint64_t task_cap;
     unsigned long long* tile_state; // scan tile records (kTileRecBytes per kTileCells cells)

@@ -134,3 +134,37 @@ def test_red_and_blue_in_one_launch(engine, n):
         assert engine.stats()["kernels"] == 1
         got = engine.pairs().astype(np.int64)
         assert np.array_equal(got[np.lexsort((got[:, 1], got[:, 0]))], want), nr
+
+
+def uneven(n, dims, rng, seed):
+    """Small boxes, and one in 700 that covers a third of the range along one axis
+    (hundreds of cells, all of one warp's boxes small but one)."""
+    rs = np.random.default_rng(seed)
+    rows = scene(n, dims, rng, seed)
+    for k in rs.choice(n, max(1, n // 700), replace=False):
+        a = int(rs.integers(0, dims))
+        rows[k, 2 * a] = rs.integers(0, rng // 2)
+        rows[k, 2 * a + 1] = rows[k, 2 * a] + rng // 3
+    return rows
+
+
+@pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("n", [6145, 77824, 77825, 100000, 262144])
+def test_boxes_of_very_different_cell_counts_in_one_launch(engine, n, dims):
+    """Parts of the boxes below, at and above a block's tile of 512 on 152 SMs."""
+    rng = 1 << 24
+    boxes = uneven(n, dims, rng, n + dims)
+    red, blue = boxes[:n // 3].copy(), boxes[n // 3:].copy()
+    red[:, -1], blue[:, -1] = np.arange(len(red)), np.arange(len(blue))
+    want = O.grid_pairs(boxes, rng)[0] if n > 20000 else O.brute_pairs(boxes)
+    w = want.astype(np.int64)
+    w = w[(w[:, 0] < len(red)) & (w[:, 1] >= len(red))] - [0, len(red)]
+    for _ in range(2):
+        assert engine.self_intersect(boxes, rng) == len(want)
+    assert engine.stats()["kernels"] == 1
+    assert np.array_equal(canon(engine.pairs()), canon(want))
+    for _ in range(2):
+        assert engine.bipartite_intersect(red, blue, rng) == len(w)
+    assert engine.stats()["kernels"] == 1
+    got = engine.pairs().astype(np.int64)
+    assert np.array_equal(got[np.lexsort((got[:, 1], got[:, 0]))], w[np.lexsort((w[:, 1], w[:, 0]))])
