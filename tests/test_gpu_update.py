@@ -123,3 +123,71 @@ def test_delta_only_scene(engine):
             sc.pairs()
     finally:
         sc.close()
+
+
+def shifted(boxes, idx, by, rng):
+    """Rows idx moved by `by` along every axis, within the range."""
+    nb = boxes[idx].astype(np.int64)
+    dims = (boxes.shape[1] - 1) // 2
+    for a in range(dims):
+        w = nb[:, 2 * a + 1] - nb[:, 2 * a]
+        nb[:, 2 * a] = np.clip(nb[:, 2 * a] + by[:, a], 0, rng - 1 - w)
+        nb[:, 2 * a + 1] = nb[:, 2 * a] + w
+    return nb.astype(np.uint32)
+
+
+@pytest.mark.parametrize("keep_pairs", [True, False])
+@pytest.mark.parametrize("dims,shift", [(2, 18), (3, 20), (3, 19)])
+def test_moves_within_cells_and_out_of_them(engine, dims, shift, keep_pairs):
+    """Boxes of 1 to hundreds of cells that stay in all their cells, in some of
+    them or in none; few boxes and all; lists that grow beyond their buffers."""
+    rs = np.random.default_rng(dims * 100 + shift)
+    n, rng, cell = 20000, gen.RANGE, 1 << shift
+    boxes = np.empty((n, 2 * dims + 1), dtype=np.uint32)
+    for a in range(dims):
+        side = np.where(np.arange(n) % 500 == 7, 7 * cell, rng // 400)
+        lo = rs.integers(0, rng - side)
+        boxes[:, 2 * a], boxes[:, 2 * a + 1] = lo, lo + rs.integers(0, side + 1)
+    boxes[:, -1] = np.arange(n)
+    sc = Scene(engine, boxes, rng, cell_shift=shift, keep_pairs=keep_pairs)
+    try:
+        cur, before = boxes.copy(), O.grid_pairs(boxes, rng)[0]
+        for k, reach in [(1, 0), (33, 3), (500, cell // 50), (500, cell), (2000, rng // 3), (n, cell // 10), (40, 8 * cell)]:
+            idx = rs.choice(n, k, replace=False).astype(np.uint32)
+            idx[0] = 7 if 7 not in idx else idx[0]  # (a large box each time)
+            nb = shifted(cur, idx, rs.integers(-reach, reach + 1, size=(k, dims)), rng)
+            nr, na = sc.move(idx, nb)
+            cur[idx] = nb
+            after = O.grid_pairs(cur, rng)[0]
+            rem, add = sc.delta()
+            assert (nr, na) == (len(rem), len(add))
+            assert np.array_equal(canon(rem), touching(before, idx)), (k, reach)
+            assert np.array_equal(canon(add), touching(after, idx)), (k, reach)
+            if keep_pairs:
+                assert np.array_equal(canon(sc.pairs()), after), (k, reach)
+            before = after
+    finally:
+        sc.close()
+
+
+def test_a_refused_move_keeps_the_last_lists(engine):
+    boxes = gen.scene3d(30000, seed=8)
+    sc = Scene(engine, boxes, gen.RANGE)
+    try:
+        idx = np.arange(100, 200, dtype=np.uint32)
+        sc.move(idx, shifted(boxes, idx, np.full((100, 3), 50000), gen.RANGE))
+        lists = [canon(v) for v in sc.delta()] + [canon(sc.pairs())]
+        many = np.arange(30000, dtype=np.uint32)  # (more room asked for than there is)
+        bad = boxes.copy()
+        bad[29999, 1] = gen.RANGE
+        twice = many.copy()
+        twice[5] = 6
+        for i, b in ((many, bad), (twice, boxes[twice]), (np.array([30000], dtype=np.uint32), boxes[:1])):
+            with pytest.raises(PbigError):
+                sc.move(i, b)
+            for want, got in zip(lists, [*sc.delta(), sc.pairs()]):
+                assert np.array_equal(want, canon(got))
+        nr, na = sc.move(many, boxes)
+        assert nr == len(lists[2]) and np.array_equal(canon(sc.pairs()), O.grid_pairs(boxes, gen.RANGE)[0])
+    finally:
+        sc.close()
