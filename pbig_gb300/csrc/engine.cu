@@ -276,6 +276,18 @@ static cudaError_t record_pipeline(pbig2_ctx* c, const Params& p, int dims, bool
         g_record_line = __LINE__;     \
         return e;                     \
     }
+    // (what is not a kernel comes first: the kernels are chained)
+    GroupArgs g{};
+    if (grouped) {
+        g.hist = c->d_scene_cursor.as<unsigned long long>();
+        g.cursor = g.hist + nsc + 1;
+        g.off = c->d_scene_pair.as<unsigned long long>();
+        g.off_host = static_cast<unsigned long long*>(c->h_pair_off.p);
+        g.block_counts = c->d_group.as<uint32_t>();
+        g.dst = c->d_out2.as<uint2>();
+        g.ctr_host = static_cast<Ctr*>(c->h_ctr.p);
+        R(cudaMemsetAsync(g.hist, 0, 2 * (nsc + 1) * 8, st));
+    }
     if (full) {
         if (tune) {
             R(launch_tune_query(p, *tune, dims, st));
@@ -283,9 +295,9 @@ static cudaError_t record_pipeline(pbig2_ctx* c, const Params& p, int dims, bool
             R(cudaMemsetAsync(p.ctr, 0, sizeof(Ctr), st));
         }
         if (p.scene_table) R(launch_scene_table(p, st));
-        R(launch_count(p, dims, st));
-        R(launch_scan(p, st));
-        R(launch_scatter(p, dims, st));
+        R(launch_count(p, dims, st, true, tune || p.scene_table));
+        R(launch_scan(p, st, true));
+        R(launch_scatter(p, dims, st, true));
     } else {
         // keep the grid and lists; clear the pair count, the error word and the item counters
         R(cudaMemsetAsync(&p.ctr->pairs, 0, sizeof(unsigned long long), st));
@@ -300,19 +312,8 @@ static cudaError_t record_pipeline(pbig2_ctx* c, const Params& p, int dims, bool
     PairOverlap ov{c->side_stream, c->ev_fork, c->ev_join,
                    c->host_split > 0 ? c->host_split : (2 * c->sm_count + 2) / 5};
     const bool overlap = c->ext_host && p.out == c->ext_out && c->host_split >= 0 && !p.records;
-    R(launch_pairs(pp, dims, c->sm_count, st, overlap ? &ov : nullptr));
-    if (grouped) {
-        GroupArgs g{};
-        g.hist = c->d_scene_cursor.as<unsigned long long>();
-        g.cursor = g.hist + nsc + 1;
-        g.off = c->d_scene_pair.as<unsigned long long>();
-        g.off_host = static_cast<unsigned long long*>(c->h_pair_off.p);
-        g.block_counts = c->d_group.as<uint32_t>();
-        g.dst = c->d_out2.as<uint2>();
-        g.ctr_host = static_cast<Ctr*>(c->h_ctr.p);
-        R(cudaMemsetAsync(g.hist, 0, 2 * (nsc + 1) * 8, st));
-        R(launch_group_by_scene(pp, g, st));
-    }
+    R(launch_pairs(pp, dims, c->sm_count, st, overlap ? &ov : nullptr, full));
+    if (grouped) R(launch_group_by_scene(pp, g, st, !overlap));
 #undef R
     return cudaSuccess;
 }

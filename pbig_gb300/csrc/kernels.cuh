@@ -226,9 +226,12 @@ constexpr uint32_t kUnmerged = 0x0fffff11u;  // a cell outside every merged bloc
 // grids: sized from p.nboxes / p.ncells (which must then be upper bounds
 // of the device-side sizes when p.dyn is set)
 // launch_count zeroes the counters and the scan's tile records first
-cudaError_t launch_count(const Params& p, int dims, cudaStream_t st);
-cudaError_t launch_scan(const Params& p, cudaStream_t st);
-cudaError_t launch_scatter(const Params& p, int dims, cudaStream_t st);
+// chained: each kernel's blocks take their places while the kernel before it
+// in the stream ends (that one has to be one of these kernels; for the count,
+// after_kernel says so)
+cudaError_t launch_count(const Params& p, int dims, cudaStream_t st, bool chained = false, bool after_kernel = false);
+cudaError_t launch_scan(const Params& p, cudaStream_t st, bool chained = false);
+cudaError_t launch_scatter(const Params& p, int dims, cudaStream_t st, bool chained = false);
 
 // The grid of a single-scene query (red/blue: both colours on one grid),
 // chosen on the device: zeroes p.ctr and writes the scene table (p.scenes,
@@ -272,7 +275,8 @@ struct PairOverlap {
     int side_sms;
 };
 
-cudaError_t launch_pairs(const Params& p, int dims, int sm_count, cudaStream_t st, const PairOverlap* ov = nullptr);
+cudaError_t launch_pairs(const Params& p, int dims, int sm_count, cudaStream_t st, const PairOverlap* ov = nullptr,
+                         bool chained = false);
 // the pairs of p.out grouped by scene into dst, the scenes' pair offsets on the
 // device and the host, and the end of the query (Params::ctr_host)
 struct GroupArgs {
@@ -285,7 +289,7 @@ struct GroupArgs {
     Ctr* ctr_host;
 };
 size_t group_count_bytes(uint32_t nscenes);
-cudaError_t launch_group_by_scene(const Params& p, const GroupArgs& g, cudaStream_t st);
+cudaError_t launch_group_by_scene(const Params& p, const GroupArgs& g, cudaStream_t st, bool chained = false);
 // p.scene_table for p.nboxes boxes (scene_table_entries of them)
 cudaError_t launch_scene_table(const Params& p, cudaStream_t st);
 uint64_t scene_table_entries(uint64_t nboxes);
