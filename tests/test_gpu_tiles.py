@@ -78,3 +78,35 @@ def test_two_colours_in_one_cell(engines, dims, shift, step):
         assert e.bipartite_intersect(boxes[:red].copy(), blue, rng, cell_shift=shift) == len(want), (n, red)
         got = e.pairs().astype(np.int64)
         assert np.array_equal(got[np.lexsort((got[:, 1], got[:, 0]))], want), (n, red)
+
+
+@pytest.mark.parametrize("n", [64, 100, 128, 300, 512, 600])
+@pytest.mark.parametrize("hits", [1, 11, 12, 13, 32, 63, 64])
+def test_rows_of_many_pairs(engines, n, hits):
+    """Boxes apart from one another, and every 20th of them a wide one that
+    overlaps `hits` others: rows below, at and above the length that the warp
+    writes together, some in one column tile and some in two."""
+    rs = np.random.default_rng(n + hits)
+    shift, rng = 14, 1 << 16
+    at = np.arange(n) * 16
+    boxes = np.zeros((n, 7), dtype=np.uint32)
+    boxes[:, 0], boxes[:, 1] = at, at + 1
+    wide = np.arange(0, n, 20)
+    first = rs.integers(0, max(1, n - hits), size=len(wide)) * 16
+    boxes[wide, 0], boxes[wide, 1] = first, np.minimum(first + 16 * (hits - 1) + 1, (1 << shift) - 1)
+    boxes[:, 3] = boxes[:, 5] = 5
+    boxes = boxes[rs.permutation(n)]
+    boxes[:, 6] = np.arange(n)
+    want = O.brute_pairs(boxes)
+    red, blue = boxes[:n // 2].copy(), boxes[n // 2:].copy()
+    blue[:, 6] = np.arange(len(blue))
+    w = want.astype(np.int64)
+    w = w[(w[:, 0] < n // 2) & (w[:, 1] >= n // 2)] - [0, n // 2]
+    for e in engines:
+        for _ in range(2):
+            assert e.self_intersect(boxes, rng, cell_shift=shift) == len(want)
+        assert np.array_equal(canon(e.pairs()), canon(want))
+        for _ in range(2):
+            assert e.bipartite_intersect(red, blue, rng, cell_shift=shift) == len(w)
+        got = e.pairs().astype(np.int64)
+        assert np.array_equal(got[np.lexsort((got[:, 1], got[:, 0]))], w[np.lexsort((w[:, 1], w[:, 0]))])
