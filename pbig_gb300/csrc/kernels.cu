@@ -150,7 +150,10 @@ __global__ void k_scene_table(Params pin) {
 // tuner's analytic model (tune_impl with T = E^2 / 2C) on the rows
 // a + floor(k * n / m), k < m = min(n, 64), of the scene [a, a + n). Every
 // sum is of integers (exact in any order), so the choice equals the host
-// model's on the same rows.
+// model's on the same rows. The sizes are counted one after the other in
+// integers and weighed side by side, a lane a size: double precision runs at a
+// sixty-fourth of the rate, and with all of it in every lane, eight scenes to
+// an SM, the kernel took 40 us; now 12.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kTuneRows = 64;
 
@@ -197,38 +200,53 @@ __device__ __forceinline__ SceneTune tune_scene_warp(const uint32_t* boxes, uint
             const int s0 = tune_s0(ext, (good ? good : 1) * (uint64_t)dims);
             const double scale = (double)n / (double)m;
             const int s_win = s0 + 3 < 31 ? s0 + 3 : 31;
-            double best_cost = 1e300;
-            for (int s = s0 - 2 > 0 ? s0 - 2 : 0; s <= 31; s++) {
-                if (s == s_win + 1 && best_cost < 1e300) break;
-                const double C = tune_cells(nrc_dev(range, s), dims);
-                if (C > max_cells) continue;
-                if (s > s_win && C > fmax(4096.0, 64.0 * (double)n)) continue;
-                double e = 0, cm = 0;
+            best.shift = 32u;
+            // the window, then every coarser size if none of it qualifies
+            for (int pass = 0; pass < 2 && best.shift == 32u; pass++) {
+                const int first = pass ? s_win + 1 : s0 - 2 > 0 ? s0 - 2 : 0, last = pass ? 31 : s_win;
+                uint32_t entries = 0;  // lane s - first: the sample's at shift s
+                bool fits = false;
+                for (int s = first; s <= last; s++) {
+                    uint32_t e = 0;
+                    bool huge = false;  // (without one, 64 boxes of less than 2^26 cells: below 2^32)
 #pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    if (!ok[j]) continue;
-                    double c = 1;
-                    for (int d = 0; d < dims; d++) c = tune_mul(c, (double)((hi[j][d] >> s) - (lo[j][d] >> s) + 1));
-                    e = tune_add(e, c);
-                    cm = fmax(cm, c);
+                    for (int j = 0; j < 2; j++) {
+                        if (!ok[j]) continue;
+                        uint64_t c = 1;
+                        for (int d = 0; d < dims; d++) c = c >= (1ull << 26) ? c : c * ((uint64_t)((hi[j][d] >> s) - (lo[j][d] >> s)) + 1);
+                        huge = huge || c >= (1ull << 26);
+                        e += (uint32_t)c;
+                    }
+                    e = __reduce_add_sync(FULL_MASK, e);
+                    huge = __any_sync(FULL_MASK, huge);
+                    if ((int)lane == s - first) {
+                        entries = e;
+                        fits = !huge && e <= 64u * (uint32_t)m;
+                    }
                 }
+                const double C = tune_cells(nrc_dev(range, min(first + (int)lane, 31)), dims);
+                double E = 0.0;
+                unsigned long long cost = ~0ull;  // (positive doubles are in the order of their bits)
+                if (fits && C <= max_cells && (!pass || C <= fmax(4096.0, 64.0 * (double)n))) {
+                    E = tune_mul((double)entries, scale);
+                    cost = (unsigned long long)__double_as_longlong(tune_cost(C, E, tune_mul(E, E) / tune_mul(2.0, C)));
+                }
+                uint32_t l = lane;  // of the least cost, the finest on a tie
 #pragma unroll
                 for (int o = 16; o; o >>= 1) {
-                    e = tune_add(e, __shfl_xor_sync(FULL_MASK, e, o));
-                    cm = fmax(cm, __shfl_xor_sync(FULL_MASK, cm, o));
+                    const unsigned long long k = __shfl_xor_sync(FULL_MASK, cost, o);
+                    const uint32_t kl = __shfl_xor_sync(FULL_MASK, l, o);
+                    if (k < cost || (k == cost && kl < l)) {
+                        cost = k;
+                        l = kl;
+                    }
                 }
-                if (e / (double)m > 64.0) continue;
-                if (cm >= (double)(1u << 26)) continue;
-                const double E = tune_mul(e, scale);
-                const double T = tune_mul(E, E) / tune_mul(2.0, C);
-                const double cost = tune_cost(C, E, T);
-                if (cost < best_cost) {
-                    best_cost = cost;
-                    best.shift = (uint32_t)s;
-                    best.est_entries = E;
+                if (cost != ~0ull) {
+                    best.shift = (uint32_t)first + l;
+                    best.est_entries = __shfl_sync(FULL_MASK, E, l);
                 }
             }
-            if (best_cost == 1e300) {  // the coarsest grid that is not a single cell
+            if (best.shift == 32u) {  // the coarsest grid that is not a single cell
                 uint32_t s = 31;
                 while (s > 0 && nrc_dev(range, (int)s - 1) <= 1) s--;
                 best.shift = s;
@@ -3096,9 +3114,8 @@ cudaError_t launch_tune_query(const Params& p, const TuneArgs& a, int dims, cuda
 cudaError_t launch_tune_scenes(const uint32_t* boxes, const unsigned long long* offs, uint32_t nscenes, int dims,
                                uint32_t range, SceneTune* out, cudaStream_t st) {
     if (nscenes == 0) return cudaSuccess;
-    const uint64_t blocks = ((uint64_t)nscenes + 7) / 8;  // 8 warps (scenes) per block
-    const uint64_t cap = (uint64_t)(g_sm_count > 0 ? g_sm_count : 152) * 16;
-    k_tune_scenes<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(boxes, offs, nscenes, dims, range, out);
+    const uint64_t cap = (uint64_t)(g_sm_count > 0 ? g_sm_count : 152) * 32;  // a warp per block: scenes on SMs of their own
+    k_tune_scenes<<<(unsigned)(nscenes < cap ? nscenes : cap), 32, 0, st>>>(boxes, offs, nscenes, dims, range, out);
     return cudaGetLastError();
 }
 
