@@ -32,7 +32,7 @@ struct alignas(16) ResCtr {
     unsigned long long add;          // and after it (may exceed capacity)
     unsigned long long full;         // pairs of the full list after the move
     unsigned int done;               // blocks of the last kernel that finished
-    unsigned int pad;
+    unsigned int span;               // most cells of a box (k_res_span)
 };
 
 struct ResGrid {
@@ -62,7 +62,23 @@ __device__ __forceinline__ uint64_t res_gid(const ResGrid& g, uint32_t i, uint32
     return ((uint64_t)k * g.nrc + j) * g.nrc + i;
 }
 
-// one thread per listed box (idx == nullptr: boxes 0..k-1): count its cells
+// the most cells that a box covers on the grid of shift sh
+template <int D>
+__global__ void k_res_span(const uint32_t* boxes, uint64_t n, uint32_t sh, unsigned int* most) {
+    constexpr int W = 2 * D + 1;
+    uint32_t m = 0;
+    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t lo[3], hi[3];
+        res_range<D>(boxes + t * W, sh, lo, hi);
+        uint64_t c = 1;
+        for (int d = 0; d < D; d++) c = min(c * ((uint64_t)(hi[d] - lo[d]) + 1), (uint64_t)0x7fffffffu);
+        m = max(m, (uint32_t)c);
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31u) == 0 && m) atomicMax(most, m);
+}
+
+// one thread per box: count its cells
 template <int D>
 __global__ void k_res_count(ResGrid g, uint32_t* cnt) {
     constexpr int W = 2 * D + 1;
@@ -597,7 +613,7 @@ __global__ void __launch_bounds__(kResThreads, kResBlocks) k_move_after(Move m) 
             h.rem = __ldcg(&c->rem);
             h.add = __ldcg(&c->add);
             h.full = __ldcg(&c->full);
-            h.done = h.pad = 0;
+            h.done = h.span = 0;
             *m.host = h;
             __threadfence_system();
         }
@@ -662,6 +678,30 @@ ResCtr read_ctr(pbig2_scene* s, cudaStream_t st, cudaError_t* e) {
     *e = cudaMemcpyAsync(&h, s->rctr.p, sizeof h, cudaMemcpyDeviceToHost, st);
     if (*e == cudaSuccess) *e = cudaStreamSynchronize(st);
     return h;
+}
+
+// With an automatic cell size the scene's grid is one size finer than the
+// query's, where that makes at most 4 cells a box and no box covers more than
+// 512: a move tests the moved boxes against whole cells, while the query tests
+// each pair of a cell once. Moves of 1 % of a million boxes of one density 81 us
+// on the query's grid, 70 on the finer one and 69 on the next; of 65 536 boxes
+// 52 and 46; of the clustered 4M-box scene 716, 568 and 621.
+int finer_grid(pbig2_scene* s, cudaStream_t st) {
+    if (s->shift == 0 || grid_cells(s->range, s->shift - 1, s->dims) > 4 * s->n) return PBIG2_OK;
+    SCK(cudaMemsetAsync(s->rctr.p, 0, sizeof(ResCtr), st));
+    const unsigned g = grid_for(s->n, 256, s->ctx->sm_count);
+    unsigned int* most = &s->rctr.as<ResCtr>()->span;
+    if (s->dims == 2) k_res_span<2><<<g, 256, 0, st>>>(s->boxes.as<uint32_t>(), s->n, s->shift - 1, most);
+    else k_res_span<3><<<g, 256, 0, st>>>(s->boxes.as<uint32_t>(), s->n, s->shift - 1, most);
+    SCK(cudaGetLastError());
+    cudaError_t e;
+    const ResCtr h = read_ctr(s, st, &e);
+    SCK(e);
+    if (h.span > 512) return PBIG2_OK;
+    s->shift--;
+    s->nrc = nrc_for(s->range, s->shift);
+    s->ncells = grid_cells(s->range, s->shift, s->dims);
+    return PBIG2_OK;
 }
 
 // the grid of the scene's current boxes: counts, capacities with slack,
@@ -791,6 +831,10 @@ PBIG2_API int pbig2_scene_create(pbig2_ctx* c, const uint32_t* boxes, uint64_t n
     if (np && pbig2_copy_pairs(c, s->full[0].as<uint32_t>(), 0, np, PBIG2_DEVICE, sm) != PBIG2_OK) return bail(PBIG2_ECUDA);
     s->nfull = np;
     s->keep_full = (flags & PBIG2_SCENE_DELTA_ONLY) == 0;
+    if (cell_shift == PBIG2_AUTO) {
+        rc = finer_grid(s, sm);
+        if (rc != PBIG2_OK) return bail(rc);
+    }
     rc = build_grid(s, sm);
     if (rc != PBIG2_OK) return bail(rc);
     *out = s;

@@ -191,3 +191,31 @@ def test_a_refused_move_keeps_the_last_lists(engine):
         assert nr == len(lists[2]) and np.array_equal(canon(sc.pairs()), O.grid_pairs(boxes, gen.RANGE)[0])
     finally:
         sc.close()
+
+
+@pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("large", [0, 1])
+def test_automatic_grids_of_scenes(engine, dims, large):
+    """Automatic cell sizes, with the finer grid that small boxes get and, where
+    a box covers most of the range, the query's."""
+    rs = np.random.default_rng(dims + 10 * large)
+    for n in (40, 7000):
+        side = int(gen.RANGE * (1.0 / n) ** (1 / dims))
+        boxes = np.empty((n, 2 * dims + 1), dtype=np.uint32)
+        lo = rs.integers(0, gen.RANGE - side, size=(n, dims))
+        boxes[:, 0:2 * dims:2], boxes[:, 1:2 * dims:2] = lo, lo + rs.integers(0, side, size=(n, dims))
+        if large:
+            boxes[n // 2, 0:2 * dims:2], boxes[n // 2, 1:2 * dims:2] = 0, gen.RANGE - 1
+        boxes[:, -1] = np.arange(n)
+        sc = Scene(engine, boxes, gen.RANGE)
+        try:
+            cur = boxes.copy()
+            assert np.array_equal(canon(sc.pairs()), O.brute_pairs(cur))
+            for step in range(3):
+                idx = rs.choice(n, n // 3, replace=False).astype(np.uint32)
+                idx[0] = n // 2 if n // 2 not in idx else idx[0]
+                cur[idx] = shifted(cur, idx, rs.integers(-side, side + 1, size=(len(idx), dims)), gen.RANGE)
+                sc.move(idx, cur[idx])
+                assert np.array_equal(canon(sc.pairs()), O.brute_pairs(cur)), (n, step)
+        finally:
+            sc.close()
