@@ -1,7 +1,7 @@
 // Host orchestration of the pair-detection pipeline and the C ABI (pbig2.h).
 //
-// One query = one pass of count -> scan -> expand -> scatter -> pairs on the
-// context's stream, after the cell size has been chosen by the autotuner.
+// One query = one pass of tune -> count -> scan -> scatter -> pairs on the
+// context's stream, or one launch of them all.
 // The reference runs the same phases with host round trips in between
 // (plan_phase / map_phase / sched_phase / match_phase, src/pbig/pbig.cu:1361,
 // 1429, 1592, 1694); here every phase stays on the device and the host reads
@@ -308,9 +308,12 @@ static cudaError_t record_pipeline(pbig2_ctx* c, const Params& p, int dims, bool
     Params pp = p;
     pp.ctr_host = grouped ? nullptr : static_cast<Ctr*>(c->h_ctr.p);
     // pairs stored over the host link: the lighter pair kernels run beside
-    // the medium-cell kernel (two fifths of the SMs unless set)
+    // the medium-cell kernel (three fifths of the SMs unless set: the big
+    // cells are the most of it. Clustered 4M-box queries on two contexts 2.29
+    // ms each at two fifths, 2.18 at three, 2.23 at 110 of 152; a million boxes
+    // of range 2^31 0.348, 0.319 and 0.331 ms)
     PairOverlap ov{c->side_stream, c->ev_fork, c->ev_join,
-                   c->host_split > 0 ? c->host_split : (2 * c->sm_count + 2) / 5};
+                   c->host_split > 0 ? c->host_split : (3 * c->sm_count + 2) / 5};
     const bool overlap = c->ext_host && p.out == c->ext_out && c->host_split >= 0 && !p.records;
     R(launch_pairs(pp, dims, c->sm_count, st, overlap ? &ov : nullptr, full));
     if (grouped) R(launch_group_by_scene(pp, g, st, !overlap));

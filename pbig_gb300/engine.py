@@ -347,8 +347,8 @@ class Engine:
 
     def set_host_split(self, sms: int) -> None:
         """SMs of the small-cell and block kernels beside the medium-cell
-        kernel when pairs go to page-locked host memory (0: automatic, a
-        quarter; negative: one after another)."""
+        kernel when pairs go to page-locked host memory (0: automatic, three
+        fifths; negative: one after another)."""
         _check(self._L.pbig2_set_option(self._ctx, 4, int(sms)))
 
     def set_one_launch(self, on: bool) -> None:
