@@ -2,9 +2,8 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl gb300|reference] [--workload NAME]
 
-A step is one self-intersection query over the whole workload (count, scan,
-scatter, pair test, compaction; the autotuner's choice is memoised after the
-first query of a context). Default workload: 4,194,304 3-D boxes drawn from a
+A step is one self-intersection query over the whole workload (choice of the
+cell size, count, scan, scatter, pair test, compaction). Default workload: 4,194,304 3-D boxes drawn from a
 mixture of 64 Gaussians (sigma 0.02, means U[0.1,0.9]^3), lognormal sides
 (median 0.002, log-sigma 0.5), fp32 quantised to the PBIG API's unsigned
 coordinates (range 2^24); synthetic, seeded, generated on the host.
@@ -207,14 +206,15 @@ class ClockSampler:
 
 def algorithmic_bytes(st: dict, n: int) -> dict:
     """Bytes each kernel must move at minimum (per launch): boxes are read
-    whole (28 B), cells as one u32 count/start, entries as one u32, pairs as
-    two u32; the pair test reads each entry and its box coordinates once."""
+    whole (28 B), cells as one u32 count/start, entries as four u32 (the
+    box's part of the cell, and its index), pairs as two u32; the pair test
+    reads each entry once."""
     C, E, P = st["cells"], st["entries"], st["pairs"]
     return {
         "count": n * BOX_BYTES + C * 4,
         "scan": 2 * C * 4,
-        "scatter": n * BOX_BYTES + C * 4 + E * 4,
-        "pairs": E * (4 + 24) + 8 * P,
+        "scatter": n * BOX_BYTES + C * 4 + E * 16,
+        "pairs": E * 16 + 8 * P,
     }
 
 
@@ -386,7 +386,7 @@ def stream_of_queries(eng, query, host, P, n, args, local, ws):
     try:
         for e, o, st in zip(engs, outs, streams):
             e.set_pair_output(o)
-            for _ in range(2):  # warm-up: buffers and the tuner's memo of the second context
+            for _ in range(2):  # warm-up: buffers of the second context
                 query(host, e, st)
         torch.cuda.synchronize()
 

@@ -67,11 +67,12 @@ typedef struct {
     uint32_t grid_retries; /* automatic cell size: passes rerun on a coarser
                               grid because a box outside the tuner's sample
                               covered 2^26 cells or more */
-    double device_ms;      /* device time of the query (CUDA events) */
-    /* device time per phase of the last pipeline pass (CUDA events on the
-     * query's stream): count, scan, expand, scatter, pair test (all three
-     * pair kernels), grouping by scene, and within the pair test: the
-     * small-cell, medium-cell and block kernels */
+    double device_ms;      /* device time of the query (the kernels' own clock) */
+    /* device time per phase of the last pipeline pass (the kernels' own
+     * clock): count, scan, expand (0: the scatter does it), scatter, pair test
+     * (all three pair kernels), grouping by scene, and within the pair test:
+     * the small-cell, medium-cell and block kernels; all 0 for a query that
+     * ran as one launch */
     double phase_ms[9];
     /* the reference's own work statistics for the same grid (sched_phase,
      * src/pbig/pbig.cu:1586-1688): numCompPairs = sum of n*n/2, jobs = sum
@@ -216,15 +217,17 @@ PBIG2_API int pbig2_get_stats(pbig2_ctx* ctx, pbig2_stats* stats);
 /* PBIG2_OPT_HOST_SPLIT (default 0 = automatic): when the pair output set by
  * pbig2_set_pair_output is page-locked host memory, the pair phase is bound
  * by the host link; the small-cell and block kernels then run on their own
- * stream over this many SMs (automatic: a quarter) beside the medium-cell
+ * stream over this many SMs (automatic: three fifths) beside the medium-cell
  * kernel on the rest, so the link is not idle while they compute. A
  * negative value runs the three kernels one after another. */
 #define PBIG2_OPT_HOST_SPLIT 4
-/* PBIG2_OPT_ONE_LAUNCH (default 1): a self query of at most 262 144 boxes
-   with an automatic cell size (or a given one whose grid has at most 2^20
-   cells), outside merged and record mode, runs as one cooperative kernel
-   launch: cell size, count, scan, scatter and pair test, separated by grid
-   barriers. A result that does not fit the buffers the launch was given is
+/* PBIG2_OPT_ONE_LAUNCH (default 1): a self or red/blue query of at most
+   262 144 boxes with an automatic cell size (or a given one whose grid has at
+   most 2^20 cells), outside merged and record mode, runs as one cooperative
+   kernel launch: cell size, count, scan, scatter and pair test, separated by
+   grid barriers; with an automatic cell size and at most 6144 boxes in a range
+   of at most 2^31, as one ordinary launch that tests every pair (the
+   statistics are those of a grid of one cell). A result that does not fit the buffers the launch was given is
    redone by the regular pipeline. 0 sends every query to the regular
    pipeline. The value 2 tests the barriers' bounded wait: in the next
    one-launch query no barrier completes, every block gives up after about a
@@ -292,7 +295,7 @@ PBIG2_API int pbig2_serve_batch(pbig2_ctx* ctx, pbig2_batch_item* items, uint32_
  * latency-critical loop that cannot afford cudaMalloc/cudaFree and their
  * device-wide synchronization. Boxes and the output pairs (pair_cap uint32
  * pairs, a<b) are caller-owned device buffers; every intermediate buffer
- * lives in a fixed 16 MiB scratch array inside the library, held by every
+ * lives in a fixed 24 MiB scratch array inside the library, held by every
  * GPU that loads the library until exit. Limits: n <= 262144 boxes, a grid
  * of at most 2^20 cells (the cell size is coarsened to fit) and at most
  * 524288 box-in-cell entries; larger queries return PBIG2_ECAPACITY. The

@@ -217,7 +217,6 @@ TuneResult tune_shift_sample(const uint32_t* boxes, uint64_t n_avail, uint64_t n
 struct GridScene {
     uint64_t box_off, n;
     uint32_t shift;
-    int grid_of;  // index of the scene whose grid this one shares (self for its own)
 };
 
 // device buffers of one query; fills the matching Params fields
@@ -834,8 +833,8 @@ static int run_single(pbig2_ctx* c, const SingleScene& q, uint32_t shift, cudaSt
     if (rc) return rc;
     c->result_ext = use_ext;
     c->out_hint = std::max<uint64_t>(c->out_hint, h.pairs + h.pairs / 8);
-    std::vector<GridScene> sc{{0, q.n, h.shift, 0}};
-    if (q.bip) sc.push_back({q.n_red, q.n - q.n_red, h.shift, 0});
+    std::vector<GridScene> sc{{0, q.n, h.shift}};
+    if (q.bip) sc.push_back({q.n_red, q.n - q.n_red, h.shift});
     *used = h.shift;
     rc = finish_query(c, h, q.n, h.cells, p.nscenes, sc, false, launches);
     c->stats.class_map = p.class_map;
@@ -973,7 +972,7 @@ static int fused_query(pbig2_ctx* c, const uint32_t* red, uint64_t n_red, const 
     c->result_ext = use_ext;
     c->out_hint = std::max<uint64_t>(c->out_hint, h.pairs + h.pairs / 8);
     c->merged_blocks = 0;
-    std::vector<GridScene> sc{{0, n, h.shift, 0}};
+    std::vector<GridScene> sc{{0, n, h.shift}};
     rc = finish_query(c, h, n, h.cells, 1, sc, false, 1);
     c->stats.class_map = p.class_map;
     c->stats.device_ms = h.t_end > h.t_start ? (double)(h.t_end - h.t_start) * 1e-6 : 0.0;  // the kernel's own clock
@@ -1219,7 +1218,7 @@ PBIG2_API int pbig2_batch_intersect(pbig2_ctx* c, const uint32_t* boxes, const u
             shift = tuned[i].shift;
             e = std::max(e, tuned[i].est_entries);
         }
-        sc[i] = GridScene{a, ns, shift, (int)i};
+        sc[i] = GridScene{a, ns, shift};
         est_e += e;
     }
     // (a batch of one scene is a query of that scene)

@@ -721,7 +721,7 @@ __device__ __forceinline__ void enumerate_cells(const Params& p, uint32_t* sbox,
             bool take = true;
             uint4 rec = make_uint4(0u, 0u, 0u, 0u);
             const uint32_t* ob = sbox + ((t & ~31u) + o) * W;
-            if (SCATTER && !MERGED) {
+            if constexpr (SCATTER && !MERGED) {
                 rec.x = term_cut(ob[0], i == 0, i + 1 == o_sx);
                 rec.y = term_cut(ob[1], j == 0, j + 1 == o_sy);
                 // (the last layer: its cells are the last sx*sy)
