@@ -69,16 +69,6 @@ __device__ __forceinline__ void stamp(const Params& p, int k) {
     if (blockIdx.x == 0 && threadIdx.x == 0) p.ctr->stamp[k] = now_ns();
 }
 
-// The kernels of a pipeline pass are chained (launch_after): each is launched
-// once every block of the one before has begun, and waits here until that one
-// is complete before it touches memory. Its blocks are on the SMs by then: a
-// scene of 500 000 boxes, nine kernels, 111 -> 101 us on the device; eight
-// scenes of 1.4 million boxes, a graph of twelve, 198 -> 173 us.
-__device__ __forceinline__ void chain_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // the run counters to page-locked host memory (one thread; the counters were
 // changed through L2 by other blocks)
 __device__ __forceinline__ void ctr_to_host(const Ctr* ctr, Ctr* host) {
@@ -3042,24 +3032,6 @@ cudaError_t kernels_init() {
 }
 
 uint64_t scene_table_entries(uint64_t nboxes) { return (nboxes >> kSceneTableShift) + 2; }
-
-// a launch behind another kernel of the pass, chained to it (chain_wait), or
-// an ordinary one
-template <class... P>
-static cudaError_t launch_after(bool chained, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
-                                P... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = chained ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
 
 cudaError_t launch_scene_table(const Params& p, cudaStream_t st) {
     const uint64_t n = scene_table_entries(p.nboxes);

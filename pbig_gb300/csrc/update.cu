@@ -149,8 +149,10 @@ __device__ __forceinline__ bool res_moved(const uint32_t* bits, uint32_t id) { r
 // Each looks at the counters of the ones before it and does nothing where
 // those found an error, a buffer too small or a cell without slack: the host
 // reads the counters once, at the end, and repeats what is missing with more
-// room. Nine kernels with five waits, the pairs before by a query, took 234 us
-// for 10 485 of a million boxes, 120 of them in kernels; these take 80 and 53.
+// room. The kernels are chained (chain_wait). Nine kernels with five waits, the
+// pairs before by a query, took 234 us for 10 485 of a million boxes, 120 of
+// them in kernels; these took 80 and 53, on the finer grid (finer_grid) 70, and
+// chained 63.
 struct Move {
     ResGrid g;
     const uint32_t* idx;  // [k] listed boxes
@@ -193,6 +195,7 @@ __device__ __forceinline__ MoveState move_state(const Move& m) {
 template <int D>
 __global__ void k_move_check(Move m) {
     constexpr int W = 2 * D + 1;
+    chain_wait();
     for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m.k; t += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t* b = m.nb + t * W;
         const uint32_t id = m.idx[t];
@@ -505,6 +508,7 @@ template <int D>
 __global__ void __launch_bounds__(kResThreads) k_move_out(Move m, uint32_t rblocks) {
     __shared__ uint32_t s_w[kResWarps];
     __shared__ unsigned long long s_at[2];
+    chain_wait();
     // (with a full list, the pairs before are being counted here)
     const MoveState c = move_state(m);
     if (c.bad || (!m.full && c.rem > m.rem_cap)) return;
@@ -516,6 +520,7 @@ __global__ void __launch_bounds__(kResThreads) k_move_out(Move m, uint32_t rbloc
 template <int D>
 __global__ void __launch_bounds__(kResThreads, kResBlocks) k_move_before(Move m) {
     __shared__ ResOut s;
+    chain_wait();
     if (move_state(m).bad) return;
     res_query<D>(m, ResDst{m.rem, m.rem_cap, &m.g.ctr->rem, nullptr, 0, nullptr}, blockIdx.x, gridDim.x, s);
 }
@@ -529,6 +534,7 @@ __global__ void __launch_bounds__(kResThreads, kResBlocks) k_move_before(Move m)
 template <int D>
 __global__ void __launch_bounds__(kResThreads) k_move_in(Move m, uint32_t* boxes) {
     constexpr int W = 2 * D + 1;
+    chain_wait();
     const MoveState c = move_state(m);
     if (c.bad || c.rem > m.rem_cap) return;
     const ResGrid& g = m.g;
@@ -599,6 +605,7 @@ template <int D>
 __global__ void __launch_bounds__(kResThreads, kResBlocks) k_move_after(Move m) {
     __shared__ ResOut s;
     ResCtr* c = m.g.ctr;
+    chain_wait();
     const MoveState before = move_state(m);
     if (!before.bad && !before.no_slack && before.rem <= m.rem_cap)
         res_query<D>(m, ResDst{m.add, m.add_cap, &c->add, m.full, m.full ? m.nold + m.add_cap : 0,
@@ -780,12 +787,13 @@ cudaError_t launch_move(pbig2_scene* s, const Move& m, MovePart part, cudaStream
     const int sms = s->ctx->sm_count;
     const unsigned gw = grid_for(m.k, kResWarps, sms), r = part == kMoveAll ? gw : 0u;
     const unsigned f = m.nold ? grid_for(m.nold, kResThreads * kFilterPer, sms) : 0u;
-    if (part == kMoveAll) k_move_check<D><<<grid_for(m.k, 256, sms), 256, 0, st>>>(m);
-    if (part == kMoveAll && !m.full) k_move_before<D><<<gw, kResThreads, 0, st>>>(m);
-    if (r + f) k_move_out<D><<<r + f, kResThreads, 0, st>>>(m, r);
-    if (part == kMoveAll) k_move_in<D><<<gw, kResThreads, 0, st>>>(m, s->boxes.as<uint32_t>());
-    k_move_after<D><<<gw, kResThreads, 0, st>>>(m);
-    return cudaGetLastError();
+    const bool all = part == kMoveAll;
+    cudaError_t e = cudaSuccess;
+    if (all) e = launch_after(false, k_move_check<D>, grid_for(m.k, 256, sms), 256, 0, st, m);
+    if (e == cudaSuccess && all && !m.full) e = launch_after(true, k_move_before<D>, gw, kResThreads, 0, st, m);
+    if (e == cudaSuccess && r + f) e = launch_after(all, k_move_out<D>, r + f, kResThreads, 0, st, m, (uint32_t)r);
+    if (e == cudaSuccess && all) e = launch_after(true, k_move_in<D>, gw, kResThreads, 0, st, m, s->boxes.as<uint32_t>());
+    return e != cudaSuccess ? e : launch_after(all || r + f, k_move_after<D>, gw, kResThreads, 0, st, m);
 }
 
 }  // namespace
