@@ -324,7 +324,10 @@ PBIG2_API const char* pbig2_noalloc_last_error(void);
  * old list without the removed pairs plus the added ones -- an O(pairs)
  * step that flags = PBIG2_SCENE_DELTA_ONLY leaves out. The scene uses
  * ctx's stream and buffers: one scene call at a time per context, and the
- * context's last-result pointers are overwritten by pbig2_scene_create. */
+ * context's last-result pointers are overwritten by pbig2_scene_create.
+ * The grid has one slot and a half per entry and four more per cell, 32 bytes
+ * each, and 2^32 - 1 of them at most: an automatic cell size is coarsened to
+ * fit, a given one that does not fit is refused (PBIG2_ECAPACITY). */
 typedef struct pbig2_scene pbig2_scene;
 #define PBIG2_SCENE_DELTA_ONLY 1u /* flags: moves report their delta only; no full list is kept */
 PBIG2_API int pbig2_scene_create(pbig2_ctx* ctx, const uint32_t* boxes, uint64_t n, uint32_t dims, uint32_t range,
@@ -346,6 +349,10 @@ PBIG2_API int pbig2_scene_copy(pbig2_scene* scene, int which, uint32_t* dst, uin
  * (no counterpart in the reference, whose 32-bit nCells wraps). Queries
  * refuse grids of 2^32 - 1 cells or more. */
 PBIG2_API uint64_t pbig2_grid_cells(uint32_t range, uint32_t shift, uint32_t dims);
+
+/* Slots of a resident scene's grid of ncells cells with `entries`
+ * box-in-cell entries: so many at most, saturating at UINT64_MAX. */
+PBIG2_API uint64_t pbig2_scene_slots(uint64_t ncells, uint64_t entries);
 
 /* Cell-size autotuner of batched and serving scenes, for boxes in host
  * memory, from a sample of at most `sample` of them. (Self and red/blue

@@ -33,13 +33,14 @@ struct alignas(16) ResCtr {
     unsigned long long full;         // pairs of the full list after the move
     unsigned int done;               // blocks of the last kernel that finished
     unsigned int span;               // most cells of a box (k_res_span)
+    unsigned long long sum;          // entries of the boxes (k_res_span), slots of the cells (k_res_caps)
 };
 
 struct ResGrid {
     const uint32_t* boxes;
     uint64_t nboxes;
     uint32_t shift, nrc, range;
-    uint64_t ncells;
+    uint64_t ncells, nslots;
     uint32_t* start;     // [ncells + 1] capacity region of each cell
     uint32_t* used;      // [ncells] slots used (live entries and tombstones)
     uint4* entries;      // two per slot: {x0, x1, y0, y1}, {z0, z1, start bits << 29 | box index (kDead: free), 0}
@@ -48,6 +49,14 @@ struct ResGrid {
 
 // slack of a cell of n boxes
 __host__ __device__ __forceinline__ uint32_t res_cap(uint32_t n) { return n + (n >> 1) + 4u; }
+// the starts are 32-bit words, the last of them the number of slots
+constexpr uint64_t kMaxSlots = 0xffffffffull;
+
+__device__ __forceinline__ void res_sum(unsigned long long* sum, unsigned long long x) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if ((threadIdx.x & 31u) == 0 && x) atomicAdd(sum, x);
+}
 
 template <int D>
 __device__ __forceinline__ void res_range(const uint32_t* b, uint32_t sh, uint32_t lo[3], uint32_t hi[3]) {
@@ -62,20 +71,23 @@ __device__ __forceinline__ uint64_t res_gid(const ResGrid& g, uint32_t i, uint32
     return ((uint64_t)k * g.nrc + j) * g.nrc + i;
 }
 
-// the most cells that a box covers on the grid of shift sh
+// the cells that the boxes cover on the grid of shift sh: the most of one, and of all
 template <int D>
-__global__ void k_res_span(const uint32_t* boxes, uint64_t n, uint32_t sh, unsigned int* most) {
+__global__ void k_res_span(const uint32_t* boxes, uint64_t n, uint32_t sh, ResCtr* ctr) {
     constexpr int W = 2 * D + 1;
     uint32_t m = 0;
+    unsigned long long sum = 0;
     for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t lo[3], hi[3];
         res_range<D>(boxes + t * W, sh, lo, hi);
-        uint64_t c = 1;
-        for (int d = 0; d < D; d++) c = min(c * ((uint64_t)(hi[d] - lo[d]) + 1), (uint64_t)0x7fffffffu);
+        uint64_t c = 1;  // (at most the grid's cells: 2^31)
+        for (int d = 0; d < D; d++) c *= (uint64_t)(hi[d] - lo[d]) + 1;
         m = max(m, (uint32_t)c);
+        sum += c;
     }
     m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31u) == 0 && m) atomicMax(most, m);
+    if ((threadIdx.x & 31u) == 0 && m) atomicMax(&ctr->span, m);
+    res_sum(&ctr->sum, sum);
 }
 
 // one thread per box: count its cells
@@ -91,9 +103,14 @@ __global__ void k_res_count(ResGrid g, uint32_t* cnt) {
     }
 }
 
-__global__ void k_res_caps(const uint32_t* cnt, uint32_t* cap, uint64_t ncells) {
-    for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += (uint64_t)gridDim.x * blockDim.x)
-        cap[c] = res_cap(cnt[c]);
+__global__ void k_res_caps(const uint32_t* cnt, uint32_t* cap, uint64_t ncells, ResCtr* ctr) {
+    unsigned long long sum = 0;
+    for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t x = res_cap(cnt[c]);
+        cap[c] = x;
+        sum += x;
+    }
+    res_sum(&ctr->sum, sum);
 }
 
 // ends (in place of the capacities, after the scan) -> starts; used = 0
@@ -112,7 +129,8 @@ __device__ __forceinline__ void res_slot(const uint32_t* b, uint32_t idw, uint4&
     e1 = make_uint4(D == 3 ? b[4] : 0u, D == 3 ? b[5] : 0u, idw, 0u);
 }
 
-// build: every box (one thread each) appended to its cells
+// build: every box (one thread each) appended to its cells (and nothing outside
+// the slots, whatever the scan made of the starts)
 template <int D>
 __global__ void k_res_fill(ResGrid g) {
     constexpr int W = 2 * D + 1;
@@ -126,7 +144,7 @@ __global__ void k_res_fill(ResGrid g) {
                     const uint64_t c = res_gid(g, i, j, kk);
                     const uint32_t f = (i == lo[0] ? 1u : 0u) | (j == lo[1] ? 2u : 0u) | (kk == lo[2] ? 4u : 0u);
                     const uint32_t slot = atomicAdd(&g.used[c], 1u);
-                    if (slot < g.start[c + 1] - g.start[c]) {
+                    if (slot < g.start[c + 1] - g.start[c] && (uint64_t)g.start[c] + slot < g.nslots) {
                         uint4 e0, e1;
                         res_slot<D>(b, (f << kIdBits) | (uint32_t)t, e0, e1);
                         g.entries[2 * (uint64_t)(g.start[c] + slot)] = e0;
@@ -621,6 +639,7 @@ __global__ void __launch_bounds__(kResThreads, kResBlocks) k_move_after(Move m) 
             h.add = __ldcg(&c->add);
             h.full = __ldcg(&c->full);
             h.done = h.span = 0;
+            h.sum = 0;
             *m.host = h;
             __threadfence_system();
         }
@@ -635,13 +654,14 @@ struct pbig2_scene {
     pbig2_ctx* ctx = nullptr;
     int dims = 3;
     uint32_t range = 0, shift = 0, nrc = 0;
-    uint64_t n = 0, ncells = 0;
+    uint64_t n = 0, ncells = 0, nslots = 0;
     DevBuf boxes, start, used, entries, cnt, tmp, state, ctrbuf, lists, idx, nb;
     DevBuf rctr;  // ResCtr, then one bit per box: listed by the move
     DevBuf full[2], rem, add;
     int cur = 0;  // full[cur] holds the current list
     bool stale = false;     // a move that failed half-way left the grid: it is built anew before the next one
     bool keep_full = true;  // maintain the full pair list on every move
+    bool automatic = false; // the cell size is the engine's choice
     uint64_t nfull = 0, nrem = 0, nadd = 0;
 
     size_t rctr_bytes() const { return sizeof(ResCtr) + ((n + 31) / 32) * 4; }
@@ -653,6 +673,7 @@ struct pbig2_scene {
         g.nrc = nrc;
         g.range = range;
         g.ncells = ncells;
+        g.nslots = nslots;
         g.start = start.as<uint32_t>();
         g.used = used.as<uint32_t>();
         g.entries = entries.as<uint4>();
@@ -687,9 +708,15 @@ ResCtr read_ctr(pbig2_scene* s, cudaStream_t st, cudaError_t* e) {
     return h;
 }
 
+void set_shift(pbig2_scene* s, uint32_t shift) {
+    s->shift = shift;
+    s->nrc = nrc_for(s->range, shift);
+    s->ncells = grid_cells(s->range, shift, s->dims);
+}
+
 // With an automatic cell size the scene's grid is one size finer than the
-// query's, where that makes at most 4 cells a box and no box covers more than
-// 512: a move tests the moved boxes against whole cells, while the query tests
+// query's, where that makes at most 4 cells a box, no box covers more than 512
+// and the slots can be numbered: a move tests the moved boxes against whole cells, while the query tests
 // each pair of a cell once. Moves of 1 % of a million boxes of one density 81 us
 // on the query's grid, 70 on the finer one and 69 on the next; of 65 536 boxes
 // 52 and 46; of the clustered 4M-box scene 716, 568 and 621.
@@ -697,24 +724,24 @@ int finer_grid(pbig2_scene* s, cudaStream_t st) {
     if (s->shift == 0 || grid_cells(s->range, s->shift - 1, s->dims) > 4 * s->n) return PBIG2_OK;
     SCK(cudaMemsetAsync(s->rctr.p, 0, sizeof(ResCtr), st));
     const unsigned g = grid_for(s->n, 256, s->ctx->sm_count);
-    unsigned int* most = &s->rctr.as<ResCtr>()->span;
-    if (s->dims == 2) k_res_span<2><<<g, 256, 0, st>>>(s->boxes.as<uint32_t>(), s->n, s->shift - 1, most);
-    else k_res_span<3><<<g, 256, 0, st>>>(s->boxes.as<uint32_t>(), s->n, s->shift - 1, most);
+    if (s->dims == 2) k_res_span<2><<<g, 256, 0, st>>>(s->boxes.as<uint32_t>(), s->n, s->shift - 1, s->rctr.as<ResCtr>());
+    else k_res_span<3><<<g, 256, 0, st>>>(s->boxes.as<uint32_t>(), s->n, s->shift - 1, s->rctr.as<ResCtr>());
     SCK(cudaGetLastError());
     cudaError_t e;
     const ResCtr h = read_ctr(s, st, &e);
     SCK(e);
-    if (h.span > 512) return PBIG2_OK;
-    s->shift--;
-    s->nrc = nrc_for(s->range, s->shift);
-    s->ncells = grid_cells(s->range, s->shift, s->dims);
+    if (h.span > 512 || pbig2_scene_slots(grid_cells(s->range, s->shift - 1, s->dims), h.sum) > kMaxSlots) return PBIG2_OK;
+    set_shift(s, s->shift - 1);
     return PBIG2_OK;
 }
 
 // the grid of the scene's current boxes: counts, capacities with slack,
-// starts (the engine's scan), then every box inserted
+// starts (the engine's scan), then every box inserted. The slots are summed in
+// 64 bits before anything is placed by them: 2^32 or more are refused.
 int build_grid(pbig2_scene* s, cudaStream_t st) {
     const int sms = s->ctx->sm_count;
+    if (pbig2_scene_slots(s->ncells, 0) + s->n > kMaxSlots)  // (every box has an entry)
+        return api_fail(PBIG2_ECAPACITY, "resident grid: 2^32 slots or more");
     SCK(s->cnt.ensure(s->ncells * 4 + 16, false, st));
     SCK(s->tmp.ensure(s->ncells * 4 + 16, false, st));
     SCK(s->start.ensure((s->ncells + 1) * 4, false, st));
@@ -728,8 +755,15 @@ int build_grid(pbig2_scene* s, cudaStream_t st) {
     if (s->dims == 2) k_res_count<2><<<grid_for(s->n, 256, sms), 256, 0, st>>>(g, s->cnt.as<uint32_t>());
     else k_res_count<3><<<grid_for(s->n, 256, sms), 256, 0, st>>>(g, s->cnt.as<uint32_t>());
     SCK(cudaGetLastError());
-    k_res_caps<<<grid_for(s->ncells, 256, sms), 256, 0, st>>>(s->cnt.as<uint32_t>(), s->tmp.as<uint32_t>(), s->ncells);
+    k_res_caps<<<grid_for(s->ncells, 256, sms), 256, 0, st>>>(s->cnt.as<uint32_t>(), s->tmp.as<uint32_t>(), s->ncells, g.ctr);
     SCK(cudaGetLastError());
+    cudaError_t e;
+    ResCtr h = read_ctr(s, st, &e);
+    SCK(e);
+    if (h.sum > kMaxSlots) return api_fail(PBIG2_ECAPACITY, "resident grid: 2^32 slots or more");
+    s->nslots = h.sum;
+    SCK(s->entries.ensure(s->nslots * 32 + 32, false, st));
+    g = s->grid();
     // exclusive scan of the capacities with the engine's scan kernels (the
     // cell ends replace the capacities in place; no work lists)
     Params p{};
@@ -743,22 +777,26 @@ int build_grid(pbig2_scene* s, cudaStream_t st) {
     SCK(launch_scan(p, st));
     k_res_starts<<<grid_for(s->ncells, 256, sms), 256, 0, st>>>(s->cnt.as<uint32_t>(), s->tmp.as<uint32_t>(), g);
     SCK(cudaGetLastError());
-    uint32_t total = 0;
-    SCK(cudaMemcpyAsync(&total, s->start.as<uint32_t>() + s->ncells, 4, cudaMemcpyDeviceToHost, st));
-    SCK(cudaStreamSynchronize(st));
-    SCK(s->entries.ensure((uint64_t)total * 32 + 32, false, st));
     // free slots hold no tombstone of an older grid: one that a box is about to
     // be appended to must not be claimed by another box of the same move
-    SCK(cudaMemsetAsync(s->entries.p, 0, (uint64_t)total * 32, st));
-    g = s->grid();
+    SCK(cudaMemsetAsync(s->entries.p, 0, s->nslots * 32, st));
     if (s->dims == 2) k_res_fill<2><<<grid_for(s->n, 256, sms), 256, 0, st>>>(g);
     else k_res_fill<3><<<grid_for(s->n, 256, sms), 256, 0, st>>>(g);
     SCK(cudaGetLastError());
-    cudaError_t e;
-    const ResCtr h = read_ctr(s, st, &e);
+    h = read_ctr(s, st, &e);
     SCK(e);
     if (h.overflow) return api_fail(PBIG2_ECUDA, "resident grid: a cell overflowed its own count");
     return PBIG2_OK;
+}
+
+// with an automatic cell size, on coarser grids until the slots can be numbered
+int build(pbig2_scene* s, cudaStream_t st) {
+    int rc = build_grid(s, st);
+    while (rc == PBIG2_ECAPACITY && s->automatic && s->ncells > 1 && s->shift < 31) {
+        set_shift(s, s->shift + 1);
+        rc = build_grid(s, st);
+    }
+    return rc;
 }
 
 // room for `need` pairs in a buffer that keeps its first `have`: a move that
@@ -800,6 +838,11 @@ cudaError_t launch_move(pbig2_scene* s, const Move& m, MovePart part, cudaStream
 
 extern "C" {
 
+PBIG2_API uint64_t pbig2_scene_slots(uint64_t ncells, uint64_t entries) {
+    const unsigned __int128 s = (unsigned __int128)entries + entries / 2 + (unsigned __int128)ncells * res_cap(0);
+    return s > ~0ull ? ~0ull : (uint64_t)s;
+}
+
 PBIG2_API int pbig2_scene_create(pbig2_ctx* c, const uint32_t* boxes, uint64_t n, uint32_t dims, uint32_t range,
                                  uint32_t cell_shift, int boxes_loc, uint32_t flags, pbig2_scene** out,
                                  uint64_t* npairs) {
@@ -820,10 +863,9 @@ PBIG2_API int pbig2_scene_create(pbig2_ctx* c, const uint32_t* boxes, uint64_t n
     s->ctx = c;
     s->dims = (int)dims;
     s->range = range;
-    s->shift = st.cell_shift;
-    s->nrc = nrc_for(range, s->shift);
     s->n = n;
-    s->ncells = grid_cells(range, s->shift, (int)dims);  // below 2^32: the query above ran on this grid
+    s->automatic = cell_shift == PBIG2_AUTO;
+    set_shift(s, st.cell_shift);  // below 2^32 cells: the query above ran on this grid
     cudaStream_t sm = c->own_stream;
     const int W = 2 * (int)dims + 1;
     auto bail = [&](int code) {
@@ -839,11 +881,11 @@ PBIG2_API int pbig2_scene_create(pbig2_ctx* c, const uint32_t* boxes, uint64_t n
     if (np && pbig2_copy_pairs(c, s->full[0].as<uint32_t>(), 0, np, PBIG2_DEVICE, sm) != PBIG2_OK) return bail(PBIG2_ECUDA);
     s->nfull = np;
     s->keep_full = (flags & PBIG2_SCENE_DELTA_ONLY) == 0;
-    if (cell_shift == PBIG2_AUTO) {
+    if (s->automatic) {
         rc = finer_grid(s, sm);
         if (rc != PBIG2_OK) return bail(rc);
     }
-    rc = build_grid(s, sm);
+    rc = build(s, sm);
     if (rc != PBIG2_OK) return bail(rc);
     *out = s;
     *npairs = np;
@@ -877,7 +919,7 @@ PBIG2_API int pbig2_scene_move(pbig2_scene* s, const uint32_t* idx, uint64_t k, 
     SCK(s->idx.ensure(k * 4 + 16, false, st));
     SCK(s->nb.ensure(k * W * 4 + 16, false, st));
     if (s->stale) {
-        const int rc = build_grid(s, st);
+        const int rc = build(s, st);
         if (rc) return rc;
         s->stale = false;
     }
@@ -935,7 +977,7 @@ PBIG2_API int pbig2_scene_move(pbig2_scene* s, const uint32_t* idx, uint64_t k, 
             if (!m.full) again.rem = h.rem;
             part = kMoveRest;
             if (h.overflow) {  // a cell ran out of slack
-                const int rc = build_grid(s, st);
+                const int rc = build(s, st);
                 if (rc) return rc;
                 m.g = s->grid();
                 h.add = guess;

@@ -33,6 +33,7 @@ EXPORTS = [
     "pbig2_scene_move", "pbig2_scene_delta", "pbig2_scene_pairs", "pbig2_scene_boxes", "pbig2_scene_copy",
     "pbig2_result_records", "pbig2_copy_records", "pbig2_decode_records", "pbig2_serve_batch",
     "pbig2_grid_cells", "pbig2_result_scene_shifts", "pbig2_class_map_auto", "pbig2_class_map_check",
+    "pbig2_scene_slots",
 ]
 
 
@@ -104,6 +105,8 @@ def lib():
         L.pbig2_tune_shift.argtypes = [vp, u64, u32, u32, u64, C.POINTER(u32)]
         L.pbig2_grid_cells.argtypes = [u32, u32, u32]
         L.pbig2_grid_cells.restype = u64
+        L.pbig2_scene_slots.argtypes = [u64, u64]
+        L.pbig2_scene_slots.restype = u64
         L.pbig2_class_map_auto.argtypes = [u32]
         L.pbig2_class_map_auto.restype = u64
         L.pbig2_class_map_check.argtypes = [u64]
