@@ -244,6 +244,10 @@ PBIG2_API int pbig2_get_stats(pbig2_ctx* ctx, pbig2_stats* stats);
    block limit -- a block grows while its boxes stay within the limit. The
    pair set does not depend on it; the merged build's statistics do. */
 #define PBIG2_OPT_MERGE_LIMIT 7
+/* PBIG2_OPT_MAX_BUFFER (default 0 = any): the most bytes of one device buffer
+   that the context and its scenes may allocate from now on. A call that needs
+   a larger one fares as on a device without the memory. */
+#define PBIG2_OPT_MAX_BUFFER 8
 
 /* The automatic class map: the work lists a query takes when no map is set
    (one_launch: a small scene's one-launch query). Measured on GB300: the
@@ -327,7 +331,8 @@ PBIG2_API const char* pbig2_noalloc_last_error(void);
  * context's last-result pointers are overwritten by pbig2_scene_create.
  * The grid has one slot and a half per entry and four more per cell, 32 bytes
  * each, and 2^32 - 1 of them at most: an automatic cell size is coarsened to
- * fit, a given one that does not fit is refused (PBIG2_ECAPACITY). */
+ * fit these and the device's memory, a given one that does not fit is refused
+ * (PBIG2_ECAPACITY, PBIG2_ENOMEM). */
 typedef struct pbig2_scene pbig2_scene;
 #define PBIG2_SCENE_DELTA_ONLY 1u /* flags: moves report their delta only; no full list is kept */
 PBIG2_API int pbig2_scene_create(pbig2_ctx* ctx, const uint32_t* boxes, uint64_t n, uint32_t dims, uint32_t range,

@@ -46,8 +46,9 @@ cudaError_t DevBuf::ensure(size_t need, bool zero, cudaStream_t st) {
     release();
     size_t b = need + need / 8;
     b = (b + 255) & ~size_t(255);
-    cudaError_t e = cudaMalloc(&p, b);
+    cudaError_t e = most && *most && b > *most ? cudaErrorMemoryAllocation : cudaMalloc(&p, b);
     if (e != cudaSuccess) {
+        (void)cudaGetLastError();  // (reported here, and not by the next launch's check)
         p = nullptr;
         return e;
     }
@@ -1024,6 +1025,7 @@ PBIG2_API int pbig2_create(int device, pbig2_ctx** out) {
     CK(cudaSetDevice(device));
     pbig2_ctx* c = new pbig2_ctx();
     c->device = device;
+    c->each_buffer([c](DevBuf& b) { b.most = &c->max_buffer; });
     cudaError_t e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking);
@@ -1043,11 +1045,7 @@ PBIG2_API int pbig2_destroy(pbig2_ctx* c) {
     cudaSetDevice(c->device);
     if (c->own_stream) cudaStreamSynchronize(c->own_stream);
     c->drop_graph();
-    for (DevBuf* b : {&c->d_boxes, &c->d_counts, &c->d_entries, &c->d_recs, &c->d_merged, &c->d_merged_ext, &c->d_bar, &c->d_fctr,
-                      &c->d_lists, &c->d_tasks, &c->d_state,
-                      &c->d_out, &c->d_out2, &c->d_ctr, &c->d_scenes, &c->d_scene_off, &c->d_scene_pair,
-                      &c->d_scene_cursor, &c->d_dims, &c->d_scene_tab, &c->d_tune, &c->d_tune_cost, &c->d_group})
-        b->release();
+    c->each_buffer([](DevBuf& b) { b.release(); });
     c->h_ctr.release();
     c->h_pair_off.release();
     c->h_stage.release();
@@ -1444,6 +1442,11 @@ PBIG2_API int pbig2_set_option(pbig2_ctx* c, int option, int64_t value) {
             return PBIG2_OK;
         }
         c->use_fused = value != 0;
+        return PBIG2_OK;
+    }
+    if (option == PBIG2_OPT_MAX_BUFFER) {
+        if (value < 0) return fail(PBIG2_EINVAL, "largest buffer of %lld bytes", (long long)value);
+        c->max_buffer = (uint64_t)value;
         return PBIG2_OK;
     }
     if (option == PBIG2_OPT_HOST_SPLIT) {

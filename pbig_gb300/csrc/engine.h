@@ -15,6 +15,7 @@ namespace pbig {
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    const uint64_t* most = nullptr;  // bytes of the largest allocation there may be (0: any)
     cudaError_t ensure(size_t need, bool zero, cudaStream_t st);
     void release();
     template <class T> T* as() const { return reinterpret_cast<T*>(p); }
@@ -52,6 +53,7 @@ struct pbig2_ctx {
     cudaStream_t own_stream = nullptr;
     pbig::DevBuf d_merged, d_merged_ext;  // merged mode: cell -> root table; the roots' extents
     pbig::DevBuf d_recs;    // record mode: box index of every entry
+    uint64_t max_buffer = 0;  // PBIG2_OPT_MAX_BUFFER
     bool merged_mode = false;
     bool rice_mode = false;      // record mode (PBIG2_OPT_RICE)
     bool result_records = false; // the last result is a record stream
@@ -99,6 +101,13 @@ struct pbig2_ctx {
                                       &d_scene_tab, &d_group})
             h = h * 1000003u + (uintptr_t)b->p;
         return (h * 1000003u + (uintptr_t)h_ctr.p) * 1000003u + (uintptr_t)h_pair_off.p;
+    }
+    template <class F>
+    void each_buffer(F f) {
+        for (pbig::DevBuf* b : {&d_boxes, &d_counts, &d_entries, &d_recs, &d_merged, &d_merged_ext, &d_bar, &d_fctr, &d_lists,
+                                &d_tasks, &d_state, &d_out, &d_out2, &d_ctr, &d_scenes, &d_scene_off, &d_scene_pair,
+                                &d_scene_cursor, &d_dims, &d_scene_tab, &d_tune, &d_tune_cost, &d_group})
+            f(*b);
     }
     void drop_graph() {
         if (graph.exec) cudaGraphExecDestroy(graph.exec);

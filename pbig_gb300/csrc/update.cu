@@ -664,6 +664,12 @@ struct pbig2_scene {
     bool automatic = false; // the cell size is the engine's choice
     uint64_t nfull = 0, nrem = 0, nadd = 0;
 
+    template <class F>
+    void each_buffer(F f) {
+        for (DevBuf* b : {&boxes, &start, &used, &entries, &cnt, &tmp, &state, &ctrbuf, &rctr, &lists, &idx, &nb, &full[0],
+                          &full[1], &rem, &add})
+            f(*b);
+    }
     size_t rctr_bytes() const { return sizeof(ResCtr) + ((n + 31) / 32) * 4; }
     ResGrid grid() {
         ResGrid g{};
@@ -790,9 +796,11 @@ int build_grid(pbig2_scene* s, cudaStream_t st) {
 }
 
 // with an automatic cell size, on coarser grids until the slots can be numbered
+// and there is memory for them
 int build(pbig2_scene* s, cudaStream_t st) {
     int rc = build_grid(s, st);
-    while (rc == PBIG2_ECAPACITY && s->automatic && s->ncells > 1 && s->shift < 31) {
+    while ((rc == PBIG2_ECAPACITY || rc == PBIG2_ENOMEM) && s->automatic && s->ncells > 1 && s->shift < 31) {
+        for (DevBuf* b : {&s->cnt, &s->tmp, &s->start, &s->used, &s->state, &s->entries}) b->release();
         set_shift(s, s->shift + 1);
         rc = build_grid(s, st);
     }
@@ -804,6 +812,7 @@ int build(pbig2_scene* s, cudaStream_t st) {
 cudaError_t room_for(DevBuf& buf, uint64_t need, uint64_t have, cudaStream_t st) {
     if (need * 8 <= buf.bytes) return cudaSuccess;
     DevBuf grown;
+    grown.most = buf.most;
     cudaError_t e = grown.ensure(need * 8, false, st);
     if (e == cudaSuccess && have) {
         e = cudaMemcpyAsync(grown.p, buf.p, have * 8, cudaMemcpyDeviceToDevice, st);
@@ -861,6 +870,7 @@ PBIG2_API int pbig2_scene_create(pbig2_ctx* c, const uint32_t* boxes, uint64_t n
     pbig2_get_stats(c, &st);
     pbig2_scene* s = new pbig2_scene();
     s->ctx = c;
+    s->each_buffer([c](DevBuf& b) { b.most = &c->max_buffer; });
     s->dims = (int)dims;
     s->range = range;
     s->n = n;
@@ -894,9 +904,7 @@ PBIG2_API int pbig2_scene_create(pbig2_ctx* c, const uint32_t* boxes, uint64_t n
 
 PBIG2_API int pbig2_scene_destroy(pbig2_scene* s) {
     if (!s) return PBIG2_OK;
-    for (DevBuf* b : {&s->boxes, &s->start, &s->used, &s->entries, &s->cnt, &s->tmp, &s->state, &s->ctrbuf, &s->rctr,
-                      &s->lists, &s->idx, &s->nb, &s->full[0], &s->full[1], &s->rem, &s->add})
-        b->release();
+    s->each_buffer([](DevBuf& b) { b.release(); });
     delete s;
     return PBIG2_OK;
 }

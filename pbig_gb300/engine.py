@@ -354,6 +354,11 @@ class Engine:
         fifths; negative: one after another)."""
         _check(self._L.pbig2_set_option(self._ctx, 4, int(sms)))
 
+    def set_max_buffer(self, size: int) -> None:
+        """The most bytes of one device buffer that the context and its scenes
+        may allocate from now on (0: any)."""
+        _check(self._L.pbig2_set_option(self._ctx, 8, int(size)))
+
     def set_one_launch(self, on: bool) -> None:
         """Run small self queries (at most 262 144 boxes) as one cooperative
         kernel launch (on by default); off: the regular pipeline."""

@@ -1,5 +1,6 @@
-"""Resident scenes whose boxes are very small against their spacing: the
-query's grid has cells that the scene's slots cannot all be numbered for."""
+"""Grids of resident scenes that do not fit: boxes so small against their
+spacing that the slots of the query's grid cannot all be numbered, and too
+little memory for the finer grid that scenes get."""
 import numpy as np
 import pytest
 
@@ -60,3 +61,29 @@ def test_a_given_size_that_does_not_fit_is_refused():
         sc = Scene(engine, boxes, RANGE, cell_shift=17)
         assert np.array_equal(canon(sc.pairs()), want(boxes))
         sc.close()
+
+
+def test_without_memory_for_the_finer_grid_a_scene_keeps_the_querys():
+    n, limit = 80000, 24 << 20
+    r = np.random.default_rng(4)
+    side = 0.6 * n ** (-1 / 3) * RANGE
+    boxes = np.empty((n, 7), dtype=np.uint32)
+    boxes[:, 0:6:2] = lo = r.integers(0, RANGE - int(side), size=(n, 3))
+    boxes[:, 1:6:2] = lo + r.integers(0, int(side), size=(n, 3))
+    boxes[:, 6] = np.arange(n)
+    with Engine(0) as engine:
+        engine.self_intersect(boxes, RANGE)
+        cells = engine.stats()["cells"]
+        assert 8 * cells <= 4 * n and 8 * cells * 4 * 32 > limit  # one size finer: taken, and its empty slots alone too many
+    with Engine(0) as engine:
+        engine.set_max_buffer(limit)
+        sc = Scene(engine, boxes, RANGE)
+        try:
+            idx = np.arange(0, n, 50, dtype=np.uint32)
+            nb = boxes[idx].copy()
+            nb[:, :6] = boxes[(idx + 25) % n, :6]
+            sc.move(idx, nb)
+            boxes[idx] = nb
+            assert np.array_equal(canon(sc.pairs()), want(boxes))
+        finally:
+            sc.close()
