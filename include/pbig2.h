@@ -329,6 +329,9 @@ PBIG2_API const char* pbig2_noalloc_last_error(void);
  * step that flags = PBIG2_SCENE_DELTA_ONLY leaves out. The scene uses
  * ctx's stream and buffers: one scene call at a time per context, and the
  * context's last-result pointers are overwritten by pbig2_scene_create.
+ * A move that is refused (PBIG2_EINVAL) leaves everything as it was. One that
+ * fails for want of memory leaves the boxes and the full list as they were, and
+ * no delta of the move before it to rely on.
  * The grid has one slot and a half per entry and four more per cell, 32 bytes
  * each, and 2^32 - 1 of them at most: an automatic cell size is coarsened to
  * fit these and the device's memory, a given one that does not fit is refused

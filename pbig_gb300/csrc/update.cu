@@ -174,7 +174,7 @@ __device__ __forceinline__ bool res_moved(const uint32_t* bits, uint32_t id) { r
 struct Move {
     ResGrid g;
     const uint32_t* idx;  // [k] listed boxes
-    const uint32_t* nb;   // [k] their new rows
+    uint32_t* nb;         // [k] their new rows; once they have moved, their old ones
     uint64_t k;
     uint32_t* moved;      // one bit per box of the scene
     uint2* rem;
@@ -567,7 +567,12 @@ __global__ void __launch_bounds__(kResThreads) k_move_in(Move m, uint32_t* boxes
         res_range<D>(boxes + (uint64_t)id * W, g.shift, lo0, hi0);
         res_range<D>(a, g.shift, lo, hi);
         __syncwarp();  // (every lane has read the old coordinates)
-        if (lane < W) boxes[(uint64_t)id * W + lane] = b[lane];
+        if (lane < W) {  // (the old row stays at hand: k_move_back)
+            uint32_t &now = boxes[(uint64_t)id * W + lane], &then = m.nb[t * W + lane];
+            const uint32_t w = now;
+            now = then;
+            then = w;
+        }
         auto put = [&](uint64_t slot, uint32_t idw) {
             uint4 e0, e1;
             res_slot<D>(a, idw, e0, e1);
@@ -617,6 +622,14 @@ __global__ void __launch_bounds__(kResThreads) k_move_in(Move m, uint32_t* boxes
     }
 }
 
+// the rows that k_move_in left at hand, back in their places
+template <int D>
+__global__ void k_move_back(Move m, uint32_t* boxes) {
+    constexpr int W = 2 * D + 1;
+    for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < m.k * W; w += (uint64_t)gridDim.x * blockDim.x)
+        boxes[(uint64_t)m.idx[w / W] * W + w % W] = m.nb[w];
+}
+
 // pairs of the listed boxes after the move, to the list of added pairs and
 // behind the filtered full list; the last block hands the counters to the host
 template <int D>
@@ -660,6 +673,7 @@ struct pbig2_scene {
     DevBuf full[2], rem, add;
     int cur = 0;  // full[cur] holds the current list
     bool stale = false;     // a move that failed half-way left the grid: it is built anew before the next one
+    bool lost = false;      // a CUDA error struck while the boxes were moving
     bool keep_full = true;  // maintain the full pair list on every move
     bool automatic = false; // the cell size is the engine's choice
     uint64_t nfull = 0, nrem = 0, nadd = 0;
@@ -699,6 +713,8 @@ namespace {
             return api_fail(_e == cudaErrorMemoryAllocation ? PBIG2_ENOMEM : PBIG2_ECUDA, _m);        \
         }                                                                                              \
     } while (0)
+
+constexpr char kLost[] = "the scene was lost to a CUDA error in a move";
 
 unsigned grid_for(uint64_t items, unsigned per_block, int sms) {
     uint64_t b = (items + per_block - 1) / per_block;
@@ -843,6 +859,79 @@ cudaError_t launch_move(pbig2_scene* s, const Move& m, MovePart part, cudaStream
     return e != cudaSuccess ? e : launch_after(all || r + f, k_move_after<D>, gw, kResThreads, 0, st, m);
 }
 
+// The passes of a move until the pairs before and after it fit their lists.
+// `part`: whether the boxes have moved. A move that fails once its kernels have
+// run leaves `stale` set.
+int move_passes(pbig2_scene* s, Move& m, uint64_t guess, ResCtr& h, MovePart& part, cudaStream_t st) {
+    const int nxt = s->cur ^ 1;
+    for (int attempt = 0;; attempt++) {
+        m.rem = s->rem.as<uint2>();
+        m.add = s->add.as<uint2>();
+        m.rem_cap = s->rem.bytes / 8;
+        m.add_cap = s->add.bytes / 8;
+        if (s->keep_full) {
+            // (the list that a larger one of these replaces is the one before the last)
+            SCK(s->full[nxt].ensure((s->nfull + (part == kMoveAll ? guess : h.add)) * 8 + 16, false, st));
+            const uint64_t room = s->full[nxt].bytes / 8 - s->nfull;
+            if (m.add_cap > room) m.add_cap = room;
+            m.old_full = s->full[s->cur].as<uint2>();
+            m.full = s->full[nxt].as<uint2>();
+            m.nold = s->nfull;
+        }
+        s->stale = true;
+        SCK(s->dims == 2 ? launch_move<2>(s, m, part, st) : launch_move<3>(s, m, part, st));
+        SCK(cudaStreamSynchronize(st));
+        h = *m.host;
+        if (h.err) {
+            s->stale = false;  // nothing was touched
+            return api_fail(PBIG2_EINVAL, h.err == kErrIndex
+                                              ? "a box is listed twice"
+                                              : "moved boxes must keep rid = their index, coordinates < range and min <= max");
+        }
+        const bool more_rem = h.rem > m.rem_cap, more_add = !more_rem && !h.overflow && h.add > m.add_cap;
+        if (!more_rem && !h.overflow && !more_add) break;
+        if (attempt == 4) return api_fail(PBIG2_ENOMEM, "pair buffer retries exhausted");
+        ResCtr again{};
+        if (more_rem) {  // the boxes have their old coordinates
+            s->nrem = 0;
+            SCK(s->rem.ensure(h.rem * 8 + h.rem / 4, false, st));
+        } else {
+            if (!m.full) again.rem = h.rem;
+            part = kMoveRest;
+            if (h.overflow) {  // a cell ran out of slack
+                const int rc = build(s, st);
+                if (rc) return rc;
+                m.g = s->grid();
+                h.add = guess;
+            } else {
+                s->nadd = 0;
+                SCK(s->add.ensure(h.add * 8 + h.add / 4, false, st));
+            }
+        }
+        // (the check marks the boxes again, or they stay marked)
+        if (more_rem) SCK(cudaMemsetAsync(s->rctr.p, 0, s->rctr_bytes(), st));
+        else SCK(cudaMemcpyAsync(s->rctr.p, &again, sizeof again, cudaMemcpyHostToDevice, st));
+    }
+    return PBIG2_OK;
+}
+
+// What is left of a move that failed on the way, for want of memory: the boxes
+// have their old rows again, so that the full list is theirs, and the grid is
+// built anew before the next move. After a CUDA error the scene is lost.
+int take_back(pbig2_scene* s, const Move& m, MovePart part, int rc, cudaStream_t st) {
+    s->nrem = s->nadd = 0;
+    if (rc == PBIG2_ECUDA) {
+        s->lost = true;
+        return rc;
+    }
+    if (part == kMoveAll) return rc;  // the boxes had not moved
+    const unsigned g = grid_for(m.k, 256, s->ctx->sm_count);
+    if (s->dims == 2) k_move_back<2><<<g, 256, 0, st>>>(m, s->boxes.as<uint32_t>());
+    else k_move_back<3><<<g, 256, 0, st>>>(m, s->boxes.as<uint32_t>());
+    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) s->lost = true;
+    return rc;
+}
+
 }  // namespace
 
 extern "C" {
@@ -918,6 +1007,7 @@ PBIG2_API int pbig2_scene_move(pbig2_scene* s, const uint32_t* idx, uint64_t k, 
         return PBIG2_OK;
     }
     if (k > s->n) return api_fail(PBIG2_EINVAL, "more moved boxes than the scene holds");
+    if (s->lost) return api_fail(PBIG2_ECUDA, kLost);
     SCK(cudaSetDevice(s->ctx->device));
     cudaStream_t st = s->ctx->own_stream;
     const int W = 2 * s->dims + 1;
@@ -940,7 +1030,6 @@ PBIG2_API int pbig2_scene_move(pbig2_scene* s, const uint32_t* idx, uint64_t k, 
     const uint64_t guess = 1024 + (mean < s->nfull ? mean : s->nfull);
     SCK(room_for(s->rem, guess, s->nrem, st));
     SCK(room_for(s->add, guess, s->nadd, st));
-    const int nxt = s->cur ^ 1;
     Move m{};
     m.g = s->grid();
     m.idx = s->idx.as<uint32_t>();
@@ -950,57 +1039,11 @@ PBIG2_API int pbig2_scene_move(pbig2_scene* s, const uint32_t* idx, uint64_t k, 
     m.host = static_cast<ResCtr*>(s->ctx->h_ctr.p);
     ResCtr h{};
     MovePart part = kMoveAll;
-    for (int attempt = 0;; attempt++) {
-        m.rem = s->rem.as<uint2>();
-        m.add = s->add.as<uint2>();
-        m.rem_cap = s->rem.bytes / 8;
-        m.add_cap = s->add.bytes / 8;
-        if (s->keep_full) {
-            // (the list that a larger one of these replaces is the one before the last)
-            SCK(s->full[nxt].ensure((s->nfull + (part == kMoveAll ? guess : h.add)) * 8 + 16, false, st));
-            const uint64_t room = s->full[nxt].bytes / 8 - s->nfull;
-            if (m.add_cap > room) m.add_cap = room;
-            m.old_full = s->full[s->cur].as<uint2>();
-            m.full = s->full[nxt].as<uint2>();
-            m.nold = s->nfull;
-        }
-        s->stale = true;
-        SCK(s->dims == 2 ? launch_move<2>(s, m, part, st) : launch_move<3>(s, m, part, st));
-        SCK(cudaStreamSynchronize(st));
-        h = *m.host;
-        if (h.err) {
-            s->stale = false;  // nothing was touched
-            return api_fail(PBIG2_EINVAL, h.err == kErrIndex
-                                              ? "a box is listed twice"
-                                              : "moved boxes must keep rid = their index, coordinates < range and min <= max");
-        }
-        const bool more_rem = h.rem > m.rem_cap, more_add = !more_rem && !h.overflow && h.add > m.add_cap;
-        if (!more_rem && !h.overflow && !more_add) break;
-        if (attempt == 4) return api_fail(PBIG2_ENOMEM, "pair buffer retries exhausted");
-        ResCtr again{};
-        if (more_rem) {  // the boxes have their old coordinates
-            s->nrem = 0;
-            SCK(s->rem.ensure(h.rem * 8 + h.rem / 4, false, st));
-        } else {
-            if (!m.full) again.rem = h.rem;
-            part = kMoveRest;
-            if (h.overflow) {  // a cell ran out of slack
-                const int rc = build(s, st);
-                if (rc) return rc;
-                m.g = s->grid();
-                h.add = guess;
-            } else {
-                s->nadd = 0;
-                SCK(s->add.ensure(h.add * 8 + h.add / 4, false, st));
-            }
-        }
-        // (the check marks the boxes again, or they stay marked)
-        if (more_rem) SCK(cudaMemsetAsync(s->rctr.p, 0, s->rctr_bytes(), st));
-        else SCK(cudaMemcpyAsync(s->rctr.p, &again, sizeof again, cudaMemcpyHostToDevice, st));
-    }
+    const int rc = move_passes(s, m, guess, h, part, st);
+    if (rc) return s->stale ? take_back(s, m, part, rc, st) : rc;
     s->stale = false;
     if (s->keep_full) {
-        s->cur = nxt;
+        s->cur ^= 1;
         s->nfull = h.full;
     }
     *n_removed = s->nrem = h.rem;
@@ -1011,6 +1054,7 @@ PBIG2_API int pbig2_scene_move(pbig2_scene* s, const uint32_t* idx, uint64_t k, 
 PBIG2_API int pbig2_scene_delta(pbig2_scene* s, const uint32_t** removed, uint64_t* n_removed, const uint32_t** added,
                                 uint64_t* n_added) {
     if (!s || !removed || !n_removed || !added || !n_added) return api_fail(PBIG2_EINVAL, "bad arguments");
+    if (s->lost) return api_fail(PBIG2_ECUDA, kLost);
     *removed = s->rem.as<uint32_t>();
     *n_removed = s->nrem;
     *added = s->add.as<uint32_t>();
@@ -1021,6 +1065,7 @@ PBIG2_API int pbig2_scene_delta(pbig2_scene* s, const uint32_t** removed, uint64
 PBIG2_API int pbig2_scene_pairs(pbig2_scene* s, const uint32_t** pairs, uint64_t* npairs) {
     if (!s || !pairs || !npairs) return api_fail(PBIG2_EINVAL, "bad arguments");
     if (!s->keep_full) return api_fail(PBIG2_EINVAL, "the scene keeps no full pair list (PBIG2_SCENE_DELTA_ONLY)");
+    if (s->lost) return api_fail(PBIG2_ECUDA, kLost);
     *pairs = s->full[s->cur].as<uint32_t>();
     *npairs = s->nfull;
     return PBIG2_OK;
@@ -1029,6 +1074,7 @@ PBIG2_API int pbig2_scene_pairs(pbig2_scene* s, const uint32_t** pairs, uint64_t
 PBIG2_API int pbig2_scene_copy(pbig2_scene* s, int which, uint32_t* dst, uint64_t count) {
     if (!s || (count && !dst) || which < 0 || which > 2) return api_fail(PBIG2_EINVAL, "bad arguments");
     if (which == 0 && !s->keep_full) return api_fail(PBIG2_EINVAL, "the scene keeps no full pair list (PBIG2_SCENE_DELTA_ONLY)");
+    if (s->lost) return api_fail(PBIG2_ECUDA, kLost);
     const uint64_t have = which == 0 ? s->nfull : which == 1 ? s->nrem : s->nadd;
     if (count > have) return api_fail(PBIG2_EINVAL, "more pairs asked for than the list holds");
     if (count == 0) return PBIG2_OK;
@@ -1041,6 +1087,7 @@ PBIG2_API int pbig2_scene_copy(pbig2_scene* s, int which, uint32_t* dst, uint64_
 
 PBIG2_API int pbig2_scene_boxes(pbig2_scene* s, const uint32_t** boxes, uint64_t* n) {
     if (!s || !boxes || !n) return api_fail(PBIG2_EINVAL, "bad arguments");
+    if (s->lost) return api_fail(PBIG2_ECUDA, kLost);
     *boxes = s->boxes.as<uint32_t>();
     *n = s->n;
     return PBIG2_OK;

@@ -426,8 +426,11 @@ class Scene:
         if nb.shape != (idx.shape[0], 2 * self.dims + 1):
             raise ValueError("new_boxes must hold one RectInfo row per index")
         r, a = C.c_uint64(), C.c_uint64()
-        _check(self._L.pbig2_scene_move(self._sc, C.c_void_p(idx.ctypes.data), idx.shape[0],
-                                        C.c_void_p(nb.ctypes.data), HOST, C.byref(r), C.byref(a)))
+        rc = self._L.pbig2_scene_move(self._sc, C.c_void_p(idx.ctypes.data), idx.shape[0],
+                                      C.c_void_p(nb.ctypes.data), HOST, C.byref(r), C.byref(a))
+        if rc not in (OK, EINVAL):  # (a refused move leaves the last one's lists)
+            self.nremoved = self.nadded = 0
+        _check(rc)
         self.nremoved, self.nadded = r.value, a.value
         return r.value, a.value
 
