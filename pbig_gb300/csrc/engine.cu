@@ -700,8 +700,8 @@ struct SingleScene {
 constexpr uint64_t kBlindBoxes = 1u << 25;
 
 // A self or red/blue query of one scene at cell shift `shift` (PBIG2_AUTO:
-// chosen on the device). used: the cell shift it ran at.
-static int run_single(pbig2_ctx* c, const SingleScene& q, uint32_t shift, cudaStream_t st, uint32_t* used) {
+// chosen on the device). used: the cell shift it ran at. blind: launched whole.
+static int run_single_in(pbig2_ctx* c, const SingleScene& q, uint32_t shift, bool blind, cudaStream_t st, uint32_t* used) {
     c->last_err = 0;
     c->fused_dirty = true;  // this pipeline leaves cell starts in the counters
     c->merged_blocks = 0;
@@ -709,7 +709,6 @@ static int run_single(pbig2_ctx* c, const SingleScene& q, uint32_t shift, cudaSt
     if (q.n > (uint64_t)kIdMask + 1)
         return fail(PBIG2_EINVAL, "a query holds at most 2^29 boxes (got %llu)", (unsigned long long)q.n);
     if (c->rice_mode && q.bip) return fail(PBIG2_EINVAL, "record mode serves self queries only");
-    const bool blind = !c->merged_mode && q.n <= kBlindBoxes;
     Need need{};
     const uint64_t have_cells = c->d_counts.bytes >= 64 ? (c->d_counts.bytes - 16) / 4 : 0;
     need.cells = blind ? std::max<uint64_t>(8 * q.n + (1u << 20), have_cells) : 0;
@@ -851,6 +850,16 @@ static bool fused_eligible(const pbig2_ctx* c, uint64_t n, int dims, uint32_t ra
     if (!c->use_fused || fused_blocks() <= 0 || c->merged_mode || c->rice_mode) return false;
     if (n == 0 || n > kFusedMaxBoxes) return false;
     return cell_shift == PBIG2_AUTO || grid_cells(range, cell_shift, dims) <= kFusedMaxCells;
+}
+
+// (the buffers of a query launched whole are sized without its estimate: where
+// there is no memory for them it is read first)
+static int run_single(pbig2_ctx* c, const SingleScene& q, uint32_t shift, cudaStream_t st, uint32_t* used) {
+    const bool blind = !c->merged_mode && q.n <= kBlindBoxes;
+    const int rc = run_single_in(c, q, shift, blind, st, used);
+    if (rc != PBIG2_ENOMEM || !blind) return rc;
+    for (DevBuf* b : {&c->d_counts, &c->d_state, &c->d_entries, &c->d_lists}) b->release();
+    return run_single_in(c, q, shift, false, st, used);
 }
 
 // a small query small enough to test every pair (a grid of one cell, which a
@@ -1124,7 +1133,7 @@ static int self_or_bip(pbig2_ctx* c, const uint32_t* red, uint64_t n_red, const 
         if (rc) return rc;
         const uint32_t* d_blue = !bip ? nullptr : two ? blue : d_boxes + n_red * W;
         rc = fused_query(c, d_boxes, n_red, d_blue, n, (int)dims, range, cell_shift, st);
-        if (rc != kFusedRedo) {
+        if (rc != kFusedRedo && rc != PBIG2_ENOMEM) {
             c->scene_shifts.assign(1, c->stats.cell_shift);
             *npairs = c->npairs;
             return rc;
