@@ -759,7 +759,7 @@ static int run_single_in(pbig2_ctx* c, const SingleScene& q, uint32_t shift, boo
             ta.raise_from = r.from;
             ta.raise_to = r.to;
         }
-    ta.max_cells = 4000000000ull;
+    ta.max_cells = kQueryMaxCells;
     ta.scenes = c->d_scenes.as<Scene>();
     ta.box_off = c->d_scene_off.as<uint32_t>();
     ta.dims = c->d_dims.as<RunDims>();

@@ -259,14 +259,13 @@ __global__ void k_tune_scenes(const uint32_t* boxes, const unsigned long long* o
 
 // ---------------------------------------------------------------------------
 // the cell size of a single-scene query: block b of kTuneBlocks weighs the
-// candidate s0 - 2 + b (s0 = log2 of the sample's mean extent) with the cost
-// model on a strided sample: C cells, E entries, and T tests. A cell holds
+// candidates s0 - 2 + b, + kTuneBlocks, ... (s0 = log2 of the sample's mean
+// extent) with the cost model on a strided sample: C cells, E entries, and T tests. A cell holds
 // about E/m entries for every box whose lower corner lies in it (m boxes in
 // the sample), so T is (E/m)^2 times the pairs of sampled corners that share a
 // cell (counted in a shared-memory hash table), times (n/m)^2, since a pair
 // survives sampling with probability (m/n)^2. The last block to finish takes
-// the cheapest, the finest on a tie, or, when none qualifies, weighs every
-// coarser size itself. It then writes the query's tables.
+// the cheapest, the finest on a tie, and writes the query's tables.
 //
 // Latency is all that counts here, so one thread does the arithmetic in double
 // precision (its rate is a sixty-fourth: 30 us with every thread at it) and
@@ -279,12 +278,12 @@ __global__ void k_tune_scenes(const uint32_t* boxes, const unsigned long long* o
 // slower.
 // ---------------------------------------------------------------------------
 constexpr int kTuneThreads = 1024;
-constexpr uint32_t kTuneBlocks = 8;          // s0 - 2 .. s0 + 5
+constexpr uint32_t kTuneBlocks = 8;          // s0 - 2 .. s0 + 5; coarser sizes are dealt out over the blocks
 constexpr uint32_t kTuneSlots = 8192;        // hash table {cell + 1, corners}, twice the sample
 constexpr int kTunePer = (int)(kTuneSample / kTuneThreads);
 constexpr size_t kTuneSmem = kTuneSlots * 2 * sizeof(uint32_t);
 static_assert(kTuneSlots == 2 * kTuneSample && kTuneThreads == 1024, "tuner table and sums");
-static_assert((1 + 2 * kTuneBlocks) * sizeof(unsigned long long) <= kTuneScratchBytes, "tuner scratch");
+static_assert((1 + 3 * kTuneBlocks) * sizeof(unsigned long long) <= kTuneScratchBytes, "tuner scratch");
 
 // a box's coordinates, wherever its row begins, in two or three 16-byte loads
 // (every row is a line or two of its own, and each load instruction looks all
@@ -309,7 +308,6 @@ __device__ __forceinline__ void load_row(const uint32_t* b, uint32_t (&v)[2 * D]
 struct TuneShared {
     uint32_t part[2][kTuneThreads / 32];
     int s0;
-    uint32_t state;  // the last block: a size was found; another block: not the last
 };
 
 // two sums over the block, each below 2^32 (every thread gets them)
@@ -333,15 +331,12 @@ __device__ __forceinline__ uint64_t tune_grid(uint32_t range, uint32_t sh) {
     return nrc >= 65536ull ? ~0ull : D == 3 ? nrc * nrc * nrc : nrc * nrc;
 }
 
-// what the cost of cell shift sh takes: the sample's entries and pairs of
-// corners in a cell; false when the size does not qualify (block-uniform)
+// this thread's part of the sample's entries at cell shift sh. (A box of too many
+// cells counts for 2^19: the sample may have 2^18 at most.)
 template <int D>
-__device__ bool tune_weigh(TuneShared& s, uint32_t* key, const uint32_t (&lo)[kTunePer][D],
-                           const uint32_t (&hi)[kTunePer][D], const bool (&ok)[kTunePer], uint32_t m, uint32_t range,
-                           uint32_t sh, uint64_t max_cells, uint32_t& entries, uint32_t& pairs) {
-    const uint32_t t = threadIdx.x, nrc = nrc_dev(range, (int)sh);
-    if (tune_grid<D>(range, sh) > max_cells) return false;
-    uint32_t e = 0, huge = 0;
+__device__ __forceinline__ uint32_t tune_entries(const uint32_t (&lo)[kTunePer][D], const uint32_t (&hi)[kTunePer][D],
+                                                 const bool (&ok)[kTunePer], uint32_t sh) {
+    uint32_t e = 0;
 #pragma unroll
     for (int j = 0; j < kTunePer; j++) {
         if (!ok[j]) continue;
@@ -351,12 +346,16 @@ __device__ bool tune_weigh(TuneShared& s, uint32_t* key, const uint32_t (&lo)[kT
             const unsigned long long k = (hi[j][d] >> sh) - (lo[j][d] >> sh) + 1;
             c = c >= (1ull << 26) ? c : c * k;
         }
-        huge |= c >= (1ull << 26) ? 1u : 0u;
-        e += (uint32_t)(c < (1ull << 19) ? c : (1ull << 19));  // (2^18 over the sample is too many)
+        e += (uint32_t)(c < (1ull << 19) ? c : (1ull << 19));
     }
-    const uint2 sums = block_sums(s, e, huge);
-    entries = sums.x;
-    if (sums.y || entries > 64u * m) return false;  // a box that would not fit; too many entries per box
+    return e;
+}
+
+// the sample's pairs of corners in a cell at cell shift sh (grids of less than 2^32 cells)
+template <int D>
+__device__ uint32_t tune_pairs(TuneShared& s, uint32_t* key, const uint32_t (&lo)[kTunePer][D], const bool (&ok)[kTunePer],
+                               uint32_t range, uint32_t sh) {
+    const uint32_t t = threadIdx.x, nrc = nrc_dev(range, (int)sh);
     uint32_t* cnt = key + kTuneSlots;
     for (uint32_t i = t; i < kTuneSlots / 2; i += kTuneThreads) reinterpret_cast<uint4*>(key)[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
@@ -375,8 +374,7 @@ __device__ bool tune_weigh(TuneShared& s, uint32_t* key, const uint32_t (&lo)[kT
         }
     }
     static_assert(kTuneSlots == 1u << 13, "13 bits of the hash");
-    pairs = block_sums(s, found, 0u).x;
-    return true;
+    return block_sums(s, found, 0u).x;
 }
 
 // the cost model (one thread): C cells, the sample's counts, m of n boxes. Of
@@ -435,55 +433,67 @@ __global__ void __launch_bounds__(kTuneThreads, 1) k_tune_query(Params p, TuneAr
         }
         __syncthreads();
         const int s0 = s.s0, s_lo = s0 - 2 > 0 ? s0 - 2 : 0, s_win = s0 + 3 < 31 ? s0 + 3 : 31;
-        const int mine = s_lo + (int)blockIdx.x;
-        uint32_t e = 0, pairs = 0;
         // s0 + 4 and s0 + 5 (of boxes of two sizes the mean says little) where s0 + 3
-        // makes at most 64 cells a box; scenes sparser than that in their range stay
-        // with s0 + 3 at most
+        // makes at most 64 cells a box
         const int s_far = tune_grid<D>(a.range, (uint32_t)s_win) <= 64 * a.n ? (s0 + 5 < 31 ? s0 + 5 : 31) : s_win;
-        const bool fits = m > 0 && mine <= s_far &&
-                          tune_weigh<D>(s, table, lo, hi, ok, m, a.range, (uint32_t)mine, a.max_cells, e, pairs);
-        double best = 1e300, E = 0.0;  // (thread 0)
-        if (t == 0) {
-            const double cost = fits ? tune_cost_query(tune_grid<D>(a.range, (uint32_t)mine), e, pairs, m, a.n, a.bip, E) : 1e300;
-            a.scratch[1 + 2 * blockIdx.x] = (unsigned long long)__double_as_longlong(cost);
-            a.scratch[2 + 2 * blockIdx.x] = (unsigned long long)__double_as_longlong(E);
-            __threadfence();
-            const bool last = atomicAdd(a.scratch, 1ull) == gridDim.x - 1;
-            if (last) {
-                __threadfence();
-                for (uint32_t b = 0; b < gridDim.x; b++) {
-                    const double c = __longlong_as_double((long long)__ldcg(a.scratch + 1 + 2 * b));
-                    if (c < best) {
-                        best = c;
-                        shift = (uint32_t)s_lo + b;
-                        est = __longlong_as_double((long long)__ldcg(a.scratch + 2 + 2 * b));
-                    }
+        const int mine = s_lo + (int)blockIdx.x;
+        const uint2 both = block_sums(s, tune_entries<D>(lo, hi, ok, (uint32_t)min(mine, 31)), tune_entries<D>(lo, hi, ok, (uint32_t)s_far));
+        // Coarser ones up to a single cell, on grids in proportion to the boxes, where
+        // none of those qualifies (boxes too sparse in their range, or a few huge ones
+        // among them; the coarsest decides, for cells and entries only fall), and where
+        // s0 + 3 makes more cells than that. Small queries, which run in one launch on
+        // coarse grids of their own if they can, stay with s0 + 3 then: on 300 000 boxes
+        // of side 2048 in a range of 2^24 it makes 2^30 cells, where 2^18 are a few
+        // microseconds' work.
+        const bool none = tune_grid<D>(a.range, (uint32_t)s_far) > a.max_cells || both.y > 64u * m;
+        const bool coarser = none || (a.n > kFusedMaxBoxes && tune_grid<D>(a.range, (uint32_t)s_win) > 64 * a.n);
+        const int s_one = a.range <= 1u ? 0 : min(32 - __clz((int)(a.range - 1u)), 31);  // the first of a single cell
+        const int last = coarser ? max(s_one, s_far) : s_far;
+        const uint64_t far = mn64(a.max_cells, a.n * 64 > 4096 ? a.n * 64 : 4096);
+        double best = 1e300, E = 0.0;  // (thread 0; the finest on a tie)
+        for (int w = mine; w <= last && m > 0; w += (int)kTuneBlocks) {
+            if (tune_grid<D>(a.range, (uint32_t)w) > (w > s_far ? far : a.max_cells)) continue;
+            const uint32_t e = w == mine ? both.x : block_sums(s, tune_entries<D>(lo, hi, ok, (uint32_t)w), 0u).x;
+            if (e > 64u * m) continue;
+            const uint32_t pairs = tune_pairs<D>(s, table, lo, ok, a.range, (uint32_t)w);
+            if (t == 0) {
+                const double cost = tune_cost_query(tune_grid<D>(a.range, (uint32_t)w), e, pairs, m, a.n, a.bip, E);
+                if (cost < best) {
+                    best = cost;
+                    shift = (uint32_t)w;
+                    est = E;
                 }
             }
-            s.state = !last || best < 1e300 ? 1u : 0u;
         }
-        __syncthreads();
-        if (s.state == 0u) {
-            // a few huge boxes in the sample can disqualify all of those: every
-            // coarser size, on grids in proportion to the boxes
-            const uint64_t far = mn64(a.max_cells, a.n * 64 > 4096 ? a.n * 64 : 4096);
-            for (int w = s_win + 1; w <= 31 && m > 0; w++) {
-                const bool qualifies = tune_weigh<D>(s, table, lo, hi, ok, m, a.range, (uint32_t)w, far, e, pairs);
-                if (t == 0 && qualifies) {
-                    const double cost = tune_cost_query(tune_grid<D>(a.range, (uint32_t)w), e, pairs, m, a.n, a.bip, E);
-                    if (cost < best) {
-                        best = cost;
-                        shift = (uint32_t)w;
-                        est = E;
+        if (t == 0) {
+            unsigned long long* mine3 = a.scratch + 1 + 3 * blockIdx.x;
+            mine3[0] = (unsigned long long)__double_as_longlong(best);
+            mine3[1] = (unsigned long long)__double_as_longlong(est);
+            mine3[2] = shift;
+            shift = kTuneShift;
+            __threadfence();
+            if (atomicAdd(a.scratch, 1ull) == gridDim.x - 1) {
+                __threadfence();
+                unsigned long long all[kTuneBlocks][3];
+#pragma unroll
+                for (uint32_t b = 0; b < kTuneBlocks; b++)
+#pragma unroll
+                    for (int k = 0; k < 3; k++) all[b][k] = __ldcg(a.scratch + 1 + 3 * b + k);
+                best = 1e300;
+#pragma unroll
+                for (uint32_t b = 0; b < kTuneBlocks; b++) {
+                    const double c = __longlong_as_double((long long)all[b][0]);
+                    if (c < best || (c == best && c < 1e300 && (uint32_t)all[b][2] < shift)) {
+                        best = c;
+                        est = __longlong_as_double((long long)all[b][1]);
+                        shift = (uint32_t)all[b][2];
                     }
                 }
-                __syncthreads();
-            }
-            if (t == 0 && best == 1e300) {  // the coarsest grid that is not a single cell
-                shift = 31;
-                while (shift > 0 && nrc_dev(a.range, (int)shift - 1) <= 1) shift--;
-                est = (double)a.n;
+                if (best == 1e300) {  // the coarsest grid that is not a single cell
+                    shift = 31;
+                    while (shift > 0 && nrc_dev(a.range, (int)shift - 1) <= 1) shift--;
+                    est = (double)a.n;
+                }
             }
         }
         if (t != 0 || shift == kTuneShift) return;  // (another block writes the tables)

@@ -272,6 +272,7 @@ cudaError_t launch_scatter(const Params& p, int dims, cudaStream_t st, bool chai
 // of more than room_cells cells sets kErrGridRoom and leaves the kernels
 // behind it nothing to do.
 constexpr uint32_t kTuneShift = 0xffffffffu;
+constexpr uint64_t kQueryMaxCells = 4000000000ull;  // the most of an automatic cell size
 constexpr uint64_t kTuneSample = 4096;
 struct TuneArgs {
     const uint32_t* red;    // boxes [0, n_red) and [n_red, n) (device memory or mapped host memory)
@@ -285,7 +286,7 @@ struct TuneArgs {
     Scene* scenes;
     uint32_t* box_off;
     RunDims* dims;
-    unsigned long long* scratch;  // 2 words per block, zero at the start and left zero
+    unsigned long long* scratch;  // a count of blocks, left zero, then each one's cost, entries and cell shift
 };
 constexpr size_t kTuneScratchBytes = 256;
 cudaError_t launch_tune_query(const Params& p, const TuneArgs& a, int dims, cudaStream_t st);
