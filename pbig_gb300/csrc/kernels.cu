@@ -2680,8 +2680,10 @@ __device__ __forceinline__ uint32_t tune_scene_fast(const Params& p, uint32_t ra
     const unsigned long long mean = ext / ((good ? good : 1ull) * (unsigned long long)dims);
     const int s0 = mean < 2 ? 0 : 63 - __clzll(mean);
     const int s_win = s0 + 3 < 31 ? s0 + 3 : 31;
-    // red and blue boxes too sparse in their range for these grids: the regular pipeline's
-    if (BIP && tune_grid<dims>(range, (uint32_t)s_win) > max_cells) return kFusedLeave;
+    // red and blue boxes too sparse in their range for these grids: the regular
+    // pipeline's, unless it took a coarser grid itself
+    if (BIP && tune_grid<dims>(range, (uint32_t)s_win) > max_cells && tune_grid<dims>(range, (uint32_t)s_win) <= kQueryMaxCells)
+        return kFusedLeave;
     const float scale = (float)n / (float)(m ? m : 1);
     const uint64_t far_cap = n * 64 > 4096 ? n * 64 : 4096;
     float best_cost = 3.0e38f;

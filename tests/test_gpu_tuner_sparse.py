@@ -82,3 +82,23 @@ def test_choice(engine, n, side, dims, huge, none):
     assert st["cells"] <= 64 * n and st["grid_retries"] == 0
     want = O.grid_pairs(boxes, RANGE, cs=1 << 18)[0]
     assert np.array_equal(O.sort_pairs(engine.pairs()), want)
+
+
+@pytest.mark.parametrize("n,side,launches", [
+    (20000, 256, 1),      # a coarse grid in the one launch, as self queries have
+    (40000, 1200, 1),
+    (50000, 100000, 1),   # the usual sizes fit the one launch
+])
+def test_small_red_blue_queries_run_in_one_launch(n, side, launches):
+    both = boxes_of(2 * n, side, n)
+    both[n::7, :6] = both[:n][: len(both[n::7]), :6]  # (pairs)
+    red, blue = both[:n].copy(), both[n:].copy()
+    blue[:, 6] -= n
+    p = O.grid_pairs(both, RANGE, cs=1 << 18)[0]
+    p = p[(p[:, 0] < n) & (p[:, 1] >= n)]
+    with Engine(0) as e:
+        assert e.bipartite_intersect(red, blue, RANGE) == len(p) > 2000
+        assert e.stats()["kernels"] == launches
+        got = e.pairs()
+    got[:, 1] += n
+    assert np.array_equal(O.sort_pairs(got), p)
