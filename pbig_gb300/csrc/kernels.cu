@@ -1630,7 +1630,12 @@ __global__ void __launch_bounds__(kPairThreads, 5) k_pairs_small(Params pin) {
 // a scaled value, which leaves the test open when no other sum is larger. The
 // sweep keeps the largest signed value it saw (32767 is the largest there is),
 // and a tile that met one is tested again on the whole coordinates (about 1 %
-// of the tiles of random boxes).
+// of the tiles of random boxes). A box ties with itself where one of its sides
+// is shorter than a scaled step, so of points every tile that meets itself did.
+// One-launch queries, whose tiles nearly all meet themselves, look at such a
+// tile again without those sums first: 262 144 points 106 -> 84 us, 100 000 66
+// -> 62. (In the kernels of large queries it gained nothing on points, and
+// their registers spilled: the crowded 4M-box scene took 1 % longer.)
 //
 // Red/blue queries stage the two colours apart, so their tiles are red rows
 // against blue columns (or the other way, whichever takes fewer steps), and a
@@ -1775,11 +1780,34 @@ __device__ __noinline__ uint32_t tile_exact(const uint32_t* boxes, const uint32_
 // the bits of the slots of groups `groups` .. 7
 __device__ __forceinline__ uint32_t tile_beyond(uint32_t groups) { return ((0xffu << groups) & 0xffu) * 0x01010101u; }
 
-// row tile against column tile x of `cols` boxes: bit s set iff this lane's
-// box and slot s overlap and the reference-cell rule reports them here
+__device__ __forceinline__ bool tile_tied(uint32_t top) {
+    const uint32_t low = top ^ 0x7fff7fffu;  // a zero half: a sum of 32767 was the largest of its pair
+    return __any_sync(FULL_MASK, ((low - 0x00010001u) & ~low & 0x80008000u) != 0u);
+}
+
+// the largest sums of a tile against itself without those of a box with itself
 template <int D>
+__device__ __forceinline__ uint32_t tile_others(const Tiles& t, const Row<D>& r, uint32_t x, uint32_t cols) {
+    const uint32_t lane = lane_id(), own = 0x8000u << (2u * (lane & 8u));  // this lane's box: its half of a pair
+    uint32_t top = 0;
+#pragma unroll 1
+    for (uint32_t g = 0; 4u * g < cols; g++) {
+        uint32_t m = tile_pair<D>(t, r, 16 * x + 2 * g), n = tile_pair<D>(t, r, 16 * x + 2 * g + 1);
+        if (g == (lane & 7u)) {
+            m |= lane < 16u ? own : 0u;
+            n |= lane < 16u ? 0u : own;
+        }
+        top = __vimax3_s16x2(top, m, n);
+    }
+    return top;
+}
+
+// row tile against column tile x of `cols` boxes: bit s set iff this lane's
+// box and slot s overlap and the reference-cell rule reports them here. OWN:
+// ties of boxes with themselves are looked for where the tiles are one (self).
+template <int D, bool OWN>
 __device__ __forceinline__ uint32_t tile_hits(const Params& p, const Tiles& t, const Row<D>& r, uint32_t rows,
-                                              uint32_t x, uint32_t cols) {
+                                              uint32_t x, uint32_t cols, bool self) {
     uint32_t miss = 0, top = 0;
     if (cols > 24u) {
 #pragma unroll
@@ -1795,11 +1823,8 @@ __device__ __forceinline__ uint32_t tile_hits(const Params& p, const Tiles& t, c
     }
     const uint32_t raw = t.raw[32 * x + lane_id()];
     uint32_t mask = ~miss;
-    if (p.open) {
-        const uint32_t low = top ^ 0x7fff7fffu;  // a zero half: a sum of 32767 was the largest of its pair
-        if (__any_sync(FULL_MASK, ((low - 0x00010001u) & ~low & 0x80008000u) != 0u))
-            mask = tile_exact<D>(p.boxes, p.blue, p.split, p.nboxes, r.raw, raw, rows, cols);
-    }
+    if (p.open && tile_tied(top) && (!OWN || !self || tile_tied(tile_others<D>(t, r, x, cols))))
+        mask = tile_exact<D>(p.boxes, p.blue, p.split, p.nboxes, r.raw, raw, rows, cols);
     const uint32_t m0 = __ballot_sync(FULL_MASK, ((raw >> kIdBits) & 1u) == 0u);
     const uint32_t m1 = __ballot_sync(FULL_MASK, ((raw >> (kIdBits + 1)) & 1u) == 0u);
     const uint32_t m2 = __ballot_sync(FULL_MASK, ((raw >> (kIdBits + 2)) & 1u) == 0u);
@@ -1906,19 +1931,19 @@ __device__ __forceinline__ void tile_put_colour(const Tiles& t, uint32_t tiles, 
 
 // row tile r of a staged cell against its column tiles from x (self: from r),
 // `count` of them at most, two per emission step
-template <int D, bool BIP, bool REC>
+template <int D, bool BIP, bool REC, bool OWN>
 __device__ __forceinline__ void row_sweep(const Params& p, const Tiles& t, WarpOut& o, const CellTiles& c, uint32_t r,
                                           uint32_t x, uint32_t count, uint32_t gid) {
     const uint32_t rows = tile_fill(c.rows, r), end = min(c.col_tiles(), x + count);
     const Row<D> row = tile_row<D>(t, c.row_tile(r));
     for (; x < end; x += 2) {
         const uint32_t xa = c.col_tile(x);
-        uint32_t ma = tile_hits<D>(p, t, row, rows, xa, tile_fill(c.cols, x));
+        uint32_t ma = tile_hits<D, OWN && !BIP>(p, t, row, rows, xa, tile_fill(c.cols, x), x == r);
         if (!BIP && x == r) ma &= after_lane();
         uint32_t mb = 0, xb = xa;
         if (x + 1 < end) {
             xb = c.col_tile(x + 1);
-            mb = tile_hits<D>(p, t, row, rows, xb, tile_fill(c.cols, x + 1));
+            mb = tile_hits<D, false>(p, t, row, rows, xb, tile_fill(c.cols, x + 1), false);
         }
         tile_emit<BIP, REC>(p, t, o, row.raw, ma, xa, mb, xb, 32 * r, 32 * x, 32 * (x + 1), gid);
     }
@@ -1983,7 +2008,7 @@ __device__ __forceinline__ void med_pass(const Params& p, unsigned char* wsm, ui
         }
         __syncwarp();
         const uint32_t R = c.row_tiles();
-        for (uint32_t r = 0; r < R; r++) row_sweep<D, BIP, REC>(p, t, o, c, r, BIP ? 0u : r, ~0u >> 1, gid);
+        for (uint32_t r = 0; r < R; r++) row_sweep<D, BIP, REC, FRESH>(p, t, o, c, r, BIP ? 0u : r, ~0u >> 1, gid);
         __syncwarp();
     };
     // items taken from a counter, so warps whose cells were larger end no
@@ -2118,7 +2143,7 @@ __device__ __forceinline__ void big_cell(const Params& p, TeamSmem& s, WarpOut& 
             r++;
         }
         if (r >= R) break;
-        row_sweep<D, BIP, REC>(p, t, o, c, r, (BIP ? 0u : r) + 2 * (u - before), 2, gid);
+        row_sweep<D, BIP, REC, SUB>(p, t, o, c, r, (BIP ? 0u : r) + 2 * (u - before), 2, gid);
     }
 }
 
@@ -2151,7 +2176,7 @@ __device__ __forceinline__ void huge_item(const Params& p, const Tiles& t, WarpO
 #pragma unroll
         for (uint32_t k = 0; k < 2; k++) {
             if (x + k >= x1) continue;
-            m[k] = tile_hits<D>(p, t, row, rows, 1 + k, tile_fill(n, x + k));
+            m[k] = tile_hits<D, false>(p, t, row, rows, 1 + k, tile_fill(n, x + k), false);
             if (x + k == r) m[k] &= after_lane();
             if (BIP) {
                 const uint32_t red = __ballot_sync(FULL_MASK, (t.raw[32 * (1 + k) + lane] & kIdMask) < p.split);
