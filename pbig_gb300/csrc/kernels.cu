@@ -2670,10 +2670,11 @@ __device__ __forceinline__ void deal_cells(const Params& p, const DealtTile& s, 
     }
 }
 
-// the query's cost model for one scene of n boxes at row 0, with T = E^2 / 2C
-// on 64 sampled boxes, in single precision over exact integer sums: the one-launch path cannot wait
-// for double-precision divisions. Grids of at most max_cells cells, so a
-// box covers at most max_cells cells and every per-box product fits 32 bits.
+// the one-launch queries' cost model for one scene of n boxes at row 0, with T =
+// E^2 / 2C on 64 sampled boxes, in single precision over exact integer sums: the
+// one-launch path cannot wait for double-precision divisions. Grids of at most
+// max_cells cells, so a box covers at most max_cells cells and every per-box
+// product fits 32 bits.
 template <int dims, bool BIP>
 __device__ __forceinline__ uint32_t tune_scene_fast(const Params& p, uint32_t range, uint64_t max_cells, uint32_t warps) {
     const uint32_t lane = lane_id();
@@ -2716,6 +2717,7 @@ __device__ __forceinline__ uint32_t tune_scene_fast(const Params& p, uint32_t ra
     for (int s = s0 - 2 > 0 ? s0 - 2 : 0; s <= 31 && m > 0; s++) {
         if (s == s_win + 1 && best != 0xffffffffu) break;
         const uint64_t nrc = nrc_dev(range, s);
+        if (s > s_win && nrc_dev(range, s - 1) == 1) break;  // (a single cell again: it costs the same)
         if (nrc > max_cells) continue;
         const uint64_t C = dims == 3 ? nrc * nrc * nrc : nrc * nrc;  // nrc <= 2^20: no overflow in 64 bits
         if (C > max_cells) continue;
@@ -2735,7 +2737,10 @@ __device__ __forceinline__ uint32_t tune_scene_fast(const Params& p, uint32_t ra
         // (fewer cells than warps leave warps idle: 30 000 boxes of one
         // density took 35 us on 512 cells and 26 us on 4096)
         const float idle = (float)warps > Cf ? (float)warps / Cf : 1.0f;
-        const float cost = (float)kQueryCell * Cf + (float)kQueryEntry * E + (BIP ? 0.5f : 1.0f) * (float)kQueryTest * idle * T;
+        const float l = E / Cf, l3 = l * l * l;
+        const float cost = (C > kFusedLocalCells ? (float)kFusedGrid : 0.0f) + (float)kQueryCell * Cf + (float)kQueryEntry * E +
+                           (float)kFusedCell * Cf * (l3 / (l3 + (float)kFusedShare)) +
+                           (BIP ? 0.5f : 1.0f) * (float)kFusedTest * idle * T;
         if (cost < best_cost) {
             best_cost = cost;
             best = (uint32_t)s;

@@ -87,6 +87,15 @@ constexpr double kTuneCell = 2.4e-12, kTuneEntry = 80.0e-12, kTuneTest = 0.9e-12
 // cell sizes each: 65 us + 3.1 ps C + 41 ps E + 0.46 ps T + 0.6 ps per pair; it
 // picks the fastest size of every one). Tests cost the same in cells of any size.
 constexpr double kQueryCell = 3.1e-12, kQueryEntry = 41.0e-12, kQueryTest = 0.46e-12;
+// One-launch queries: their cells and entries cost the same, but a cell of five
+// boxes or more (a share l^3 / (l^3 + 160) of the cells where l boxes fall on one)
+// takes a warp's time whatever it holds, tests run in a few warps each, and a
+// grid of more than kFusedLocalCells another barrier. Fitted to the device time
+// of 49 queries of 10 000 to 262 144 boxes (even, thin, clumped, red/blue, 2-D
+// and 3-D) at up to five cell sizes each: its choices are 3 % slower than the
+// fastest size on average, those of the constants above were 11 %.
+constexpr double kFusedGrid = 3.0e-6, kFusedCell = 0.5e-9, kFusedTest = 2.0e-12;
+constexpr double kFusedShare = 160.0;
 
 __host__ __device__ inline double tune_mul(double a, double b) {
 #ifdef __CUDA_ARCH__

@@ -64,7 +64,7 @@ def test_a_given_size_that_does_not_fit_is_refused():
 
 
 def test_without_memory_for_the_finer_grid_a_scene_keeps_the_querys():
-    n, limit = 80000, 24 << 20
+    n, limit = 300000, 40 << 20
     r = np.random.default_rng(4)
     side = 0.6 * n ** (-1 / 3) * RANGE
     boxes = np.empty((n, 7), dtype=np.uint32)
@@ -74,7 +74,7 @@ def test_without_memory_for_the_finer_grid_a_scene_keeps_the_querys():
     with Engine(0) as engine:
         engine.self_intersect(boxes, RANGE)
         cells = engine.stats()["cells"]
-        assert 8 * cells <= 4 * n and 8 * cells * 4 * 32 > limit  # one size finer: taken, and its empty slots alone too many
+        assert 8 * cells <= 4 * n and 32 * (8 * cells * 4 + n + n // 2) > limit  # one size finer: taken, and too many slots
     with Engine(0) as engine:
         engine.set_max_buffer(limit)
         sc = Scene(engine, boxes, RANGE)
