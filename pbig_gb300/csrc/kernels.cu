@@ -1844,6 +1844,33 @@ __device__ __forceinline__ uint32_t after_lane() { return 0xfffffffeu << lane_id
 // rows above 12 written together 232, 794 and 407, above 9 230, 811 and 407,
 // above 16 236, 793 and 415.
 constexpr uint32_t kRowHits = 12;
+
+// More pairs than the buffer holds, straight to the pair array: a lane a column
+// of each tile, so that a store covers its row's pairs one after the other. (A
+// lane a row, each store's pairs were up to 512 bytes apart: 84 million pairs of
+// 20 000 boxes in one cell took 2780 us, now 1060.) k: the
+// lane's pairs, `at` of the total before them.
+template <bool BIP>
+__device__ __forceinline__ void row_store(const Params& p, uint32_t ma, const uint32_t* ca, uint32_t mb, const uint32_t* cb,
+                                       uint32_t row, uint32_t k, uint32_t at, uint32_t total) {
+    const uint32_t lane = lane_id(), below = (1u << lane) - 1u;
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(&p.ctr->pairs, (unsigned long long)total);
+    base = __shfl_sync(FULL_MASK, base, 0);
+    if (base + total > p.out_cap && lane == 0) atomicOr(&p.ctr->err, kErrOutOvf);
+    const uint32_t va = ca[lane], vb = cb[lane];
+    for (uint32_t rows = __ballot_sync(FULL_MASK, k != 0u); rows; rows &= rows - 1) {
+        const uint32_t l = __ffs(rows) - 1;
+        const uint32_t a = __shfl_sync(FULL_MASK, ma, l), b = __shfl_sync(FULL_MASK, mb, l);
+        const uint32_t r = __shfl_sync(FULL_MASK, row, l);
+        const unsigned long long g = base + __shfl_sync(FULL_MASK, at, l);
+        const unsigned long long ga = g + __popc(a & below), gb = g + __popc(a) + __popc(b & below);
+        if (((a >> lane) & 1u) && ga < p.out_cap) p.out[ga] = out_pair<BIP, false>(p, make_uint2(r, va));
+        if (((b >> lane) & 1u) && gb < p.out_cap) p.out[gb] = out_pair<BIP, false>(p, make_uint2(r, vb));
+    }
+    __syncwarp();
+}
+
 template <bool BIP>
 __device__ __forceinline__ void row_emit(const Params& p, WarpOut& o, uint32_t ma, const uint32_t* ca, uint32_t mb,
                                          const uint32_t* cb, uint32_t row) {
@@ -1854,8 +1881,8 @@ __device__ __forceinline__ void row_emit(const Params& p, WarpOut& o, uint32_t m
     if (total == 0) return;
     if (o.n + total > o.cap) {
         wflush<BIP, false>(p, o);
-        if (total > o.cap) {  // past the buffer
-            wemit<BIP>(p, o, ma, [&](uint32_t b) { return ca[b]; }, mb, [&](uint32_t b) { return cb[b]; }, row);
+        if (total > o.cap) {  // past the buffer: every row by the whole warp
+            row_store<BIP>(p, ma, ca, mb, cb, row, k, incl - k, total);
             return;
         }
     }
