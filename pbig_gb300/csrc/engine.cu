@@ -902,7 +902,7 @@ static int fused_query(pbig2_ctx* c, const uint32_t* red, uint64_t n_red, const 
     } else {
         const uint64_t cells_cap = cell_shift == PBIG2_AUTO ? kFusedMaxCells : grid_cells(range, cell_shift, dims);
         const uint64_t entry_cap = std::max<uint64_t>({c->fused_entry_hint, 8 * n + 4096, c->d_entries.bytes / sizeof(uint4)});
-        const uint64_t task_cap = std::max<uint64_t>(c->d_tasks.bytes / 16, 4096);
+        const uint64_t task_cap = std::max<uint64_t>({c->fused_task_hint, c->d_tasks.bytes / 16, 4096});
         void* counts_before = c->d_counts.p;
         CK(c->d_counts.ensure(cells_cap * 4 + 16, false, st));
         if (c->d_counts.p != counts_before) c->fused_dirty = true;
@@ -976,6 +976,7 @@ static int fused_query(pbig2_ctx* c, const uint32_t* red, uint64_t n_red, const 
     if (h.err & kErrIndex) return fail(PBIG2_ECUDA, "inconsistent cell lists (error bits 0x%x)", h.err);
     if ((h.err & (kErrEntryOvf | kErrTaskOvf | kErrOutOvf)) || h.entries > p.entry_cap || h.pairs > p.out_cap) {
         c->fused_entry_hint = std::max<uint64_t>(c->fused_entry_hint, h.entries + h.entries / 8 + 4096);
+        if (h.err & kErrTaskOvf) c->fused_task_hint = std::max<uint64_t>(c->fused_task_hint, (uint64_t)h.need_tasks + 1024);
         if (!use_ext || h.pairs <= p.out_cap) c->out_hint = std::max<uint64_t>(c->out_hint, h.pairs + h.pairs / 8);
         return kFusedRedo;
     }

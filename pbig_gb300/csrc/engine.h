@@ -121,7 +121,7 @@ struct pbig2_ctx {
     unsigned int bar_base = 0;
     int fused_slot = 0;
     bool fused_dirty = true;     // the counters may hold values another pipeline left (or are new)
-    uint64_t fused_entry_hint = 0;
+    uint64_t fused_entry_hint = 0, fused_task_hint = 0;
     bool want_grid = false;      // the running query's cell size is what the caller is after
     bool fused_stall_test = false;  // the next launch's barriers never complete (test of the bounded wait)
     // work-list class map of later queries (PBIG2_OPT_CLASS_MAP; 0: automatic)

@@ -74,3 +74,12 @@ def test_pairs_beyond_the_callers_buffer(engines):
         assert not e.result_in(room[: len(want) // 2]) and np.array_equal(canon(e.pairs()), want)
         assert bool((room[len(want) // 2:] == -1).all())
         e.set_pair_output(None)
+
+
+def test_a_query_of_many_tile_tasks_runs_in_one_launch_again():
+    """A launch short of room for its tile tasks goes to the pipeline once."""
+    boxes = dense(12000, 2, 0.3, 5)
+    with Engine(0) as e:
+        e.self_intersect(boxes, RANGE, cell_shift=19)
+        count = e.self_intersect(boxes, RANGE, cell_shift=19)
+        assert e.stats()["kernels"] == 1 and count == len(O.grid_pairs(boxes, RANGE, cs=1 << 19)[0])
