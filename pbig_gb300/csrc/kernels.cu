@@ -2750,39 +2750,45 @@ __device__ __forceinline__ uint32_t tune_scene_fast(const Params& p, uint32_t ra
         return kFusedLeave;
     const float scale = (float)n / (float)(m ? m : 1);
     const uint64_t far_cap = n * 64 > 4096 ? n * 64 : 4096;
-    float best_cost = 3.0e38f;
     uint32_t best = 0xffffffffu;
-    for (int s = s0 - 2 > 0 ? s0 - 2 : 0; s <= 31 && m > 0; s++) {
-        if (s == s_win + 1 && best != 0xffffffffu) break;
-        const uint64_t nrc = nrc_dev(range, s);
-        if (s > s_win && nrc_dev(range, s - 1) == 1) break;  // (a single cell again: it costs the same)
-        if (nrc > max_cells) continue;
-        const uint64_t C = dims == 3 ? nrc * nrc * nrc : nrc * nrc;  // nrc <= 2^20: no overflow in 64 bits
-        if (C > max_cells) continue;
-        if (s > s_win && C > far_cap) continue;
-        uint32_t e = 0;
+    // the window, then every coarser size if none of it qualifies: entries counted
+    // in integers, size after size, and weighed side by side, a lane a size
+    for (int pass = 0; pass < 2 && best == 0xffffffffu && m > 0; pass++) {
+        const int first = pass ? s_win + 1 : s0 - 2 > 0 ? s0 - 2 : 0, last = pass ? 31 : s_win;
+        const uint64_t limit = pass ? mn64(max_cells, far_cap) : max_cells;
+        uint32_t entries = 0xffffffffu;  // lane s - first: the sample's at shift s, if it qualifies
+        for (int s = first; s <= last; s++) {
+            if (tune_grid<dims>(range, (uint32_t)s) > limit) continue;
+            uint32_t e = 0;
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            if (!ok[j]) continue;
-            uint32_t c = 1;
-            for (int d = 0; d < dims; d++) c *= (hi[j][d] >> s) - (lo[j][d] >> s) + 1;
-            e += c;  // <= 2 * max_cells
+            for (int j = 0; j < 2; j++) {
+                if (!ok[j]) continue;
+                uint32_t c = 1;
+                for (int d = 0; d < dims; d++) c *= (hi[j][d] >> s) - (lo[j][d] >> s) + 1;
+                e += c;  // <= 2 * max_cells
+            }
+            e = __reduce_add_sync(FULL_MASK, e);
+            if ((int)lane == s - first && e <= 64u * (uint32_t)m) entries = e;
+            if (nrc_dev(range, s) <= 1u) break;  // (coarser ones are this cell again)
         }
-        e = __reduce_add_sync(FULL_MASK, e);
-        if (e > 64u * (uint32_t)m) continue;
-        const float E = (float)e * scale, Cf = (float)C;
-        const float T = E * E / (2.0f * Cf);
-        // (fewer cells than warps leave warps idle: 30 000 boxes of one
-        // density took 35 us on 512 cells and 26 us on 4096)
-        const float idle = (float)warps > Cf ? (float)warps / Cf : 1.0f;
-        const float l = E / Cf, l3 = l * l * l;
-        const float cost = (C > kFusedLocalCells ? (float)kFusedGrid : 0.0f) + (float)kQueryCell * Cf + (float)kQueryEntry * E +
-                           (float)kFusedCell * Cf * (l3 / (l3 + (float)kFusedShare)) +
-                           (BIP ? 0.5f : 1.0f) * (float)kFusedTest * idle * T;
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = (uint32_t)s;
+        uint32_t bits = 0x7f800000u;  // of the cost (positive floats are in the order of their bits)
+        if (entries != 0xffffffffu) {
+            const uint64_t C = tune_grid<dims>(range, (uint32_t)first + lane);
+            const float E = (float)entries * scale, Cf = (float)C;
+            const float T = E * E / (2.0f * Cf);
+            // (fewer cells than warps leave warps idle: 30 000 boxes of one
+            // density took 35 us on 512 cells and 26 us on 4096)
+            const float l = E / Cf, l3 = l * l * l;
+            // (a cell of l boxes has about l^2 / 16384 tile tasks, a warp's each)
+            const float units = Cf * fmaxf(1.0f, l * l * (1.0f / 16384.0f));
+            const float idle = (float)warps > units ? (float)warps / units : 1.0f;
+            bits = __float_as_uint((C > kFusedLocalCells ? (float)kFusedGrid : 0.0f) + (float)kQueryCell * Cf + (float)kQueryEntry * E +
+                                   (float)kFusedCell * Cf * (l3 / (l3 + (float)kFusedShare)) +
+                                   (BIP ? 0.5f : 1.0f) * (float)kFusedTest * idle * T);
         }
+        const uint32_t least = __reduce_min_sync(FULL_MASK, bits);
+        // (the finest on a tie)
+        if (least < 0x7f800000u) best = (uint32_t)first + __ffs(__ballot_sync(FULL_MASK, bits == least)) - 1u;
     }
     if (best == 0xffffffffu) {  // the coarsest grid that is not a single cell
         uint32_t s = 31;

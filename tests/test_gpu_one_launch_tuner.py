@@ -34,7 +34,8 @@ def choice(b, warps, bip=False):
             return None
         E = e * (n / m)
         per = (E / C) ** 3
-        tests = E * E / (2 * C) * max(1, warps / C) * (0.5 if bip else 1)
+        units = C * max(1, (E / C) ** 2 / 16384)  # a warp's each
+        tests = E * E / (2 * C) * max(1, warps / units) * (0.5 if bip else 1)
         return (3e-6 if C > 8192 else 0) + 3.1e-12 * C + 41e-12 * E + 0.5e-9 * C * per / (per + 160) + 2e-12 * tests
 
     costs = {s: cost(s, 1 << 20) for s in range(max(0, s0 - 2), s0 + 4)}
