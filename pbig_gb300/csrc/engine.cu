@@ -303,6 +303,7 @@ static cudaError_t record_pipeline(pbig2_ctx* c, const Params& p, int dims, bool
         R(cudaMemsetAsync(&p.ctr->pairs, 0, sizeof(unsigned long long), st));
         R(cudaMemsetAsync(&p.ctr->rec_pairs, 0, sizeof(unsigned long long), st));
         R(cudaMemsetAsync(&p.ctr->err, 0, sizeof(unsigned int), st));
+        R(cudaMemsetAsync(&p.ctr->need_tasks, 0, sizeof(unsigned int), st));
         R(cudaMemsetAsync(&p.ctr->med_next, 0, 3 * sizeof(unsigned int), st));  // med_next, big_next, done
     }
     Params pp = p;

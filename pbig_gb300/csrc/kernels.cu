@@ -834,42 +834,41 @@ __device__ __forceinline__ uint32_t list_size(const Params& p, int k) {
 }
 
 // tile tasks of the last k row tiles of a cell: ceil(i / kTaskCols), i = 1 .. k
-__device__ __forceinline__ uint64_t tile_tasks(uint64_t k) {
-    const uint64_t a = k / kTaskCols, b = k % kTaskCols;
-    return a * (a + 1) / 2 * kTaskCols + b * (a + 1);
+__device__ __forceinline__ uint32_t tile_tasks(uint32_t k) {
+    const uint32_t a = k / kTaskCols, b = k % kTaskCols;
+    return (a + 1) * (a * (kTaskCols / 2) + b);
 }
+constexpr uint32_t kMostRows = 1u << 17;  // (2^30 tasks; cells of more boxes ask for more than there can be)
 
 // huge cells i0, i0 + stride, ..., a warp each and its lanes a row tile: a
 // thread to a cell took 0.6 ms to write the 25 000 tasks of one of 20 000 boxes,
-// and the boxes of its block waited (with a warp the scatter takes 28 us in all).
-template <bool FRESH = false>
-__device__ __forceinline__ void expand_cells(const Params& p, uint32_t i0, uint32_t stride) {
-    const uint32_t nh = mn64(FRESH ? __ldcg(&p.ctr->n_list[kListHuge]) : p.ctr->n_list[kListHuge], p.list_cap[kListHuge]);
+// 1.06 ms the query; with a warp it takes 0.51.
+// (pl: the kernel's own parameters, as in scan_chunk)
+__device__ __forceinline__ void expand_cells(const Params& p, const Params& pl, uint32_t huge, uint32_t i0, uint32_t stride) {
+    const uint32_t nh = (uint32_t)mn64(huge, pl.list_cap[kListHuge]);
     for (uint32_t i = i0; i < nh; i += stride) {
-        const uint2 sn = p.lists[p.list_off[kListHuge] + i];
-        const uint32_t n = sn.y;
-        const uint32_t R = (n + 31) >> 5;
-        const uint64_t cnt = tile_tasks(R);
+        const uint2 sn = p.lists[pl.list_off[kListHuge] + i];
+        const uint32_t R = (sn.y + 31) >> 5, cap = (uint32_t)mn64(p.task_cap, 0x7fffffffu);
+        const uint32_t cnt = R <= kMostRows ? tile_tasks(R) : 0x7fffffffu;
         uint32_t b = 0;
         if (lane_id() == 0) {
-            b = atomicAdd(&p.ctr->need_tasks, (uint32_t)mn64(cnt, 0x7fffffffu));
-            if (b + cnt > p.task_cap) atomicOr(&p.ctr->err, kErrTaskOvf);
+            b = atomicAdd(&p.ctr->need_tasks, cnt);
+            if ((uint64_t)b + cnt > cap) atomicOr(&p.ctr->err, kErrTaskOvf);
         }
         b = __shfl_sync(FULL_MASK, b, 0);
+        if (b >= cap || R > kMostRows) continue;
         for (uint32_t r = lane_id(); r < R; r += 32) {
-            uint64_t k = b + (cnt - tile_tasks(R - r));
-            for (uint32_t x0 = r; x0 < R && k < p.task_cap; x0 += kTaskCols, k++) p.tasks[k] = make_uint4(sn.x, n, r, x0);
+            uint32_t k = b + cnt - tile_tasks(R - r);
+            for (uint32_t x0 = r; x0 < R && k < cap; x0 += kTaskCols, k++) p.tasks[k] = make_uint4(sn.x, sn.y, r, x0);
         }
     }
 }
 
-// (with the tile tasks of huge cells: a launch of their own took 4 to 6 us)
 template <int D, bool MERGED>
 __global__ void __launch_bounds__(kBoxThreads) k_scatter(Params pin) {
     __shared__ __align__(16) uint32_t sbox[kBoxThreads * (2 * D + 1)];
     chain_wait();
     stamp(pin, kStampScatter);
-    expand_cells(pin, (blockIdx.x * kBoxThreads + threadIdx.x) / 32, gridDim.x * (kBoxThreads / 32));
     box_pass<D, true, MERGED>(resolve(pin), sbox, blockIdx.x, gridDim.x);
 }
 
@@ -1609,16 +1608,21 @@ __device__ __forceinline__ void small_pass(const Params& p, uint4* s, uint2* s_o
     if (REC) rec_hits(p, o);
 }
 
+// (with the tile tasks of huge cells, which the block kernel takes: a launch of
+// their own took 4 to 6 us, and in the scatter they cost it registers that its
+// blocks need to fill the SMs: 89 us became 108 on 4 million points)
 template <int D, bool BIP, bool REC = false>
 __global__ void __launch_bounds__(kPairThreads, 5) k_pairs_small(Params pin) {
     chain_wait();
     const Params p = resolve(pin);
     stamp(p, kStampSmall);
+    const uint32_t huge = p.ctr->n_list[kListHuge];  // (there by the time it is needed)
     __shared__ uint4 s_slot[kPairWarps][kSmallSlots];
     __shared__ uint2 s_out[kPairWarps][kWarpOut];
     const uint32_t warp = threadIdx.x >> 5;
     small_pass<D, BIP, REC>(p, s_slot[warp], s_out[warp], (uint64_t)blockIdx.x * kPairWarps + warp,
                             (uint64_t)gridDim.x * kPairWarps);
+    expand_cells(p, pin, huge, blockIdx.x * kPairWarps + warp, gridDim.x * kPairWarps);
 }
 
 // ---- tiles ------------------------------------------------------------------
@@ -2959,7 +2963,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Params pin, FusedArg
     FUSED_BARRIER()
     // P3: tile tasks of huge cells, scatter (against the cell ends)
     if (fits) {
-        expand_cells<true>(p, (uint32_t)gw, (uint32_t)nw);
+        expand_cells(p, pin, __ldcg(&p.ctr->n_list[kListHuge]), (uint32_t)gw, (uint32_t)nw);
         Params pe = p;
         if (p.ncells <= kFusedLocalCells) pe.counts = a.ends;
         for (uint64_t b0 = part0; b0 < part1; b0 += kFusedThreads) {
