@@ -287,15 +287,23 @@ static_assert((1 + 3 * kTuneBlocks) * sizeof(unsigned long long) <= kTuneScratch
 
 // a box's coordinates, wherever its row begins, in two or three 16-byte loads
 // (every row is a line or two of its own, and each load instruction looks all
-// of a warp's lines up: with a load per word the sample alone took 12 us). The
-// loads cover aligned 16 bytes that hold at least a byte of the row, so they
-// stay in its memory page.
+// of a warp's lines up: with a load per word the sample alone took 12 us). Rows
+// [0, n) of the array at `rows`; one whose 16 bytes reach out of it is read word
+// by word.
 template <int D>
-__device__ __forceinline__ void load_row(const uint32_t* b, uint32_t (&v)[2 * D]) {
-    const uint32_t o = (uint32_t)(reinterpret_cast<uintptr_t>(b) >> 2) & 3u;
+__device__ __forceinline__ void load_row(const uint32_t* rows, uint64_t n, uint64_t i, uint32_t (&v)[2 * D]) {
+    constexpr uint32_t W = 2 * D + 1;
+    const uint32_t* b = rows + i * W;
+    const RowLoads at = row_loads((uint64_t)b, 2 * D, (uint64_t)rows, (uint64_t)(rows + n * W));
+    if (at.count == 0u) {
+#pragma unroll
+        for (int k = 0; k < 2 * D; k++) v[k] = __ldg(b + k);
+        return;
+    }
+    const uint32_t o = at.before;
     const uint4* q = reinterpret_cast<const uint4*>(b - o);
     const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-    const uint4 q0 = __ldg(q), q1 = o + 2 * D > 4 ? __ldg(q + 1) : z, q2 = o + 2 * D > 8 ? __ldg(q + 2) : z;
+    const uint4 q0 = __ldg(q), q1 = at.count > 1u ? __ldg(q + 1) : z, q2 = at.count > 2u ? __ldg(q + 2) : z;
     uint32_t w[11] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, q2.y, q2.z};
     if (o & 1u) {
 #pragma unroll
@@ -389,7 +397,6 @@ template <int D>
 __global__ void __launch_bounds__(kTuneThreads, 1) k_tune_query(Params p, TuneArgs a) {
     extern __shared__ __align__(16) uint32_t table[];
     __shared__ TuneShared s;
-    constexpr uint32_t W = 2 * D + 1;
     const uint32_t t = threadIdx.x;
     chain_wait();
     const unsigned long long began = now_ns();
@@ -407,9 +414,9 @@ __global__ void __launch_bounds__(kTuneThreads, 1) k_tune_query(Params p, TuneAr
             ok[j] = k < m;
             static_assert(kTuneSample == 1u << 12, "row k * n / m of a full sample");
             const uint64_t g = !ok[j] ? 0ull : a.n > kTuneSample ? (uint64_t)k * a.n >> 12 : k;
-            const uint32_t* b = g < a.n_red ? a.red + g * W : a.blue + (g - a.n_red) * W;
+            const bool red = g < a.n_red;
             uint32_t v[2 * D] = {};
-            if (ok[j]) load_row<D>(b, v);
+            if (ok[j]) load_row<D>(red ? a.red : a.blue, red ? a.n_red : a.n - a.n_red, red ? g : g - a.n_red, v);
 #pragma unroll
             for (int d = 0; d < D; d++) {
                 lo[j][d] = v[2 * d];

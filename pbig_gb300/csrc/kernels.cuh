@@ -280,6 +280,18 @@ cudaError_t launch_scatter(const Params& p, int dims, cudaStream_t st, bool chai
 // of at most max_cells cells. A choice of raise_from becomes raise_to. A grid
 // of more than room_cells cells sets kErrGridRoom and leaves the kernels
 // behind it nothing to do.
+// The 16-byte loads, on their boundaries, that hold the `words` words at address
+// b of an array [begin, end): `count` of them from `before` words ahead of b, or
+// none where one would reach out of the array (its first and last rows).
+struct RowLoads {
+    uint32_t before, count;
+};
+__host__ __device__ inline RowLoads row_loads(uint64_t b, uint32_t words, uint64_t begin, uint64_t end) {
+    const uint32_t before = (uint32_t)(b >> 2) & 3u, count = (before + words + 3) / 4;
+    const uint64_t first = b - 4ull * before;
+    return RowLoads{before, first >= begin && first + 16ull * count <= end ? count : 0u};
+}
+
 constexpr uint32_t kTuneShift = 0xffffffffu;
 constexpr uint64_t kQueryMaxCells = 4000000000ull;  // the most of an automatic cell size
 constexpr uint64_t kTuneSample = 4096;
