@@ -985,7 +985,8 @@ static int fused_query(pbig2_ctx* c, const uint32_t* red, uint64_t n_red, const 
     c->out_hint = std::max<uint64_t>(c->out_hint, h.pairs + h.pairs / 8);
     c->merged_blocks = 0;
     std::vector<GridScene> sc{{0, n, h.shift}};
-    rc = finish_query(c, h, n, h.cells, 1, sc, false, 1);
+    if (bip) sc.push_back({n_red, n - n_red, h.shift});
+    rc = finish_query(c, h, n, h.cells, p.nscenes, sc, false, 1);
     c->stats.class_map = p.class_map;
     c->stats.device_ms = h.t_end > h.t_start ? (double)(h.t_end - h.t_start) * 1e-6 : 0.0;  // the kernel's own clock
     return rc;
