@@ -695,6 +695,22 @@ struct SingleScene {
     uint32_t range;
 };
 
+// Queries of this size, dims and range that had to run on a coarser grid before
+// (coarser_grid_helps): every box is looked at before the tuner's choice is
+// taken, so a scene with such a box runs once, and one without keeps its own
+// cell size. (The scenes were told apart by size alone, and a plain one ran on
+// the grid of the last that had a huge box.)
+static bool was_raised(const pbig2_ctx* c, const SingleScene& q) {
+    for (const auto& r : c->raised)
+        if (r.n == q.n && r.dims == q.dims && r.range == q.range && r.bip == q.bip) return true;
+    return false;
+}
+static void remember_raise(pbig2_ctx* c, const SingleScene& q) {
+    if (was_raised(c, q)) return;
+    if (c->raised.size() >= 64) c->raised.erase(c->raised.begin());
+    c->raised.push_back({q.n, q.dims, q.range, q.bip});
+}
+
 // up to this many boxes a query is launched whole, the grid and its size known
 // to the device alone, into buffers for eight cells and six entries a box (a
 // query that needs more runs again); beyond, the tuner's result is read first
@@ -754,24 +770,24 @@ static int run_single_in(pbig2_ctx* c, const SingleScene& q, uint32_t shift, boo
     ta.bip = q.bip ? 1u : 0u;
     ta.range = q.range;
     ta.shift = shift == PBIG2_AUTO ? kTuneShift : shift;
-    ta.raise_from = ta.raise_to = 32;
-    for (const auto& r : c->raised)
-        if (r.n == q.n && r.dims == q.dims && r.range == q.range) {
-            ta.raise_from = r.from;
-            ta.raise_to = r.to;
-        }
     ta.max_cells = kQueryMaxCells;
     ta.scenes = c->d_scenes.as<Scene>();
     ta.box_off = c->d_scene_off.as<uint32_t>();
     ta.dims = c->d_dims.as<RunDims>();
     ta.scratch = c->d_tune_cost.as<unsigned long long>();
+    if (shift == PBIG2_AUTO && was_raised(c, q)) {
+        unsigned int* least = c->d_tune_cost.as<unsigned int>() + kTuneScratchBytes / sizeof(unsigned int) - 1;
+        CK(cudaMemsetAsync(least, 0, sizeof *least, st));
+        CK(launch_least_shift(ta, q.dims, least, st));
+        ta.least = least;
+    }
 
     need.entries = std::max<uint64_t>(6 * q.n + 4096, c->d_entries.bytes / sizeof(uint4));
     need.out = std::max<uint64_t>({c->out_hint, q.n * 4, 1u << 16, c->d_out.bytes / 8});
     need.tasks = std::max<uint64_t>(c->d_tasks.bytes / 16, 4096);
     need.full = true;
     Ctr h{};
-    int launches = 0, rc = PBIG2_OK;
+    int launches = ta.least ? 1 : 0, rc = PBIG2_OK;
     if (!blind) {
         ta.room_cells = ~0ull;
         CK(launch_tune_query(p, ta, q.dims, st));
@@ -1094,17 +1110,6 @@ static bool coarser_grid_helps(const pbig2_ctx* c, int rc) {
     return rc == PBIG2_EINPUT && (c->last_err & kErrCellOvf) != 0;
 }
 
-// later queries of this size that choose the same cell size start at the one that fitted
-static void remember_raise(pbig2_ctx* c, uint64_t n, int dims, uint32_t range, uint32_t from, uint32_t to) {
-    for (auto& r : c->raised)
-        if (r.n == n && r.dims == dims && r.range == range) {
-            r.from = from;
-            r.to = to;
-            return;
-        }
-    if (c->raised.size() >= 64) c->raised.erase(c->raised.begin());
-    c->raised.push_back({n, dims, range, from, to});
-}
 
 static int self_or_bip(pbig2_ctx* c, const uint32_t* red, uint64_t n_red, const uint32_t* blue, uint64_t n_blue,
                        uint32_t dims, uint32_t range, uint32_t cell_shift, int loc, void* stream, uint64_t* npairs) {
@@ -1159,7 +1164,7 @@ static int self_or_bip(pbig2_ctx* c, const uint32_t* red, uint64_t n_red, const 
     if (cell_shift == PBIG2_AUTO && coarser_grid_helps(c, rc)) {
         const uint32_t first = shift;
         while (coarser_grid_helps(c, rc) && shift < 31) rc = run_single(c, q, shift + 1, st, &shift);
-        remember_raise(c, n, (int)dims, range, first, shift);
+        remember_raise(c, q);
         c->stats.grid_retries = shift - first;
     }
     c->scene_shifts.assign(1, shift);

@@ -127,8 +127,8 @@ struct pbig2_ctx {
     // work-list class map of later queries (PBIG2_OPT_CLASS_MAP; 0: automatic)
     unsigned long long class_map = 0;
     uint32_t merge_limit = 256;  // merged mode's block limit (PBIG2_OPT_MERGE_LIMIT)
-    // scenes whose automatic cell size had to be raised (a box outside the
-    // tuner's sample did not fit): a choice of `from` becomes `to`
-    struct Raised { uint64_t n; int dims; uint32_t range, from, to; };
+    // queries whose automatic cell size had to be raised (a box outside the
+    // tuner's sample did not fit)
+    struct Raised { uint64_t n; int dims; uint32_t range; bool bip; };
     std::vector<Raised> raised;
 };

@@ -283,7 +283,7 @@ constexpr uint32_t kTuneSlots = 8192;        // hash table {cell + 1, corners}, 
 constexpr int kTunePer = (int)(kTuneSample / kTuneThreads);
 constexpr size_t kTuneSmem = kTuneSlots * 2 * sizeof(uint32_t);
 static_assert(kTuneSlots == 2 * kTuneSample && kTuneThreads == 1024, "tuner table and sums");
-static_assert((1 + 3 * kTuneBlocks) * sizeof(unsigned long long) <= kTuneScratchBytes, "tuner scratch");
+static_assert((1 + 3 * kTuneBlocks) * sizeof(unsigned long long) < kTuneScratchBytes, "tuner scratch, launch_least_shift's word at its end");
 
 // a box's coordinates, wherever its row begins, in two or three 16-byte loads
 // (every row is a line or two of its own, and each load instruction looks all
@@ -391,6 +391,37 @@ __device__ double tune_cost_query(uint64_t C, uint32_t entries, uint32_t pairs, 
     const double per_box = (double)entries / (double)m, f = per_box * ((double)n / (double)m);
     E = per_box * (double)n;
     return kQueryCell * (double)C + kQueryEntry * E + (bip ? 0.5 : 1.0) * kQueryTest * ((double)pairs * f * f);
+}
+
+// the finest cell shift at which every valid box covers less than 2^26 cells
+// (the tuner's sample can miss the box that does not; of queries that met one)
+template <int D>
+__global__ void __launch_bounds__(256) k_least_shift(TuneArgs a, unsigned int* least) {
+    constexpr uint32_t W = 2 * D + 1;
+    uint32_t s = 0;  // at which all of this thread's boxes so far fit
+    for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < a.n; g += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t* b = g < a.n_red ? a.red + g * W : a.blue + (g - a.n_red) * W;
+        uint32_t lo[D], hi[D];
+        bool valid = true;
+#pragma unroll
+        for (int d = 0; d < D; d++) {
+            lo[d] = __ldg(b + 2 * d);
+            hi[d] = __ldg(b + 2 * d + 1);
+            valid = valid && lo[d] <= hi[d] && hi[d] < a.range;
+        }
+        while (valid && s < 31u) {
+            unsigned long long c = 1;
+#pragma unroll
+            for (int d = 0; d < D; d++) {
+                const unsigned long long k = (hi[d] >> s) - (lo[d] >> s) + 1ull;
+                c = c >= (1ull << 26) ? c : c * k;
+            }
+            if (c < (1ull << 26)) break;
+            s++;
+        }
+    }
+    s = __reduce_max_sync(FULL_MASK, s);
+    if (lane_id() == 0 && s) atomicMax(least, s);
 }
 
 template <int D>
@@ -504,7 +535,7 @@ __global__ void __launch_bounds__(kTuneThreads, 1) k_tune_query(Params p, TuneAr
             }
         }
         if (t != 0 || shift == kTuneShift) return;  // (another block writes the tables)
-        if (shift == a.raise_from) shift = a.raise_to;
+        if (a.least) shift = max(shift, __ldcg(a.least));
     }
     if (t != 0) return;
     if (a.shift == kTuneShift) a.scratch[0] = 0;
@@ -3171,6 +3202,14 @@ cudaError_t launch_scan(const Params& p, cudaStream_t st, bool chained) {
     const unsigned g2 = (unsigned)(rblocks < cap ? (rblocks ? rblocks : 1) : cap);
     const cudaError_t e = launch_after(chained, k_scan_reduce, g2, kReduceThreads, 0, st, p);
     return e != cudaSuccess ? e : launch_after(chained, k_scan_cells, g, kScanThreads, 0, st, p);
+}
+
+cudaError_t launch_least_shift(const TuneArgs& a, int dims, unsigned int* least, cudaStream_t st) {
+    const uint64_t blocks = (a.n + 255) / 256, cap = (uint64_t)(g_sm_count > 0 ? g_sm_count : 152) * 8;
+    const unsigned g = (unsigned)(blocks < cap ? (blocks ? blocks : 1) : cap);
+    if (dims == 2) k_least_shift<2><<<g, 256, 0, st>>>(a, least);
+    else k_least_shift<3><<<g, 256, 0, st>>>(a, least);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_tune_query(const Params& p, const TuneArgs& a, int dims, cudaStream_t st) {

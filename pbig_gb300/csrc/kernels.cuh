@@ -277,7 +277,7 @@ cudaError_t launch_scatter(const Params& p, int dims, cudaStream_t st, bool chai
 // p.scene_box_off), `dims` and ctr->cells, shift, est_entries, so that the
 // kernels behind it need nothing from the host. `shift`: the cell shift, or
 // kTuneShift for the cost model on a strided sample of 4096 boxes, over grids
-// of at most max_cells cells. A choice of raise_from becomes raise_to. A grid
+// of at most max_cells cells, and no finer than *least (if given). A grid
 // of more than room_cells cells sets kErrGridRoom and leaves the kernels
 // behind it nothing to do.
 // The 16-byte loads, on their boundaries, that hold the `words` words at address
@@ -302,7 +302,7 @@ struct TuneArgs {
     uint32_t bip;           // two scenes
     uint32_t range;
     uint32_t shift;
-    uint32_t raise_from, raise_to;
+    const unsigned int* least;
     uint64_t max_cells, room_cells;
     Scene* scenes;
     uint32_t* box_off;
@@ -310,6 +310,8 @@ struct TuneArgs {
     unsigned long long* scratch;  // a count of blocks, left zero, then each one's cost, entries and cell shift
 };
 constexpr size_t kTuneScratchBytes = 256;
+// the finest cell shift at which every valid box covers less than 2^26 cells, into *least (0 before)
+cudaError_t launch_least_shift(const TuneArgs& a, int dims, unsigned int* least, cudaStream_t st);
 cudaError_t launch_tune_query(const Params& p, const TuneArgs& a, int dims, cudaStream_t st);
 // per-scene cell sizes of a batched query (one warp per scene, a strided
 // sample of up to 64 boxes of each scene, T estimated as E^2 / 2C); offs:
