@@ -71,8 +71,9 @@ typedef struct {
     /* device time per phase of the last pipeline pass (the kernels' own
      * clock): count, scan, expand (0: the scatter does it), scatter, pair test
      * (all three pair kernels), grouping by scene, and within the pair test:
-     * the small-cell, medium-cell and block kernels; all 0 for a query that
-     * ran as one launch */
+     * the small-cell, medium-cell and block kernels (0 where they ran beside
+     * each other, PBIG2_OPT_HOST_SPLIT); all 0 for a query that ran as one
+     * launch */
     double phase_ms[9];
     /* the reference's own work statistics for the same grid (sched_phase,
      * src/pbig/pbig.cu:1586-1688): numCompPairs = sum of n*n/2, jobs = sum

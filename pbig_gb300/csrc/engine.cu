@@ -316,6 +316,7 @@ static cudaError_t record_pipeline(pbig2_ctx* c, const Params& p, int dims, bool
     PairOverlap ov{c->side_stream, c->ev_fork, c->ev_join,
                    c->host_split > 0 ? c->host_split : (3 * c->sm_count + 2) / 5};
     const bool overlap = c->ext_host && p.out == c->ext_out && c->host_split >= 0 && !p.records;
+    c->pairs_overlap = overlap;
     R(launch_pairs(pp, dims, c->sm_count, st, overlap ? &ov : nullptr, full));
     if (grouped) R(launch_group_by_scene(pp, g, st, !overlap));
 #undef R
@@ -342,11 +343,13 @@ static int finish_query(pbig2_ctx* c, const Ctr& h, uint64_t nboxes, uint64_t nc
     const auto between = [&](int a, int b) {
         return h.stamp[a] && h.stamp[b] > h.stamp[a] ? (double)(h.stamp[b] - h.stamp[a]) * 1e-6 : 0.0;
     };
+    const bool beside = c->pairs_overlap && !grouped;  // (kernels beside each other have no times of their own)
+    const int pairs_begin = beside && h.stamp[kStampMed] < h.stamp[kStampSmall] ? kStampMed : kStampSmall;
     const int pairs_end = grouped ? kStampGroup : kStampEnd;
     const double phase[9] = {between(kStampCount, kStampScan), between(kStampScan, kStampScatter), 0.0,
-                             between(kStampScatter, kStampSmall), between(kStampSmall, pairs_end),
-                             grouped ? between(kStampGroup, kStampEnd) : 0.0, between(kStampSmall, kStampMed),
-                             between(kStampMed, kStampBlock), between(kStampBlock, pairs_end)};
+                             between(kStampScatter, pairs_begin), between(pairs_begin, pairs_end),
+                             grouped ? between(kStampGroup, kStampEnd) : 0.0, beside ? 0.0 : between(kStampSmall, kStampMed),
+                             beside ? 0.0 : between(kStampMed, kStampBlock), beside ? 0.0 : between(kStampBlock, pairs_end)};
     c->last_err = h.err;
     pbig2_stats& s = c->stats;
     s.boxes = nboxes;

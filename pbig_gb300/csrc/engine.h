@@ -74,6 +74,7 @@ struct pbig2_ctx {
     cudaStream_t side_stream = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     bool result_ext = false;  // the last result went to ext_out
+    bool pairs_overlap = false;  // the last pass ran its pair kernels beside each other
     // last result
     const uint2* result = nullptr;
     uint64_t npairs = 0;

@@ -31,3 +31,24 @@ def test_scenes_and_boxes(n, one_launch):
             e.self_intersect(red, RANGE)
             st = e.stats()
             assert (st["scenes"], st["boxes"]) == (1, n)
+
+
+def test_phases_of_pair_kernels_beside_each_other():
+    """Pairs bound for page-locked memory: one time for the three pair kernels,
+    none of their own; alone they have theirs."""
+    import torch
+    boxes = boxes_of(300000, 3)
+    host = torch.empty(4000000, 2, dtype=torch.int32).pin_memory()
+    names = ("pairs_small", "pairs_med", "pairs_block")
+    with Engine(0) as e:
+        e.set_pair_output(host)
+        e.self_intersect(boxes, RANGE)
+        ph = e.stats()["phase_ms"]
+        assert e.result_in(host) and ph["pairs"] > 0 and [ph[k] for k in names] == [0, 0, 0]
+        e.set_host_split(-1)
+        e.self_intersect(boxes, RANGE)
+        ph = e.stats()["phase_ms"]
+        assert all(ph[k] > 0 for k in names) and abs(sum(ph[k] for k in names) - ph["pairs"]) < 1e-6
+        e.set_pair_output(None)
+        e.self_intersect(boxes, RANGE)
+        assert all(e.stats()["phase_ms"][k] > 0 for k in names)
