@@ -668,7 +668,8 @@ struct pbig2_scene {
     int dims = 3;
     uint32_t range = 0, shift = 0, nrc = 0;
     uint64_t n = 0, ncells = 0, nslots = 0;
-    DevBuf boxes, start, used, entries, cnt, tmp, state, ctrbuf, lists, idx, nb;
+    DevBuf boxes, entries, idx, nb;
+    DevBuf cells;  // of the grid: starts, slots used; while it is built: counts, capacities, the scan's state and counters
     DevBuf rctr;  // ResCtr, then one bit per box: listed by the move
     DevBuf full[2], rem, add;
     int cur = 0;  // full[cur] holds the current list
@@ -680,10 +681,17 @@ struct pbig2_scene {
 
     template <class F>
     void each_buffer(F f) {
-        for (DevBuf* b : {&boxes, &start, &used, &entries, &cnt, &tmp, &state, &ctrbuf, &rctr, &lists, &idx, &nb, &full[0],
-                          &full[1], &rem, &add})
-            f(*b);
+        for (DevBuf* b : {&boxes, &entries, &cells, &rctr, &idx, &nb, &full[0], &full[1], &rem, &add}) f(*b);
     }
+    // `cells`: four arrays of a word per cell and one more, then the scan's tile
+    // records, counters and (unused) lists; one allocation, for they are all large
+    // and are taken each time a scene is made
+    size_t cell_pitch() const { return ((ncells + 1) * 4 + 255) & ~size_t(255); }
+    size_t scan_at() const { return 4 * cell_pitch(); }
+    size_t ctr_at() const { return scan_at() + ((scan_state_bytes(ncells) + 255) & ~size_t(255)); }
+    size_t cells_bytes() const { return ctr_at() + ((sizeof(Ctr) + 255) & ~size_t(255)) + 256; }
+    unsigned char* cell_bytes(size_t at) { return cells.as<unsigned char>() + at; }
+    uint32_t* cell_words(int k) { return reinterpret_cast<uint32_t*>(cell_bytes(k * cell_pitch())); }
     size_t rctr_bytes() const { return sizeof(ResCtr) + ((n + 31) / 32) * 4; }
     ResGrid grid() {
         ResGrid g{};
@@ -694,8 +702,8 @@ struct pbig2_scene {
         g.range = range;
         g.ncells = ncells;
         g.nslots = nslots;
-        g.start = start.as<uint32_t>();
-        g.used = used.as<uint32_t>();
+        g.start = cell_words(0);
+        g.used = cell_words(1);
         g.entries = entries.as<uint4>();
         g.ctr = rctr.as<ResCtr>();
         return g;
@@ -764,20 +772,15 @@ int build_grid(pbig2_scene* s, cudaStream_t st) {
     const int sms = s->ctx->sm_count;
     if (pbig2_scene_slots(s->ncells, 0) + s->n > kMaxSlots)  // (every box has an entry)
         return api_fail(PBIG2_ECAPACITY, "resident grid: 2^32 slots or more");
-    SCK(s->cnt.ensure(s->ncells * 4 + 16, false, st));
-    SCK(s->tmp.ensure(s->ncells * 4 + 16, false, st));
-    SCK(s->start.ensure((s->ncells + 1) * 4, false, st));
-    SCK(s->used.ensure(s->ncells * 4, false, st));
-    SCK(s->state.ensure(scan_state_bytes(s->ncells), false, st));
-    SCK(s->ctrbuf.ensure(sizeof(Ctr), false, st));
-    SCK(s->lists.ensure(256, false, st));
-    SCK(cudaMemsetAsync(s->cnt.p, 0, s->ncells * 4, st));
+    SCK(s->cells.ensure(s->cells_bytes(), false, st));
+    uint32_t *cnt = s->cell_words(2), *cap = s->cell_words(3);
+    SCK(cudaMemsetAsync(cnt, 0, s->ncells * 4, st));
     SCK(cudaMemsetAsync(s->rctr.p, 0, sizeof(ResCtr), st));
     ResGrid g = s->grid();
-    if (s->dims == 2) k_res_count<2><<<grid_for(s->n, 256, sms), 256, 0, st>>>(g, s->cnt.as<uint32_t>());
-    else k_res_count<3><<<grid_for(s->n, 256, sms), 256, 0, st>>>(g, s->cnt.as<uint32_t>());
+    if (s->dims == 2) k_res_count<2><<<grid_for(s->n, 256, sms), 256, 0, st>>>(g, cnt);
+    else k_res_count<3><<<grid_for(s->n, 256, sms), 256, 0, st>>>(g, cnt);
     SCK(cudaGetLastError());
-    k_res_caps<<<grid_for(s->ncells, 256, sms), 256, 0, st>>>(s->cnt.as<uint32_t>(), s->tmp.as<uint32_t>(), s->ncells, g.ctr);
+    k_res_caps<<<grid_for(s->ncells, 256, sms), 256, 0, st>>>(cnt, cap, s->ncells, g.ctr);
     SCK(cudaGetLastError());
     cudaError_t e;
     ResCtr h = read_ctr(s, st, &e);
@@ -789,15 +792,14 @@ int build_grid(pbig2_scene* s, cudaStream_t st) {
     // exclusive scan of the capacities with the engine's scan kernels (the
     // cell ends replace the capacities in place; no work lists)
     Params p{};
-    p.counts = s->tmp.as<uint32_t>();
+    p.counts = cap;
     p.ncells = s->ncells;
-    p.tile_state = s->state.as<unsigned long long>();
-    p.ctr = s->ctrbuf.as<Ctr>();
-    p.lists = s->lists.as<uint2>();
-    SCK(cudaMemsetAsync(p.ctr, 0, sizeof(Ctr), st));
-    SCK(cudaMemsetAsync(p.tile_state, 0, scan_state_bytes(p.ncells), st));
+    p.tile_state = reinterpret_cast<unsigned long long*>(s->cell_bytes(s->scan_at()));
+    p.ctr = reinterpret_cast<Ctr*>(s->cell_bytes(s->ctr_at()));
+    p.lists = reinterpret_cast<uint2*>(s->cell_bytes(s->cells_bytes() - 256));
+    SCK(cudaMemsetAsync(p.tile_state, 0, s->ctr_at() - s->scan_at() + sizeof(Ctr), st));  // (and p.ctr behind it)
     SCK(launch_scan(p, st));
-    k_res_starts<<<grid_for(s->ncells, 256, sms), 256, 0, st>>>(s->cnt.as<uint32_t>(), s->tmp.as<uint32_t>(), g);
+    k_res_starts<<<grid_for(s->ncells, 256, sms), 256, 0, st>>>(cnt, cap, g);
     SCK(cudaGetLastError());
     // free slots hold no tombstone of an older grid: one that a box is about to
     // be appended to must not be claimed by another box of the same move
@@ -816,7 +818,7 @@ int build_grid(pbig2_scene* s, cudaStream_t st) {
 int build(pbig2_scene* s, cudaStream_t st) {
     int rc = build_grid(s, st);
     while ((rc == PBIG2_ECAPACITY || rc == PBIG2_ENOMEM) && s->automatic && s->ncells > 1 && s->shift < 31) {
-        for (DevBuf* b : {&s->cnt, &s->tmp, &s->start, &s->used, &s->state, &s->entries}) b->release();
+        for (DevBuf* b : {&s->cells, &s->entries}) b->release();
         set_shift(s, s->shift + 1);
         rc = build_grid(s, st);
     }
