@@ -69,7 +69,7 @@ typedef struct {
                               covered 2^26 cells or more */
     double device_ms;      /* device time of the query (the kernels' own clock) */
     /* device time per phase of the last pipeline pass (the kernels' own
-     * clock): count, scan, expand (0: the scatter does it), scatter, pair test
+     * clock): count, scan, expand (0: the small-cell kernel does it), scatter, pair test
      * (all three pair kernels), grouping by scene, and within the pair test:
      * the small-cell, medium-cell and block kernels (0 where they ran beside
      * each other, PBIG2_OPT_HOST_SPLIT); all 0 for a query that ran as one
@@ -237,8 +237,8 @@ PBIG2_API int pbig2_get_stats(pbig2_ctx* ctx, pbig2_stats* stats);
 /* PBIG2_OPT_CLASS_MAP (default 0 = automatic): which pair kernel takes a cell
    of n boxes. Nibble L (L = ceil(log2 n), 1..15; 15 also for larger cells)
    names the list: 0..3 lane groups of 4, 8, 16, 32 lanes (cells up to that
-   many boxes), 4 one warp per cell staged whole (up to 128), 5 one block per
-   cell (up to 512), 6 tile tasks (any size; required for L = 15). A map that
+   many boxes), 4 one warp per cell staged whole (up to 128), 5 a team of
+   four warps per cell (up to 512), 6 tile tasks (any size; required for L = 15). A map that
    sends a bucket to a list too small for it is refused. */
 #define PBIG2_OPT_CLASS_MAP 6
 /* PBIG2_OPT_MERGE_LIMIT (default 256, the reference's NTPB): merged mode's

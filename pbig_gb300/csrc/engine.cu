@@ -950,7 +950,6 @@ static int fused_query(pbig2_ctx* c, const uint32_t* red, uint64_t n_red, const 
     hc->barriers = 0xffffffffu;
     a.ctr_host = hc;
     if (all) {
-        hc->done = 0;
         p.ctr_host = hc;
         CK(launch_all_pairs(p, a.ctr_next, dims, st));
     } else {

@@ -28,11 +28,6 @@ struct HostPinned {
     void release();
 };
 
-struct SceneIn {
-    uint64_t box_off, n;
-    uint32_t shift;   // chosen cell shift
-};
-
 // cell-size autotuner (host): cost model over candidate shifts, fed from a
 // sample of boxes. `words` = 2*dims+1.
 struct TuneResult {

@@ -3059,8 +3059,6 @@ static int g_sm_count = 0;
 
 static size_t med_smem() { return (size_t)kPairWarps * kMedWarpBytes; }
 
-size_t pair_smem_bytes() { return sizeof(TeamSmem); }
-
 template <int D, bool B, bool R = false>
 static cudaError_t init_variant() {
     cudaError_t e = cudaFuncSetAttribute(k_pairs_med<D, B, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)med_smem());

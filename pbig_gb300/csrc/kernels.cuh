@@ -1,5 +1,5 @@
 // Device-side data structures and kernel launchers of the pair-detection
-// pipeline (count -> scan -> expand -> scatter -> pair test).
+// pipeline (count -> scan -> scatter -> pair test).
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -15,7 +15,7 @@ enum : uint32_t {
     kErrOutOvf = 16u,     // pair buffer too small
     kErrWait = 32u,       // a bounded spin-wait gave up
     kErrTaskOvf = 64u,    // tile-task buffer too small
-    kErrCellOvf = 128u,   // one box covers >= 2^31 cells
+    kErrCellOvf = 128u,   // one box covers >= 2^26 cells
     kErrIndex = 256u,     // more than 2^29 boxes in one launch
     kErrRecCell = 512u,   // record mode: a cell of 65536 boxes or more (the record format's limit)
     kErrGridRoom = 1024u  // the chosen grid has more cells than the buffers: nothing was run on it
@@ -28,12 +28,12 @@ constexpr uint32_t kIdMask = (1u << kIdBits) - 1u;
 
 // class lists built by the scan, one {start, n} record per cell: cells with
 // 2..4, 5..8, 9..16, 17..32 boxes (several per warp), 33..kMedMax (one per
-// warp, staged whole), kMedMax+1..kBigMax (one block, staged whole) and
+// warp, staged whole), kMedMax+1..kBigMax (one per team of four warps, staged whole) and
 // larger (32x32 tile tasks)
 constexpr int kNumLists = 7;
 constexpr int kListMed = 4, kListBig = 5, kListHuge = 6;
 constexpr uint32_t kMedMax = 128;   // largest cell staged by one warp
-constexpr uint32_t kBigMax = 512;   // largest cell staged by one block
+constexpr uint32_t kBigMax = 512;   // largest cell staged by a team
 
 // Which list a cell goes to is a class map: nibble L (L = ceil(log2 n), 1..15;
 // 15 also for larger cells) holds the list of cells of n in (2^(L-1), 2^L].
@@ -351,7 +351,6 @@ uint64_t scene_table_entries(uint64_t nboxes);
 constexpr uint64_t kTileCells = 4096, kTileRecBytes = 64;
 __host__ __device__ inline uint64_t scan_tiles(uint64_t ncells) { return (ncells + kTileCells - 1) / kTileCells; }
 inline size_t scan_state_bytes(uint64_t ncells) { return scan_tiles(ncells) * kTileRecBytes; }
-size_t pair_smem_bytes();
 cudaError_t kernels_init();
 
 // ---- one-launch queries of small scenes -----------------------------------
