@@ -251,12 +251,15 @@ PBIG2_API int pbig2_get_stats(pbig2_ctx* ctx, pbig2_stats* stats);
 #define PBIG2_OPT_MAX_BUFFER 8
 
 /* The automatic class map: the work lists a query takes when no map is set
-   (one_launch: a small scene's one-launch query). Measured on GB300: the
-   default map (each cell to the smallest list that holds it) is the fastest
-   on the clustered 4M-box, red/blue and 4096-scene workloads; in a one-launch
-   query cells of 5..32 boxes go to the one-warp-per-cell pass instead (all
-   passes run at one block per SM there, and a warp per cell keeps more
-   independent load chains in flight). No
+   (one_launch: a small scene's one-launch query). Measured on GB300 (device
+   time): the default map (each cell to the smallest list that holds it) is the
+   fastest on the clustered and crowded 4M-box scenes and on 512 scenes (0.77,
+   1.74 and 1.76 ms; with 65..128 boxes to the teams 0.79, 1.83 and 2.11), and
+   within 1 % on red/blue 2M. In a one-launch query cells of 5..32 boxes go to
+   the one-warp-per-cell pass instead (all passes run at one block per SM there,
+   and a warp per cell keeps more independent load chains in flight): a scene of
+   30 000 boxes 26.4 against 27.5 us, a plain 2-D one of 65 536 28.9 against
+   31.3, though 50 000 red and blue boxes 32.0 against 29.5. No
    counterpart in the reference: its cell classes are fixed at build time. */
 PBIG2_API uint64_t pbig2_class_map_auto(uint32_t one_launch);
 /* 0 when every bucket of the class map names a list that can hold its cells,

@@ -3,10 +3,10 @@
 //   k_count    boxes -> per-cell counts                (src/pbig/pbig.cu:174-221)
 //   k_scan     counts -> cell starts + cell work lists (host thrust scan, pbig.cu:1497-1505,
 //              and the job list of sched_phase, pbig.cu:1586-1688)
-//   k_scatter  boxes -> cell entry lists               (d_mapping, pbig.cu:321-427), and tile tasks
-//              for cells too big for shared memory     (sched_phase's 256-row jobs)
+//   k_scatter  boxes -> cell entry lists               (d_mapping, pbig.cu:321-427)
 //   k_pairs    per-cell all-pairs test with the reference-cell rule and compacted output
-//              (d_matching + prefix_scan, pbig.cu:429-543, 562-603, 641-932)
+//              (d_matching + prefix_scan, pbig.cu:429-543, 562-603, 641-932), with tile tasks for
+//              cells too big for shared memory         (sched_phase's 256-row jobs)
 //
 // Box records are the reference's RectInfo (rect.h): 2*D+1 unsigned words.
 // Cell ids follow the reference linearisation gid = (k*nrc + j)*nrc + i.
