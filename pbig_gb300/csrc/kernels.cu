@@ -294,16 +294,15 @@ template <int D>
 __device__ __forceinline__ void load_row(const uint32_t* rows, uint64_t n, uint64_t i, uint32_t (&v)[2 * D]) {
     constexpr uint32_t W = 2 * D + 1;
     const uint32_t* b = rows + i * W;
-    const RowLoads at = row_loads((uint64_t)b, 2 * D, (uint64_t)rows, (uint64_t)(rows + n * W));
-    if (at.count == 0u) {
+    const uint32_t o = (uint32_t)((uint64_t)b >> 2) & 3u;
+    if ((i == 0 || i + 1 == n) && row_loads((uint64_t)b, 2 * D, (uint64_t)rows, (uint64_t)(rows + n * W)).count == 0u) {
 #pragma unroll
         for (int k = 0; k < 2 * D; k++) v[k] = __ldg(b + k);
         return;
     }
-    const uint32_t o = at.before;
     const uint4* q = reinterpret_cast<const uint4*>(b - o);
     const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-    const uint4 q0 = __ldg(q), q1 = at.count > 1u ? __ldg(q + 1) : z, q2 = at.count > 2u ? __ldg(q + 2) : z;
+    const uint4 q0 = __ldg(q), q1 = o + 2 * D > 4 ? __ldg(q + 1) : z, q2 = o + 2 * D > 8 ? __ldg(q + 2) : z;
     uint32_t w[11] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, q2.y, q2.z};
     if (o & 1u) {
 #pragma unroll
@@ -475,27 +474,31 @@ __global__ void __launch_bounds__(kTuneThreads, 1) k_tune_query(Params p, TuneAr
         // makes at most 64 cells a box
         const int s_far = tune_grid<D>(a.range, (uint32_t)s_win) <= 64 * a.n ? (s0 + 5 < 31 ? s0 + 5 : 31) : s_win;
         const int mine = s_lo + (int)blockIdx.x;
-        const uint2 both = block_sums(s, tune_entries<D>(lo, hi, ok, (uint32_t)min(mine, 31)), tune_entries<D>(lo, hi, ok, (uint32_t)s_far));
+        const uint32_t first = block_sums(s, tune_entries<D>(lo, hi, ok, (uint32_t)min(mine, 31)), 0u).x;
         // Coarser ones up to a single cell, on grids in proportion to the boxes, where
         // none of those qualifies (boxes too sparse in their range, or a few huge ones
-        // among them; the coarsest decides, for cells and entries only fall), and where
-        // s0 + 3 makes more cells than that. Small queries, which run in one launch on
-        // coarse grids of their own if they can, stay with s0 + 3 then: on 300 000 boxes
-        // of side 2048 in a range of 2^24 it makes 2^30 cells, where 2^18 are a few
-        // microseconds' work.
-        const bool none = tune_grid<D>(a.range, (uint32_t)s_far) > a.max_cells || both.y > 64u * m;
+        // among them; the coarsest decides, for cells and entries only fall, and a block
+        // whose own size does need not ask it), and where s0 + 3 makes more cells than
+        // that: on 300 000 boxes of side 2048 in a range of 2^24 it makes 2^30, where
+        // 2^18 are a few microseconds' work. (Small queries, which run in one launch on
+        // coarse grids of their own if they can, stay with s0 + 3.)
+        const bool none = !(mine <= s_far && tune_grid<D>(a.range, (uint32_t)mine) <= a.max_cells && first <= 64u * m) &&
+                          (tune_grid<D>(a.range, (uint32_t)s_far) > a.max_cells ||
+                           block_sums(s, tune_entries<D>(lo, hi, ok, (uint32_t)s_far), 0u).x > 64u * m);
         const bool coarser = none || (a.n > kFusedMaxBoxes && tune_grid<D>(a.range, (uint32_t)s_win) > 64 * a.n);
         const int s_one = a.range <= 1u ? 0 : min(32 - __clz((int)(a.range - 1u)), 31);  // the first of a single cell
         const int last = coarser ? max(s_one, s_far) : s_far;
         const uint64_t far = mn64(a.max_cells, a.n * 64 > 4096 ? a.n * 64 : 4096);
-        double best = 1e300, E = 0.0;  // (thread 0; the finest on a tie)
+        unsigned long long best = ~0ull;  // (thread 0: the bits of the least cost, which are in its order; the finest on a tie)
         for (int w = mine; w <= last && m > 0; w += (int)kTuneBlocks) {
             if (tune_grid<D>(a.range, (uint32_t)w) > (w > s_far ? far : a.max_cells)) continue;
-            const uint32_t e = w == mine ? both.x : block_sums(s, tune_entries<D>(lo, hi, ok, (uint32_t)w), 0u).x;
+            const uint32_t e = w == mine ? first : block_sums(s, tune_entries<D>(lo, hi, ok, (uint32_t)w), 0u).x;
             if (e > 64u * m) continue;
             const uint32_t pairs = tune_pairs<D>(s, table, lo, ok, a.range, (uint32_t)w);
             if (t == 0) {
-                const double cost = tune_cost_query(tune_grid<D>(a.range, (uint32_t)w), e, pairs, m, a.n, a.bip, E);
+                double E;
+                const unsigned long long cost = (unsigned long long)__double_as_longlong(
+                    tune_cost_query(tune_grid<D>(a.range, (uint32_t)w), e, pairs, m, a.n, a.bip, E));
                 if (cost < best) {
                     best = cost;
                     shift = (uint32_t)w;
@@ -505,7 +508,7 @@ __global__ void __launch_bounds__(kTuneThreads, 1) k_tune_query(Params p, TuneAr
         }
         if (t == 0) {
             unsigned long long* mine3 = a.scratch + 1 + 3 * blockIdx.x;
-            mine3[0] = (unsigned long long)__double_as_longlong(best);
+            mine3[0] = best;
             mine3[1] = (unsigned long long)__double_as_longlong(est);
             mine3[2] = shift;
             shift = kTuneShift;
@@ -517,17 +520,16 @@ __global__ void __launch_bounds__(kTuneThreads, 1) k_tune_query(Params p, TuneAr
                 for (uint32_t b = 0; b < kTuneBlocks; b++)
 #pragma unroll
                     for (int k = 0; k < 3; k++) all[b][k] = __ldcg(a.scratch + 1 + 3 * b + k);
-                best = 1e300;
+                best = ~0ull;
 #pragma unroll
                 for (uint32_t b = 0; b < kTuneBlocks; b++) {
-                    const double c = __longlong_as_double((long long)all[b][0]);
-                    if (c < best || (c == best && c < 1e300 && (uint32_t)all[b][2] < shift)) {
-                        best = c;
+                    if (all[b][0] < best || (all[b][0] == best && (uint32_t)all[b][2] < shift)) {
+                        best = all[b][0];
                         est = __longlong_as_double((long long)all[b][1]);
                         shift = (uint32_t)all[b][2];
                     }
                 }
-                if (best == 1e300) {  // the coarsest grid that is not a single cell
+                if (best == ~0ull) {  // the coarsest grid that is not a single cell
                     shift = 31;
                     while (shift > 0 && nrc_dev(a.range, (int)shift - 1) <= 1) shift--;
                     est = (double)a.n;
