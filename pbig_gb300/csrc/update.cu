@@ -32,8 +32,8 @@ struct alignas(16) ResCtr {
     unsigned long long add;          // and after it (may exceed capacity)
     unsigned long long full;         // pairs of the full list after the move
     unsigned int done;               // blocks of the last kernel that finished
-    unsigned int span;               // most cells of a box (k_res_span)
-    unsigned long long sum;          // entries of the boxes (k_res_span), slots of the cells (k_res_caps)
+    unsigned int wide;               // a box covers more cells than it may (k_res_count)
+    unsigned long long sum;          // slots of the cells (k_res_caps)
 };
 
 struct ResGrid {
@@ -71,32 +71,19 @@ __device__ __forceinline__ uint64_t res_gid(const ResGrid& g, uint32_t i, uint32
     return ((uint64_t)k * g.nrc + j) * g.nrc + i;
 }
 
-// the cells that the boxes cover on the grid of shift sh: the most of one, and of all
+// one thread per box: count its cells, unless they are more than `widest` (ctr->wide)
 template <int D>
-__global__ void k_res_span(const uint32_t* boxes, uint64_t n, uint32_t sh, ResCtr* ctr) {
-    constexpr int W = 2 * D + 1;
-    uint32_t m = 0;
-    unsigned long long sum = 0;
-    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t lo[3], hi[3];
-        res_range<D>(boxes + t * W, sh, lo, hi);
-        uint64_t c = 1;  // (at most the grid's cells: 2^31)
-        for (int d = 0; d < D; d++) c *= (uint64_t)(hi[d] - lo[d]) + 1;
-        m = max(m, (uint32_t)c);
-        sum += c;
-    }
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31u) == 0 && m) atomicMax(&ctr->span, m);
-    res_sum(&ctr->sum, sum);
-}
-
-// one thread per box: count its cells
-template <int D>
-__global__ void k_res_count(ResGrid g, uint32_t* cnt) {
+__global__ void k_res_count(ResGrid g, uint32_t* cnt, uint32_t widest) {
     constexpr int W = 2 * D + 1;
     for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < g.nboxes; t += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t lo[3], hi[3];
         res_range<D>(g.boxes + t * W, g.shift, lo, hi);
+        uint64_t c = 1;  // (at most the grid's cells: below 2^32)
+        for (int d = 0; d < D; d++) c *= (uint64_t)(hi[d] - lo[d]) + 1;
+        if (c > widest) {
+            atomicOr(&g.ctr->wide, 1u);
+            continue;
+        }
         for (uint32_t k = lo[2]; k <= hi[2]; k++)
             for (uint32_t j = lo[1]; j <= hi[1]; j++)
                 for (uint32_t i = lo[0]; i <= hi[0]; i++) atomicAdd(&cnt[res_gid(g, i, j, k)], 1u);
@@ -169,7 +156,7 @@ __device__ __forceinline__ bool res_moved(const uint32_t* bits, uint32_t id) { r
 // reads the counters once, at the end, and repeats what is missing with more
 // room. The kernels are chained (chain_wait). Nine kernels with five waits, the
 // pairs before by a query, took 234 us for 10 485 of a million boxes, 120 of
-// them in kernels; these took 80 and 53, on the finer grid (finer_grid) 70, and
+// them in kernels; these took 80 and 53, on the finer grid (build_first) 70, and
 // chained 63.
 struct Move {
     ResGrid g;
@@ -651,7 +638,7 @@ __global__ void __launch_bounds__(kResThreads, kResBlocks) k_move_after(Move m) 
             h.rem = __ldcg(&c->rem);
             h.add = __ldcg(&c->add);
             h.full = __ldcg(&c->full);
-            h.done = h.span = 0;
+            h.done = h.wide = 0;
             h.sum = 0;
             *m.host = h;
             __threadfence_system();
@@ -744,31 +731,11 @@ void set_shift(pbig2_scene* s, uint32_t shift) {
     s->ncells = grid_cells(s->range, shift, s->dims);
 }
 
-// With an automatic cell size the scene's grid is one size finer than the
-// query's, where that makes at most 4 cells a box, no box covers more than 512
-// and the slots can be numbered: a move tests the moved boxes against whole cells, while the query tests
-// each pair of a cell once. Moves of 1 % of a million boxes of one density 81 us
-// on the query's grid, 70 on the finer one and 69 on the next; of 65 536 boxes
-// 52 and 46; of the clustered 4M-box scene 716, 568 and 621.
-int finer_grid(pbig2_scene* s, cudaStream_t st) {
-    if (s->shift == 0 || grid_cells(s->range, s->shift - 1, s->dims) > 4 * s->n) return PBIG2_OK;
-    SCK(cudaMemsetAsync(s->rctr.p, 0, sizeof(ResCtr), st));
-    const unsigned g = grid_for(s->n, 256, s->ctx->sm_count);
-    if (s->dims == 2) k_res_span<2><<<g, 256, 0, st>>>(s->boxes.as<uint32_t>(), s->n, s->shift - 1, s->rctr.as<ResCtr>());
-    else k_res_span<3><<<g, 256, 0, st>>>(s->boxes.as<uint32_t>(), s->n, s->shift - 1, s->rctr.as<ResCtr>());
-    SCK(cudaGetLastError());
-    cudaError_t e;
-    const ResCtr h = read_ctr(s, st, &e);
-    SCK(e);
-    if (h.span > 512 || pbig2_scene_slots(grid_cells(s->range, s->shift - 1, s->dims), h.sum) > kMaxSlots) return PBIG2_OK;
-    set_shift(s, s->shift - 1);
-    return PBIG2_OK;
-}
-
 // the grid of the scene's current boxes: counts, capacities with slack,
 // starts (the engine's scan), then every box inserted. The slots are summed in
-// 64 bits before anything is placed by them: 2^32 or more are refused.
-int build_grid(pbig2_scene* s, cudaStream_t st) {
+// 64 bits before anything is placed by them: 2^32 or more are refused, and so is
+// a box of more than `widest` cells.
+int build_grid(pbig2_scene* s, cudaStream_t st, uint32_t widest = 0xffffffffu) {
     const int sms = s->ctx->sm_count;
     if (pbig2_scene_slots(s->ncells, 0) + s->n > kMaxSlots)  // (every box has an entry)
         return api_fail(PBIG2_ECAPACITY, "resident grid: 2^32 slots or more");
@@ -777,15 +744,15 @@ int build_grid(pbig2_scene* s, cudaStream_t st) {
     SCK(cudaMemsetAsync(cnt, 0, s->ncells * 4, st));
     SCK(cudaMemsetAsync(s->rctr.p, 0, sizeof(ResCtr), st));
     ResGrid g = s->grid();
-    if (s->dims == 2) k_res_count<2><<<grid_for(s->n, 256, sms), 256, 0, st>>>(g, cnt);
-    else k_res_count<3><<<grid_for(s->n, 256, sms), 256, 0, st>>>(g, cnt);
+    if (s->dims == 2) k_res_count<2><<<grid_for(s->n, 256, sms), 256, 0, st>>>(g, cnt, widest);
+    else k_res_count<3><<<grid_for(s->n, 256, sms), 256, 0, st>>>(g, cnt, widest);
     SCK(cudaGetLastError());
     k_res_caps<<<grid_for(s->ncells, 256, sms), 256, 0, st>>>(cnt, cap, s->ncells, g.ctr);
     SCK(cudaGetLastError());
     cudaError_t e;
     ResCtr h = read_ctr(s, st, &e);
     SCK(e);
-    if (h.sum > kMaxSlots) return api_fail(PBIG2_ECAPACITY, "resident grid: 2^32 slots or more");
+    if (h.wide || h.sum > kMaxSlots) return api_fail(PBIG2_ECAPACITY, "resident grid: 2^32 slots or more, or a box too wide for it");
     s->nslots = h.sum;
     SCK(s->entries.ensure(s->nslots * 32 + 32, false, st));
     g = s->grid();
@@ -823,6 +790,23 @@ int build(pbig2_scene* s, cudaStream_t st) {
         rc = build_grid(s, st);
     }
     return rc;
+}
+
+// With an automatic cell size the scene's grid is one size finer than the
+// query's, where that makes at most 4 cells a box, no box covers more than 512
+// and it fits: a move tests the moved boxes against whole cells, while the query
+// tests each pair of a cell once. Moves of 1 % of a million boxes of one density
+// 81 us on the query's grid, 70 on the finer one and 69 on the next; of 65 536
+// boxes 52 and 46; of the clustered 4M-box scene 716, 568 and 621.
+int build_first(pbig2_scene* s, cudaStream_t st) {
+    if (s->automatic && s->shift > 0 && grid_cells(s->range, s->shift - 1, s->dims) <= 4 * s->n) {
+        set_shift(s, s->shift - 1);
+        const int rc = build_grid(s, st, 512);
+        if (rc != PBIG2_ECAPACITY && rc != PBIG2_ENOMEM) return rc;
+        for (DevBuf* b : {&s->cells, &s->entries}) b->release();
+        set_shift(s, s->shift + 1);
+    }
+    return build(s, st);
 }
 
 // room for `need` pairs in a buffer that keeps its first `have`: a move that
@@ -982,11 +966,7 @@ PBIG2_API int pbig2_scene_create(pbig2_ctx* c, const uint32_t* boxes, uint64_t n
     if (np && pbig2_copy_pairs(c, s->full[0].as<uint32_t>(), 0, np, PBIG2_DEVICE, sm) != PBIG2_OK) return bail(PBIG2_ECUDA);
     s->nfull = np;
     s->keep_full = (flags & PBIG2_SCENE_DELTA_ONLY) == 0;
-    if (s->automatic) {
-        rc = finer_grid(s, sm);
-        if (rc != PBIG2_OK) return bail(rc);
-    }
-    rc = build(s, sm);
+    rc = build_first(s, sm);
     if (rc != PBIG2_OK) return bail(rc);
     *out = s;
     *npairs = np;
