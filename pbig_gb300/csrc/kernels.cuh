@@ -272,14 +272,6 @@ cudaError_t launch_count(const Params& p, int dims, cudaStream_t st, bool chaine
 cudaError_t launch_scan(const Params& p, cudaStream_t st, bool chained = false);
 cudaError_t launch_scatter(const Params& p, int dims, cudaStream_t st, bool chained = false);
 
-// The grid of a single-scene query (red/blue: both colours on one grid),
-// chosen on the device: zeroes p.ctr and writes the scene table (p.scenes,
-// p.scene_box_off), `dims` and ctr->cells, shift, est_entries, so that the
-// kernels behind it need nothing from the host. `shift`: the cell shift, or
-// kTuneShift for the cost model on a strided sample of 4096 boxes, over grids
-// of at most max_cells cells, and no finer than *least (if given). A grid
-// of more than room_cells cells sets kErrGridRoom and leaves the kernels
-// behind it nothing to do.
 // The 16-byte loads, on their boundaries, that hold the `words` words at address
 // b of an array [begin, end): `count` of them from `before` words ahead of b, or
 // none where one would reach out of the array (its first and last rows).
@@ -292,6 +284,14 @@ __host__ __device__ inline RowLoads row_loads(uint64_t b, uint32_t words, uint64
     return RowLoads{before, first >= begin && first + 16ull * count <= end ? count : 0u};
 }
 
+// The grid of a single-scene query (red/blue: both colours on one grid),
+// chosen on the device: zeroes p.ctr and writes the scene table (p.scenes,
+// p.scene_box_off), `dims` and ctr->cells, shift, est_entries, so that the
+// kernels behind it need nothing from the host. `shift`: the cell shift, or
+// kTuneShift for the cost model on a strided sample of 4096 boxes, over grids
+// of at most max_cells cells, and no finer than *least (if given). A grid
+// of more than room_cells cells sets kErrGridRoom and leaves the kernels
+// behind it nothing to do.
 constexpr uint32_t kTuneShift = 0xffffffffu;
 constexpr uint64_t kQueryMaxCells = 4000000000ull;  // the most of an automatic cell size
 constexpr uint64_t kTuneSample = 4096;
